@@ -322,7 +322,7 @@ def cross_entropy(logits, targets, grad_scale: Optional[float] = None, prob_eps:
     rows, V = logits.shape
     dl = logits if inplace else torch.empty_like(logits)
     losses = torch.empty(rows, dtype=torch.float32, device=logits.device)
-    loss = torch.zeros(1, dtype=torch.float32, device=logits.device)
+    loss = torch.empty(1, dtype=torch.float32, device=logits.device)
     gs = 1.0 / rows if grad_scale is None else grad_scale
     _check(lib().cme_cross_entropy(_dt(logits), _p(logits), _p(targets), _p(dl), _p(losses), _p(loss), rows, V,
                                    ctypes.c_longlong(V), ctypes.c_float(gs), ctypes.c_float(prob_eps),

@@ -1,0 +1,46 @@
+"""Row-wise kernels at the edges of their register and shared-memory tiles, against float64 PyTorch.
+
+bf16 results are rounded once: at most 2^-8 relative, for a single value as for the 2-norm."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DTYPES = [torch.float32, torch.bfloat16]
+
+
+def _ops():
+    from cme213_final_project_b200 import ops
+    return ops
+
+
+def _rand(shape, dtype, seed, scale=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, generator=g, device="cuda") * scale).to(dtype)
+
+
+def _rel(got, want):
+    return ((got.double() - want).norm() / want.norm().clamp_min(1e-30)).item()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("rows,V", [(1, 1), (9, 31), (300, 64), (300, 65), (64, 128), (64, 129), (33, 512), (33, 1024),
+                                    (17, 1025), (17, 2049), (5, 4095), (5, 4097)])
+def test_cross_entropy_short_rows(dtype, rows, V):
+    ops = _ops()
+    logits = _rand((rows, V), dtype, 6, 3.0)
+    if 2 < V <= 4096:
+        logits[0, 0] = float("-inf")                       # a masked symbol
+        logits[rows - 1, 1] = torch.finfo(dtype).min
+    g = torch.Generator(device="cuda").manual_seed(7)
+    targets = torch.randint(2 if V > 2 else 0, V, (rows,), generator=g, device="cuda", dtype=torch.int32)
+    x = logits.double().requires_grad_(True)
+    losses = -torch.log_softmax(x, -1).gather(1, targets.long()[:, None])[:, 0]
+    want = torch.autograd.grad(losses.mean(), x)[0]
+    for inplace in (False, True):
+        src = logits.clone()
+        loss, grad, per_row = ops.cross_entropy(src, targets, inplace=inplace)
+        # __expf: 2^-21 relative, the sum of V of them, one rounding of the gradient
+        assert (per_row.double() - losses.detach()).abs().max().item() < 2e-5
+        assert abs(loss.item() - losses.mean().item()) < 2e-5
+        assert (grad.double() - want).abs().max().item() < (2.0 ** -8 if dtype == torch.bfloat16 else 4e-6) / rows
+        assert inplace or torch.equal(src, logits)
