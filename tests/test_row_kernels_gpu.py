@@ -44,3 +44,29 @@ def test_cross_entropy_short_rows(dtype, rows, V):
         assert abs(loss.item() - losses.mean().item()) < 2e-5
         assert (grad.double() - want).abs().max().item() < (2.0 ** -8 if dtype == torch.bfloat16 else 4e-6) / rows
         assert inplace or torch.equal(src, logits)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("rows,D", [(1, 8), (7, 256), (20000, 264), (9001, 768), (5000, 1024), (4096, 512), (13, 516)])
+def test_layernorm_rows_through_the_ring(dtype, residual, rows, D):
+    """One row to several rounds of the persistent grid (the ring wraps), one to four vectors per lane."""
+    ops = _ops()
+    x, res, dy = (_rand((rows, D), dtype, s) for s in (1, 2, 3))
+    gamma, beta = _rand((D,), dtype, 4, 0.1) + 1, _rand((D,), dtype, 5, 0.1)
+    y, mean, rstd, summed = ops.layernorm_fwd(x, gamma, beta, residual=res if residual else None, save_sum=residual)
+    xin = x.double() + res.double() if residual else x.double()
+    mu = xin.mean(-1, keepdim=True)
+    rs = ((xin - mu).square().mean(-1, keepdim=True) + 1e-5).rsqrt()
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 4e-6
+    assert _rel(y, (xin - mu) * rs * gamma.double() + beta.double()) < tol
+    assert _rel(rstd, rs[:, 0]) < (tol if D % (8 if dtype == torch.bfloat16 else 4) else 4e-6)
+    src = summed if residual else x
+    leaves = [src.double().requires_grad_(True), gamma.double().requires_grad_(True), beta.double().requires_grad_(True)]
+    m = leaves[0].mean(-1, keepdim=True)
+    r = ((leaves[0] - m).square().mean(-1, keepdim=True) + 1e-5).rsqrt()
+    want = torch.autograd.grad((leaves[0] - m) * r * leaves[1] + leaves[2], leaves, dy.double())
+    mean2, rstd2 = m.detach()[:, 0].float(), r.detach()[:, 0].float()
+    dx, dg, db = ops.layernorm_bwd(dy, src, gamma, mean2, rstd2, dres=res if residual else None)
+    assert _rel(dx, want[0] + res.double() if residual else want[0]) < tol
+    assert _rel(dg, want[1]) < max(tol, 2e-5) and _rel(db, want[2]) < max(tol, 2e-5)
