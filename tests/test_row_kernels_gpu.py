@@ -70,3 +70,30 @@ def test_layernorm_rows_through_the_ring(dtype, residual, rows, D):
     dx, dg, db = ops.layernorm_bwd(dy, src, gamma, mean2, rstd2, dres=res if residual else None)
     assert _rel(dx, want[0] + res.double() if residual else want[0]) < tol
     assert _rel(dg, want[1]) < max(tol, 2e-5) and _rel(db, want[2]) < max(tol, 2e-5)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n", [1, 3, 4, 1027, 2_500_002])
+def test_optimizer_tails_and_ranges(dtype, n):
+    """Counts that are not whole vectors, no-decay ranges that begin and end inside a group of four."""
+    ops = _ops()
+    master, m = _rand((n,), torch.float32, 14, 0.02), _rand((n,), torch.float32, 15, 1e-4)
+    v, grads = _rand((n,), torch.float32, 16, 1e-3).square_(), _rand((n,), dtype, 17, 1e-3)
+    nd = [r for r in [[0, 1], [5, 11], [601, 1001], [n - 2, n]] if 0 <= r[0] < r[1] <= n]
+    nd = [r for i, r in enumerate(nd) if i == 0 or r[0] >= nd[i - 1][1]]
+    nodecay = torch.tensor(nd, dtype=torch.int64, device="cuda").reshape(-1, 2)
+    normsq = ops.grad_normsq(grads)
+    assert abs(normsq.item() / grads.double().square().sum().item() - 1) < 1e-5
+    keep = torch.ones(n, device="cuda", dtype=torch.float64)
+    for a, b in nd:
+        keep[a:b] = 0
+    g = grads.double() * min(1.0, 0.01 / float(normsq.sqrt()))
+    m2, v2 = 0.9 * m.double() + 0.1 * g, 0.95 * v.double() + 0.05 * g * g
+    want = master.double() * (1 - 3e-4 * 0.1 * keep) - 3e-4 * (m2 / (1 - 0.9 ** 5)) / ((v2 / (1 - 0.95 ** 5)).sqrt() + 1e-8)
+    step, lr = torch.full((1,), 5, dtype=torch.int32, device="cuda"), torch.full((1,), 3e-4, device="cuda")
+    comp = torch.empty(n, dtype=torch.bfloat16, device="cuda")
+    ops.adam_step(master, grads, m, v, step, lr, compute=comp, normsq=normsq, beta2=0.95, weight_decay=0.1, clip_norm=0.01,
+                  nodecay=nodecay)
+    assert (master.double() - want).abs().max().item() < 1e-7
+    assert _rel(m, m2) < 1e-5 and _rel(v, v2) < 1e-5
+    assert torch.equal(comp, master.to(torch.bfloat16))
