@@ -72,27 +72,6 @@ __global__ void splitk_reduce_vec4_kernel(const float4* __restrict__ P, int spli
     }
 }
 
-// out[b][c][r] = in[b][r][c] for fp32 matrices (32 x 32 tiles through shared memory).  The tf32 products take
-// K-major operands only -- with an MN-major fp32 operand the tensor core returned zeros here -- so operands stored
-// the other way are copied into the workspace transposed first.
-__global__ void __launch_bounds__(256) transpose_f32_kernel(const float* __restrict__ in, float* __restrict__ out, int rows,
-                                                            int cols, long long ld_in, long long stride_in,
-                                                            long long stride_out) {
-    __shared__ float tile[32][33];
-    pdl_wait();
-    const float* src = in + (long long)blockIdx.z * stride_in;
-    float* dst = out + (long long)blockIdx.z * stride_out;
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = ty; j < 32; j += 8)
-        if (r0 + j < rows && c0 + tx < cols) tile[j][tx] = src[(long long)(r0 + j) * ld_in + c0 + tx];
-    __syncthreads();
-#pragma unroll
-    for (int j = ty; j < 32; j += 8)
-        if (c0 + j < cols && r0 + tx < rows) dst[(long long)(c0 + j) * rows + r0 + tx] = tile[tx][j];
-}
-
 // ---------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------
@@ -115,7 +94,8 @@ EncodeTiledFn get_encoder() {
 
 // 3-D tensor map: dims (inner, rows, batch), 128-byte swizzle, box (128 bytes of inner, box_rows, 1).
 int make_tmap(CUtensorMap* out, const void* base, long long inner, long long rows, long long ld, long long batch,
-              long long batch_stride, int box_rows, bool f32 = false, bool round_tf32 = false) {
+              long long batch_stride, int box_rows, bool f32 = false, bool round_tf32 = false,
+              bool mn_major = false) {
     EncodeTiledFn enc = get_encoder();
     CME_REQUIRE(enc != nullptr, CME_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     const int es = f32 ? 4 : 2;
@@ -129,7 +109,7 @@ int make_tmap(CUtensorMap* out, const void* base, long long inner, long long row
                                         : round_tf32 ? CU_TENSOR_MAP_DATA_TYPE_TFLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     CUresult r = enc(out, dt, 3,
                      const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     round_tf32 && mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     CME_REQUIRE(r == CUDA_SUCCESS, CME_ERR_CUDA,
                 "cuTensorMapEncodeTiled failed (%d): inner=%lld rows=%lld ld=%lld batch=%lld bstride=%lld box_rows=%d",
                 (int)r, inner, rows, ld, batch, batch_stride, box_rows);
@@ -231,12 +211,8 @@ int gemm_tcgen05_supported(const CmeGemm* g) {
     if (tf32 && (!g->allow_tf32 || g->c_dtype != CME_F32 || g->bias || g->residual || g->aux_out || g->aux_in ||
                  g->act || g->dact || g->N % 4 || g->ldc % 4 || (g->batch > 1 && g->strideC % 4)))
         return 0;
-    if (tf32 && (g->a_trans || !g->b_trans)) {
-        // an operand stored MN-major is transposed into the workspace first: its new row pitch is K
-        const long long na = g->a_trans ? (long long)(g->strideA ? g->batch : 1) * g->M * g->K : 0;
-        const long long nb = !g->b_trans ? (long long)(g->strideB ? g->batch : 1) * g->N * g->K : 0;
-        if (g->K % 4 || !g->workspace || (na + nb) * 4 + 512 > g->workspace_bytes / 2) return 0;
-    }
+    // the tf32 variants only store: an accumulating product adds its fp32 result from the workspace
+    if (tf32 && g->accumulate && (!g->workspace || (long long)g->batch * g->M * g->N * 4 > g->workspace_bytes)) return 0;
     if (!tf32 && g->ab_dtype != CME_BF16) return 0;
     if (g->M <= 0 || g->N <= 0 || g->K <= 0 || g->batch <= 0) return 0;
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
@@ -265,38 +241,6 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream) {
     const int g_num_sms = ds->num_sms, g_max_pairs = ds->max_pairs;
     int* const g_status = ds->status + CME_STATUS_GEMM;
     const bool tf32 = g->ab_dtype == CME_F32;
-    if (tf32 && (g->a_trans || !g->b_trans)) {
-        // K-major copies of the operands that are stored MN-major (see transpose_f32_kernel), carved from the front
-        // of the workspace; the product then runs on the copies with what is left of the workspace
-        CmeGemm gg = *g;
-        char* w = static_cast<char*>(g->workspace);
-        auto carve = [&](long long floats) {
-            float* p = reinterpret_cast<float*>(w);
-            w += (floats * 4 + 255) / 256 * 256;
-            return p;
-        };
-        if (g->a_trans) {                                     // stored [K, M] -> [M, K]
-            const int nb = g->strideA ? g->batch : 1;
-            float* t = carve((long long)nb * g->M * g->K);
-            CME_CUDA(cme_launch_dependent(transpose_f32_kernel, dim3(cme_cdiv(g->M, 32), cme_cdiv(g->K, 32), nb), dim3(256),
-                                          0, stream, static_cast<const float*>(g->A), t, g->K, g->M, g->lda, g->strideA,
-                                          (long long)g->M * g->K));
-            CME_LAUNCH_CHECK();
-            gg.A = t; gg.lda = g->K; gg.a_trans = 0; gg.strideA = g->strideA ? (long long)g->M * g->K : 0;
-        }
-        if (!g->b_trans) {                                    // stored [K, N] -> [N, K]
-            const int nb = g->strideB ? g->batch : 1;
-            float* t = carve((long long)nb * g->N * g->K);
-            CME_CUDA(cme_launch_dependent(transpose_f32_kernel, dim3(cme_cdiv(g->N, 32), cme_cdiv(g->K, 32), nb), dim3(256),
-                                          0, stream, static_cast<const float*>(g->B), t, g->K, g->N, g->ldb, g->strideB,
-                                          (long long)g->N * g->K));
-            CME_LAUNCH_CHECK();
-            gg.B = t; gg.ldb = g->K; gg.b_trans = 1; gg.strideB = g->strideB ? (long long)g->N * g->K : 0;
-        }
-        gg.workspace = w;
-        gg.workspace_bytes = g->workspace_bytes - (w - static_cast<char*>(g->workspace));
-        return gemm_tcgen05_launch(&gg, stream);
-    }
     const int BK = tf32 ? 32 : 64;                            // K elements per 128-byte k-block
     int tiles_m = cme_cdiv(g->M, BM);
     const int num_kb = cme_cdiv(g->K, BK);
@@ -332,12 +276,12 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream) {
     int rc;
     // A: K-major -> map (K, M), box (64, 128); MN-major -> map (M, K), box (64, 64)
     if (!g->a_trans) rc = make_tmap(&ta, g->A, g->K, g->M, g->lda, g->strideA ? g->batch : 1, g->strideA, BM, tf32, tf32);
-    else             rc = make_tmap(&ta, g->A, g->M, g->K, g->lda, g->strideA ? g->batch : 1, g->strideA, BK, tf32, tf32);
+    else             rc = make_tmap(&ta, g->A, g->M, g->K, g->lda, g->strideA ? g->batch : 1, g->strideA, BK, tf32, tf32, true);
     if (rc) return rc;
     // B: stored [N, K] (b_trans) is K-major -> map (K, N), box (64, bn); stored [K, N] -> map (N, K), box (64, 64)
     if (g->b_trans) rc = make_tmap(&tb, g->B, g->K, g->N, g->ldb, g->strideB ? g->batch : 1, g->strideB,
                                    pair ? bn / 2 : bn, tf32, tf32);
-    else            rc = make_tmap(&tb, g->B, g->N, g->K, g->ldb, g->strideB ? g->batch : 1, g->strideB, BK, tf32, tf32);
+    else            rc = make_tmap(&tb, g->B, g->N, g->K, g->ldb, g->strideB ? g->batch : 1, g->strideB, BK, tf32, tf32, true);
     if (rc) return rc;
 
     EpiParams ep{};

@@ -512,10 +512,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     for (int k = 0; k < BK_BYTES / MMA_K_BYTES; ++k) {
                         // K-major: step 32 bytes (16 bf16 / 8 tf32 elements) inside the 128-byte row.
                         // MN-major: step KROWS k-rows of 128 bytes; column groups are GROUP_BYTES apart.
-                        const uint64_t da = A_MN ? make_smem_desc(sA + k * KROWS * 128, GROUP_BYTES, 1024)
-                                                 : make_smem_desc(sA + k * MMA_K_BYTES, 0, 1024);
-                        const uint64_t db = B_MN ? make_smem_desc(sB + k * KROWS * 128, GROUP_BYTES, 1024)
-                                                 : make_smem_desc(sB + k * MMA_K_BYTES, 0, 1024);
+                        auto mn_desc = [](uint32_t at) {
+                            return C::TF32 ? make_smem_desc_mn32(at, GROUP_BYTES) : make_smem_desc(at, GROUP_BYTES, 1024);
+                        };
+                        const uint64_t da = A_MN ? mn_desc(sA + k * KROWS * 128) : make_smem_desc(sA + k * MMA_K_BYTES, 0, 1024);
+                        const uint64_t db = B_MN ? mn_desc(sB + k * KROWS * 128) : make_smem_desc(sB + k * MMA_K_BYTES, 0, 1024);
                         const uint32_t accf = (kb > kb0 || k > 0) ? 1u : 0u;
                         if constexpr (C::TF32) {
                             if constexpr (PAIR) mma_tf32_ss_pair(tmem_d, da, db, idesc, accf);

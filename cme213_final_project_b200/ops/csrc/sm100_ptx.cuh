@@ -290,6 +290,19 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
     d |= (uint64_t)2 << 61;
     return d;
 }
+// MN-major operand tile of 32-bit elements (rows of 32 elements = 128 bytes along M/N, one row per k): the tensor core
+// transposes 32-bit elements only from a tile whose 32-byte pieces are permuted inside each 128-byte row (layout type 1,
+// what CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B writes), in groups of 4 k-rows: SBO = 512.
+//   LBO = byte distance between consecutive 32-element groups along M/N.
+__device__ __forceinline__ uint64_t make_smem_desc_mn32(uint32_t smem_addr, uint32_t lbo_bytes) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)1 << 61;
+    return d;
+}
 
 // Instruction descriptor for kind::f16 / kind::tf32 with fp32 accumulation:
 //   [4,6) D format (1 = f32), [7,10) A format, [10,13) B format (0 = f16, 1 = bf16, 2 = tf32),
