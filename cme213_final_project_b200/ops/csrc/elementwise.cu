@@ -312,12 +312,16 @@ int bias_act_res_t(const void* x, const void* bias, const void* res, void* pre, 
 }
 
 // dbias[c] (+)= sum over the `slabs` rows of partial[slabs][cols], added in a fixed order: a block covers 32 columns
-// with 8 row groups; each thread sums every 8th row (four independent chains), then the 8 groups are added in
-// shared memory.  The rows come from a GEMM epilogue that sums its stored output per 32-row slab.
+// with 32 row groups; each thread sums every 32nd row (four independent chains), then the 32 groups are added in
+// shared memory.  The rows come from a GEMM epilogue that sums its stored output per 32-row slab.  One block per 32
+// columns leaves the chip mostly idle, so the time is that of a thread's chain of loads: 32 groups instead of 8 make it
+// a quarter as long: 512 rows of 3072 columns 15.5 -> 6.5 us.
+constexpr int SLAB_GROUPS = 32;
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(SLAB_GROUPS * 32)
 colsum_slabs_finalize_kernel(const float* __restrict__ partial, int slabs, int cols, T* dbias, int accumulate) {
-    __shared__ float sm[8][33];
+    constexpr int NG = SLAB_GROUPS;
+    __shared__ float sm[NG][33];
     pdl_wait();
     const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
     const int c = blockIdx.x * 32 + cx;
@@ -325,13 +329,13 @@ colsum_slabs_finalize_kernel(const float* __restrict__ partial, int slabs, int c
     if (c < cols) {
         float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
         int r = ry;
-        for (; r + 24 < slabs; r += 32) {
+        for (; r + 3 * NG < slabs; r += 4 * NG) {
             s0 += partial[(long long)r * cols + c];
-            s1 += partial[(long long)(r + 8) * cols + c];
-            s2 += partial[(long long)(r + 16) * cols + c];
-            s3 += partial[(long long)(r + 24) * cols + c];
+            s1 += partial[(long long)(r + NG) * cols + c];
+            s2 += partial[(long long)(r + 2 * NG) * cols + c];
+            s3 += partial[(long long)(r + 3 * NG) * cols + c];
         }
-        for (; r < slabs; r += 8) s0 += partial[(long long)r * cols + c];
+        for (; r < slabs; r += NG) s0 += partial[(long long)r * cols + c];
         s = (s0 + s1) + (s2 + s3);
     }
     sm[ry][cx] = s;
@@ -339,7 +343,7 @@ colsum_slabs_finalize_kernel(const float* __restrict__ partial, int slabs, int c
     if (ry == 0 && c < cols) {
         float t = 0.f;
 #pragma unroll
-        for (int g = 0; g < 8; ++g) t += sm[g][cx];
+        for (int g = 0; g < NG; ++g) t += sm[g][cx];
         dbias[c] = from_f32<T>(accumulate ? to_f32<T>(dbias[c]) + t : t);
     }
 }
@@ -407,10 +411,10 @@ CME_API int cme_colsum_slabs_finalize(int dtype, const float* partial, int slabs
     cudaStream_t st = (cudaStream_t)stream;
     CME_REQUIRE(slabs > 0 && cols > 0, CME_ERR_SHAPE, "colsum finalize: empty input");
     if (dtype == CME_BF16)
-        CME_CUDA(cme_launch_dependent(colsum_slabs_finalize_kernel<__nv_bfloat16>, dim3(cme_cdiv(cols, 32)), dim3(256), 0,
+        CME_CUDA(cme_launch_dependent(colsum_slabs_finalize_kernel<__nv_bfloat16>, dim3(cme_cdiv(cols, 32)), dim3(SLAB_GROUPS * 32), 0,
                                       st, partial, slabs, cols, (__nv_bfloat16*)dbias, accumulate));
     else
-        CME_CUDA(cme_launch_dependent(colsum_slabs_finalize_kernel<float>, dim3(cme_cdiv(cols, 32)), dim3(256), 0, st,
+        CME_CUDA(cme_launch_dependent(colsum_slabs_finalize_kernel<float>, dim3(cme_cdiv(cols, 32)), dim3(SLAB_GROUPS * 32), 0, st,
                                       partial, slabs, cols, (float*)dbias, accumulate));
     CME_LAUNCH_CHECK();
     return CME_OK;
