@@ -425,8 +425,10 @@ def attention_bwd(q, k, v, out, lse, dout, B: int, H: int, T: int, layout: str =
     if scratch is not None:
         acc, sem = scratch
     else:
-        acc = torch.zeros(q.numel(), dtype=torch.float32, device=q.device)
-        sem = torch.zeros(B * H * ((T + 127) // 128), dtype=torch.int32, device=q.device)
+        # mode 0 clears the scratch itself and counts nothing; the other modes start from zeros
+        make = torch.zeros if dq_mode else torch.empty
+        acc = make(q.numel(), dtype=torch.float32, device=q.device)
+        sem = make(B * H * ((T + 127) // 128), dtype=torch.int32, device=q.device)
     a.q, a.k, a.v, a.o, a.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr()
     a.d_o, a.dq, a.dk, a.dv = dout.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
     a.delta, a.dq_accum = delta.data_ptr(), acc.data_ptr()

@@ -42,6 +42,11 @@ constexpr int CME_ATTN_FINISH_MAX_QBLOCKS = 64;      // dq_mode 2: query blocks 
 
 int attention_simt_fwd(const CmeAttn* a, cudaStream_t st);
 int attention_simt_bwd(const CmeAttn* a, cudaStream_t st);
+int attention_short_supported(const CmeAttn* a, int bwd);
+int attention_short_fwd(const CmeAttn* a, cudaStream_t st);
+int attention_short_bwd(const CmeAttn* a, cudaStream_t st);
+// Whether backend 0 runs the one-launch kernel for short sequences (no dQ scratch then).
+int attention_takes_short(const CmeAttn* a, int bwd);
 int attention_gemm_supported(const CmeAttn* a);
 int attention_gemm_fwd(const CmeAttn* a, cudaStream_t st);
 int attention_gemm_bwd(const CmeAttn* a, cudaStream_t st);
@@ -49,3 +54,4 @@ long long attention_gemm_ws_bytes(int nb, int T);
 int attention_tc_supported(const CmeAttn* a);
 int attention_tc_fwd(const CmeAttn* a, cudaStream_t st);
 int attention_tc_bwd(const CmeAttn* a, cudaStream_t st);
+int attention_tc_check_bwd(const CmeAttn* a);            // what attention_tc_bwd refuses

@@ -471,10 +471,19 @@ int attention_simt_bwd(const CmeAttn* a, cudaStream_t st) {
     return a->dtype == CME_BF16 ? bwd_t<__nv_bfloat16>(a, st) : bwd_t<float>(a, st);
 }
 
-// backend: 0 auto (fused tensor-core kernel, else batched-GEMM path, else SIMT), 1 fused tensor-core only,
-//          2 SIMT only, 3 batched-GEMM path only
+// The short-sequence kernel stands in for the two paths that round P to bf16 as it does; bf16 calls that neither takes
+// (e.g. head size 32 in split layout) keep the fp32 probabilities of the SIMT kernel.  Up to 64 tokens because one
+// block then holds the whole head; the flash kernel's 128-row tile is at least half padding there, and its backward is three
+// launches.
+int attention_takes_short(const CmeAttn* a, int bwd) {
+    return attention_short_supported(a, bwd) && (attention_tc_supported(a) || attention_gemm_supported(a));
+}
+
+// backend: 0 auto (one-launch kernel up to 64 tokens, else fused tensor-core kernel, else batched-GEMM path, else SIMT),
+//          1 fused tensor-core only, 2 SIMT only, 3 batched-GEMM path only
 CME_API int cme_attention_fwd(const CmeAttn* a, int backend, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
+    if (backend == 0 && attention_takes_short(a, 0)) return attention_short_fwd(a, st);
     if ((backend == 0 || backend == 1) && attention_tc_supported(a)) return attention_tc_fwd(a, st);
     CME_REQUIRE(backend != 1, CME_ERR_SHAPE, "attention shape not supported by the tensor-core kernel");
     if ((backend == 0 || backend == 3) && attention_gemm_supported(a)) return attention_gemm_fwd(a, st);
@@ -483,6 +492,13 @@ CME_API int cme_attention_fwd(const CmeAttn* a, int backend, void* stream) {
 }
 CME_API int cme_attention_bwd(const CmeAttn* a, int backend, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
+    if (backend == 0 && attention_takes_short(a, 1)) {
+        if (attention_tc_supported(a)) {           // the same calls are refused as without this kernel
+            const int rc = attention_tc_check_bwd(a);
+            if (rc) return rc;
+        }
+        return attention_short_bwd(a, st);
+    }
     if ((backend == 0 || backend == 1) && attention_tc_supported(a)) return attention_tc_bwd(a, st);
     CME_REQUIRE(backend != 1, CME_ERR_SHAPE, "attention shape not supported by the tensor-core kernel");
     if ((backend == 0 || backend == 3) && attention_gemm_supported(a)) return attention_gemm_bwd(a, st);

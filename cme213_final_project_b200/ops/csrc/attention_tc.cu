@@ -950,16 +950,25 @@ int attention_tc_fwd(const CmeAttn* a, cudaStream_t st) {
 
 int attention_delta_launch(const CmeAttn* a, cudaStream_t st);
 
-int attention_tc_bwd(const CmeAttn* a, cudaStream_t st) {
+int attention_tc_check_bwd(const CmeAttn* a) {
     CME_REQUIRE(attention_tc_supported(a), CME_ERR_SHAPE, "attention: shape not supported by the tensor-core kernel");
     CME_REQUIRE(a->lse && a->delta && a->dq_accum && a->d_o && a->dq && a->dk && a->dv, CME_ERR_SHAPE,
                 "attention backward: missing buffer");
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    CME_REQUIRE(al16(a->d_o) && al16(a->dq) && al16(a->dk) && al16(a->dv), CME_ERR_SHAPE,
+    CME_REQUIRE(al16(a->d_o) && al16(a->dq) && al16(a->dk) && al16(a->dv) && al16(a->dq_accum), CME_ERR_SHAPE,
                 "attention backward: gradient buffers must be 16-byte aligned");
+    CME_REQUIRE(a->dq_mode >= 0 && a->dq_mode <= 2 && (a->dq_mode == 0 || a->dq_sem != nullptr), CME_ERR_SHAPE,
+                "attention backward: dq_mode 1 and 2 need the counter array");
+    CME_REQUIRE(a->dq_mode != 2 || cme_cdiv(a->T, BQ) <= CME_ATTN_FINISH_MAX_QBLOCKS, CME_ERR_LIMIT,
+                "attention backward: dq_mode 2 handles up to %d query blocks", CME_ATTN_FINISH_MAX_QBLOCKS);
+    return CME_OK;
+}
+
+int attention_tc_bwd(const CmeAttn* a, cudaStream_t st) {
+    int rc = attention_tc_check_bwd(a);
+    if (rc) return rc;
     int* const g_attn_status = cme_attn_status_ptr();
     CME_REQUIRE(g_attn_status != nullptr, CME_ERR_CUDA, "attention: device state unavailable");
-    int rc;
     if ((rc = attention_delta_launch(a, st))) return rc;
     const long long rows = (long long)a->nb * a->nh * a->T;
     CUtensorMap mq, mk, mv, mdo, mdq;
@@ -969,10 +978,6 @@ int attention_tc_bwd(const CmeAttn* a, cudaStream_t st) {
     if ((rc = make_map4(&mdo, a->d_o, a->T, a->nh, a->nb, a->ost, a->osh, a->osb, 128))) return rc;
     if ((rc = make_map_dq(&mdq, a->dq_accum, a->T, a->nb * a->nh))) return rc;
     const int mode = a->dq_mode;
-    CME_REQUIRE(mode >= 0 && mode <= 2 && (mode == 0 || a->dq_sem != nullptr), CME_ERR_SHAPE,
-                "attention backward: dq_mode 1 and 2 need the counter array");
-    CME_REQUIRE(mode != 2 || cme_cdiv(a->T, BQ) <= CME_ATTN_FINISH_MAX_QBLOCKS, CME_ERR_LIMIT,
-                "attention backward: dq_mode 2 handles up to %d query blocks", CME_ATTN_FINISH_MAX_QBLOCKS);
     if (mode == 0 && !a->dq_accum_clean) CME_CUDA(cudaMemsetAsync(a->dq_accum, 0, (size_t)rows * HD * sizeof(float), st));
     static bool attr[CME_MAX_DEVICES] = {};               // function attributes are per device
     int dev = 0;

@@ -620,7 +620,7 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
         // needed again -- instead of by a clear in front of every launch on this stream.  Both start clear (bind), and
         // a step ends with both cleared again, since the caller joins the second stream before the next step.
         const bool side_clear = ov && at.dq_mode == 0 && (d.attn_backend == 0 || d.attn_backend == 1) &&
-                                attention_tc_supported(&at);
+                                attention_tc_supported(&at) && !(d.attn_backend == 0 && attention_takes_short(&at, 1));
         const int b01 = l & 1;
         if (side_clear) {
             at.dq_accum = b01 ? e.dq_accum2 : e.dq_accum;

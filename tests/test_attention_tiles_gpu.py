@@ -40,6 +40,59 @@ def _rel(got, want):
 BF16_REL = 2 * 2.0 ** -8
 
 
+@pytest.mark.parametrize("B,H,T,HD,layout,causal", [
+    (2, 4, 64, 32, "flat", False), (2, 4, 64, 128, "flat", False), (3, 2, 56, 40, "flat", True), (1, 2, 8, 8, "flat", False),
+    (2, 3, 64, 64, "split", True), (2, 3, 63, 64, "split", False), (1, 2, 17, 64, "split", True), (1, 1, 1, 64, "split", True),
+    (1, 4, 64, 120, "flat", True)])
+def test_short_sequences_in_one_launch(B, H, T, HD, layout, causal):
+    from cme213_final_project_b200 import ops
+    q, k, v, do = _inputs(B, H, T, HD, torch.bfloat16, 3)
+    before = ops.launch_count()
+    out, lse = ops.attention_fwd(q, k, v, B, H, T, layout, causal)
+    grads = ops.attention_bwd(q, k, v, out, lse, do, B, H, T, layout, causal)
+    assert ops.launch_count() - before == 2
+    ref, ref_lse, ref_grads = _reference(q, k, v, do, B, H, T, layout, causal)
+    assert _rel(out, ref) < BF16_REL
+    assert (lse.double() - ref_lse).abs().max().item() < 1e-4
+    for got, want in zip(grads, ref_grads):
+        # one visible key: dS = P (dP - delta) cancels to rounding noise of the bf16 output, compare with dO's size
+        if T == 1:
+            assert (got.double() - want).abs().max().item() < 2.0 ** -6
+        else:
+            assert _rel(got, want) < 2 * BF16_REL
+    again = ops.attention_bwd(q, k, v, out, lse, do, B, H, T, layout, causal)
+    assert all(torch.equal(a, b) for a, b in zip(grads, again))
+
+
+def test_short_sequences_write_nothing_outside_their_rows():
+    """A ragged fused [tokens, 3D] projection: rows beyond T and columns beyond the head stay as they were."""
+    import ctypes
+    from cme213_final_project_b200 import ops
+    B, H, T, HD = 2, 2, 40, 64
+    D = H * HD
+    g = torch.Generator(device="cuda").manual_seed(5)
+    qkv = torch.randn(B * T + 8, 3 * D, generator=g, device="cuda").to(torch.bfloat16)
+    q, k, v = (qkv[:B * T, i * D:(i + 1) * D].contiguous() for i in range(3))
+    do = torch.randn(B * T, D, generator=g, device="cuda").to(torch.bfloat16)
+    want, lse_want = ops.attention_fwd(q, k, v, B, H, T, "split", True)
+    grads = ops.attention_bwd(q, k, v, want, lse_want, do, B, H, T, "split", True)
+    out = torch.full((B * T + 8, D), 7.0, device="cuda", dtype=torch.bfloat16)
+    dqkv = torch.full_like(qkv, 7.0)
+    lse, delta = torch.zeros(2, B * H * T, device="cuda")
+    acc = torch.zeros(B * T * D, device="cuda")
+    a = ops._attn_desc(q, B, H, T, "split", True)
+    a.sb, a.st = T * 3 * D, 3 * D
+    base, dbase = qkv.data_ptr(), dqkv.data_ptr()
+    a.q, a.k, a.v, a.o, a.lse = base, base + 2 * D, base + 4 * D, out.data_ptr(), lse.data_ptr()
+    ops._check(ops.lib().cme_attention_fwd(ctypes.byref(a), 0, ops._stream()))
+    a.d_o, a.dq, a.dk, a.dv = do.data_ptr(), dbase, dbase + 2 * D, dbase + 4 * D
+    a.delta, a.dq_accum = delta.data_ptr(), acc.data_ptr()
+    ops._check(ops.lib().cme_attention_bwd(ctypes.byref(a), 0, ops._stream()))
+    assert torch.equal(out[:B * T], want) and torch.equal(lse, lse_want)
+    assert torch.equal(dqkv[:B * T], torch.cat(grads, 1))
+    assert (out[B * T:] == 7).all() and (dqkv[B * T:] == 7).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("B,H,T,HD,layout,causal", [
     (2, 4, 64, 128, "flat", False), (2, 2, 65, 32, "split", True), (1, 3, 130, 96, "split", False), (1, 2, 33, 100, "split", True),
