@@ -10,7 +10,7 @@
 #include "gemm.h"
 
 extern "C" int cme_gemm(const CmeGemm*, int, void*);
-int attention_delta_launch(const CmeAttn* a, cudaStream_t st);
+int attention_delta_launch(const CmeAttn* a, cudaStream_t st, float* clear = nullptr);
 
 namespace {
 

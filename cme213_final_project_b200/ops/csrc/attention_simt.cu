@@ -213,24 +213,45 @@ __global__ void attn_delta_kernel(const CmeAttn a) {
     s = warp_sum(s);
     if ((threadIdx.x & 31) == 0) a.delta[row] = s;
 }
-// bf16, head size 64, 16-byte aligned rows: 8 lanes per row (one 128-bit load each), 4 rows per warp.
-__global__ void attn_delta_hd64_kernel(const CmeAttn a) {
-    const int rows = a.nb * a.nh * a.T;
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, sub = threadIdx.x & 7;
-    float s = 0.f;
-    if (row < rows) {
-        const int bh = row / a.T, t = row % a.T;
-        const long long off = head_base_o(a, bh) + (long long)t * a.ost + sub * 8;
-        float x[8], y[8];
-        unpack8(*reinterpret_cast<const Bf16x8*>((const __nv_bfloat16*)a.d_o + off), x);
-        unpack8(*reinterpret_cast<const Bf16x8*>((const __nv_bfloat16*)a.o + off), y);
+// bf16, head size 64, 16-byte aligned rows: 8 lanes per row (one 128-bit load of each operand per lane), two rows per
+// lane so that four loads are in flight.  `clear`: 64 floats per row, set to zero in the same pass (the scratch the
+// backward adds its parts of dQ to), which saves a clearing pass between this kernel and the backward: 16 x 12
+// heads x 1024 tokens 12.9 us + a 9.5 us clear before, 12.8 us for both now.
+__global__ void __launch_bounds__(256) attn_delta_hd64_kernel(const CmeAttn a, float* __restrict__ clear) {
+    pdl_wait();
+    const int rows = a.nb * a.nh * a.T, sub = threadIdx.x & 7;
+    uint4 x[2], y[2];
+    int row[2];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s += x[i] * y[i];
+    for (int k = 0; k < 2; ++k) {
+        row[k] = blockIdx.x * 64 + (threadIdx.x >> 3) + 32 * k;
+        x[k] = y[k] = make_uint4(0, 0, 0, 0);
+        if (row[k] < rows) {
+            const int bh = row[k] / a.T, t = row[k] % a.T;
+            const long long off = head_base_o(a, bh) + (long long)t * a.ost + sub * 8;
+            x[k] = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)a.d_o + off);
+            y[k] = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)a.o + off);
+        }
     }
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 4);
-    if (row < rows && sub == 0) a.delta[row] = s;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        float u[8], w[8], s = 0.f;
+        unpack8(x[k], u);
+        unpack8(y[k], w);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s += u[i] * w[i];
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 4);
+        if (row[k] < rows) {
+            if (sub == 0) a.delta[row[k]] = s;
+            if (clear) {
+                float4* z = reinterpret_cast<float4*>(clear + (long long)row[k] * 64) + sub;
+                z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+                z[8] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+    }
 }
 
 // delta[r] = sum_d dO[r][d] * O[r][d] for the rows whose dO tile has just been staged, one warp per row.
@@ -447,14 +468,18 @@ int check(const CmeAttn* a, bool bwd) {
 
 }  // namespace
 
-// delta[bh, t] = sum_d dO * O, shared with the tensor-core backward.
-int attention_delta_launch(const CmeAttn* a, cudaStream_t st) {
+// delta[bh, t] = sum_d dO * O, shared with the tensor-core backward; `clear` (or null): fp32 scratch of 64 per row to zero.
+int attention_delta_launch(const CmeAttn* a, cudaStream_t st, float* clear) {
     const int rows = a->nb * a->nh * a->T;
     const bool al = ((reinterpret_cast<uintptr_t>(a->d_o) | reinterpret_cast<uintptr_t>(a->o)) & 15) == 0 &&
                     a->ost % 8 == 0 && a->osh % 8 == 0 && a->osb % 8 == 0;
-    if (a->dtype == CME_BF16 && a->HD == 64 && al)
-        attn_delta_hd64_kernel<<<cme_cdiv((long long)rows * 8, 256), 256, 0, st>>>(*a);
-    else if (a->dtype == CME_BF16) attn_delta_kernel<__nv_bfloat16><<<cme_cdiv(rows, 8), 256, 0, st>>>(*a);
+    if (a->dtype == CME_BF16 && a->HD == 64 && al) {
+        CME_CUDA(cme_launch_dependent(attn_delta_hd64_kernel, dim3(cme_cdiv(rows, 64)), dim3(256), 0, st, *a, clear));
+        CME_LAUNCH_CHECK();
+        return CME_OK;
+    }
+    if (clear) CME_CUDA(cudaMemsetAsync(clear, 0, (size_t)rows * 64 * sizeof(float), st));
+    if (a->dtype == CME_BF16) attn_delta_kernel<__nv_bfloat16><<<cme_cdiv(rows, 8), 256, 0, st>>>(*a);
     else attn_delta_kernel<float><<<cme_cdiv(rows, 8), 256, 0, st>>>(*a);
     CME_LAUNCH_CHECK();
     return CME_OK;

@@ -827,30 +827,17 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (warp == BWD_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, BWD_TMEM_COLS); }
 }
 
-// dq[b, h, t, :] = scale * sum over key blocks of the partial dQ slices (bf16, strided destination).
-// Causal: only key blocks at or before the query's block contributed (and were written).
-__global__ void dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int T, int nh,
-                                  long long sb, long long sh, long long st, float scale, long long rows, int nkb,
-                                  int causal) {
+// dq[b, h, t, :] = scale * acc[b * nh + h, t, :] (bf16, strided destination).  One thread per 8 elements, one (batch, head)
+// per grid row, so that no index needs a division by the sequence length (50 + 25 MB: 18.4 -> 10.5 us).
+__global__ void __launch_bounds__(256)
+dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int T, int nh, long long sb, long long sh,
+                  long long st, float scale) {
     pdl_wait();
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;      // one thread per 8 elements
-    if (i >= rows * (HD / 8)) return;
-    const long long r = i / (HD / 8);
-    const int c = (int)(i % (HD / 8)) * 8;
-    const int bh = (int)(r / T), t = (int)(r % T);
-    const int last = causal ? min(nkb - 1, t / BKV) : nkb - 1;
-    float f[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = 0.f;
-    for (int kb = 0; kb <= last; ++kb) {
-        const float* src = acc + ((long long)kb * rows + r) * HD + c;
-        const float4 a = *reinterpret_cast<const float4*>(src);
-        const float4 b2 = *reinterpret_cast<const float4*>(src + 4);
-        f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
-        f[4] += b2.x; f[5] += b2.y; f[6] += b2.z; f[7] += b2.w;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] *= scale;
+    const int i = blockIdx.x * 256 + threadIdx.x, t = i >> 3, c = (i & 7) * 8, bh = blockIdx.y;
+    if (t >= T) return;
+    const float4* src = reinterpret_cast<const float4*>(acc + ((long long)bh * T + t) * HD + c);
+    const float4 u = __ldcs(src), v = __ldcs(src + 1);
+    const float f[8] = {u.x * scale, u.y * scale, u.z * scale, u.w * scale, v.x * scale, v.y * scale, v.z * scale, v.w * scale};
     *reinterpret_cast<uint4*>(dq + (long long)(bh / nh) * sb + (long long)(bh % nh) * sh + (long long)t * st + c) = pack8(f);
 }
 
@@ -948,7 +935,7 @@ int attention_tc_fwd(const CmeAttn* a, cudaStream_t st) {
     return CME_OK;
 }
 
-int attention_delta_launch(const CmeAttn* a, cudaStream_t st);
+int attention_delta_launch(const CmeAttn* a, cudaStream_t st, float* clear = nullptr);
 
 int attention_tc_check_bwd(const CmeAttn* a) {
     CME_REQUIRE(attention_tc_supported(a), CME_ERR_SHAPE, "attention: shape not supported by the tensor-core kernel");
@@ -969,8 +956,8 @@ int attention_tc_bwd(const CmeAttn* a, cudaStream_t st) {
     if (rc) return rc;
     int* const g_attn_status = cme_attn_status_ptr();
     CME_REQUIRE(g_attn_status != nullptr, CME_ERR_CUDA, "attention: device state unavailable");
-    if ((rc = attention_delta_launch(a, st))) return rc;
-    const long long rows = (long long)a->nb * a->nh * a->T;
+    // delta, and in the same pass over the rows the zeros that the dQ parts are added to
+    if ((rc = attention_delta_launch(a, st, a->dq_mode == 0 && !a->dq_accum_clean ? a->dq_accum : nullptr))) return rc;
     CUtensorMap mq, mk, mv, mdo, mdq;
     if ((rc = make_map4(&mq, a->q, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
     if ((rc = make_map4(&mk, a->k, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
@@ -978,7 +965,6 @@ int attention_tc_bwd(const CmeAttn* a, cudaStream_t st) {
     if ((rc = make_map4(&mdo, a->d_o, a->T, a->nh, a->nb, a->ost, a->osh, a->osb, 128))) return rc;
     if ((rc = make_map_dq(&mdq, a->dq_accum, a->T, a->nb * a->nh))) return rc;
     const int mode = a->dq_mode;
-    if (mode == 0 && !a->dq_accum_clean) CME_CUDA(cudaMemsetAsync(a->dq_accum, 0, (size_t)rows * HD * sizeof(float), st));
     static bool attr[CME_MAX_DEVICES] = {};               // function attributes are per device
     int dev = 0;
     CME_CUDA(cudaGetDevice(&dev));
@@ -993,10 +979,9 @@ int attention_tc_bwd(const CmeAttn* a, cudaStream_t st) {
     attn_bwd_tc_kernel<<<grid, BWD_THREADS, BWD_SMEM, st>>>(mq, mk, mv, mdo, mdq, p);
     CME_LAUNCH_CHECK();
     if (mode != 0) return CME_OK;                  // dQ was completed inside the kernel
-    const long long nthreads = rows * (HD / 8);
-    CME_CUDA(cme_launch_dependent(dq_convert_kernel, dim3(cme_cdiv(nthreads, 256)), dim3(256), 0, st,
+    CME_CUDA(cme_launch_dependent(dq_convert_kernel, dim3(cme_cdiv(a->T, 32), a->nb * a->nh), dim3(256), 0, st,
                                   (const float*)a->dq_accum, (__nv_bfloat16*)a->dq, a->T, a->nh, a->sb, a->sh, a->st,
-                                  a->scale, rows, 1, 0));
+                                  a->scale));
     CME_LAUNCH_CHECK();
     return CME_OK;
 }
