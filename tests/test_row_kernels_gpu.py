@@ -97,3 +97,55 @@ def test_optimizer_tails_and_ranges(dtype, n):
     assert (master.double() - want).abs().max().item() < 1e-7
     assert _rel(m, m2) < 1e-5 and _rel(v, v2) < 1e-5
     assert torch.equal(comp, master.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("V,D,B,T,ids", [(7, 8, 2, 4, "uniform"), (65, 384, 16, 64, "uniform"), (50304, 264, 2, 512, "uniform"),
+                                         (3000, 768, 4, 512, "one"), (3000, 136, 4, 512, "few"), (1, 16, 3, 40, "one"),
+                                         (50304, 64, 64, 1023, "few"), (300, 100, 4, 33, "few")])
+def test_token_table_gradient_by_stripes(dtype, V, D, B, T, ids):
+    """Rows without a token, rows with one, rows that many tokens share (summed by the whole block), ids outside the
+    table; twice the same bits; accumulation on top of what is there."""
+    ops = _ops()
+    n = B * T
+    g = torch.Generator(device="cuda").manual_seed(8)
+    tokens = torch.randint(0, V, (n,), generator=g, device="cuda", dtype=torch.int32)
+    if ids == "one":
+        tokens.fill_(V - 1)
+    elif ids == "few":
+        tokens = tokens % min(V, 5)
+        tokens[::7] = V - 1
+        tokens[3], tokens[11] = -1, V                      # no row: ignored
+    dout = _rand((n, D), dtype, 9)
+    ok = (tokens >= 0) & (tokens < V)
+    want = torch.zeros(V, D, dtype=torch.float64, device="cuda").index_add_(0, tokens[ok].long(), dout[ok].double())
+    want_pos = dout.double().reshape(B, T, D).sum(0)
+    dtok, dpos = ops.embedding_bwd(tokens, dout, V, T)
+    again, _ = ops.embedding_bwd(tokens, dout, V, T)
+    if n <= 65535 and D % 8 == 0:
+        assert torch.equal(dtok, again)
+        # fp32 sums of up to n terms, rounded once
+        tol = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
+    else:
+        tol = 3e-2 if dtype == torch.bfloat16 else 1e-5    # atomics round once per token
+    assert _rel(dtok, want) < tol
+    assert _rel(dpos, want_pos) < (2.0 ** -8 if dtype == torch.bfloat16 else 1e-6)
+    base, base_pos = _rand((V, D), dtype, 10), _rand((T, D), dtype, 11)
+    got, got_pos = base.clone(), base_pos.clone()
+    ops.embedding_bwd(tokens, dout, V, T, dtok=got, dpos=got_pos, accumulate=True)
+    assert _rel(got, want + base.double()) < tol
+    assert _rel(got_pos, want_pos + base_pos.double()) < (2.0 ** -8 if dtype == torch.bfloat16 else 1e-6)
+    untouched = torch.ones(V, dtype=torch.bool, device="cuda")
+    untouched[tokens[ok].long()] = False
+    assert torch.equal(got[untouched], base[untouched])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("D,T", [(768, 100), (100, 7)])
+def test_embedding_gather_rows(dtype, D, T):
+    ops = _ops()
+    tok, pos = _rand((500, D), dtype, 12), _rand((T, D), dtype, 13)
+    tokens = torch.randint(0, 500, (3 * T,), device="cuda", dtype=torch.int32)
+    tokens[0], tokens[1] = -3, 900                         # clamped to the table
+    want = (tok.float()[tokens.long().clamp(0, 499)] + pos.float().repeat(3, 1)).to(dtype)
+    assert torch.equal(ops.embedding_fwd(tokens, tok, pos), want)
