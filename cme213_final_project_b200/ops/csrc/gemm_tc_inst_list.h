@@ -54,6 +54,7 @@ CME_GEMM_TC_EXTERN(128, false, false, SPEC_F32)
 #if CME_GEMM_TC_GROUP == -1 || CME_GEMM_TC_GROUP == 7      // 64-wide tiles, GELU epilogues
 CME_GEMM_TC_EXTERN(64, false, false, SPEC_BIAS_GELU_AUX)
 CME_GEMM_TC_EXTERN(64, false, false, SPEC_DGELU)
+CME_GEMM_TC_EXTERN(256, false, false, SPEC_F32)            // split-K partials of wide tiles on single CTAs
 #endif
 
 #if CME_GEMM_TC_GROUP == -1 || CME_GEMM_TC_GROUP == 8      // MLP pair with the derivative kept by forward: forward side

@@ -39,10 +39,11 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ P, int splits, lo
     }
 }
 
-// Same, four consecutive columns per thread (N, ldc and strideC multiples of 4): 16-byte reads of every partial.
+// Same, four consecutive columns per thread: 16-byte reads of every partial.  The partials' rows are N4 float4 long, which
+// may be padding beyond N; `vec`: C takes four columns at once (N, ldc, strideC multiples of 4, C aligned).
 __global__ void splitk_reduce_vec4_kernel(const float4* __restrict__ P, int splits, long long per_split4, void* Cout,
-                                          int c_f32, int accumulate, int M, int N4, long long ldc, long long strideC,
-                                          int batch) {
+                                          int c_f32, int accumulate, int M, int N, int N4, long long ldc, long long strideC,
+                                          int batch, int vec) {
     pdl_wait();
     const long long total = (long long)batch * M * N4;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -54,9 +55,24 @@ __global__ void splitk_reduce_vec4_kernel(const float4* __restrict__ P, int spli
         }
         const long long mn4 = (long long)M * N4;
         const long long b = i / mn4, rem = i - b * mn4;
-        const long long r = rem / N4, c = (rem - r * N4) * 4;
+        const long long r = rem / N4;
+        const int c = (int)(rem - r * N4) * 4;
         const long long off = b * strideC + r * ldc + c;
-        if (c_f32) {
+        if (!vec) {
+            const float t[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (c + j < N) {
+                    if (c_f32) {
+                        float* C = reinterpret_cast<float*>(Cout) + off + j;
+                        *C = accumulate ? *C + t[j] : t[j];
+                    } else {
+                        __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(Cout) + off + j;
+                        *C = __float2bfloat16_rn(accumulate ? __bfloat162float(*C) + t[j] : t[j]);
+                    }
+                }
+            }
+        } else if (c_f32) {
             float4* C = reinterpret_cast<float4*>(reinterpret_cast<float*>(Cout) + off);
             if (accumulate) { const float4 o = *C; s.x += o.x; s.y += o.y; s.z += o.z; s.w += o.w; }
             *C = s;
@@ -152,7 +168,7 @@ CME_API int cme_gemm_status_word(int** out) {
 //   four 64-deep k-blocks per split.
 static void plan_tiles(int M, int N, int K, int batch, bool plain_epi, long long workspace_bytes, int num_sms,
                        int max_pairs, int force_bn, int force_splits, int* bn_out, bool* pair_out, int* splits_out,
-                       int bk = 64) {
+                       int bk = 64, int mn_operands = 0) {
     const int num_kb = cme_cdiv(K, bk);
     int bn = force_bn, splits = force_splits;
     bool pair = false;
@@ -162,9 +178,17 @@ static void plan_tiles(int M, int N, int K, int batch, bool plain_epi, long long
         int best_bn = 128, best_s = 1;
         bool best_pair = false;
         const int bns[4] = {256, 256, 128, 64};
-        // clocks per 16-deep MMA step and SM: the 128-row tiles are limited by how fast shared memory can be
-        // refilled from L2 ((128 + bn) x 32 bytes per step), the pair tile (128 + 128 per SM) by the tensor pipe
-        const double cost[4] = {136.0, 168.0, 100.0, 72.0};
+        // Clocks per MMA step (32 bytes of K) and SM, from sweeps over tile widths and splits.  With one tile per SM a
+        // 128-byte k-block takes about 550 clocks whatever the tile's width (2048 x 512 x 2048 bf16, 32 k-blocks: 13.1 us
+        // at 64 and at 128 columns, 13.9 us at 256, base 3.3-4 us): the ring's round trip to L2, not the tensor pipe, sets
+        // it, so narrow tiles buy no time per k-block, and splitting K over idle SMs does.  With every SM loading, 256
+        // columns on one CTA reach the 64 bytes per clock that an SM takes in (185).
+        // tf32 operands stored along M or N arrive as 32-column groups, two to four times as many copies per k-block.
+        const double b16[4] = {136.0, 168.0, 138.0, 140.0};
+        const double t32[4] = {150.0 + 35.0 * mn_operands, 150.0 + 65.0 * mn_operands, 150.0 + 30.0 * mn_operands,
+                               145.0 + 15.0 * mn_operands};
+        const double* cost = bk == 32 ? t32 : b16;
+        const double pair_start = 2000.0;            // cluster launch and the pair's handshakes, once per CTA
         for (int i = 0; i < 4; ++i) {
             const bool pr = i == 0;
             if (pr && (max_pairs <= 0 || M <= BM)) continue;
@@ -180,7 +204,7 @@ static void plan_tiles(int M, int N, int K, int batch, bool plain_epi, long long
                 const double kb = (double)cme_cdiv(num_kb, s);
                 // 4 MMAs per k-block; epilogue / pipeline fill ~ 6 k-blocks of the widest tile per unit;
                 // a split adds one fp32 write + read of the output per split
-                double est = waves * ((kb + 2.0) * 4.0 * cost[i] + 6.0 * 4.0 * bns[i] / 2.0);
+                double est = waves * ((kb + 2.0) * 4.0 * cost[i] + 6.0 * 4.0 * bns[i] / 2.0) + (pr ? pair_start : 0.0);
                 if (s > 1) est += 6000.0 + (double)s * M * N * batch / num_sms / 16.0;   // + one more launch
                 if (est < best) { best = est; best_bn = bns[i]; best_s = s; best_pair = pr; }
             }
@@ -248,7 +272,7 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream) {
     int bn = 0, splits = 0;
     bool pair = false;
     plan_tiles(g->M, g->N, g->K, g->batch, plain_epi, g->workspace ? g->workspace_bytes : 0, g_num_sms, g_max_pairs,
-               g->force_bn, g->force_splits, &bn, &pair, &splits, BK);
+               g->force_bn, g->force_splits, &bn, &pair, &splits, BK, (g->a_trans != 0) + (g->b_trans == 0));
     // A tf32 product that accumulates into C goes through the fp32 workspace like a split-K product (one "split"
     // is then added to C by the reduction kernel): the tf32 kernel variants only store.
     const bool via_ws = splits > 1 || (tf32 && g->accumulate);
@@ -308,8 +332,14 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream) {
         ep.stream_aux = (stream_aux && g->aux_deriv && (g->act == CME_ACT_GELU || g->dact == CME_ACT_GELU)) ? 1 : 0;
     }
     ep.status = g_status;
+    // Partial rows are padded to whole 16-byte words where the workspace has room: they then leave by TMA stores and are
+    // read back four columns at a time also when N is odd, like the 65-column output head's weight gradient (with the
+    // cost table above: parity-h128 step 130.0 -> 127.7 us).
+    const int n_pad = (g->N + 3) / 4 * 4;
+    const int ldw = (long long)splits * g->batch * g->M * n_pad * 4 <= g->workspace_bytes &&
+                            (reinterpret_cast<uintptr_t>(g->workspace) & 15) == 0 ? n_pad : g->N;
     if (via_ws) {
-        ep.C = g->workspace; ep.ldc = g->N; ep.strideC = (long long)g->M * g->N; ep.c_f32 = 1;
+        ep.C = g->workspace; ep.ldc = ldw; ep.strideC = (long long)g->M * ldw; ep.c_f32 = 1;
     } else {
         ep.C = g->C; ep.ldc = g->ldc; ep.strideC = g->strideC; ep.c_f32 = g->c_dtype == CME_F32;
         ep.bias = reinterpret_cast<const __nv_bfloat16*>(g->bias);
@@ -388,17 +418,16 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream) {
     CME_REQUIRE(rc != -1, CME_ERR_SHAPE, "gemm: no kernel instantiation for tile %d pair %d", bn, (int)pair);
     if (rc) return rc;
     if (via_ws) {
-        const long long per = (long long)g->batch * g->M * g->N;
+        const long long per = (long long)g->batch * g->M * ldw;
         const bool f32 = g->c_dtype == CME_F32;
         const bool vec = g->N % 4 == 0 && g->ldc % 4 == 0 && (g->batch == 1 || g->strideC % 4 == 0) &&
-                         (reinterpret_cast<uintptr_t>(g->C) & (f32 ? 15 : 7)) == 0 &&
-                         (reinterpret_cast<uintptr_t>(g->workspace) & 15) == 0;
-        if (vec) {
+                         (reinterpret_cast<uintptr_t>(g->C) & (f32 ? 15 : 7)) == 0;
+        if (ldw % 4 == 0 && (reinterpret_cast<uintptr_t>(g->workspace) & 15) == 0) {
             const long long per4 = per / 4;
             const int blocks = (int)((per4 + 255) / 256 < 8 * g_num_sms ? (per4 + 255) / 256 : 8 * g_num_sms);
             CME_CUDA(cme_launch_dependent(splitk_reduce_vec4_kernel, dim3(blocks), dim3(256), 0, stream,
                                           reinterpret_cast<const float4*>(g->workspace), splits, per4, g->C, (int)f32,
-                                          g->accumulate, g->M, g->N / 4, g->ldc, g->strideC, g->batch));
+                                          g->accumulate, g->M, g->N, ldw / 4, g->ldc, g->strideC, g->batch, (int)vec));
         } else {
             const int blocks = (int)((per + 255) / 256 < 4096 ? (per + 255) / 256 : 4096);
             splitk_reduce_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const float*>(g->workspace), splits, per,
