@@ -48,6 +48,19 @@ class CmeGemm(ctypes.Structure):
     ]
 
 
+# Argument types of the entry points that the wrappers below call: with them declared, addresses and sizes go over as
+# plain Python numbers (no wrapper object per argument).  v: address, i: int, l: long long, f: float, u: unsigned.
+_PROTOTYPES = {
+    "cme_gemm": "viv", "cme_colsum_slabs_finalize": "iviiviv", "cme_layernorm_fwd": "ivvvvvvvviifv",
+    "cme_layernorm_bwd_blocks": "i", "cme_layernorm_bwd": "ivvvvvvvvvviiiv", "cme_bias_act_residual": "ivvvvvliiv",
+    "cme_colsum_splits": "ii", "cme_dact_colsum": "ivvvvviiiiv", "cme_scale": "ivlfv", "cme_cast": "ivivlv",
+    "cme_add": "ivvvlv", "cme_relu_bwd": "ivvvlv", "cme_init_uniform": "ivlfuv", "cme_embedding_fwd": "ivvvviiiiv",
+    "cme_embedding_bwd": "ivvvviiiiiv", "cme_cross_entropy": "ivvvvviilfffiv", "cme_grad_normsq": "ivlvvv",
+    "cme_adam": "ivvvvvlvvvffffffviv", "cme_attention_fwd": "viv", "cme_attention_bwd": "viv",
+}
+_CTYPES = {"v": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float, "u": ctypes.c_uint}
+
+
 def _load() -> Optional[ctypes.CDLL]:
     global _lib, _tried
     if _lib is not None or _tried:
@@ -62,6 +75,9 @@ def _load() -> Optional[ctypes.CDLL]:
     lib.cme_last_error.restype = ctypes.c_char_p
     lib.fnv1a_u32.restype = ctypes.c_ulonglong
     lib.fnv1a_u32.argtypes = [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_ulonglong]
+    lib.cme_attention_gemm_ws_bytes.restype = ctypes.c_longlong
+    for name, args in _PROTOTYPES.items():
+        getattr(lib, name).argtypes = [_CTYPES[c] for c in args]
     _lib = lib
     return lib
 
@@ -91,12 +107,24 @@ def _stream() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def _st() -> int:
+    """The current stream's handle as a number, for the entry points with declared argument types."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def _a(t: Optional[torch.Tensor]) -> Optional[int]:
+    """A tensor's address as a number (likewise)."""
+    return None if t is None else t.data_ptr()
+
+
+_DTYPES = {torch.float32: F32, torch.bfloat16: BF16}
+
+
 def _dt(t: torch.Tensor) -> int:
-    if t.dtype == torch.float32:
-        return F32
-    if t.dtype == torch.bfloat16:
-        return BF16
-    raise NativeError(f"unsupported dtype {t.dtype}")
+    d = _DTYPES.get(t.dtype)
+    if d is None:
+        raise NativeError(f"unsupported dtype {t.dtype}")
+    return d
 
 
 def _p(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
@@ -125,6 +153,9 @@ def workspace(nbytes: int = 64 << 20) -> torch.Tensor:
 # --------------------------------------------------------------------------------------------------
 # GEMM
 # --------------------------------------------------------------------------------------------------
+_GEMM_BACKENDS = {"auto": 0, "tcgen05": 1, "simt": 2}
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bool = False,
          out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
          bias: Optional[torch.Tensor] = None, act: Optional[str] = None, aux_out: Optional[torch.Tensor] = None,
@@ -159,31 +190,23 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bo
         shape = (batch, M, N) if (a.dim() == 3 or b.dim() == 3) else (M, N)
         out = torch.empty(shape, dtype=odt, device=a.device)
     ws = workspace()
-    g = CmeGemm()
-    g.M, g.N, g.K, g.batch = M, N, K, batch
-    g.A, g.lda, g.strideA, g.a_trans = a.data_ptr(), a2[1], (a2[0] * a2[1] if a.dim() == 3 else 0), int(a_trans)
-    g.B, g.ldb, g.strideB, g.b_trans = b.data_ptr(), b2[1], (b2[0] * b2[1] if b.dim() == 3 else 0), int(b_trans)
-    g.C, g.ldc, g.strideC, g.c_dtype = out.data_ptr(), N, M * N, _dt(out)
-    g.ab_dtype = _dt(a)
-    g.bias = 0 if bias is None else bias.data_ptr()
-    g.residual, g.ldres = (0 if residual is None else residual.data_ptr()), N
-    g.aux_out = 0 if aux_out is None else aux_out.data_ptr()
-    g.aux_in = 0 if aux_in is None else aux_in.data_ptr()
-    g.ldaux = N
-    g.act, g.dact, g.accumulate = ACT[act], ACT[dact], int(accumulate)
-    g.workspace, g.workspace_bytes = ws.data_ptr(), ws.numel() * 4
-    g.force_bn, g.force_splits = force_bn, force_splits
-    g.aux_deriv = int(aux_deriv)
-    g.allow_tf32 = int(allow_tf32)
-    slabs = ctypes.c_int(0)
+    a3, b3 = a.dim() == 3, b.dim() == 3
+    slabs = part = None
     if dbias is not None:
+        slabs = ctypes.c_int(0)
         part = torch.empty((M + 31) // 32 * N, dtype=torch.float32, device=a.device)
-        g.colsum, g.colsum_slabs = part.data_ptr(), ctypes.pointer(slabs)
-    _check(lib().cme_gemm(ctypes.byref(g), {"auto": 0, "tcgen05": 1, "simt": 2}[backend], _stream()))
+    g = CmeGemm(M, N, K, batch,
+                a.data_ptr(), a2[1], a2[0] * a2[1] if a3 else 0, a_trans,
+                b.data_ptr(), b2[1], b2[0] * b2[1] if b3 else 0, b_trans,
+                out.data_ptr(), N, M * N, _dt(out), _dt(a),
+                _a(bias), _a(residual), N, _a(aux_out), _a(aux_in), N,
+                ACT[act], ACT[dact], accumulate, ws.data_ptr(), ws.numel() * 4, force_bn, force_splits, aux_deriv,
+                _a(part), None if slabs is None else ctypes.pointer(slabs), allow_tf32)
+    _check(lib().cme_gemm(ctypes.byref(g), _GEMM_BACKENDS[backend], _st()))
     if dbias is not None:
         gemm.last_colsum_slabs = slabs.value          # 0: the epilogue did not sum (tests look at this)
         if slabs.value:
-            _check(lib().cme_colsum_slabs_finalize(_dt(dbias), _p(part), slabs.value, N, _p(dbias), 0, _stream()))
+            _check(lib().cme_colsum_slabs_finalize(_dt(dbias), _a(part), slabs.value, N, _a(dbias), 0, _st()))
         else:
             dact_colsum(out.reshape(-1, N), want_g=False, dbias=dbias)
     return out
@@ -208,8 +231,8 @@ def layernorm_fwd(x, gamma, beta, eps: float = 1e-5, residual=None, save_sum: bo
     mean = torch.empty(rows, dtype=torch.float32, device=x.device)
     rstd = torch.empty_like(mean)
     r = torch.empty_like(x) if (save_sum and residual is not None) else None
-    _check(lib().cme_layernorm_fwd(_dt(x), _p(x), _p(residual), _p(r), _p(gamma), _p(beta), _p(y), _p(mean), _p(rstd),
-                                   rows, D, ctypes.c_float(eps), _stream()))
+    _check(lib().cme_layernorm_fwd(_dt(x), _a(x), _a(residual), _a(r), _a(gamma), _a(beta), _a(y), _a(mean), _a(rstd),
+                                   rows, D, eps, _st()))
     return y, mean, rstd, r
 
 
@@ -222,8 +245,8 @@ def layernorm_bwd(dy, x, gamma, mean, rstd, dres=None, dgamma=None, dbeta=None, 
         dgamma, dbeta, accumulate = torch.empty_like(gamma), torch.empty_like(gamma), False
     nb = lib().cme_layernorm_bwd_blocks(rows)
     scratch = torch.empty(nb * 2 * D, dtype=torch.float32, device=x.device)
-    _check(lib().cme_layernorm_bwd(_dt(x), _p(dy), _p(x), _p(gamma), _p(mean), _p(rstd), _p(dres), _p(dx), _p(dgamma),
-                                   _p(dbeta), _p(scratch), rows, D, int(accumulate), _stream()))
+    _check(lib().cme_layernorm_bwd(_dt(x), _a(dy), _a(x), _a(gamma), _a(mean), _a(rstd), _a(dres), _a(dx), _a(dgamma),
+                                   _a(dbeta), _a(scratch), rows, D, int(accumulate), _st()))
     return dx, dgamma, dbeta
 
 
@@ -237,8 +260,8 @@ def bias_act_residual(x, bias=None, act=None, residual=None, save_pre: bool = Fa
     rows = x.numel() // cols
     out = torch.empty_like(x)
     pre = torch.empty_like(x) if save_pre else None
-    _check(lib().cme_bias_act_residual(_dt(x), _p(x), _p(bias), _p(residual), _p(pre), _p(out),
-                                       ctypes.c_longlong(rows), cols, ACT[act], _stream()))
+    _check(lib().cme_bias_act_residual(_dt(x), _a(x), _a(bias), _a(residual), _a(pre), _a(out), rows, cols, ACT[act],
+                                       _st()))
     return out, pre
 
 
@@ -251,42 +274,41 @@ def dact_colsum(dout, pre=None, act=None, want_g: bool = True, dbias=None, accum
     if dbias is None:
         dbias, accumulate = torch.empty(cols, dtype=dout.dtype, device=dout.device), False
     scratch = torch.empty(lib().cme_colsum_splits(rows, cols) * cols, dtype=torch.float32, device=dout.device)
-    _check(lib().cme_dact_colsum(_dt(dout), _p(dout), _p(pre), _p(g), _p(dbias), _p(scratch), rows, cols, ACT[act],
-                                 int(accumulate), _stream()))
+    _check(lib().cme_dact_colsum(_dt(dout), _a(dout), _a(pre), _a(g), _a(dbias), _a(scratch), rows, cols, ACT[act],
+                                 int(accumulate), _st()))
     return g, dbias
 
 
 def scale_(x, s: float):
     _cuda(x)
-    _check(lib().cme_scale(_dt(x), _p(x), ctypes.c_longlong(x.numel()), ctypes.c_float(s), _stream()))
+    _check(lib().cme_scale(_dt(x), _a(x), x.numel(), s, _st()))
     return x
 
 
 def cast(x, dtype):
     _cuda(x)
     y = torch.empty(x.shape, dtype=dtype, device=x.device)
-    _check(lib().cme_cast(_dt(x), _p(x), _dt(y), _p(y), ctypes.c_longlong(x.numel()), _stream()))
+    _check(lib().cme_cast(_dt(x), _a(x), _dt(y), _a(y), x.numel(), _st()))
     return y
 
 
 def add(a, b):
     _cuda(a, b)
     out = torch.empty_like(a)
-    _check(lib().cme_add(_dt(a), _p(a), _p(b), _p(out), ctypes.c_longlong(a.numel()), _stream()))
+    _check(lib().cme_add(_dt(a), _a(a), _a(b), _a(out), a.numel(), _st()))
     return out
 
 
 def relu_bwd(x, dy):
     _cuda(x, dy)
     dx = torch.empty_like(dy)
-    _check(lib().cme_relu_bwd(_dt(x), _p(x), _p(dy), _p(dx), ctypes.c_longlong(x.numel()), _stream()))
+    _check(lib().cme_relu_bwd(_dt(x), _a(x), _a(dy), _a(dx), x.numel(), _st()))
     return dx
 
 
 def init_uniform_(out, scale: float, seed: int):
     _cuda(out)
-    _check(lib().cme_init_uniform(_dt(out), _p(out), ctypes.c_longlong(out.numel()), ctypes.c_float(scale),
-                                  ctypes.c_uint(seed & 0xFFFFFFFF), _stream()))
+    _check(lib().cme_init_uniform(_dt(out), _a(out), out.numel(), scale, seed & 0xFFFFFFFF, _st()))
     return out
 
 
@@ -297,7 +319,7 @@ def embedding_fwd(tokens, tok, pos):
     _cuda(tokens, tok, pos)
     BT, (V, D), T = tokens.numel(), tok.shape, pos.shape[0]
     out = torch.empty(BT, D, dtype=tok.dtype, device=tok.device)
-    _check(lib().cme_embedding_fwd(_dt(tok), _p(tokens), _p(tok), _p(pos), _p(out), BT, T, D, V, _stream()))
+    _check(lib().cme_embedding_fwd(_dt(tok), _a(tokens), _a(tok), _a(pos), _a(out), BT, T, D, V, _st()))
     return out
 
 
@@ -307,8 +329,8 @@ def embedding_bwd(tokens, dout, V: int, T: int, dtok=None, dpos=None, accumulate
     if dtok is None:
         dtok, dpos, accumulate = (torch.empty(V, D, dtype=dout.dtype, device=dout.device),
                                   torch.empty(T, D, dtype=dout.dtype, device=dout.device), False)
-    _check(lib().cme_embedding_bwd(_dt(dout), _p(tokens), _p(dout), _p(dtok), _p(dpos), BT, T, D, V, int(accumulate),
-                                   _stream()))
+    _check(lib().cme_embedding_bwd(_dt(dout), _a(tokens), _a(dout), _a(dtok), _a(dpos), BT, T, D, V, int(accumulate),
+                                   _st()))
     return dtok, dpos
 
 
@@ -324,9 +346,8 @@ def cross_entropy(logits, targets, grad_scale: Optional[float] = None, prob_eps:
     losses = torch.empty(rows, dtype=torch.float32, device=logits.device)
     loss = torch.empty(1, dtype=torch.float32, device=logits.device)
     gs = 1.0 / rows if grad_scale is None else grad_scale
-    _check(lib().cme_cross_entropy(_dt(logits), _p(logits), _p(targets), _p(dl), _p(losses), _p(loss), rows, V,
-                                   ctypes.c_longlong(V), ctypes.c_float(gs), ctypes.c_float(prob_eps),
-                                   ctypes.c_float(1.0), 0, _stream()))
+    _check(lib().cme_cross_entropy(_dt(logits), _a(logits), _a(targets), _a(dl), _a(losses), _a(loss), rows, V,
+                                   V, gs, prob_eps, 1.0, 0, _st()))
     return loss, dl, losses
 
 
@@ -334,7 +355,7 @@ def grad_normsq(g):
     _cuda(g)
     partial = torch.empty(1024, dtype=torch.float32, device=g.device)
     out = torch.empty(1, dtype=torch.float32, device=g.device)
-    _check(lib().cme_grad_normsq(_dt(g), _p(g), ctypes.c_longlong(g.numel()), _p(partial), _p(out), _stream()))
+    _check(lib().cme_grad_normsq(_dt(g), _a(g), g.numel(), _a(partial), _a(out), _st()))
     return out
 
 
@@ -344,11 +365,9 @@ def adam_step(master, grads, m, v, step_dev, lr_dev, *, compute=None, normsq=Non
     ``lr_dev`` (fp32 [1]) live on the device; ``nodecay`` is an int64 ``[k, 2]`` tensor of sorted ranges."""
     _cuda(master, grads, m, v, step_dev, lr_dev, compute, normsq, nodecay)
     nn = 0 if nodecay is None else nodecay.shape[0]
-    _check(lib().cme_adam(_dt(grads), _p(master), _p(compute), _p(grads), _p(m), _p(v),
-                          ctypes.c_longlong(master.numel()), _p(step_dev), _p(lr_dev), _p(normsq),
-                          ctypes.c_float(beta1), ctypes.c_float(beta2), ctypes.c_float(eps),
-                          ctypes.c_float(weight_decay), ctypes.c_float(grad_scale), ctypes.c_float(clip_norm),
-                          _p(nodecay), nn, _stream()))
+    _check(lib().cme_adam(_dt(grads), _a(master), _a(compute), _a(grads), _a(m), _a(v), master.numel(),
+                          _a(step_dev), _a(lr_dev), _a(normsq), beta1, beta2, eps, weight_decay, grad_scale, clip_norm,
+                          _a(nodecay), nn, _st()))
 
 
 # --------------------------------------------------------------------------------------------------
@@ -375,17 +394,10 @@ _BACKENDS = {"auto": 0, "tc": 1, "simt": 2, "gemm": 3}
 def _attn_desc(q, B, H, T, layout, causal):
     D = q.shape[-1]
     HD = D // H
-    a = CmeAttn()
-    a.T, a.HD, a.causal, a.scale, a.dtype = T, HD, int(causal), 1.0 / (HD ** 0.5), _dt(q)
-    if layout == "flat":
-        a.nb, a.nh, a.sb, a.sh, a.st = B * H, 1, T * HD, 0, HD
-    else:
-        a.nb, a.nh, a.sb, a.sh, a.st = B, H, T * D, HD, D
-    a.osb, a.osh, a.ost = a.sb, a.sh, a.st
+    nb, nh, sb, sh, st = (B * H, 1, T * HD, 0, HD) if layout == "flat" else (B, H, T * D, HD, D)
+    a = CmeAttn(nb, nh, T, HD, sb, sh, st, sb, sh, st, bool(causal), 1.0 / (HD ** 0.5), _dt(q))
     if layout == "flat" and T <= 512 and q.dtype == torch.bfloat16:      # scratch of the batched-GEMM path
-        l = lib()
-        l.cme_attention_gemm_ws_bytes.restype = ctypes.c_longlong
-        nbytes = int(l.cme_attention_gemm_ws_bytes(B * H, T))
+        nbytes = int(lib().cme_attention_gemm_ws_bytes(B * H, T))
         ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=q.device)
         a._ws_keepalive = ws
         a.ws = (ws.data_ptr() + 255) // 256 * 256
@@ -402,7 +414,7 @@ def attention_fwd(q, k, v, B: int, H: int, T: int, layout: str = "split", causal
     out = torch.empty_like(q)
     lse = torch.empty(B * H * T, dtype=torch.float32, device=q.device)
     a.q, a.k, a.v, a.o, a.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr()
-    _check(lib().cme_attention_fwd(ctypes.byref(a), _BACKENDS[backend], _stream()))
+    _check(lib().cme_attention_fwd(ctypes.byref(a), _BACKENDS[backend], _st()))
     return out, lse
 
 
@@ -433,7 +445,7 @@ def attention_bwd(q, k, v, out, lse, dout, B: int, H: int, T: int, layout: str =
     a.d_o, a.dq, a.dk, a.dv = dout.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
     a.delta, a.dq_accum = delta.data_ptr(), acc.data_ptr()
     a.dq_sem, a.dq_mode = sem.data_ptr(), int(dq_mode)
-    _check(lib().cme_attention_bwd(ctypes.byref(a), _BACKENDS[backend], _stream()))
+    _check(lib().cme_attention_bwd(ctypes.byref(a), _BACKENDS[backend], _st()))
     return dq, dk, dv
 
 
