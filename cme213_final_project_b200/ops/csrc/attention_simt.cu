@@ -10,19 +10,23 @@
 
 namespace {
 
-// What bounds these kernels is the fp32 multiply-add rate, so every product is register-tiled: a warp owns 8 rows, a
-// lane 2 of them (ty, ty + 4) and every eighth streamed row (tx + 8 j) or 4 consecutive columns in 32 (tx * 4 + 32 g).
-// A 4-deep step of a score product is 10 shared-memory vector loads for 64 multiply-adds (one load per multiply-add
-// before); no load has a bank conflict, since a row's pitch is an odd number of 16-byte words.  A warp keeps whole
-// rows of the score tile, so the softmax needs shuffles among 8 lanes only and P never crosses a warp in forward.
+// What bounds these kernels is the fp32 multiply-add rate and, next to it, shared-memory reads: a 16-byte load per lane
+// takes the SM's shared memory four clocks, in which its schedulers issue sixteen multiply-adds.  So every product is
+// register-tiled.  Forward: a warp owns 16 whole rows, a lane 4 of them (ty + 4 i) and every eighth streamed row
+// (tx + 8 j), or 4 consecutive columns in 32 (tx * 4 + 32 g): 12 loads for 128 multiply-adds in a 4-deep step (two loads
+// per multiply-add before there were tiles, 10 for 64 with 2 rows per lane), the softmax needs shuffles among 8 lanes only
+// and P never crosses a warp.  Backward: the warps form 4 groups of 16 rows x 2 halves -- of the streamed rows in the
+// score products, of the head's columns in the others -- so that a lane's 4-row tiles of two outputs fit its registers.
+// No load has a bank conflict, since a row's pitch is an odd number of 16-byte words.
 // The head size is padded with zeros to a multiple of 32 (template G = ceil(HD / 32)).
-// 32 x 4 heads x 64 tokens x head size 128, fp32: forward + backward call 297 us -> 65 us
-// (its floor at the fp32 rate, 0.94 GFLOP at 74 TFLOP/s, is 13 us).
+// 32 x 4 heads x 64 tokens x head size 128, fp32, forward + backward call: 297 us without tiles, 58 us
+// with 2 rows per lane, 51 us now (its floor at the fp32 rate, 0.94 GFLOP at 74 TFLOP/s, is 13 us).
 constexpr int CT = 64;               // rows streamed per step
-constexpr int WR = 8;                // rows a warp owns
+constexpr int WR = 16;               // rows a warp owns
+constexpr int LR = WR / 4;           // rows a lane has of them
 constexpr int SP = CT + 4;           // pitch of the probability tiles
 constexpr int MAX_HD = 128;
-constexpr int BWD_NW = 8;            // backward: 64 rows per block
+constexpr int BWD_ROWS = 64, BWD_THREADS = 256;
 template <int G> struct Pitch { static constexpr int P = 32 * G + 4; };
 
 __device__ __forceinline__ long long head_base(const CmeAttn& a, int bh) {
@@ -74,53 +78,76 @@ __device__ __forceinline__ void load_rows(float* dst, const T* src, long long st
 }
 
 // s[i][j] += A[ty + 4 i] . B[tx + 8 j]
-template <int G>
-__device__ __forceinline__ void dot_2x8(const float* A, const float* B, int ty, int tx, float (&s)[2][8]) {
+template <int G, int NJ>
+__device__ __forceinline__ void dot_rows(const float* A, const float* B, int ty, int tx, float (&s)[LR][NJ]) {
     constexpr int P = Pitch<G>::P;
-#pragma unroll 4
+#pragma unroll 2
     for (int d = 0; d < 32 * G; d += 4) {
-        const float4 a0 = *reinterpret_cast<const float4*>(A + ty * P + d);
-        const float4 a1 = *reinterpret_cast<const float4*>(A + (ty + 4) * P + d);
+        float4 a[LR];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int i = 0; i < LR; ++i) a[i] = *reinterpret_cast<const float4*>(A + (ty + 4 * i) * P + d);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
             const float4 b = *reinterpret_cast<const float4*>(B + (tx + 8 * j) * P + d);
-            s[0][j] = fmaf(a0.w, b.w, fmaf(a0.z, b.z, fmaf(a0.y, b.y, fmaf(a0.x, b.x, s[0][j]))));
-            s[1][j] = fmaf(a1.w, b.w, fmaf(a1.z, b.z, fmaf(a1.y, b.y, fmaf(a1.x, b.x, s[1][j]))));
+#pragma unroll
+            for (int i = 0; i < LR; ++i)
+                s[i][j] = fmaf(a[i].w, b.w, fmaf(a[i].z, b.z, fmaf(a[i].y, b.y, fmaf(a[i].x, b.x, s[i][j]))));
         }
     }
 }
 
-// o[i][g] += w(i, j) * B[j][tx * 4 + 32 g ...] over the CT streamed rows; W is the weight tile [row][CT] (pitch SP).
-template <int G>
-__device__ __forceinline__ void weighted_rows(const float* W, const float* B, int ty, int tx, float (&o)[2][G][4]) {
+// VW consecutive columns from shared memory.
+template <int VW> __device__ __forceinline__ void lds(const float* p, float* f);
+template <> __device__ __forceinline__ void lds<4>(const float* p, float* f) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+}
+template <> __device__ __forceinline__ void lds<2>(const float* p, float* f) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    f[0] = v.x; f[1] = v.y;
+}
+
+// o[i][k] += w(i, j) * B[j][c0 + 8 VW k ...] over the CT streamed rows, c0 the lane's first column.  W: the weight tile, element
+// (row, j) at row * WROW + j * WCOL, its first row being the lane's.
+template <int G, int VW, int NK, int WROW, int WCOL>
+__device__ __forceinline__ void weighted_rows(const float* W, const float* B, float (&o)[LR][NK][VW]) {
     constexpr int P = Pitch<G>::P;
 #pragma unroll 2
     for (int j = 0; j < CT; j += 4) {
-        const float4 w0 = *reinterpret_cast<const float4*>(W + ty * SP + j);
-        const float4 w1 = *reinterpret_cast<const float4*>(W + (ty + 4) * SP + j);
-        const float wa[4] = {w0.x, w0.y, w0.z, w0.w}, wb[4] = {w1.x, w1.y, w1.z, w1.w};
+        float w[LR][4];
+#pragma unroll
+        for (int i = 0; i < LR; ++i) {
+            if (WCOL == 1) {
+                lds<4>(W + 4 * i * WROW + j, w[i]);
+            } else {
+#pragma unroll
+                for (int jj = 0; jj < 4; ++jj) w[i][jj] = W[4 * i * WROW + (j + jj) * WCOL];
+            }
+        }
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const float4 b = *reinterpret_cast<const float4*>(B + (j + jj) * P + 32 * g + tx * 4);
-                o[0][g][0] = fmaf(wa[jj], b.x, o[0][g][0]); o[0][g][1] = fmaf(wa[jj], b.y, o[0][g][1]);
-                o[0][g][2] = fmaf(wa[jj], b.z, o[0][g][2]); o[0][g][3] = fmaf(wa[jj], b.w, o[0][g][3]);
-                o[1][g][0] = fmaf(wb[jj], b.x, o[1][g][0]); o[1][g][1] = fmaf(wb[jj], b.y, o[1][g][1]);
-                o[1][g][2] = fmaf(wb[jj], b.z, o[1][g][2]); o[1][g][3] = fmaf(wb[jj], b.w, o[1][g][3]);
+            for (int k = 0; k < NK; ++k) {
+                float b[VW];
+                lds<VW>(B + (j + jj) * P + 8 * VW * k, b);
+#pragma unroll
+                for (int i = 0; i < LR; ++i)
+#pragma unroll
+                    for (int c = 0; c < VW; ++c) o[i][k][c] = fmaf(w[i][jj], b[c], o[i][k][c]);
             }
         }
     }
 }
 
-// Four consecutive columns of an output row (the row is known to be inside the tensor).
-template <typename T>
+// VW consecutive columns of an output row (the row is known to be inside the tensor).
+template <typename T, int VW>
 __device__ __forceinline__ void store_cols(T* row, int c, int HD, const float* v, float mul, bool vec) {
-    const float t[4] = {v[0] * mul, v[1] * mul, v[2] * mul, v[3] * mul};
-    if (c >= HD) return;
-    if (vec) { st4<T>(row + c, t); return; }
+    float t[VW];
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < VW; ++k) t[k] = v[k] * mul;
+    if (VW == 4 && vec && c < HD) { st4<T>(row + c, t); return; }
+#pragma unroll
+    for (int k = 0; k < VW; ++k)
         if (c + k < HD) row[c + k] = from_f32<T>(t[k]);
 }
 
@@ -137,13 +164,16 @@ __global__ void __launch_bounds__(NW * 32) attn_fwd_kernel(const CmeAttn a, cons
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3;
     const long long base = head_base(a, bh);
     load_rows<T, G, RT, NT>(sQ, (const T*)a.q + base, a.st, q0, a.T, HD, a.scale, vec);
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[2][G][4];
+    float m[LR], l[LR], o[LR][G][4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < LR; ++i) {
+        m[i] = -INFINITY;
+        l[i] = 0.f;
 #pragma unroll
         for (int g = 0; g < G; ++g)
 #pragma unroll
             for (int c = 0; c < 4; ++c) o[i][g][c] = 0.f;
+    }
     const int kend = a.causal ? min(a.T, q0 + RT) : a.T;
     float* wP = sP + warp * WR * SP;
     for (int k0 = 0; k0 < kend; k0 += CT) {
@@ -151,10 +181,10 @@ __global__ void __launch_bounds__(NW * 32) attn_fwd_kernel(const CmeAttn a, cons
         load_rows<T, G, CT, NT>(sK, (const T*)a.k + base, a.st, k0, a.T, HD, 1.f, vec);
         load_rows<T, G, CT, NT>(sV, (const T*)a.v + base, a.st, k0, a.T, HD, 1.f, vec);
         __syncthreads();
-        float s[2][8] = {};
-        dot_2x8<G>(sQ + warp * WR * P, sK, ty, tx, s);
+        float s[LR][8] = {};
+        dot_rows<G, 8>(sQ + warp * WR * P, sK, ty, tx, s);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < LR; ++i) {
             const int q = q0 + warp * WR + ty + 4 * i;
             float mx = -INFINITY;
 #pragma unroll
@@ -184,16 +214,16 @@ __global__ void __launch_bounds__(NW * 32) attn_fwd_kernel(const CmeAttn a, cons
                 for (int c = 0; c < 4; ++c) o[i][g][c] *= alpha;
         }
         __syncwarp();
-        weighted_rows<G>(wP, sV, ty, tx, o);
+        weighted_rows<G, 4, G, SP, 1>(wP + ty * SP, sV + tx * 4, o);
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < LR; ++i) {
         const int q = q0 + warp * WR + ty + 4 * i;
         if (q < a.T) {
             const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
             T* out = (T*)a.o + head_base_o(a, bh) + (long long)q * a.ost;
 #pragma unroll
-            for (int g = 0; g < G; ++g) store_cols<T>(out, tx * 4 + 32 * g, HD, o[i][g], inv, vec);
+            for (int g = 0; g < G; ++g) store_cols<T, 4>(out, tx * 4 + 32 * g, HD, o[i][g], inv, vec);
             if (tx == 0 && a.lse) a.lse[(long long)bh * a.T + q] = m[i] + logf(l[i]);
         }
     }
@@ -255,8 +285,9 @@ __global__ void __launch_bounds__(256) attn_delta_hd64_kernel(const CmeAttn a, f
 }
 
 // delta[r] = sum_d dO[r][d] * O[r][d] for the rows whose dO tile has just been staged, one warp per row.
-template <typename T, int G, int NW>
+template <typename T, int G>
 __device__ __forceinline__ void delta_rows(float* dst, const float* sdO, const T* o, long long ost, int r0, int T_, int HD) {
+    constexpr int NW = BWD_THREADS / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < CT / NW; ++k) {
@@ -280,9 +311,11 @@ __device__ __forceinline__ void delta_rows(float* dst, const float* sdO, const T
 // blockIdx.z == 1: the block owns 64 queries and streams keys:    dQ = scale * sum_j dS_ij K_j
 // Both kinds run in one launch, and delta = rowsum(dO * O) is made from the staged rows instead of by a kernel before.
 template <typename T, int G>
-__global__ void __launch_bounds__(BWD_NW * 32) attn_bwd_kernel(const CmeAttn a, const bool vec) {
-    constexpr int P = Pitch<G>::P, NT = BWD_NW * 32, RT = BWD_NW * WR;
-    static_assert(RT == CT, "own and streamed tiles have the same height");
+__global__ void __launch_bounds__(BWD_THREADS) attn_bwd_kernel(const CmeAttn a, const bool vec) {
+    constexpr int P = Pitch<G>::P, NT = BWD_THREADS, RT = BWD_ROWS;
+    // a lane's columns: VW at half * 16 G + tx * VW, then every 8 VW
+    constexpr int VW = G % 2 == 0 ? 4 : 2, NK = 2 * G / VW;
+    static_assert(RT == CT && NT / 32 == 2 * RT / WR, "own and streamed tiles of one height, two warps per 16 rows");
     extern __shared__ __align__(16) float sm[];
     float* sA = sm;                    // own rows       K | Q
     float* sB = sA + RT * P;           //                V | dO
@@ -295,105 +328,92 @@ __global__ void __launch_bounds__(BWD_NW * 32) attn_bwd_kernel(const CmeAttn a, 
     const bool kv = blockIdx.z == 0;
     const int bh = blockIdx.y, r0 = blockIdx.x * RT, HD = a.HD;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3;
+    const int w0 = (warp & 3) * WR, half = warp >> 2, c0 = half * 16 * G + tx * VW;
     const long long base = head_base(a, bh), obase = head_base_o(a, bh);
     const T* q = (const T*)a.q + base; const T* k = (const T*)a.k + base; const T* v = (const T*)a.v + base;
     const T* d_o = (const T*)a.d_o + obase; const T* o = (const T*)a.o + obase;
     const float* lse = a.lse + (long long)bh * a.T;
     load_rows<T, G, RT, NT>(sA, kv ? k : q, a.st, r0, a.T, HD, 1.f, vec);
     load_rows<T, G, RT, NT>(sB, kv ? v : d_o, kv ? a.st : a.ost, r0, a.T, HD, 1.f, vec);
-    float acc1[2][G][4], acc2[2][G][4];
+    float acc1[LR][NK][VW], acc2[LR][NK][VW];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < LR; ++i)
 #pragma unroll
-        for (int g = 0; g < G; ++g)
+        for (int g = 0; g < NK; ++g)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) { acc1[i][g][c] = 0.f; acc2[i][g][c] = 0.f; }
+            for (int c = 0; c < VW; ++c) { acc1[i][g][c] = 0.f; acc2[i][g][c] = 0.f; }
     if (!kv) {
         __syncthreads();
-        delta_rows<T, G, BWD_NW>(sDl, sB, o, a.ost, r0, a.T, HD);
+        delta_rows<T, G>(sDl, sB, o, a.ost, r0, a.T, HD);
     }
-    const float* wA = sA + warp * WR * P;
-    const float* wB = sB + warp * WR * P;
-    float* wP = sP + warp * WR * SP;
-    float* wS = sS + warp * WR * SP;
     // causal: queries see keys <= their index.  dQ blocks stop early; dK / dV blocks start late.
-    const int c_begin = (kv && a.causal) ? r0 : 0;
-    const int c_end = (!kv && a.causal) ? min(a.T, r0 + RT) : a.T;
-    for (int c0 = c_begin; c0 < c_end; c0 += CT) {
+    const int s_begin = (kv && a.causal) ? r0 : 0;
+    const int s_end = (!kv && a.causal) ? min(a.T, r0 + RT) : a.T;
+    for (int s0 = s_begin; s0 < s_end; s0 += CT) {
         __syncthreads();
-        load_rows<T, G, CT, NT>(sC, kv ? q : k, a.st, c0, a.T, HD, 1.f, vec);
-        load_rows<T, G, CT, NT>(sD, kv ? d_o : v, kv ? a.ost : a.st, c0, a.T, HD, 1.f, vec);
+        load_rows<T, G, CT, NT>(sC, kv ? q : k, a.st, s0, a.T, HD, 1.f, vec);
+        load_rows<T, G, CT, NT>(sD, kv ? d_o : v, kv ? a.ost : a.st, s0, a.T, HD, 1.f, vec);
         __syncthreads();
-        if (kv) delta_rows<T, G, BWD_NW>(sDl, sD, o, a.ost, c0, a.T, HD);
-        float s[2][8] = {}, dp[2][8] = {};
-        dot_2x8<G>(wA, sC, ty, tx, s);
-        dot_2x8<G>(wB, sD, ty, tx, dp);
+        if (kv) delta_rows<T, G>(sDl, sD, o, a.ost, s0, a.T, HD);
+        float s[LR][4] = {}, dp[LR][4] = {};
+        dot_rows<G, 4>(sA + w0 * P, sC + half * 32 * P, ty, tx, s);
+        dot_rows<G, 4>(sB + w0 * P, sD + half * 32 * P, ty, tx, dp);
         if (kv) __syncthreads();                   // delta is written by all warps
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < LR; ++i) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int own = warp * WR + ty + 4 * i, str = tx + 8 * j;
-                const int qi = kv ? c0 + str : r0 + own, ki = kv ? r0 + own : c0 + str;
+            for (int j = 0; j < 4; ++j) {
+                const int own = w0 + ty + 4 * i, str = half * 32 + tx + 8 * j;
+                const int qi = kv ? s0 + str : r0 + own, ki = kv ? r0 + own : s0 + str;
                 const bool ok = qi < a.T && ki < a.T && (!a.causal || ki <= qi);
                 const float p = ok ? __expf(s[i][j] * a.scale - lse[qi]) : 0.f;
-                if (kv) wP[(ty + 4 * i) * SP + str] = p;
-                wS[(ty + 4 * i) * SP + str] = ok ? p * (dp[i][j] - sDl[kv ? str : own]) : 0.f;
+                if (kv) sP[own * SP + str] = p;
+                sS[own * SP + str] = ok ? p * (dp[i][j] - sDl[kv ? str : own]) : 0.f;
             }
         }
-        __syncwarp();
+        __syncthreads();                           // the other half of these rows' scores is another warp's
+        const float* wP = sP + (w0 + ty) * SP;
+        const float* wS = sS + (w0 + ty) * SP;
         if (kv) {
-            weighted_rows<G>(wP, sD, ty, tx, acc1);        // dV += P^T dO
-            weighted_rows<G>(wS, sC, ty, tx, acc2);        // dK += dS^T Q
+            weighted_rows<G, VW, NK, SP, 1>(wP, sD + c0, acc1);        // dV += P^T dO
+            weighted_rows<G, VW, NK, SP, 1>(wS, sC + c0, acc2);        // dK += dS^T Q
         } else {
-            weighted_rows<G>(wS, sC, ty, tx, acc1);        // dQ += dS K
+            weighted_rows<G, VW, NK, SP, 1>(wS, sC + c0, acc1);        // dQ += dS K
         }
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int r = r0 + warp * WR + ty + 4 * i;
+    for (int i = 0; i < LR; ++i) {
+        const int r = r0 + w0 + ty + 4 * i;
         if (r < a.T) {
             const long long off = base + (long long)r * a.st;
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const int c = tx * 4 + 32 * g;
+            for (int g = 0; g < NK; ++g) {
+                const int c = c0 + 8 * VW * g;
                 if (kv) {
-                    store_cols<T>((T*)a.dv + off, c, HD, acc1[i][g], 1.f, vec);
-                    store_cols<T>((T*)a.dk + off, c, HD, acc2[i][g], a.scale, vec);
+                    store_cols<T, VW>((T*)a.dv + off, c, HD, acc1[i][g], 1.f, vec);
+                    store_cols<T, VW>((T*)a.dk + off, c, HD, acc2[i][g], a.scale, vec);
                 } else {
-                    store_cols<T>((T*)a.dq + off, c, HD, acc1[i][g], a.scale, vec);
+                    store_cols<T, VW>((T*)a.dq + off, c, HD, acc1[i][g], a.scale, vec);
                 }
             }
         }
     }
     if (gridDim.z == 1) {                          // T <= 64: dQ_i = scale * sum_j dS_ij K_j from the tile at hand
-        __syncthreads();
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < LR; ++i)
 #pragma unroll
-            for (int g = 0; g < G; ++g)
+            for (int g = 0; g < NK; ++g)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) acc1[i][g][c] = 0.f;
-        const int i0 = warp * WR + ty;
-#pragma unroll 4
-        for (int j = 0; j < RT; ++j) {
-            const float wa = sS[j * SP + i0], wb = sS[j * SP + i0 + 4];
+                for (int c = 0; c < VW; ++c) acc1[i][g][c] = 0.f;
+        weighted_rows<G, VW, NK, 1, SP>(sS + w0 + ty, sA + c0, acc1);  // the tile read down its columns
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const float4 b = *reinterpret_cast<const float4*>(sA + j * P + 32 * g + tx * 4);
-                acc1[0][g][0] = fmaf(wa, b.x, acc1[0][g][0]); acc1[0][g][1] = fmaf(wa, b.y, acc1[0][g][1]);
-                acc1[0][g][2] = fmaf(wa, b.z, acc1[0][g][2]); acc1[0][g][3] = fmaf(wa, b.w, acc1[0][g][3]);
-                acc1[1][g][0] = fmaf(wb, b.x, acc1[1][g][0]); acc1[1][g][1] = fmaf(wb, b.y, acc1[1][g][1]);
-                acc1[1][g][2] = fmaf(wb, b.z, acc1[1][g][2]); acc1[1][g][3] = fmaf(wb, b.w, acc1[1][g][3]);
-            }
+        for (int i = 0; i < LR; ++i) {
+            const int r = w0 + ty + 4 * i;
+            if (r < a.T)
+#pragma unroll
+                for (int g = 0; g < NK; ++g)
+                    store_cols<T, VW>((T*)a.dq + base + (long long)r * a.st, c0 + 8 * VW * g, HD, acc1[i][g], a.scale, vec);
         }
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-            if (i0 + 4 * i < a.T)
-#pragma unroll
-                for (int g = 0; g < G; ++g)
-                    store_cols<T>((T*)a.dq + base + (long long)(i0 + 4 * i) * a.st, tx * 4 + 32 * g, HD, acc1[i][g], a.scale,
-                                  vec);
     }
 }
 
@@ -428,25 +448,25 @@ template <typename T, int G, int NW> int fwd_launch(const CmeAttn* a, cudaStream
     return CME_OK;
 }
 template <typename T, int G> int bwd_launch(const CmeAttn* a, cudaStream_t st) {
-    constexpr int P = Pitch<G>::P, RT = BWD_NW * WR;
+    constexpr int P = Pitch<G>::P, RT = BWD_ROWS;
     constexpr size_t smem = (4 * RT * P + 2 * RT * SP + CT) * sizeof(float);
     static_assert(smem <= 227 * 1024, "one block's shared memory");
     auto k = attn_bwd_kernel<T, G>;
     int rc = allow_smem(k, smem);
     if (rc) return rc;
-    CME_CUDA(cme_launch_dependent(k, dim3(cme_cdiv(a->T, RT), a->nb * a->nh, a->T <= RT ? 1 : 2), dim3(BWD_NW * 32), smem,
+    CME_CUDA(cme_launch_dependent(k, dim3(cme_cdiv(a->T, RT), a->nb * a->nh, a->T <= RT ? 1 : 2), dim3(BWD_THREADS), smem,
                                   st, *a, rows_vectorisable(a, true)));
     CME_LAUNCH_CHECK();
     return CME_OK;
 }
 template <typename T> int fwd_t(const CmeAttn* a, cudaStream_t st) {
     // 32 query rows per block; 16 where that leaves SMs without a block
-    const bool few = (long long)cme_cdiv(a->T, 4 * WR) * a->nb * a->nh < 148;
+    const bool few = (long long)cme_cdiv(a->T, 2 * WR) * a->nb * a->nh < 148;
     switch (cme_cdiv(a->HD, 32)) {
-        case 1: return few ? fwd_launch<T, 1, 2>(a, st) : fwd_launch<T, 1, 4>(a, st);
-        case 2: return few ? fwd_launch<T, 2, 2>(a, st) : fwd_launch<T, 2, 4>(a, st);
-        case 3: return few ? fwd_launch<T, 3, 2>(a, st) : fwd_launch<T, 3, 4>(a, st);
-        default: return few ? fwd_launch<T, 4, 2>(a, st) : fwd_launch<T, 4, 4>(a, st);
+        case 1: return few ? fwd_launch<T, 1, 1>(a, st) : fwd_launch<T, 1, 2>(a, st);
+        case 2: return few ? fwd_launch<T, 2, 1>(a, st) : fwd_launch<T, 2, 2>(a, st);
+        case 3: return few ? fwd_launch<T, 3, 1>(a, st) : fwd_launch<T, 3, 2>(a, st);
+        default: return few ? fwd_launch<T, 4, 1>(a, st) : fwd_launch<T, 4, 2>(a, st);
     }
 }
 template <typename T> int bwd_t(const CmeAttn* a, cudaStream_t st) {
