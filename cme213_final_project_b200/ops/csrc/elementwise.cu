@@ -148,16 +148,6 @@ __global__ void dact_colsum_scalar_kernel(const T* dout, const T* pre, T* g, flo
     }
     partial[(long long)blockIdx.y * cols + c] = s;
 }
-template <typename T>
-__global__ void colsum_finalize_kernel(const float* partial, int splits, int cols, T* out, int accumulate) {
-    pdl_wait();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.f;
-    for (int k = 0; k < splits; ++k) s += partial[(long long)k * cols + c];
-    out[c] = from_f32<T>(accumulate ? to_f32<T>(out[c]) + s : s);
-}
-
 template <typename T> __global__ void scale_kernel(T* x, long long n, float s) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         x[i] = from_f32<T>(to_f32<T>(x[i]) * s);
@@ -553,7 +543,8 @@ int bias_act_res_t(const void* x, const void* bias, const void* res, void* pre, 
 
 // dbias[c] (+)= sum over the `slabs` rows of partial[slabs][cols], added in a fixed order: a block covers 32 columns
 // with 32 row groups; each thread sums every 32nd row (four independent chains), then the 32 groups are added in
-// shared memory.  The rows come from a GEMM epilogue that sums its stored output per 32-row slab.  One block per 32
+// shared memory.  The rows come from a GEMM epilogue that sums its stored output per 32-row slab, or from
+// dact_colsum_kernel's row splits.  One block per 32
 // columns leaves the chip mostly idle, so the time is that of a thread's chain of loads: 32 groups instead of 8 make it
 // a quarter as long: 512 rows of 3072 columns 15.5 -> 6.5 us.
 constexpr int SLAB_GROUPS = 32;
@@ -605,7 +596,7 @@ int dact_colsum_t(const void* dout, const void* pre, void* g, void* dbias, float
     }
     CME_LAUNCH_CHECK();
     if (dbias) {
-        CME_CUDA(cme_launch_dependent(colsum_finalize_kernel<T>, dim3(cme_cdiv(cols, 256)), dim3(256), 0, st,
+        CME_CUDA(cme_launch_dependent(colsum_slabs_finalize_kernel<T>, dim3(cme_cdiv(cols, 32)), dim3(SLAB_GROUPS * 32), 0, st,
                                       (const float*)scratch, splits, cols, (T*)dbias, accumulate));
         CME_LAUNCH_CHECK();
     }
