@@ -44,14 +44,15 @@ __device__ __forceinline__ float dact_f(float pre, int act) {
 
 // out[m, n] = act(x[m, n] + bias[n]) + residual[m, n]; any of bias / residual / pre_out may be null.
 // One thread per vector of the row-major [rows, cols] matrix; cols is a multiple of the vector width.
-template <typename T>
-__global__ void bias_act_res_kernel(const T* __restrict__ x, const T* __restrict__ bias, const T* __restrict__ res,
-                                    T* __restrict__ pre_out, T* __restrict__ out, long long nvec, int cols, int act) {
+// The column comes from a 32-bit remainder (Index = unsigned) whenever the vectors can be counted in 31 bits.
+template <typename T, typename Index>
+__global__ void __launch_bounds__(256) bias_act_res_kernel(const T* __restrict__ x, const T* __restrict__ bias, const T* __restrict__ res,
+                                    T* __restrict__ pre_out, T* __restrict__ out, Index nvec, int cols, int act) {
     constexpr int W = Vw<T>::N;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long e = i * W;
-        const int c = (int)(e % cols);
+    const Index cvec = cols / W, step = (Index)gridDim.x * blockDim.x;
+    for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += step) {
+        const long long e = (long long)i * W;
+        const int c = (int)(i % cvec) * W;
         float v[W];
         ldv<T>(x + e, v);
         if (bias) {
@@ -531,9 +532,12 @@ int bias_act_res_t(const void* x, const void* bias, const void* res, void* pre, 
     const bool vec = cols % W == 0 && aligned16((const T*)x) && aligned16((const T*)out) &&
                      (!bias || aligned16((const T*)bias)) && (!res || aligned16((const T*)res)) &&
                      (!pre || aligned16((const T*)pre));
-    if (vec)
-        bias_act_res_kernel<T><<<grid_for(n / W), 256, 0, st>>>((const T*)x, (const T*)bias, (const T*)res, (T*)pre,
-                                                                 (T*)out, n / W, cols, act);
+    if (vec && n / W < (1ll << 31))
+        bias_act_res_kernel<T, unsigned><<<grid_for(n / W), 256, 0, st>>>((const T*)x, (const T*)bias, (const T*)res, (T*)pre,
+                                                                           (T*)out, (unsigned)(n / W), cols, act);
+    else if (vec)
+        bias_act_res_kernel<T, unsigned long long><<<grid_for(n / W), 256, 0, st>>>(
+            (const T*)x, (const T*)bias, (const T*)res, (T*)pre, (T*)out, (unsigned long long)(n / W), cols, act);
     else
         bias_act_res_scalar_kernel<T><<<grid_for(n), 256, 0, st>>>((const T*)x, (const T*)bias, (const T*)res,
                                                                     (T*)pre, (T*)out, n, cols, act);
