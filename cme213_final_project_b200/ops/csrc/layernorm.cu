@@ -337,12 +337,15 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __rest
 }
 
 // dgamma[c] (+)= sum_b partial[b][0][c];  dbeta[c] (+)= sum_b partial[b][1][c]
-// Block (16 columns x 16 block-groups): each thread sums every 16th partial, then a fixed-order shared-memory
-// reduction over the 16 groups (deterministic).
+// Block (16 columns x 64 block-groups): each thread sums every 64th partial, then a fixed-order shared-memory reduction
+// over the groups (deterministic).  The time is that of a thread's chain of loads, so it is kept to a handful: with 16
+// groups 296 partials of 2 x 768 columns took 3.5 us, now 2.9 us.
+constexpr int LN_FIN_GROUPS = 64;
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(16 * LN_FIN_GROUPS)
 ln_bwd_finalize_kernel(const float* __restrict__ partial, int nblocks, int D, T* dgamma, T* dbeta, int accumulate) {
-    __shared__ float sm[16][17];
+    constexpr int NG = LN_FIN_GROUPS;
+    __shared__ float sm[NG][17];
     pdl_wait();
     const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;
     const int c = blockIdx.x * 16 + cx;
@@ -350,21 +353,26 @@ ln_bwd_finalize_kernel(const float* __restrict__ partial, int nblocks, int D, T*
     if (c < 2 * D) {
         float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;      // independent chains: the loads of four blocks overlap
         int b = ry;
-        for (; b + 48 < nblocks; b += 64) {
+        for (; b + 3 * NG < nblocks; b += 4 * NG) {
             s0 += partial[(long long)b * 2 * D + c];
-            s1 += partial[(long long)(b + 16) * 2 * D + c];
-            s2 += partial[(long long)(b + 32) * 2 * D + c];
-            s3 += partial[(long long)(b + 48) * 2 * D + c];
+            s1 += partial[(long long)(b + NG) * 2 * D + c];
+            s2 += partial[(long long)(b + 2 * NG) * 2 * D + c];
+            s3 += partial[(long long)(b + 3 * NG) * 2 * D + c];
         }
-        for (; b < nblocks; b += 16) s0 += partial[(long long)b * 2 * D + c];
+        for (; b < nblocks; b += NG) s0 += partial[(long long)b * 2 * D + c];
         s = (s0 + s1) + (s2 + s3);
     }
     sm[ry][cx] = s;
     __syncthreads();
-    if (ry == 0 && c < 2 * D) {
+    if (ry < 4 && c < 2 * D) {                             // 64 groups -> 4, then 4 -> 1
         float t = 0.f;
 #pragma unroll
-        for (int r = 0; r < 16; ++r) t += sm[r][cx];
+        for (int r = 0; r < NG / 4; ++r) t += sm[ry * (NG / 4) + r][cx];
+        sm[ry * (NG / 4)][cx] = t;
+    }
+    __syncthreads();
+    if (ry == 0 && c < 2 * D) {
+        const float t = (sm[0][cx] + sm[NG / 4][cx]) + (sm[NG / 2][cx] + sm[3 * NG / 4][cx]);
         T* dst = (c < D) ? dgamma + c : dbeta + (c - D);
         *dst = from_f32<T>(accumulate ? to_f32<T>(*dst) + t : t);
     }
@@ -480,7 +488,7 @@ int ln_bwd_t(const void* dy, const void* x, const void* g, const float* mean, co
         CME_CUDA(cudaStreamWaitEvent(fin_st, fin_ev, 0));
         st = fin_st;
     }
-    CME_CUDA(cme_launch_dependent(ln_bwd_finalize_kernel<T>, dim3(cme_cdiv(2 * D, 16)), dim3(256), 0, st,
+    CME_CUDA(cme_launch_dependent(ln_bwd_finalize_kernel<T>, dim3(cme_cdiv(2 * D, 16)), dim3(16 * LN_FIN_GROUPS), 0, st,
                                   (const float*)scratch, nblocks, D, (T*)dgamma, (T*)dbeta, accumulate));
     CME_LAUNCH_CHECK();
     return CME_OK;
