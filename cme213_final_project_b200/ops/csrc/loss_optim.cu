@@ -255,13 +255,27 @@ cudaError_t ce_short(const void* logits, const int* targets, void* dlogits, floa
 #undef CME_CES
 }
 
-// out (+)= weight * sum(x[0..n)); single block, fixed order.
+// out (+)= weight * sum(x[0..n)); single block, fixed order.  One block's time is its chain of loads, so each thread has
+// four 16-byte loads in flight where x is aligned (16384 row losses: 5.9 us with a 4-byte load per step, 2.5 us now).
 __global__ void __launch_bounds__(1024) reduce_scalar_kernel(const float* __restrict__ x, int n, float weight, float* out,
                                                              int accumulate) {
     __shared__ float scratch[32];
     pdl_wait();
     float s = 0.f;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) s += x[i];
+    int done = 0;
+    if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        const float4* v = reinterpret_cast<const float4*>(x);
+        const int nv = n / 4, step = blockDim.x;
+        done = nv * 4;
+        for (int i = threadIdx.x; i < nv; i += 4 * step) {
+            float4 u[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) u[k] = i + k * step < nv ? v[i + k * step] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) s += (u[k].x + u[k].y) + (u[k].z + u[k].w);
+        }
+    }
+    for (int i = done + threadIdx.x; i < n; i += blockDim.x) s += x[i];
     s = block_sum(s, scratch);
     if (threadIdx.x == 0) *out = (accumulate ? *out : 0.f) + s * weight;
 }
