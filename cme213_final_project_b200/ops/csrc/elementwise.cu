@@ -308,23 +308,29 @@ tok_bwd_scan_kernel(const int* __restrict__ tokens, const T* __restrict__ dout, 
     }
 }
 // Token-table gradient by stripes of the vocabulary: block (stripe, chunk) owns the rows id = stripe, stripe + S, ... and
-// one chunk of 32 16-byte vectors of columns.  It sorts the tokens of its rows by row in shared memory (counting sort,
-// stable), then every row of the stripe is summed in fp32 in token order and written exactly once.
+// one chunk of 32 16-byte vectors of columns.  It picks its tokens out of the list, sorts them by row in shared memory
+// (counting sort, stable), then every row of the stripe is summed in fp32 in token order and written exactly once.
 //     dtok[v, :] (+)= sum_{bt : tokens[bt] == v} dout[bt, :]
 // Against a warp per token with bf16 atomics into a cleared table: no clearing pass, one rounding per element instead of
 // one per token, the same bits every time, and no queue at the rows of frequent words.  Interleaved stripes spread those,
 // whose ids are near one another, over the blocks.
-// All of it is latency, so there is one wave of blocks (two per SM) and loads are issued in batches: sixteen token ids per
-// lane (64 KB of them from L2 for 16384 tokens; the second pass finds them in L1), and eight tokens of a table row.  Rows
-// without a token are stores only; the others are handed out to the 16 warps one by one; rows with more than HOT tokens
-// are summed by the whole block in fixed shares.
-// 16384 tokens, 50304 x 768 bf16: clear + atomics 34 us, this about 37 us with the sums in fp32; with the position table and
-// the gather the call went from 58.1 to 56.0 us and its gradient from 4.5e-3 to 1.8e-3 off the exact sums.  16384 tokens, 65 x
-// 384 (where a block per vocabulary row had been used): 78 -> 16 us.
-constexpr int STRIPE_WARPS = 16, STRIPE_HOT = 64, STRIPE_MAX_BT = 65535, STRIPE_BATCH = 16, STRIPE_ENTRIES = 8;
+// All of it is latency and bookkeeping, so there is one wave of blocks (two per SM), the token list is read once (its few
+// tokens of the stripe are kept in shared memory for the two passes of the sort), and loads are issued in batches: sixteen
+// token ids per lane, eight tokens of a table row.  Rows without a token are stores only; the others are handed out to the
+// 16 warps one by one; rows with many tokens are summed by the whole block in fixed shares.
+// 16384 tokens, 50304 x 768 bf16: clear + atomics 34 us, this 35 us with the sums in fp32 (40 us when both passes of the sort
+// read the list and one warp added up the shares of a long row, 52 us with all three chunks in one block); with the position
+// table and the gather the call went from 58.1 to 51.5 us and its gradient from 4.5e-3 to 1.8e-3 off the exact sums.  2048
+// tokens, 65 x 128: 5.4 us, 8.9 us while a row of up to 64 tokens was left to one warp although the stripe had no other.
+constexpr int STRIPE_WARPS = 16, STRIPE_BATCH = 16, STRIPE_ENTRIES = 8, STRIPE_MAX_BT = 65535;
+constexpr size_t STRIPE_SMEM = 200 * 1024;
+constexpr int STRIPE_HOT = 64, STRIPE_HOT_FEW = 8;       // the block sums rows with more tokens: eight rounds of a warp's loads
+                                                         // where the stripe has a row for every warp, else one
 struct StripePlan {
     int S, R, chunks;            // stripes, rows per stripe (ceil), column chunks
     unsigned magic;              // ceil(2^32 / S): id / S == umulhi(id, magic) while V * S < 2^32
+    int per, nhot;               // tokens per warp (a multiple of 32), room for rows summed by the block
+    bool keep;                   // shared memory has room for the warps' lists
     size_t smem;
 };
 inline StripePlan stripe_plan(int BT, int D, int V, int W) {
@@ -334,26 +340,33 @@ inline StripePlan stripe_plan(int BT, int D, int V, int W) {
     p.S = (int)(s < V ? s : V);
     p.R = cme_cdiv(V, p.S);
     p.magic = (unsigned)(((1ull << 32) + p.S - 1) / p.S);     // S == 1 wraps to 0: handled in the kernel
+    p.per = (cme_cdiv(BT, STRIPE_WARPS) + 31) / 32 * 32;
+    p.nhot = p.R < STRIPE_WARPS ? p.R : BT / STRIPE_HOT + 1;
     // partial sums | counts [16][R] u16 (4-byte multiple) | starts [R + 1] i32 | hot rows i32 | rows with tokens i32 | sorted
-    // positions [BT] u16
+    // positions [BT] u16 | the warps' positions [16][per] u16
     const size_t cnt = ((size_t)STRIPE_WARPS * p.R * 2 + 3) / 4 * 4;
-    p.smem = (size_t)STRIPE_WARPS * 32 * W * 4 + cnt + ((size_t)p.R + 1) * 4 + (BT / STRIPE_HOT + 1) * 4 +
-             (size_t)p.R * 4 + (size_t)BT * 2;
+    p.smem = (size_t)STRIPE_WARPS * 32 * W * 4 + cnt + ((size_t)p.R + 1) * 4 + (size_t)p.nhot * 4 + (size_t)p.R * 4 +
+             (size_t)BT * 2;
+    const size_t lists = (size_t)STRIPE_WARPS * p.per * 2;
+    p.keep = p.smem + lists <= STRIPE_SMEM;
+    if (p.keep) p.smem += lists;
     return p;
 }
 template <typename T>
 __global__ void __launch_bounds__(STRIPE_WARPS * 32, 2)
 tok_bwd_stripe_kernel(const int* __restrict__ tokens, const T* __restrict__ dout, T* __restrict__ dtok, int BT, int D, int V,
-                      int S, int R, unsigned magic, int accumulate) {
-    constexpr int W = Vw<T>::N, NW = STRIPE_WARPS;
+                      const StripePlan plan, int accumulate) {
+    constexpr int W = Vw<T>::N, NW = STRIPE_WARPS, NE = STRIPE_ENTRIES;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     __shared__ int n_hot, n_used, next_used;
+    const int S = plan.S, R = plan.R, per = plan.per;
     float* part = reinterpret_cast<float*>(sm_raw);                        // [NW][W][32]
     unsigned short* cnt = reinterpret_cast<unsigned short*>(part + NW * W * 32);   // [NW][R]
     int* start = reinterpret_cast<int*>(sm_raw + (size_t)NW * W * 32 * 4 + ((size_t)NW * R * 2 + 3) / 4 * 4);   // [R + 1]
-    int* hot = start + R + 1;                                              // [BT / HOT + 1]
-    int* used = hot + BT / STRIPE_HOT + 1;                                 // [R] rows with 1 to HOT tokens, any order
+    int* hot = start + R + 1;                                              // [nhot]
+    int* used = hot + plan.nhot;                                           // [R] the other rows with tokens, any order
     unsigned short* sorted = reinterpret_cast<unsigned short*>(used + R);  // [BT]
+    unsigned short* found = sorted + BT;                                   // [NW][per] positions of the stripe's tokens
     pdl_wait();
     const int stripe = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int c = (blockIdx.y * 32 + lane) * W;
@@ -361,47 +374,61 @@ tok_bwd_stripe_kernel(const int* __restrict__ tokens, const T* __restrict__ dout
     for (int i = threadIdx.x; i < NW * R; i += NW * 32) cnt[i] = 0;
     if (threadIdx.x == 0) n_hot = n_used = next_used = 0;
     __syncthreads();
-    const int per = (((BT + NW - 1) / NW) + 31) / 32 * 32, t0 = warp * per, t1 = min(BT, t0 + per);
+    const int t0 = warp * per, t1 = min(BT, t0 + per);
     unsigned short* wc = cnt + warp * R;
+    unsigned short* wf = found + warp * per;
     // local row of a token id, or -1 if it is not of this stripe
     auto local = [&](int id) -> int {
         if (id < 0 || id >= V) return -1;
-        const int q = S == 1 ? id : (int)__umulhi((unsigned)id, magic);
+        const int q = S == 1 ? id : (int)__umulhi((unsigned)id, plan.magic);
         return id - q * S == stripe ? q : -1;
     };
-    // pass 1 counts each warp's tokens per row; pass 2 puts their positions in order behind the earlier warps' ones
+    // the warp's tokens of this stripe, in order (without room for them, all its tokens)
+    const bool keep = plan.keep;
+    int nf = keep ? 0 : max(t1 - t0, 0);
+    for (int base = t0; keep && base < t1; base += 32 * STRIPE_BATCH) {
+        int id[STRIPE_BATCH];
+#pragma unroll
+        for (int k = 0; k < STRIPE_BATCH; ++k) id[k] = base + 32 * k + lane < t1 ? tokens[base + 32 * k + lane] : -1;
+#pragma unroll
+        for (int k = 0; k < STRIPE_BATCH; ++k) {
+            const bool mine = local(id[k]) >= 0;
+            const unsigned m = __ballot_sync(0xffffffffu, mine);
+            if (mine) wf[nf + __popc(m & ((1u << lane) - 1))] = (unsigned short)(base + 32 * k + lane);
+            nf += __popc(m);
+        }
+    }
+    __syncwarp();
+    // pass 0 counts the warp's tokens per row; pass 1 puts their positions in order behind the earlier warps' ones
     for (int pass = 0; pass < 2; ++pass) {
-        for (int base = t0; base < t1; base += 32 * STRIPE_BATCH) {
-            int row[STRIPE_BATCH];
-#pragma unroll
-            for (int k = 0; k < STRIPE_BATCH; ++k) row[k] = base + 32 * k + lane < t1 ? tokens[base + 32 * k + lane] : -1;
-#pragma unroll
-            for (int k = 0; k < STRIPE_BATCH; ++k) {
-                row[k] = local(row[k]);
-                if (!__any_sync(0xffffffffu, row[k] >= 0)) continue;
-                const unsigned same = __match_any_sync(0xffffffffu, row[k]);
-                const int before = __popc(same & ((1u << lane) - 1));
-                if (row[k] >= 0) {
-                    const int at = wc[row[k]];
-                    if (pass) sorted[start[row[k]] + at + before] = (unsigned short)(base + 32 * k + lane);
-                }
-                __syncwarp();
-                if (row[k] >= 0 && before == 0) wc[row[k]] = (unsigned short)(wc[row[k]] + __popc(same));
-                __syncwarp();
+        for (int base = 0; base < nf; base += 32) {
+            const int pos = base + lane < nf ? (keep ? wf[base + lane] : t0 + base + lane) : -1;
+            const int row = pos >= 0 ? local(tokens[pos]) : -1;
+            if (!__any_sync(0xffffffffu, row >= 0)) continue;
+            const unsigned same = __match_any_sync(0xffffffffu, row);
+            const int before = __popc(same & ((1u << lane) - 1));
+            if (row >= 0) {
+                const int at = wc[row];
+                if (pass) sorted[start[row] + at + before] = (unsigned short)pos;
             }
+            __syncwarp();
+            if (row >= 0 && before == 0) wc[row] = (unsigned short)(wc[row] + __popc(same));
+            __syncwarp();
         }
         __syncthreads();
         if (pass) break;
         // each row's counts become the warps' offsets in the row; `start` the rows' lengths, then their first places
+        const int hot_at = R >= NW ? STRIPE_HOT : STRIPE_HOT_FEW;
         for (int r = threadIdx.x; r < R; r += NW * 32) {
             int n = 0;
+#pragma unroll
             for (int w = 0; w < NW; ++w) {
                 const int k = cnt[w * R + r];
                 cnt[w * R + r] = (unsigned short)n;
                 n += k;
             }
             start[r] = n;
-            if (n > STRIPE_HOT) hot[atomicAdd(&n_hot, 1)] = r;
+            if (n > hot_at) hot[atomicAdd(&n_hot, 1)] = r;
             else if (n > 0) used[atomicAdd(&n_used, 1)] = r;
         }
         __syncthreads();
@@ -432,26 +459,16 @@ tok_bwd_stripe_kernel(const int* __restrict__ tokens, const T* __restrict__ dout
             if (id < V && start[r + 1] == start[r]) stv<T>(dtok + id * D + c, zero);
         }
     }
-    for (;;) {
-        int u = 0;
-        if (lane == 0) u = atomicAdd(&next_used, 1);
-        u = __shfl_sync(0xffffffffu, u, 0);
-        if (u >= n_used) break;
-        if (!in) continue;
-        const int r = used[u], n0 = start[r], n = start[r + 1] - n0;
-        T* dst = dtok + ((long long)r * S + stripe) * D + c;
-        float s[W];
+    // s += the rows dout[sorted[e0 .. e1)], NE loads in flight
+    auto add_tokens = [&](float (&s)[W], int e0, int e1) {
+        for (int e = e0; e < e1; e += NE) {
+            uint4 raw[NE];
 #pragma unroll
-        for (int j = 0; j < W; ++j) s[j] = 0.f;
-        if (accumulate) ldv<T>(dst, s);
-        for (int e0 = 0; e0 < n; e0 += STRIPE_ENTRIES) {
-            uint4 raw[STRIPE_ENTRIES];
+            for (int k = 0; k < NE; ++k)
+                if (e + k < e1) raw[k] = *reinterpret_cast<const uint4*>(src + (long long)sorted[e + k] * D);
 #pragma unroll
-            for (int k = 0; k < STRIPE_ENTRIES; ++k)
-                if (e0 + k < n) raw[k] = *reinterpret_cast<const uint4*>(src + (long long)sorted[n0 + e0 + k] * D);
-#pragma unroll
-            for (int k = 0; k < STRIPE_ENTRIES; ++k) {
-                if (e0 + k < n) {
+            for (int k = 0; k < NE; ++k) {
+                if (e + k < e1) {
                     float x[W];
                     unpack_words<T>(raw[k], x);
 #pragma unroll
@@ -459,38 +476,48 @@ tok_bwd_stripe_kernel(const int* __restrict__ tokens, const T* __restrict__ dout
                 }
             }
         }
+    };
+    for (;;) {
+        int u = 0;
+        if (lane == 0) u = atomicAdd(&next_used, 1);
+        u = __shfl_sync(0xffffffffu, u, 0);
+        if (u >= n_used) break;
+        if (!in) continue;
+        const int r = used[u];
+        T* dst = dtok + ((long long)r * S + stripe) * D + c;
+        float s[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) s[j] = 0.f;
+        if (accumulate) ldv<T>(dst, s);
+        add_tokens(s, start[r], start[r + 1]);
         stv<T>(dst, s);
     }
     const int nh = n_hot;
     for (int h = 0; h < nh; ++h) {
         const int r = hot[h], n0 = start[r], n = start[r + 1] - n0;
-        const long long id = (long long)r * S + stripe;
+        T* dst = dtok + ((long long)r * S + stripe) * D + c;
         const int share = (n + NW - 1) / NW, e0 = min(n, warp * share), e1 = min(n, e0 + share);
         float s[W];
 #pragma unroll
         for (int j = 0; j < W; ++j) s[j] = 0.f;
-        if (in) {
-#pragma unroll 8
-            for (int e = e0; e < e1; ++e) {
-                float x[W];
-                ldv<T>(src + (long long)sorted[n0 + e] * D, x);
-#pragma unroll
-                for (int j = 0; j < W; ++j) s[j] += x[j];
-            }
-        }
+        if (in) add_tokens(s, n0 + e0, n0 + e1);
 #pragma unroll
         for (int j = 0; j < W; ++j) part[(warp * W + j) * 32 + lane] = s[j];
         __syncthreads();
+        if (warp < W) {                                    // warp j adds up column j of every lane's vector
+            float t = 0.f;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) t += part[(w * W + warp) * 32 + lane];
+            part[warp * 32 + lane] = t;                    // (its own slots of warp 0's sums)
+        }
+        __syncthreads();
         if (warp == 0 && in) {
-            if (accumulate) ldv<T>(dtok + id * D + c, s);
 #pragma unroll
-            for (int j = 0; j < W; ++j) {
-                float t = accumulate ? s[j] : 0.f;
+            for (int j = 0; j < W; ++j) s[j] = 0.f;
+            if (accumulate) ldv<T>(dst, s);
 #pragma unroll
-                for (int w = 0; w < NW; ++w) t += part[(w * W + j) * 32 + lane];
-                s[j] = t;
-            }
-            stv<T>(dtok + id * D + c, s);
+            for (int j = 0; j < W; ++j) s[j] += part[j * 32 + lane];
+            stv<T>(dst, s);
         }
         __syncthreads();
     }
@@ -731,12 +758,18 @@ int tok_bwd_t(const int* tokens, const void* dout, void* dtok, int BT, int D, in
     const bool scan = (long long)V * BT <= (1ll << 22) && D <= 1536;
     if (D % W == 0 && BT <= STRIPE_MAX_BT && aligned16((const T*)dout) && aligned16((const T*)dtok)) {
         const StripePlan p = stripe_plan(BT, D, V, W);
-        if ((unsigned long long)V * p.S < (1ull << 32) && p.smem <= 200 * 1024) {
+        // Stripes replace the block per vocabulary row wherever that would run (16384 tokens, 65 x 384: 21 us with the position
+        // table against 140; 64512 tokens: 136 against 478).  On larger tables they replace the atomics for 16-bit types while
+        // the lists fit (50304 x 768, 16384 tokens: 44 against 50 us; 8192 x 512, 4096 tokens: 19.5 against 21.4).  Atomics keep
+        // fp32, whose sums they do not round any more (80 against 62 us, and 21.5 against 19.2), and the longer token lists,
+        // which every block would walk three times (64512 tokens: 267 against 128 us).
+        const bool better = scan || (sizeof(T) == 2 && p.keep);
+        if (better && (unsigned long long)V * p.S < (1ull << 32) && p.smem <= STRIPE_SMEM) {
             auto k = tok_bwd_stripe_kernel<T>;
             if (p.smem > 48 * 1024)
-                CME_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+                CME_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STRIPE_SMEM));
             CME_CUDA(cme_launch_dependent(k, dim3(p.S, p.chunks), dim3(STRIPE_WARPS * 32), p.smem, st, tokens, (const T*)dout,
-                                          (T*)dtok, BT, D, V, p.S, p.R, p.magic, accumulate));
+                                          (T*)dtok, BT, D, V, p, accumulate));
             CME_LAUNCH_CHECK();
             return CME_OK;
         }

@@ -102,7 +102,7 @@ def test_optimizer_tails_and_ranges(dtype, n):
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("V,D,B,T,ids", [(7, 8, 2, 4, "uniform"), (65, 384, 16, 64, "uniform"), (50304, 264, 2, 512, "uniform"),
                                          (3000, 768, 4, 512, "one"), (3000, 136, 4, 512, "few"), (1, 16, 3, 40, "one"),
-                                         (50304, 64, 64, 1023, "few"), (300, 100, 4, 33, "few")])
+                                         (50304, 64, 32, 1023, "few"), (65, 64, 63, 1024, "few"), (300, 100, 4, 33, "few")])
 def test_token_table_gradient_by_stripes(dtype, V, D, B, T, ids):
     """Rows without a token, rows with one, rows that many tokens share (summed by the whole block), ids outside the
     table; twice the same bits; accumulation on top of what is there."""
@@ -122,7 +122,7 @@ def test_token_table_gradient_by_stripes(dtype, V, D, B, T, ids):
     want_pos = dout.double().reshape(B, T, D).sum(0)
     dtok, dpos = ops.embedding_bwd(tokens, dout, V, T)
     again, _ = ops.embedding_bwd(tokens, dout, V, T)
-    if n <= 65535 and D % 8 == 0:
+    if D % 8 == 0 and (dtype == torch.bfloat16 or V * n <= 1 << 22):
         assert torch.equal(dtok, again)
         # fp32 sums of up to n terms, rounded once
         tol = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
