@@ -137,17 +137,12 @@ def _cuda(*ts) -> None:
             raise NativeError("native ops need contiguous CUDA tensors")
 
 
-_workspaces = {}
+def workspace(nbytes: int = 64 << 20, device="cuda") -> torch.Tensor:
+    """fp32 scratch for one product launched through the Python wrappers (the partial sums of a split reduction).
 
-
-def workspace(nbytes: int = 64 << 20) -> torch.Tensor:
-    """Per-device fp32 scratch shared by split-K GEMMs launched through the Python wrappers."""
-    dev = torch.cuda.current_device()
-    w = _workspaces.get(dev)
-    if w is None or w.numel() * 4 < nbytes:
-        w = torch.empty(nbytes // 4, dtype=torch.float32, device="cuda")
-        _workspaces[dev] = w
-    return w
+    Taken anew for each call from torch's allocator, which hands freed memory out again on the same stream only: products
+    on several streams, or issued by several threads, never share it, and it goes back when the call has been issued."""
+    return torch.empty(nbytes // 4, dtype=torch.float32, device=device)
 
 
 # --------------------------------------------------------------------------------------------------
@@ -189,7 +184,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bo
     if out is None:
         shape = (batch, M, N) if (a.dim() == 3 or b.dim() == 3) else (M, N)
         out = torch.empty(shape, dtype=odt, device=a.device)
-    ws = workspace()
+    ws = workspace(device=a.device)
     a3, b3 = a.dim() == 3, b.dim() == 3
     slabs = part = None
     if dbias is not None:
