@@ -39,6 +39,8 @@ struct CmeGemm {
     float* colsum; int* colsum_slabs;                     // optional column sums of C (device scratch, host count)
     int allow_tf32;                                       // fp32 operands may be multiplied as tf32 (10-bit mantissa
                                                           // inputs, fp32 accumulation): plain products with fp32 output
+                                                          // whose operands lie along K, or along M / N with K % 4 == 0
+                                                          // and within half of the workspace; all others are exact
 };
 
 int gemm_tcgen05_supported(const CmeGemm* g);
