@@ -192,12 +192,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bo
         slabs = ctypes.c_int(0)
         part = torch.empty((M + 31) // 32 * N, dtype=torch.float32, device=a.device)
     g = CmeGemm(M, N, K, batch,
-                a.data_ptr(), a2[1], a2[0] * a2[1] if a3 else 0, a_trans,
-                b.data_ptr(), b2[1], b2[0] * b2[1] if b3 else 0, b_trans,
+                a.data_ptr(), a2[1], a2[0] * a2[1] if a3 else 0, int(a_trans),
+                b.data_ptr(), b2[1], b2[0] * b2[1] if b3 else 0, int(b_trans),
                 out.data_ptr(), N, M * N, _dt(out), _dt(a),
                 _a(bias), _a(residual), N, _a(aux_out), _a(aux_in), N,
-                ACT[act], ACT[dact], accumulate, ws.data_ptr(), ws.numel() * 4, force_bn, force_splits, aux_deriv,
-                _a(part), None if slabs is None else ctypes.pointer(slabs), allow_tf32)
+                ACT[act], ACT[dact], int(accumulate), ws.data_ptr(), ws.numel() * 4, force_bn, force_splits, int(aux_deriv),
+                _a(part), None if slabs is None else ctypes.pointer(slabs), int(allow_tf32))
     _check(lib().cme_gemm(ctypes.byref(g), _GEMM_BACKENDS[backend], _st()))
     if dbias is not None:
         gemm.last_colsum_slabs = slabs.value          # 0: the epilogue did not sum (tests look at this)
@@ -391,7 +391,7 @@ def _attn_desc(q, B, H, T, layout, causal):
     D = q.shape[-1]
     HD = D // H
     nb, nh, sb, sh, st = (B * H, 1, T * HD, 0, HD) if layout == "flat" else (B, H, T * D, HD, D)
-    a = CmeAttn(nb, nh, T, HD, sb, sh, st, sb, sh, st, bool(causal), 1.0 / (HD ** 0.5), _dt(q))
+    a = CmeAttn(nb, nh, T, HD, sb, sh, st, sb, sh, st, int(causal), 1.0 / (HD ** 0.5), _dt(q))
     if layout == "flat" and T <= 512 and q.dtype == torch.bfloat16:      # scratch of the batched-GEMM path
         nbytes = int(lib().cme_attention_gemm_ws_bytes(B * H, T))
         ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=q.device)
