@@ -337,17 +337,17 @@ struct AdamArgs {
     const long long* nodecay; int n_nodecay;      // sorted [start, end) pairs exempt from weight decay
 };
 
-// The first no-decay range with end > i (n_nodecay if there is none).
-__device__ __forceinline__ int adam_range_at(const AdamArgs& a, long long i) {
-    int lo = 0, hi = a.n_nodecay;
+// The first of `n` sorted no-decay ranges, from `lo` on, with end > i (n if there is none).
+__device__ __forceinline__ int adam_range_at(const long long* ranges, int n, int lo, long long i) {
+    int hi = n;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (a.nodecay[2 * mid + 1] > i) hi = mid; else lo = mid + 1;
+        if (ranges[2 * mid + 1] > i) hi = mid; else lo = mid + 1;
     }
     return lo;
 }
 __device__ __forceinline__ bool adam_decays(const AdamArgs& a, long long i) {
-    const int lo = adam_range_at(a, i);
+    const int lo = adam_range_at(a.nodecay, a.n_nodecay, 0, i);
     return !(lo < a.n_nodecay && a.nodecay[2 * lo] <= i);
 }
 
@@ -384,11 +384,13 @@ __global__ void __launch_bounds__(256) adam_kernel(const AdamArgs a) {
 }
 
 
-// Four elements per thread-iteration (128-bit accesses on the fp32 state, read and written once: streaming, so that they
-// do not displace the bf16 weights the next forward reads).  Requires 16-byte aligned arenas; the last n % 4 elements and
-// groups that straddle the end of a no-decay range are decided element by element.  124 M elements with bf16
-// gradients: 3.49 GB in 562-569 us, 0.92 of a 6.65 TB/s copy, norm pass included 659 -> 628 us.
-template <typename TG>
+constexpr int ADAM_LIST = 512;             // ranges that a block keeps in shared memory (8 KB); longer lists are read in place
+
+// Four elements per thread-iteration (128-bit accesses on the fp32 state).  Requires 16-byte aligned arenas; the last n % 4
+// elements and groups in which a no-decay range begins or ends are decided element by element.  RANGES: there is weight
+// decay and a list of ranges.  124 M elements with bf16 gradients, 3.49 GB: 561 us without ranges, 556 us with 150, 0.96 of a
+// 6.54 TB/s copy (574 and 575 us with accesses marked as streaming, which pay at 10 M only, 46 for 49 us).
+template <typename TG, bool RANGES>
 __global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
     const int t = *a.step;
     const float lr = *a.lr;
@@ -400,21 +402,25 @@ __global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
         if (norm > a.clip_norm) gs *= a.clip_norm / norm;
     }
     const long long nv = a.n >> 2;
-    // The no-decay range at or after the element at hand, kept in registers: found by bisection for a thread's first group,
-    // while that group's loads are under way, then walked, since indices only grow.  A bisection per group is seven dependent
-    // loads for each four elements (124 M elements 586 us, 563 us walked); a walk from the first range takes a thread of a
-    // small arena through all of them (150 ranges: 1 M elements 28 us, 8.3 us so).
-    const long long none = 0x7fffffffffffffffll;
-    const bool wd = a.weight_decay > 0.f;
-    const float keep = 1.f - lr * a.weight_decay;
-    int seg = -1;
-    long long seg_start = none, seg_end = none;
+    // The no-decay range at or after the element at hand stays in registers; where it is over, the next one is searched for
+    // in a copy of the list in shared memory.  From global memory that is a chain of dependent loads: all of the list where
+    // it was walked (150 ranges: 1 M elements 28 us, 16 M 113 us), seven loads a group where it was bisected (8.4 and 82 us).
+    __shared__ long long list[RANGES ? 2 * ADAM_LIST : 1];
+    const bool copied = a.n_nodecay <= ADAM_LIST;
+    if (RANGES && copied) {
+        for (int k = threadIdx.x; k < 2 * a.n_nodecay; k += blockDim.x) list[k] = a.nodecay[k];
+        __syncthreads();
+    }
+    const long long* ranges = copied ? list : a.nodecay;
+    const float keep = a.weight_decay > 0.f ? 1.f - lr * a.weight_decay : 1.f;
+    int seg = 0;
+    long long seg_start = 0, seg_end = 0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
         const long long e = i << 2;
         float g[4];
-        float4 m4 = __ldcs(reinterpret_cast<const float4*>(a.m + e));
-        float4 v4 = __ldcs(reinterpret_cast<const float4*>(a.v + e));
-        float4 p4 = __ldcs(reinterpret_cast<const float4*>(a.master + e));
+        float4 m4 = *reinterpret_cast<const float4*>(a.m + e);
+        float4 v4 = *reinterpret_cast<const float4*>(a.v + e);
+        float4 p4 = *reinterpret_cast<const float4*>(a.master + e);
         if constexpr (sizeof(TG) == 2) {
             const uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(a.grads) + e);
             float2 lo = bf2_to_f2(u.x), hi = bf2_to_f2(u.y);
@@ -423,22 +429,20 @@ __global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
             const float4 u = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.grads) + e);
             g[0] = u.x; g[1] = u.y; g[2] = u.z; g[3] = u.w;
         }
-        float decay[4] = {1.f, 1.f, 1.f, 1.f};
-        if (wd) {
-            auto range = [&] {
-                seg_start = seg < a.n_nodecay ? a.nodecay[2 * seg] : none;
-                seg_end = seg < a.n_nodecay ? a.nodecay[2 * seg + 1] : none;
+        float decay[4] = {keep, keep, keep, keep};
+        if (RANGES) {
+            auto advance = [&](long long to) {
+                if (seg_end > to) return;
+                seg = adam_range_at(ranges, a.n_nodecay, seg, to);
+                seg_start = seg < a.n_nodecay ? ranges[2 * seg] : 0x7fffffffffffffffll;
+                seg_end = seg < a.n_nodecay ? ranges[2 * seg + 1] : 0x7fffffffffffffffll;
             };
-            if (seg < 0) { seg = adam_range_at(a, e); range(); }       // (the loads above are under way)
-            while (seg_end <= e) { ++seg; range(); }
-            if (seg_start >= e + 4) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) decay[j] = keep;
-            } else if (seg_start > e || seg_end < e + 4) {             // ranges begin or end inside the group
+            advance(e);
+            if (seg_start < e + 4) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    while (seg_end <= e + j) { ++seg; range(); }
-                    decay[j] = seg_start <= e + j ? 1.f : keep;
+                    advance(e + j);                // (a range may end inside the group and another begin)
+                    if (seg_start <= e + j) decay[j] = 1.f;
                 }
             }
         }
@@ -449,9 +453,9 @@ __global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
             adam_moments(a, gj, mp[j], vp[j]);
             pp[j] = pp[j] * decay[j] - lr * (mp[j] * ibc1) / (sqrtf(vp[j] * ibc2) + a.eps);
         }
-        __stcs(reinterpret_cast<float4*>(a.m + e), m4);
-        __stcs(reinterpret_cast<float4*>(a.v + e), v4);
-        __stcs(reinterpret_cast<float4*>(a.master + e), p4);
+        *reinterpret_cast<float4*>(a.m + e) = m4;
+        *reinterpret_cast<float4*>(a.v + e) = v4;
+        *reinterpret_cast<float4*>(a.master + e) = p4;
         if (a.compute)
             *reinterpret_cast<uint2*>(a.compute + e) = make_uint2(f2_to_bf2(p4.x, p4.y), f2_to_bf2(p4.z, p4.w));
     }
@@ -460,7 +464,7 @@ __global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
         const float gj = to_f32<TG>(reinterpret_cast<const TG*>(a.grads)[e]) * gs;
         float mi = a.m[e], vi = a.v[e];
         adam_moments(a, gj, mi, vi);
-        const float p = a.master[e] * (wd && adam_decays(a, e) ? keep : 1.f) - lr * (mi * ibc1) / (sqrtf(vi * ibc2) + a.eps);
+        const float p = a.master[e] * (RANGES && !adam_decays(a, e) ? 1.f : keep) - lr * (mi * ibc1) / (sqrtf(vi * ibc2) + a.eps);
         a.m[e] = mi;
         a.v[e] = vi;
         a.master[e] = p;
@@ -583,8 +587,10 @@ CME_API int cme_adam(int grad_dtype, float* master, void* compute_bf16, const vo
     if (vec) {
         blocks = (n / 4 + 255) / 256;
         if (blocks > 148 * 16) blocks = 148 * 16;
-        if (grad_dtype == CME_BF16) adam_vec4_kernel<__nv_bfloat16><<<(int)blocks, 256, 0, st>>>(a);
-        else adam_vec4_kernel<float><<<(int)blocks, 256, 0, st>>>(a);
+        const bool ranges = weight_decay > 0.f && n_nodecay > 0;
+        auto kernel = grad_dtype == CME_BF16 ? (ranges ? adam_vec4_kernel<__nv_bfloat16, true> : adam_vec4_kernel<__nv_bfloat16, false>)
+                                             : (ranges ? adam_vec4_kernel<float, true> : adam_vec4_kernel<float, false>);
+        kernel<<<(int)blocks, 256, 0, st>>>(a);
     } else if (grad_dtype == CME_BF16) adam_kernel<__nv_bfloat16><<<(int)blocks, 256, 0, st>>>(a);
     else adam_kernel<float><<<(int)blocks, 256, 0, st>>>(a);
     CME_LAUNCH_CHECK();

@@ -6,7 +6,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,count,length", [(40_000, 150, 64), (40_000, 1, 1), (4096, 600, 3), (6_000_002, 150, 3072), (6_000_002, 3, 5)])
+@pytest.mark.parametrize("n,count,length", [(40_000, 150, 64), (40_000, 1, 1), (4096, 512, 3), (4096, 513, 3), (4096, 600, 3), (6_000_002, 150, 3072), (6_000_002, 3, 5)])
 def test_many_ranges(n, count, length):
     from cme213_final_project_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(3)
