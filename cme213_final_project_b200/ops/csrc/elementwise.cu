@@ -572,42 +572,56 @@ int bias_act_res_t(const void* x, const void* bias, const void* res, void* pre, 
     return CME_OK;
 }
 
-// dbias[c] (+)= sum over the `slabs` rows of partial[slabs][cols], added in a fixed order: a block covers 32 columns
-// with 32 row groups; each thread sums every 32nd row (four independent chains), then the 32 groups are added in
-// shared memory.  The rows come from a GEMM epilogue that sums its stored output per 32-row slab, or from
-// dact_colsum_kernel's row splits.  One block per 32
-// columns leaves the chip mostly idle, so the time is that of a thread's chain of loads: 32 groups instead of 8 make it
-// a quarter as long: 512 rows of 3072 columns 15.5 -> 6.5 us.
-constexpr int SLAB_GROUPS = 32;
-template <typename T>
-__global__ void __launch_bounds__(SLAB_GROUPS * 32)
+// dbias[c] (+)= sum over the `slabs` rows of partial[slabs][cols], added in a fixed order: NG row groups per column, each
+// of whose threads sums every NG-th row (four independent chains), then the groups' sums are added in shared memory.  The
+// rows come from a GEMM epilogue that sums its stored output per 32-row slab, or from dact_colsum_kernel's row splits.
+template <typename T, int NG>
+__global__ void __launch_bounds__(NG == 1 ? 256 : NG * 32)
 colsum_slabs_finalize_kernel(const float* __restrict__ partial, int slabs, int cols, T* dbias, int accumulate) {
-    constexpr int NG = SLAB_GROUPS;
+    constexpr int NC = NG == 1 ? 256 : 32;         // columns per block
+    constexpr int NL = 4;                          // a thread's loads in flight
     __shared__ float sm[NG][33];
     pdl_wait();
-    const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
-    const int c = blockIdx.x * 32 + cx;
+    const int cx = threadIdx.x % NC, ry = threadIdx.x / NC;
+    const int c = blockIdx.x * NC + cx;
     float s = 0.f;
     if (c < cols) {
-        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-        int r = ry;
-        for (; r + 3 * NG < slabs; r += 4 * NG) {
-            s0 += partial[(long long)r * cols + c];
-            s1 += partial[(long long)(r + NG) * cols + c];
-            s2 += partial[(long long)(r + 2 * NG) * cols + c];
-            s3 += partial[(long long)(r + 3 * NG) * cols + c];
+        float t[NL] = {0.f, 0.f, 0.f, 0.f};
+        for (int r = ry; r < slabs; r += NL * NG) {
+            float v[NL];
+#pragma unroll
+            for (int k = 0; k < NL; ++k) v[k] = r + k * NG < slabs ? partial[(long long)(r + k * NG) * cols + c] : 0.f;
+#pragma unroll
+            for (int k = 0; k < NL; ++k) t[k] += v[k];
         }
-        for (; r < slabs; r += NG) s0 += partial[(long long)r * cols + c];
-        s = (s0 + s1) + (s2 + s3);
+        s = (t[0] + t[1]) + (t[2] + t[3]);
     }
-    sm[ry][cx] = s;
-    __syncthreads();
+    if (NG > 1) {
+        sm[ry][cx] = s;
+        __syncthreads();
+    }
     if (ry == 0 && c < cols) {
         float t = 0.f;
 #pragma unroll
-        for (int g = 0; g < NG; ++g) t += sm[g][cx];
+        for (int g = 0; g < NG; ++g) t += NG > 1 ? sm[g][cx] : s;
         dbias[c] = from_f32<T>(accumulate ? to_f32<T>(dbias[c]) + t : t);
     }
+}
+// The time is that of a thread's chain of loads while the blocks fit the chip: 32 groups where 8 need more than three rounds
+// of loads (512 columns, us with 8 / 32 groups: 16 rows 1.3 / 1.5, 64 rows 1.5 / 1.6, 128 rows 1.7 / 1.7, 512 rows 3.6 / 2.6,
+// 2048 rows 11 / 6.1).  Beyond 32768 columns the blocks come in several waves and fewer groups pay for longer (50304
+// columns, 1 / 8 / 32 groups: 16 rows 1.9 / 2.8 / 6.8, 512 rows 78 / 17 / 19, 2048 rows 339 / 74 / 68).
+template <typename T>
+int colsum_finish(const float* partial, int slabs, int cols, T* dbias, int accumulate, cudaStream_t st) {
+    auto run = [&](auto kernel, int columns, int threads) -> int {
+        CME_CUDA(cme_launch_dependent(kernel, dim3(cme_cdiv(cols, columns)), dim3(threads), 0, st, partial, slabs, cols, dbias, accumulate));
+        CME_LAUNCH_CHECK();
+        return CME_OK;
+    };
+    const bool wide = cols > 32768;
+    if (wide && slabs <= 16) return run(colsum_slabs_finalize_kernel<T, 1>, 256, 256);
+    if (slabs <= (wide ? 512 : 96)) return run(colsum_slabs_finalize_kernel<T, 8>, 32, 256);
+    return run(colsum_slabs_finalize_kernel<T, 32>, 32, 1024);
 }
 
 template <typename T>
@@ -626,12 +640,7 @@ int dact_colsum_t(const void* dout, const void* pre, void* g, void* dbias, float
                                                             act);
     }
     CME_LAUNCH_CHECK();
-    if (dbias) {
-        CME_CUDA(cme_launch_dependent(colsum_slabs_finalize_kernel<T>, dim3(cme_cdiv(cols, 32)), dim3(SLAB_GROUPS * 32), 0, st,
-                                      (const float*)scratch, splits, cols, (T*)dbias, accumulate));
-        CME_LAUNCH_CHECK();
-    }
-    return CME_OK;
+    return dbias ? colsum_finish<T>(scratch, splits, cols, (T*)dbias, accumulate, st) : CME_OK;
 }
 
 }  // namespace
@@ -672,14 +681,8 @@ CME_API int cme_colsum_slabs_finalize(int dtype, const float* partial, int slabs
                                       void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     CME_REQUIRE(slabs > 0 && cols > 0, CME_ERR_SHAPE, "colsum finalize: empty input");
-    if (dtype == CME_BF16)
-        CME_CUDA(cme_launch_dependent(colsum_slabs_finalize_kernel<__nv_bfloat16>, dim3(cme_cdiv(cols, 32)), dim3(SLAB_GROUPS * 32), 0,
-                                      st, partial, slabs, cols, (__nv_bfloat16*)dbias, accumulate));
-    else
-        CME_CUDA(cme_launch_dependent(colsum_slabs_finalize_kernel<float>, dim3(cme_cdiv(cols, 32)), dim3(SLAB_GROUPS * 32), 0, st,
-                                      partial, slabs, cols, (float*)dbias, accumulate));
-    CME_LAUNCH_CHECK();
-    return CME_OK;
+    return DISPATCH_T(dtype, colsum_finish<__nv_bfloat16>(partial, slabs, cols, (__nv_bfloat16*)dbias, accumulate, st),
+                      colsum_finish<float>(partial, slabs, cols, (float*)dbias, accumulate, st));
 }
 
 CME_API int cme_scale(int dtype, void* x, long long n, float s, void* stream) {
