@@ -228,22 +228,23 @@ __global__ void pos_bwd_kernel(const T* __restrict__ dout, T* __restrict__ dpos,
     for (int b = 0; b < B; ++b) s += to_f32<T>(dout[(long long)b * T_ * D + i]);
     dpos[i] = from_f32<T>(s);
 }
-// Same for rows of whole 16-byte vectors: a block takes 32 vectors of the [T, D] table and splits the batch over its 8
-// warps, whose sums are added in warp order (the scalar form walks the whole batch in every thread, 2 bytes a load):
-// 16 x 1024 x 768 bf16 9.5 -> about 6 us, 64 x 256 x 384 6.3 -> 6.0 us.
-template <typename T>
+// Same for rows of whole 16-byte vectors.  SPLIT: a block takes 32 vectors of the [T, D] table and splits the batch over its 8
+// warps, whose sums are added in warp order (the scalar form walks the whole batch in every thread, 2 bytes a load): 64 x
+// 256 x 384 bf16 4.2 -> 2.6 us, 63 x 1024 x 64 4.4 -> 2.4 us.  Else a thread has a vector and walks the batch.
+template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(256)
 pos_bwd_vec_kernel(const T* __restrict__ dout, T* __restrict__ dpos, int B, long long nvec, int accumulate) {
     constexpr int W = Vw<T>::N;
-    __shared__ float part[8][W][32];
+    __shared__ float part[SPLIT ? 8 : 1][W][32];
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long v = (long long)blockIdx.x * 32 + lane;
-    const int per = (B + 7) / 8, b0 = warp * per, b1 = min(B, b0 + per);
+    const long long v = SPLIT ? (long long)blockIdx.x * 32 + lane : (long long)blockIdx.x * 256 + threadIdx.x;
+    const int per = SPLIT ? (B + 7) / 8 : B, b0 = SPLIT ? warp * per : 0, b1 = min(B, b0 + per);
     float s[W];
 #pragma unroll
     for (int j = 0; j < W; ++j) s[j] = 0.f;
     if (v < nvec) {
+        if (!SPLIT && accumulate) ldv<T>(dpos + v * W, s);
 #pragma unroll 4
         for (int b = b0; b < b1; ++b) {
             float x[W];
@@ -252,20 +253,20 @@ pos_bwd_vec_kernel(const T* __restrict__ dout, T* __restrict__ dpos, int B, long
             for (int j = 0; j < W; ++j) s[j] += x[j];
         }
     }
+    if (SPLIT) {
 #pragma unroll
-    for (int j = 0; j < W; ++j) part[warp][j][lane] = s[j];
-    __syncthreads();
-    if (warp == 0 && v < nvec) {
+        for (int j = 0; j < W; ++j) part[warp][j][lane] = s[j];
+        __syncthreads();
+        if (warp > 0 || v >= nvec) return;
+#pragma unroll
+        for (int j = 0; j < W; ++j) s[j] = 0.f;
         if (accumulate) ldv<T>(dpos + v * W, s);
 #pragma unroll
-        for (int j = 0; j < W; ++j) {
-            float t = accumulate ? s[j] : 0.f;
+        for (int j = 0; j < W; ++j)
 #pragma unroll
-            for (int w = 0; w < 8; ++w) t += part[w][j][lane];
-            s[j] = t;
-        }
-        stv<T>(dpos + v * W, s);
+            for (int w = 0; w < 8; ++w) s[j] += part[w][j][lane];
     }
+    if (v < nvec) stv<T>(dpos + v * W, s);
 }
 // Small vocabularies: one block (8 warps) per vocabulary row.  Each warp scans its own contiguous eighth of the
 // token list with ballots and sums the matching rows of dout in token order; the eight partial rows are then added
@@ -798,11 +799,15 @@ template <typename T>
 int pos_bwd_t(const void* dout, void* dpos, int BT, int T_, int D, int accumulate, cudaStream_t st) {
     constexpr int W = Vw<T>::N;
     const long long n = (long long)T_ * D;
-    if (D % W == 0 && aligned16((const T*)dout) && aligned16((const T*)dpos))
-        CME_CUDA(cme_launch_dependent(pos_bwd_vec_kernel<T>, dim3(cme_cdiv(n / W, 32)), dim3(256), 0, st, (const T*)dout, (T*)dpos,
-                                      BT / T_, n / W, accumulate));
-    else
+    if (D % W == 0 && aligned16((const T*)dout) && aligned16((const T*)dpos)) {
+        // Whole blocks of vectors for two blocks an SM leave nothing to split while the batch is a thread's few loads
+        // (1024 x 768 fp32, us split / whole: batch 1 4.8 / 1.6, 8 5.6 / 2.9, 16 7.0 / 4.2).
+        const bool split = BT / T_ > 16 || n / W < 256 * 296;
+        CME_CUDA(cme_launch_dependent(split ? pos_bwd_vec_kernel<T, true> : pos_bwd_vec_kernel<T, false>, dim3(cme_cdiv(n / W, split ? 32 : 256)),
+                                      dim3(256), 0, st, (const T*)dout, (T*)dpos, BT / T_, n / W, accumulate));
+    } else {
         pos_bwd_kernel<T><<<cme_cdiv(n, 256), 256, 0, st>>>((const T*)dout, (T*)dpos, BT / T_, T_, D, accumulate);
+    }
     CME_LAUNCH_CHECK();
     return CME_OK;
 }

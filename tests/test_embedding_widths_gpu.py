@@ -20,8 +20,8 @@ def test_gather_of_every_width(dtype, D):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("B", [1, 2, 7, 8, 9, 33])
-@pytest.mark.parametrize("T,D", [(1, 8), (33, 72), (64, 256)])
+@pytest.mark.parametrize("B", [1, 2, 8, 16, 17, 33])
+@pytest.mark.parametrize("T,D", [(1, 8), (33, 72), (64, 256), (1024, 768), (301, 1024), (592, 1024)])
 def test_position_gradient_of_few_and_many_rows(dtype, B, T, D):
     from cme213_final_project_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(3)
