@@ -44,6 +44,9 @@ template <> __device__ __forceinline__ void unpack_raw<__nv_bfloat16>(const uint
 // exactly the 16-byte words it will read itself, so waiting for its own copies is all the synchronisation there is.
 // Registers alone kept one row in flight per warp, and the memory idle while its statistics were reduced.
 constexpr int LN_STAGES = 3;
+// Row numbers are unsigned: the row fetched ahead of the last ones may lie beyond the largest int.
+constexpr unsigned row_ahead(unsigned row, unsigned step, int n) { return row + n * step; }
+static_assert(row_ahead(0x7fffffffu, 2048 * LN_WARPS, LN_STAGES) > 0x7fffffffu, "grids of up to 2048 blocks do not wrap around");
 __device__ __forceinline__ void ring_copy(uint4* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
@@ -62,11 +65,12 @@ ln_fwd_vec_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restric
     constexpr int W = VecOf<T>::N, S = LN_STAGES;
     extern __shared__ uint4 ring[];                     // [LN_WARPS][S][1 or 2][NV][32]
     pdl_wait();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = D / W, step = gridDim.x * LN_WARPS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = D / W;
+    const unsigned step = gridDim.x * LN_WARPS, n_rows = rows;
     const int stage = (b ? 2 : 1) * NV * 32;
     uint4* mine = ring + warp * S * stage + lane;
-    auto fetch = [&](int row, int s) {
-        if (row < rows) {
+    auto fetch = [&](unsigned row, int s) {
+        if (row < n_rows) {
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
                 const int v = lane + 32 * i;
@@ -78,11 +82,11 @@ ln_fwd_vec_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restric
         }
         ring_commit();
     };
-    int row = blockIdx.x * LN_WARPS + warp;
+    unsigned row = blockIdx.x * LN_WARPS + warp;
 #pragma unroll
-    for (int s = 0; s < S - 1; ++s) fetch(row + s * step, s);
-    for (int s = 0; row < rows; row += step, s = s + 1 == S ? 0 : s + 1) {
-        fetch(row + (S - 1) * step, s == 0 ? S - 1 : s - 1);
+    for (int s = 0; s < S - 1; ++s) fetch(row_ahead(row, step, s), s);
+    for (int s = 0; row < n_rows; row += step, s = s + 1 == S ? 0 : s + 1) {
+        fetch(row_ahead(row, step, S - 1), s == 0 ? S - 1 : s - 1);
         ring_wait<S - 1>();
         const uint4* in = mine + s * stage;
         const long long off = (long long)row * D;
@@ -187,11 +191,12 @@ ln_bwd_vec_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __
     constexpr int SLOTS = NV * W * 32;
     extern __shared__ uint4 ring[];   // [LN_WARPS][S][2 or 3][NV][32]; at the end [LN_WARPS][2][SLOTS] floats
     pdl_wait();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = D / W, step = gridDim.x * LN_WARPS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = D / W;
+    const unsigned step = gridDim.x * LN_WARPS, n_rows = rows;
     const int stage = 3 * NV * 32;
     uint4* mine = ring + warp * S * stage + lane;
-    auto fetch = [&](int row, int s) {
-        if (row < rows) {
+    auto fetch = [&](unsigned row, int s) {
+        if (row < n_rows) {
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
                 const int v = lane + 32 * i;
@@ -215,14 +220,14 @@ ln_bwd_vec_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __
 #pragma unroll
         for (int j = 0; j < W; ++j) adg[i][j] = adb[i][j] = 0.f;
     }
-    int row = blockIdx.x * LN_WARPS + warp;
+    unsigned row = blockIdx.x * LN_WARPS + warp;
 #pragma unroll
-    for (int s = 0; s < S - 1; ++s) fetch(row + s * step, s);
-    float mu_next = row < rows ? mean[row] : 0.f, rs_next = row < rows ? rstd[row] : 0.f;
-    for (int s = 0; row < rows; row += step, s = s + 1 == S ? 0 : s + 1) {
-        fetch(row + (S - 1) * step, s == 0 ? S - 1 : s - 1);
+    for (int s = 0; s < S - 1; ++s) fetch(row_ahead(row, step, s), s);
+    float mu_next = row < n_rows ? mean[row] : 0.f, rs_next = row < n_rows ? rstd[row] : 0.f;
+    for (int s = 0; row < n_rows; row += step, s = s + 1 == S ? 0 : s + 1) {
+        fetch(row_ahead(row, step, S - 1), s == 0 ? S - 1 : s - 1);
         const float mu = mu_next, rs = rs_next;
-        if (row + step < rows) { mu_next = mean[row + step]; rs_next = rstd[row + step]; }
+        if (row + step < n_rows) { mu_next = mean[row + step]; rs_next = rstd[row + step]; }
         ring_wait<S - 1>();
         const uint4* in = mine + s * stage;
         const long long off = (long long)row * D;
