@@ -55,8 +55,8 @@ __device__ __forceinline__ void ring_commit() { asm volatile("cp.async.commit_gr
 template <int N> __device__ __forceinline__ void ring_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // y = LN(a [+ b]) * gamma + beta; optionally writes r = a + b, mean and rstd.  Rows of at most 32 * NV 16-byte vectors, one
-// warp per row, the grid what is resident at once.  Bound by memory: 16384 x 768 bf16 with the
-// residual add and its sum stored (101 MB) took 21.0 us with one row per warp and block, 18 us now.
+// warp per row, the grid what is resident at once.  Bound by memory: 16384 x 768 bf16 from memory with the residual add and
+// its sum stored (101 MB) 18.7 us; with one row per warp and four vectors per lane whatever the row's length, 22.0 us.
 template <typename T, int NV>
 __global__ void __launch_bounds__(LN_WARPS * 32, NV <= 3 ? 3 : 2)
 ln_fwd_vec_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ r_out, const T* __restrict__ gamma,
@@ -134,6 +134,64 @@ ln_fwd_vec_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restric
             if (mean_out) mean_out[row] = mean;
             if (rstd_out) rstd_out[row] = rstd;
         }
+    }
+}
+
+// Same bits with one row per warp, from global memory to registers.
+template <typename T, int NV>
+__global__ void __launch_bounds__(LN_WARPS * 32)
+ln_fwd_row_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ r_out, const T* __restrict__ gamma,
+                  const T* __restrict__ beta, T* __restrict__ y, float* __restrict__ mean_out,
+                  float* __restrict__ rstd_out, int rows, int D, float eps) {
+    constexpr int W = VecOf<T>::N;
+    pdl_wait();
+    const int lane = threadIdx.x & 31, nvec = D / W;
+    const int row = blockIdx.x * LN_WARPS + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const long long off = (long long)row * D;
+    float x[NV][W];
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int v = lane + 32 * i;
+        if (v < nvec) {
+            load_vec<T>(a + off + v * W, x[i]);
+            if (b) {
+                float t[W];
+                load_vec<T>(b + off + v * W, t);
+#pragma unroll
+                for (int j = 0; j < W; ++j) x[i][j] += t[j];
+                if (r_out) store_vec<T>(r_out + off + v * W, x[i]);
+            }
+#pragma unroll
+            for (int j = 0; j < W; ++j) s += x[i][j];
+        }
+    }
+    const float mean = warp_sum(s) / D;
+    float q = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        if (lane + 32 * i < nvec) {
+#pragma unroll
+            for (int j = 0; j < W; ++j) { const float d = x[i][j] - mean; q += d * d; }
+        }
+    }
+    const float rstd = rsqrtf(warp_sum(q) / D + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int v = lane + 32 * i;
+        if (v < nvec) {
+            float g[W], bt[W], o[W];
+            load_vec<T>(gamma + v * W, g);
+            load_vec<T>(beta + v * W, bt);
+#pragma unroll
+            for (int j = 0; j < W; ++j) o[j] = (x[i][j] - mean) * rstd * g[j] + bt[j];
+            store_vec<T>(y + off + v * W, o);
+        }
+    }
+    if (lane == 0) {
+        if (mean_out) mean_out[row] = mean;
+        if (rstd_out) rstd_out[row] = rstd;
     }
 }
 
@@ -406,6 +464,17 @@ inline int even_grid(int rows, int resident) {
 template <typename T, int NV>
 int ln_fwd_vec_launch(const T* a, const T* b, T* r, const T* g, const T* be, T* y, float* mean, float* rstd, int rows, int D,
                       float eps, cudaStream_t st) {
+    // The ring pays while the grid is a round or two (2048 x 768 bf16, residual, us row by row / ring: 4.2 / 4.0, 2048 x 1024 7.0 /
+    // 4.6) and where the rows come from memory and not from L2 (65536 x 768 43 / 41, 65536 x 1024 64 / 56).  Between the two
+    // more warps are worth more: 8192 x 768 from L2 5.8 / 6.5, 16384 x 512 6.7 / 8.3, 16384 x 1024 12.1 / 14.6, 8192 x 384 fp32
+    // 4.0 / 5.2.  fp32 rows beyond L2 are written faster row by row as well (65536 x 384, residual, 64 / 73).
+    const double in_bytes = (double)rows * D * sizeof(T) * (b ? 2 : 1);
+    if (rows >= 8192 && (in_bytes <= 36e6 || (sizeof(T) == 4 && in_bytes >= 90e6))) {
+        CME_CUDA(cme_launch_dependent(ln_fwd_row_kernel<T, NV>, dim3(cme_cdiv(rows, LN_WARPS)), dim3(LN_WARPS * 32), 0, st, a, b, r, g, be,
+                                      y, mean, rstd, rows, D, eps));
+        CME_LAUNCH_CHECK();
+        return CME_OK;
+    }
     const size_t smem = (size_t)LN_WARPS * LN_STAGES * (b ? 2 : 1) * NV * 512;
     auto k = ln_fwd_vec_kernel<T, NV>;
     static int resident[2][CME_MAX_DEVICES];       // [residual][device]
