@@ -400,45 +400,60 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __rest
 }
 
 // dgamma[c] (+)= sum_b partial[b][0][c];  dbeta[c] (+)= sum_b partial[b][1][c]
-// Block (16 columns x 64 block-groups): each thread sums every 64th partial, then a fixed-order shared-memory reduction
-// over the groups (deterministic).  The time is that of a thread's chain of loads, so it is kept to a handful: with 16
-// groups 296 partials of 2 x 768 columns took 3.5 us, now 2.9 us.
-constexpr int LN_FIN_GROUPS = 64;
-template <typename T>
-__global__ void __launch_bounds__(16 * LN_FIN_GROUPS)
+// Block (16 columns x NG block-groups): each thread sums every NG-th partial, then a fixed-order shared-memory reduction
+// over the groups (deterministic).  The time is that of a thread's chain of loads, so it is kept to a handful.
+template <typename T, int NG>
+__global__ void __launch_bounds__(16 * NG)
 ln_bwd_finalize_kernel(const float* __restrict__ partial, int nblocks, int D, T* dgamma, T* dbeta, int accumulate) {
-    constexpr int NG = LN_FIN_GROUPS;
+    constexpr int NL = NG == 64 ? 10 : 4;                  // a thread's loads in flight: 640 partials, more than there are
     __shared__ float sm[NG][17];
     pdl_wait();
     const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;
     const int c = blockIdx.x * 16 + cx;
     float s = 0.f;
     if (c < 2 * D) {
-        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;      // independent chains: the loads of four blocks overlap
-        int b = ry;
-        for (; b + 3 * NG < nblocks; b += 4 * NG) {
-            s0 += partial[(long long)b * 2 * D + c];
-            s1 += partial[(long long)(b + NG) * 2 * D + c];
-            s2 += partial[(long long)(b + 2 * NG) * 2 * D + c];
-            s3 += partial[(long long)(b + 3 * NG) * 2 * D + c];
+        float t[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int b = ry; b < nblocks; b += NL * NG) {
+            float v[NL];
+#pragma unroll
+            for (int k = 0; k < NL; ++k) v[k] = b + k * NG < nblocks ? partial[(long long)(b + k * NG) * 2 * D + c] : 0.f;
+#pragma unroll
+            for (int k = 0; k < NL; ++k) t[k % 4] += v[k];
         }
-        for (; b < nblocks; b += NG) s0 += partial[(long long)b * 2 * D + c];
-        s = (s0 + s1) + (s2 + s3);
+        s = (t[0] + t[1]) + (t[2] + t[3]);
     }
     sm[ry][cx] = s;
     __syncthreads();
-    if (ry < 4 && c < 2 * D) {                             // 64 groups -> 4, then 4 -> 1
-        float t = 0.f;
+    if (NG == 64) {
+        if (ry < 4 && c < 2 * D) {                         // 64 groups -> 4
+            float t = 0.f;
 #pragma unroll
-        for (int r = 0; r < NG / 4; ++r) t += sm[ry * (NG / 4) + r][cx];
-        sm[ry * (NG / 4)][cx] = t;
+            for (int r = 0; r < NG / 4; ++r) t += sm[ry * (NG / 4) + r][cx];
+            sm[ry * (NG / 4)][cx] = t;
+        }
+        __syncthreads();
     }
-    __syncthreads();
     if (ry == 0 && c < 2 * D) {
-        const float t = (sm[0][cx] + sm[NG / 4][cx]) + (sm[NG / 2][cx] + sm[3 * NG / 4][cx]);
+        float t = 0.f;
+        if (NG == 64) {
+            t = (sm[0][cx] + sm[NG / 4][cx]) + (sm[NG / 2][cx] + sm[3 * NG / 4][cx]);
+        } else {
+#pragma unroll
+            for (int r = 0; r < NG; ++r) t += sm[r][cx];
+        }
         T* dst = (c < D) ? dgamma + c : dbeta + (c - D);
         *dst = from_f32<T>(accumulate ? to_f32<T>(*dst) + t : t);
     }
+}
+template <typename T>
+int ln_bwd_finalize(const float* partial, int nblocks, int D, T* dgamma, T* dbeta, int accumulate, cudaStream_t st) {
+    // Blocks of 1024 threads cost more than they save while 16 groups read everything in two rounds (whole backward, 768
+    // bf16 columns, us with 16 / 64 groups: 32 partials 5.6 / 5.8, 128 5.9 / 6.2; 384 columns, 512 partials 7.96 / 7.75).
+    const bool many = nblocks > 128;
+    CME_CUDA(cme_launch_dependent(many ? ln_bwd_finalize_kernel<T, 64> : ln_bwd_finalize_kernel<T, 16>, dim3(cme_cdiv(2 * D, 16)),
+                                  dim3(many ? 1024 : 256), 0, st, partial, nblocks, D, dgamma, dbeta, accumulate));
+    CME_LAUNCH_CHECK();
+    return CME_OK;
 }
 
 // Every operand (null ones aside) starts on a 16-byte boundary.
@@ -562,10 +577,7 @@ int ln_bwd_t(const void* dy, const void* x, const void* g, const float* mean, co
         CME_CUDA(cudaStreamWaitEvent(fin_st, fin_ev, 0));
         st = fin_st;
     }
-    CME_CUDA(cme_launch_dependent(ln_bwd_finalize_kernel<T>, dim3(cme_cdiv(2 * D, 16)), dim3(16 * LN_FIN_GROUPS), 0, st,
-                                  (const float*)scratch, nblocks, D, (T*)dgamma, (T*)dbeta, accumulate));
-    CME_LAUNCH_CHECK();
-    return CME_OK;
+    return ln_bwd_finalize<T>(scratch, nblocks, D, (T*)dgamma, (T*)dbeta, accumulate, st);
 }
 
 }  // namespace
