@@ -192,10 +192,12 @@ static void plan_tiles(int M, int N, int K, int batch, bool plain_epi, long long
         // 128-byte k-block takes about 550 clocks whatever the tile's width (2048 x 512 x 2048 bf16, 32 k-blocks: 13.1 us
         // at 64 and at 128 columns, 13.9 us at 256, base 3.3-4 us): the ring's round trip to L2, not the tensor pipe, sets
         // it, so narrow tiles buy no time per k-block, and splitting K over idle SMs does.  With every SM loading, 256
-        // columns on one CTA reach the 64 bytes per clock that an SM takes in (185).
-        // tf32 operands stored along M or N arrive as 32-column groups, two to four times as many copies per k-block.
+        // columns on one CTA come near the 64 bytes per clock that an SM takes in (192 by that rate, 168 fits the sweeps).
+        // tf32 operands stored along M or N arrive as 32-column groups, two to four times as many copies per k-block.  With
+        // both along K the pair tile has to win where it can fill the SMs: over 130 products it is then 0.5 % off the best
+        // forced plan on average, 2.6 % with the single CTA's 150 (8192 x 768 x 2304 60.9 us as planned then, 52.0 on pairs).
         const double b16[4] = {136.0, 168.0, 138.0, 140.0};
-        const double t32[4] = {150.0 + 35.0 * mn_operands, 150.0 + 65.0 * mn_operands, 150.0 + 30.0 * mn_operands,
+        const double t32[4] = {mn_operands ? 150.0 + 35.0 * mn_operands : 140.0, 150.0 + 65.0 * mn_operands, 150.0 + 30.0 * mn_operands,
                                145.0 + 15.0 * mn_operands};
         const double* cost = bk == 32 ? t32 : b16;
         const double pair_start = 2000.0;            // cluster launch and the pair's handshakes, once per CTA
@@ -235,6 +237,15 @@ CME_API int cme_gemm_plan(int M, int N, int K, int batch, int plain_epilogue, lo
     plan_tiles(M, N, K, batch, plain_epilogue != 0, workspace_bytes, num_sms, max_pairs, force_bn, force_splits, &bn,
                &pair, &splits);
     out[0] = bn; out[1] = pair ? 1 : 0; out[2] = splits;
+    return CME_OK;
+}
+
+// The same for a plain tf32 product with `mn_operands` operands (0, 1, 2) stored along M or N.
+CME_API int cme_gemm_plan_tf32(int M, int N, int K, int mn_operands, long long workspace_bytes, int num_sms, int max_pairs, int* out) {
+    CME_REQUIRE(M > 0 && N > 0 && K > 0 && num_sms > 0, CME_ERR_SHAPE, "gemm plan: empty problem");
+    bool pair = false;
+    plan_tiles(M, N, K, 1, true, workspace_bytes, num_sms, max_pairs, 0, 0, &out[0], &pair, &out[2], 32, mn_operands);
+    out[1] = pair ? 1 : 0;
     return CME_OK;
 }
 

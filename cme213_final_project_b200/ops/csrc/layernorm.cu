@@ -448,7 +448,7 @@ ln_bwd_finalize_kernel(const float* __restrict__ partial, int nblocks, int D, T*
 template <typename T>
 int ln_bwd_finalize(const float* partial, int nblocks, int D, T* dgamma, T* dbeta, int accumulate, cudaStream_t st) {
     // Blocks of 1024 threads cost more than they save while 16 groups read everything in two rounds (whole backward, 768
-    // bf16 columns, us with 16 / 64 groups: 32 partials 5.6 / 5.8, 128 5.9 / 6.2; 384 columns, 512 partials 7.96 / 7.75).
+    // bf16 columns, us with 16 / 64 groups: 32 partials 5.6 / 5.8, 128 partials 5.9 / 6.3).
     const bool many = nblocks > 128;
     CME_CUDA(cme_launch_dependent(many ? ln_bwd_finalize_kernel<T, 64> : ln_bwd_finalize_kernel<T, 16>, dim3(cme_cdiv(2 * D, 16)),
                                   dim3(many ? 1024 : 256), 0, st, partial, nblocks, D, dgamma, dbeta, accumulate));
