@@ -66,6 +66,7 @@ struct CmeDeviceState {
     int max_pairs;         // co-resident CTA pairs of the pair GEMM kernel (-1: not queried yet, 0: unusable)
 };
 int cme_device_state(CmeDeviceState** out);
+int cme_num_sms(int* out);
 int cme_check_status_word(int which, int* host_out);
 
 #ifdef __CUDACC__

@@ -73,8 +73,16 @@ int cme_device_state(CmeDeviceState** out) {
     return CME_OK;
 }
 
+// SMs of the current device.  Allocates nothing, so a first call may be captured.
+int cme_num_sms(int* out) {
+    int dev = 0;
+    CME_CUDA(cudaGetDevice(&dev));
+    CME_CUDA(cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev));
+    return CME_OK;
+}
+
 // Sets up the current device (SM count, status words).  Call once per device before the first stream capture;
-// every launcher calls it too, so eager use needs no explicit call.
+// every launcher whose kernel waits calls it too, so eager use needs no explicit call.
 CME_API int cme_init_device() {
     CmeDeviceState* st;
     return cme_device_state(&st);

@@ -461,13 +461,12 @@ template <typename... P> bool aligned16(P... p) { return ((reinterpret_cast<uint
 
 // Blocks of `kernel` that are resident on the current device at once with `smem` bytes each.
 template <typename K> int resident_blocks(K kernel, size_t smem, int* out) {
-    int per_sm = 0;
-    CmeDeviceState* ds;
-    const int rc = cme_device_state(&ds);
+    int per_sm = 0, num_sms = 0;
+    const int rc = cme_num_sms(&num_sms);
     if (rc) return rc;
     if (smem > 48 * 1024) CME_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CME_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, LN_WARPS * 32, smem));
-    *out = ds->num_sms * (per_sm > 0 ? per_sm : 1);
+    *out = num_sms * (per_sm > 0 ? per_sm : 1);
     return CME_OK;
 }
 // Blocks for `rows`: what is resident at once, evened out so that every block runs the same number of rounds.
