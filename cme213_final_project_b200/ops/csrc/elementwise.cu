@@ -317,16 +317,15 @@ tok_bwd_scan_kernel(const int* __restrict__ tokens, const T* __restrict__ dout, 
 // Against a warp per token with bf16 atomics into a cleared table: no clearing pass, one rounding per element instead of
 // one per token, the same bits every time, and no queue at the rows of frequent words.  Interleaved stripes spread those,
 // whose ids are near one another, over the blocks.
-// All of it is latency and bookkeeping, so there is one wave of blocks (two per SM), the token list is read once (its few
+// All of it is latency and bookkeeping, so there is one wave of blocks (two per SM while their shared memory fits, about
+// 19000 tokens at 50304 x 768 bf16, then one: 32768 tokens 64 -> 54 us), the token list is read once (its few
 // tokens of the stripe are kept in shared memory for the two passes of the sort), and loads are issued in batches: sixteen
 // token ids per lane, eight tokens of a table row.  Rows without a token are stores only; the others are handed out to the
-// 16 warps one by one; rows with many tokens are summed by the whole block in fixed shares.
-// 16384 tokens, 50304 x 768 bf16: clear + atomics 34 us, this 35 us with the sums in fp32 (40 us when both passes of the sort
-// read the list and one warp added up the shares of a long row, 52 us with all three chunks in one block); with the position
-// table and the gather the call went from 58.1 to 51.5 us and its gradient from 4.5e-3 to 1.8e-3 off the exact sums.  2048
-// tokens, 65 x 128: 5.4 us, 8.9 us while a row of up to 64 tokens was left to one warp although the stripe had no other.
+// 16 warps one by one; rows with many tokens are summed by the whole block in fixed shares (of a stripe with fewer rows than
+// warps from nine tokens on: 2048 tokens, 65 x 128, 5.4 us, 8.9 us where a row of 64 is left to one warp).
 constexpr int STRIPE_WARPS = 16, STRIPE_BATCH = 16, STRIPE_ENTRIES = 8, STRIPE_MAX_BT = 65535;
 constexpr size_t STRIPE_SMEM = 200 * 1024;
+constexpr size_t STRIPE_SMEM_TWO = 112 * 1024;           // 228 KB of an SM for two blocks and the 1 KB that each takes
 constexpr int STRIPE_HOT = 64, STRIPE_HOT_FEW = 8;       // the block sums rows with more tokens: eight rounds of a warp's loads
                                                          // where the stripe has a row for every warp, else one
 struct StripePlan {
@@ -336,23 +335,27 @@ struct StripePlan {
     bool keep;                   // shared memory has room for the warps' lists
     size_t smem;
 };
-inline StripePlan stripe_plan(int BT, int D, int V, int W) {
+inline StripePlan stripe_plan(int BT, int D, int V, int W, int num_sms) {
     StripePlan p;
     p.chunks = cme_cdiv(D, 32 * W);
-    const long long s = p.chunks < 296 ? 296 / p.chunks : 1;      // two blocks per SM, all resident at once
-    p.S = (int)(s < V ? s : V);
-    p.R = cme_cdiv(V, p.S);
-    p.magic = (unsigned)(((1ull << 32) + p.S - 1) / p.S);     // S == 1 wraps to 0: handled in the kernel
     p.per = (cme_cdiv(BT, STRIPE_WARPS) + 31) / 32 * 32;
-    p.nhot = p.R < STRIPE_WARPS ? p.R : BT / STRIPE_HOT + 1;
-    // partial sums | counts [16][R] u16 (4-byte multiple) | starts [R + 1] i32 | hot rows i32 | rows with tokens i32 | sorted
-    // positions [BT] u16 | the warps' positions [16][per] u16
-    const size_t cnt = ((size_t)STRIPE_WARPS * p.R * 2 + 3) / 4 * 4;
-    p.smem = (size_t)STRIPE_WARPS * 32 * W * 4 + cnt + ((size_t)p.R + 1) * 4 + (size_t)p.nhot * 4 + (size_t)p.R * 4 +
-             (size_t)BT * 2;
-    const size_t lists = (size_t)STRIPE_WARPS * p.per * 2;
-    p.keep = p.smem + lists <= STRIPE_SMEM;
-    if (p.keep) p.smem += lists;
+    // One wave: two blocks per SM while two fit its shared memory, else one.
+    for (int per_sm = 2; per_sm > 0; --per_sm) {
+        const int s = num_sms * per_sm / p.chunks;
+        p.S = s < 1 ? 1 : s < V ? s : V;
+        p.R = cme_cdiv(V, p.S);
+        p.magic = (unsigned)(((1ull << 32) + p.S - 1) / p.S);     // S == 1 wraps to 0: handled in the kernel
+        p.nhot = p.R < STRIPE_WARPS ? p.R : BT / STRIPE_HOT + 1;
+        // partial sums | counts [16][R] u16 (4-byte multiple) | starts [R + 1] i32 | hot rows i32 | rows with tokens i32 |
+        // sorted positions [BT] u16 | the warps' positions [16][per] u16
+        const size_t cnt = ((size_t)STRIPE_WARPS * p.R * 2 + 3) / 4 * 4;
+        p.smem = (size_t)STRIPE_WARPS * 32 * W * 4 + cnt + ((size_t)p.R + 1) * 4 + (size_t)p.nhot * 4 + (size_t)p.R * 4 +
+                 (size_t)BT * 2;
+        const size_t lists = (size_t)STRIPE_WARPS * p.per * 2;
+        p.keep = p.smem + lists <= STRIPE_SMEM;
+        if (p.keep) p.smem += lists;
+        if (p.smem <= STRIPE_SMEM_TWO || (long long)p.S * p.chunks <= num_sms) break;
+    }
     return p;
 }
 template <typename T>
@@ -766,12 +769,19 @@ int tok_bwd_t(const int* tokens, const void* dout, void* dtok, int BT, int D, in
     constexpr int W = Vw<T>::N;
     const bool scan = (long long)V * BT <= (1ll << 22) && D <= 1536;
     if (D % W == 0 && BT <= STRIPE_MAX_BT && aligned16((const T*)dout) && aligned16((const T*)dtok)) {
-        const StripePlan p = stripe_plan(BT, D, V, W);
-        // Stripes replace the block per vocabulary row wherever that would run (16384 tokens, 65 x 384: 21 us with the position
-        // table against 140; 64512 tokens: 136 against 478).  On larger tables they replace the atomics for 16-bit types while
-        // the lists fit (50304 x 768, 16384 tokens: 44 against 50 us; 8192 x 512, 4096 tokens: 19.5 against 21.4).  Atomics keep
-        // fp32, whose sums they do not round any more (80 against 62 us, and 21.5 against 19.2), and the longer token lists,
-        // which every block would walk three times (64512 tokens: 267 against 128 us).
+        int num_sms = 0;
+        const int rc = cme_num_sms(&num_sms);
+        if (rc) return rc;
+        const StripePlan p = stripe_plan(BT, D, V, W, num_sms);
+        // Stripes replace the block per vocabulary row wherever that would run (65 x 384 bf16, us: 16384 tokens 64 / 11, 39000 152 /
+        // 22, three quarters of 16384 one id 707 / 97; lists of up to 512 tokens, where that takes 2.5 to 5 us, 1 to 2 us more).
+        // On larger tables they replace the atomics for 16-bit types while the lists fit, because those round every sum
+        // to 16 bits once per token (4.5e-3 off the exact sums instead of 1.8e-3) and in another order each time.  What that
+        // costs or saves, token gradient alone, inputs from memory, us atomics with their clearing pass / stripes: 50304 x 768
+        // 1024 tokens 22.6 / 19.7, 16384 33 / 35, 32768 50 / 54, three quarters of 16384 one id 150 / 160; 50304 x 256 4096 tokens
+        // 10.7 / 12.7, 16384 14.6 / 20.8; 50304 x 64 16384 tokens 6.9 / 19.0; 8192 x 512 16384 tokens 16.6 / 20.4, three quarters
+        // one id 128 / 154.  Atomics keep fp32, whose sums they do not round any more, and longer lists, which every block
+        // would walk three times (64512 tokens, 50304 x 768, with the position table: 128 / 267 us).
         const bool better = scan || (sizeof(T) == 2 && p.keep);
         if (better && (unsigned long long)V * p.S < (1ull << 32) && p.smem <= STRIPE_SMEM) {
             auto k = tok_bwd_stripe_kernel<T>;
@@ -823,8 +833,9 @@ CME_API int cme_embedding_fwd(int dtype, const int* tokens, const void* tok, con
 }
 
 // dtok (+)= scatter of dout rows by token id; dpos (+)= sum over the batch.  With accumulate = 0 the outputs are
-// overwritten.  The stripe kernel takes every call whose rows are whole 16-byte vectors and whose positions fit 16 bits;
-// the rest: a block per vocabulary row for small vocabularies, else atomics into a table that is zero-filled first.
+// overwritten.  The stripe kernel takes small vocabularies, and 16-bit tables of any size while a block's shared memory holds
+// the token lists, where rows are whole 16-byte vectors and positions fit 16 bits; the rest: a block per vocabulary row for
+// small vocabularies, else atomics into a table that is zero-filled first.
 CME_API int cme_embedding_bwd(int dtype, const int* tokens, const void* dout, void* dtok, void* dpos, int BT, int T,
                               int D, int V, int accumulate, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
