@@ -229,8 +229,7 @@ __global__ void __launch_bounds__(NW * 32) attn_fwd_kernel(const CmeAttn a, cons
     }
 }
 
-// delta[bh, t] = sum_d dO * O
-template <typename T>
+// delta[bh, t] = sum_d dO * O, bf16 of any head size (the CUDA-core backward makes its own).
 __global__ void attn_delta_kernel(const CmeAttn a) {
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int rows = a.nb * a.nh * a.T;
@@ -239,7 +238,7 @@ __global__ void attn_delta_kernel(const CmeAttn a) {
     const long long off = head_base_o(a, bh) + (long long)t * a.ost;
     float s = 0.f;
     for (int d = threadIdx.x & 31; d < a.HD; d += 32)
-        s += to_f32<T>(((const T*)a.d_o)[off + d]) * to_f32<T>(((const T*)a.o)[off + d]);
+        s += __bfloat162float(((const __nv_bfloat16*)a.d_o)[off + d]) * __bfloat162float(((const __nv_bfloat16*)a.o)[off + d]);
     s = warp_sum(s);
     if ((threadIdx.x & 31) == 0) a.delta[row] = s;
 }
@@ -488,19 +487,18 @@ int check(const CmeAttn* a, bool bwd) {
 
 }  // namespace
 
-// delta[bh, t] = sum_d dO * O, shared with the tensor-core backward; `clear` (or null): fp32 scratch of 64 per row to zero.
+// delta[bh, t] = sum_d dO * O for the bf16 tensor-core backwards; `clear` (or null): fp32 scratch of 64 per row to zero.
 int attention_delta_launch(const CmeAttn* a, cudaStream_t st, float* clear) {
     const int rows = a->nb * a->nh * a->T;
     const bool al = ((reinterpret_cast<uintptr_t>(a->d_o) | reinterpret_cast<uintptr_t>(a->o)) & 15) == 0 &&
                     a->ost % 8 == 0 && a->osh % 8 == 0 && a->osb % 8 == 0;
-    if (a->dtype == CME_BF16 && a->HD == 64 && al) {
+    if (a->HD == 64 && al) {
         CME_CUDA(cme_launch_dependent(attn_delta_hd64_kernel, dim3(cme_cdiv(rows, 64)), dim3(256), 0, st, *a, clear));
         CME_LAUNCH_CHECK();
         return CME_OK;
     }
     if (clear) CME_CUDA(cudaMemsetAsync(clear, 0, (size_t)rows * 64 * sizeof(float), st));
-    if (a->dtype == CME_BF16) attn_delta_kernel<__nv_bfloat16><<<cme_cdiv(rows, 8), 256, 0, st>>>(*a);
-    else attn_delta_kernel<float><<<cme_cdiv(rows, 8), 256, 0, st>>>(*a);
+    attn_delta_kernel<<<cme_cdiv(rows, 8), 256, 0, st>>>(*a);
     CME_LAUNCH_CHECK();
     return CME_OK;
 }
