@@ -69,6 +69,12 @@ int cme_device_state(CmeDeviceState** out);
 int cme_num_sms(int* out);
 int cme_check_status_word(int which, int* host_out);
 
+// Whether grid-stride loops over n items may count in 32 unsigned bits: the last step goes a grid's threads past the end.
+constexpr bool cme_index32(long long n) { return n < (1ll << 31); }
+constexpr long long CME_MAX_GRID_THREADS = 148ll * 64 * 1024;
+static_assert(!cme_index32(1ll << 31) && cme_index32((1ll << 31) - 1) && (1ll << 31) - 1 + CME_MAX_GRID_THREADS < (1ll << 32),
+              "an index past the end does not wrap around");
+
 #ifdef __CUDACC__
 
 // Programmatic dependent launch for the many short kernels of a step.  A kernel launched through

@@ -46,8 +46,9 @@ __device__ __forceinline__ float dact_f(float pre, int act) {
 // One thread per vector of the row-major [rows, cols] matrix; cols is a multiple of the vector width.
 // The column comes from a 32-bit remainder (Index = unsigned) whenever the vectors can be counted in 31 bits.
 template <typename T, typename Index>
-__global__ void __launch_bounds__(256) bias_act_res_kernel(const T* __restrict__ x, const T* __restrict__ bias, const T* __restrict__ res,
-                                    T* __restrict__ pre_out, T* __restrict__ out, Index nvec, int cols, int act) {
+__global__ void __launch_bounds__(256)
+bias_act_res_kernel(const T* __restrict__ x, const T* __restrict__ bias, const T* __restrict__ res, T* __restrict__ pre_out,
+                    T* __restrict__ out, Index nvec, int cols, int act) {
     constexpr int W = Vw<T>::N;
     const Index cvec = cols / W, step = (Index)gridDim.x * blockDim.x;
     for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += step) {
@@ -565,7 +566,7 @@ int bias_act_res_t(const void* x, const void* bias, const void* res, void* pre, 
     const bool vec = cols % W == 0 && aligned16((const T*)x) && aligned16((const T*)out) &&
                      (!bias || aligned16((const T*)bias)) && (!res || aligned16((const T*)res)) &&
                      (!pre || aligned16((const T*)pre));
-    if (vec && n / W < (1ll << 31))
+    if (vec && cme_index32(n / W))
         bias_act_res_kernel<T, unsigned><<<grid_for(n / W), 256, 0, st>>>((const T*)x, (const T*)bias, (const T*)res, (T*)pre,
                                                                            (T*)out, (unsigned)(n / W), cols, act);
     else if (vec)
@@ -620,7 +621,8 @@ colsum_slabs_finalize_kernel(const float* __restrict__ partial, int slabs, int c
 template <typename T>
 int colsum_finish(const float* partial, int slabs, int cols, T* dbias, int accumulate, cudaStream_t st) {
     auto run = [&](auto kernel, int columns, int threads) -> int {
-        CME_CUDA(cme_launch_dependent(kernel, dim3(cme_cdiv(cols, columns)), dim3(threads), 0, st, partial, slabs, cols, dbias, accumulate));
+        CME_CUDA(cme_launch_dependent(kernel, dim3(cme_cdiv(cols, columns)), dim3(threads), 0, st, partial, slabs, cols, dbias,
+                                      accumulate));
         CME_LAUNCH_CHECK();
         return CME_OK;
     };
@@ -773,15 +775,18 @@ int tok_bwd_t(const int* tokens, const void* dout, void* dtok, int BT, int D, in
         const int rc = cme_num_sms(&num_sms);
         if (rc) return rc;
         const StripePlan p = stripe_plan(BT, D, V, W, num_sms);
-        // Stripes replace the block per vocabulary row wherever that would run (65 x 384 bf16, us: 16384 tokens 64 / 11, 39000 152 /
-        // 22, three quarters of 16384 one id 707 / 97; lists of up to 512 tokens, where that takes 2.5 to 5 us, 1 to 2 us more).
+        // Stripes replace the block per vocabulary row wherever that would run (65 x 384 bf16, us rows / stripes: 16384 tokens
+        // 64 / 11, 39000 152 / 22, three quarters of 16384 one id 707 / 97; lists of up to 512 tokens take 1 to 2 us more than its
+        // 2.5 to 5, and 6 to 48 us less where half of them are one id).
         // On larger tables they replace the atomics for 16-bit types while the lists fit, because those round every sum
         // to 16 bits once per token (4.5e-3 off the exact sums instead of 1.8e-3) and in another order each time.  What that
-        // costs or saves, token gradient alone, inputs from memory, us atomics with their clearing pass / stripes: 50304 x 768
-        // 1024 tokens 22.6 / 19.7, 16384 33 / 35, 32768 50 / 54, three quarters of 16384 one id 150 / 160; 50304 x 256 4096 tokens
-        // 10.7 / 12.7, 16384 14.6 / 20.8; 50304 x 64 16384 tokens 6.9 / 19.0; 8192 x 512 16384 tokens 16.6 / 20.4, three quarters
-        // one id 128 / 154.  Atomics keep fp32, whose sums they do not round any more, and longer lists, which every block
-        // would walk three times (64512 tokens, 50304 x 768, with the position table: 128 / 267 us).
+        // costs or saves, token gradient alone, inputs from memory, us atomics with their clearing pass / stripes:
+        //   50304 x 768   1024 tokens 22.6 / 19.7   16384 33.1 / 35.4   32768 50 / 54   three quarters of 16384 one id 150 / 160
+        //   50304 x 256   4096 tokens 10.7 / 12.7   16384 14.6 / 20.8
+        //   50304 x 64    4096 tokens  5.5 / 11.0   16384  6.9 / 19.0
+        //   8192 x 512    4096 tokens 10.5 / 11.7   16384 16.6 / 20.4   three quarters of 16384 one id 128 / 154
+        // Atomics keep fp32, whose sums they do not round any more, and longer lists, which every block would walk three
+        // times (64512 tokens, 50304 x 768, with the position table: 128 / 267 us).
         const bool better = scan || (sizeof(T) == 2 && p.keep);
         if (better && (unsigned long long)V * p.S < (1ull << 32) && p.smem <= STRIPE_SMEM) {
             auto k = tok_bwd_stripe_kernel<T>;
@@ -813,8 +818,9 @@ int pos_bwd_t(const void* dout, void* dpos, int BT, int T_, int D, int accumulat
         // Whole blocks of vectors for two blocks an SM leave nothing to split while the batch is a thread's few loads
         // (1024 x 768 fp32, us split / whole: batch 1 4.8 / 1.6, 8 5.6 / 2.9, 16 7.0 / 4.2).
         const bool split = BT / T_ > 16 || n / W < 256 * 296;
-        CME_CUDA(cme_launch_dependent(split ? pos_bwd_vec_kernel<T, true> : pos_bwd_vec_kernel<T, false>, dim3(cme_cdiv(n / W, split ? 32 : 256)),
-                                      dim3(256), 0, st, (const T*)dout, (T*)dpos, BT / T_, n / W, accumulate));
+        auto kernel = split ? pos_bwd_vec_kernel<T, true> : pos_bwd_vec_kernel<T, false>;
+        CME_CUDA(cme_launch_dependent(kernel, dim3(cme_cdiv(n / W, split ? 32 : 256)), dim3(256), 0, st, (const T*)dout, (T*)dpos,
+                                      BT / T_, n / W, accumulate));
     } else {
         pos_bwd_kernel<T><<<cme_cdiv(n, 256), 256, 0, st>>>((const T*)dout, (T*)dpos, BT / T_, T_, D, accumulate);
     }

@@ -45,9 +45,9 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ P, int splits, lo
 // kernel was bound by them, not by memory (two partials of 3072 x 768:
 // 10.9 -> 4.8 us; four of 2048 x 512: 9.0 -> 3.8 us).
 template <typename Index>
-__global__ void __launch_bounds__(256) splitk_reduce_vec4_kernel(const float4* __restrict__ P, int splits, long long per_split4, void* Cout,
-                                          int c_f32, int accumulate, int M, int N, int N4, long long ldc, long long strideC,
-                                          int batch, int vec) {
+__global__ void __launch_bounds__(256)
+splitk_reduce_vec4_kernel(const float4* __restrict__ P, int splits, long long per_split4, void* Cout, int c_f32, int accumulate,
+                          int M, int N, int N4, long long ldc, long long strideC, int batch, int vec) {
     pdl_wait();
     const Index total = (Index)batch * M * N4, step = (Index)gridDim.x * blockDim.x;
     for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
@@ -135,7 +135,8 @@ int make_tmap(CUtensorMap* out, const void* base, long long inner, long long row
                                         : round_tf32 ? CU_TENSOR_MAP_DATA_TYPE_TFLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     CUresult r = enc(out, dt, 3,
                      const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     round_tf32 && mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     round_tf32 && mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     CME_REQUIRE(r == CUDA_SUCCESS, CME_ERR_CUDA,
                 "cuTensorMapEncodeTiled failed (%d): inner=%lld rows=%lld ld=%lld batch=%lld bstride=%lld box_rows=%d",
                 (int)r, inner, rows, ld, batch, batch_stride, box_rows);
@@ -197,8 +198,8 @@ static void plan_tiles(int M, int N, int K, int batch, bool plain_epi, long long
         // both along K the pair tile has to win where it can fill the SMs: over 130 products it is then 0.5 % off the best
         // forced plan on average, 2.6 % with the single CTA's 150 (8192 x 768 x 2304 60.9 us as planned then, 52.0 on pairs).
         const double b16[4] = {136.0, 168.0, 138.0, 140.0};
-        const double t32[4] = {mn_operands ? 150.0 + 35.0 * mn_operands : 140.0, 150.0 + 65.0 * mn_operands, 150.0 + 30.0 * mn_operands,
-                               145.0 + 15.0 * mn_operands};
+        const double t32[4] = {mn_operands ? 150.0 + 35.0 * mn_operands : 140.0, 150.0 + 65.0 * mn_operands,
+                               150.0 + 30.0 * mn_operands, 145.0 + 15.0 * mn_operands};
         const double* cost = bk == 32 ? t32 : b16;
         const double pair_start = 2000.0;            // cluster launch and the pair's handshakes, once per CTA
         for (int i = 0; i < 4; ++i) {
@@ -241,7 +242,8 @@ CME_API int cme_gemm_plan(int M, int N, int K, int batch, int plain_epilogue, lo
 }
 
 // The same for a plain tf32 product with `mn_operands` operands (0, 1, 2) stored along M or N.
-CME_API int cme_gemm_plan_tf32(int M, int N, int K, int mn_operands, long long workspace_bytes, int num_sms, int max_pairs, int* out) {
+CME_API int cme_gemm_plan_tf32(int M, int N, int K, int mn_operands, long long workspace_bytes, int num_sms, int max_pairs,
+                               int* out) {
     CME_REQUIRE(M > 0 && N > 0 && K > 0 && num_sms > 0, CME_ERR_SHAPE, "gemm plan: empty problem");
     bool pair = false;
     plan_tiles(M, N, K, 1, true, workspace_bytes, num_sms, max_pairs, 0, 0, &out[0], &pair, &out[2], 32, mn_operands);
@@ -455,8 +457,8 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream) {
         if (ldw % 4 == 0 && (reinterpret_cast<uintptr_t>(g->workspace) & 15) == 0) {
             const long long per4 = per / 4;
             const int blocks = (int)((per4 + 255) / 256 < 8 * g_num_sms ? (per4 + 255) / 256 : 8 * g_num_sms);
-            // (half of the range: the index steps once more past the end)
-            auto kernel = per4 < (1ll << 31) ? splitk_reduce_vec4_kernel<unsigned> : splitk_reduce_vec4_kernel<unsigned long long>;
+            auto kernel = cme_index32(per4) ? splitk_reduce_vec4_kernel<unsigned>
+                                            : splitk_reduce_vec4_kernel<unsigned long long>;
             CME_CUDA(cme_launch_dependent(kernel, dim3(blocks), dim3(256), 0, stream,
                                           reinterpret_cast<const float4*>(g->workspace), splits, per4, g->C, (int)f32,
                                           g->accumulate, g->M, g->N, ldw / 4, g->ldc, g->strideC, g->batch, (int)vec));

@@ -46,7 +46,7 @@ template <> __device__ __forceinline__ void unpack_raw<__nv_bfloat16>(const uint
 constexpr int LN_STAGES = 3;
 // Row numbers are unsigned: the row fetched ahead of the last ones may lie beyond the largest int.
 constexpr unsigned row_ahead(unsigned row, unsigned step, int n) { return row + n * step; }
-static_assert(row_ahead(0x7fffffffu, 2048 * LN_WARPS, LN_STAGES) > 0x7fffffffu, "grids of up to 2048 blocks do not wrap around");
+static_assert(row_ahead(0x7fffffffu, 2048 * LN_WARPS, LN_STAGES) > 0x7fffffffu, "no wrap around with up to 2048 blocks");
 __device__ __forceinline__ void ring_copy(uint4* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
@@ -450,8 +450,9 @@ int ln_bwd_finalize(const float* partial, int nblocks, int D, T* dgamma, T* dbet
     // Blocks of 1024 threads cost more than they save while 16 groups read everything in two rounds (whole backward, 768
     // bf16 columns, us with 16 / 64 groups: 32 partials 5.6 / 5.8, 128 partials 5.9 / 6.3).
     const bool many = nblocks > 128;
-    CME_CUDA(cme_launch_dependent(many ? ln_bwd_finalize_kernel<T, 64> : ln_bwd_finalize_kernel<T, 16>, dim3(cme_cdiv(2 * D, 16)),
-                                  dim3(many ? 1024 : 256), 0, st, partial, nblocks, D, dgamma, dbeta, accumulate));
+    auto kernel = many ? ln_bwd_finalize_kernel<T, 64> : ln_bwd_finalize_kernel<T, 16>;
+    CME_CUDA(cme_launch_dependent(kernel, dim3(cme_cdiv(2 * D, 16)), dim3(many ? 1024 : 256), 0, st, partial, nblocks, D, dgamma,
+                                  dbeta, accumulate));
     CME_LAUNCH_CHECK();
     return CME_OK;
 }
@@ -478,14 +479,14 @@ inline int even_grid(int rows, int resident) {
 template <typename T, int NV>
 int ln_fwd_vec_launch(const T* a, const T* b, T* r, const T* g, const T* be, T* y, float* mean, float* rstd, int rows, int D,
                       float eps, cudaStream_t st) {
-    // The ring pays while the grid is a round or two (2048 x 768 bf16, residual, us row by row / ring: 4.2 / 4.0, 2048 x 1024 7.0 /
-    // 4.6) and where the rows come from memory and not from L2 (65536 x 768 43 / 41, 65536 x 1024 64 / 56).  Between the two
-    // more warps are worth more: 8192 x 768 from L2 5.8 / 6.5, 16384 x 512 6.7 / 8.3, 16384 x 1024 12.1 / 14.6, 8192 x 384 fp32
-    // 4.0 / 5.2.  fp32 rows beyond L2 are written faster row by row as well (65536 x 384, residual, 64 / 73).
+    // The ring pays while the grid is a round or two (bf16, residual, us row by row / ring: 2048 x 768 4.2 / 4.0, 2048 x 1024
+    // 7.0 / 4.6) and where the rows come from memory and not from L2 (65536 x 768 43 / 41, 65536 x 1024 64 / 56).  Between the
+    // two more warps are worth more: 8192 x 768 from L2 5.8 / 6.5, 16384 x 512 6.7 / 8.3, 16384 x 1024 12.1 / 14.6, 8192 x 384
+    // fp32 4.0 / 5.2.  fp32 rows beyond L2 are faster row by row as well (65536 x 384, residual, 64 / 73).
     const double in_bytes = (double)rows * D * sizeof(T) * (b ? 2 : 1);
     if (rows >= 8192 && (in_bytes <= 36e6 || (sizeof(T) == 4 && in_bytes >= 90e6))) {
-        CME_CUDA(cme_launch_dependent(ln_fwd_row_kernel<T, NV>, dim3(cme_cdiv(rows, LN_WARPS)), dim3(LN_WARPS * 32), 0, st, a, b, r, g, be,
-                                      y, mean, rstd, rows, D, eps));
+        CME_CUDA(cme_launch_dependent(ln_fwd_row_kernel<T, NV>, dim3(cme_cdiv(rows, LN_WARPS)), dim3(LN_WARPS * 32), 0, st, a, b,
+                                      r, g, be, y, mean, rstd, rows, D, eps));
         CME_LAUNCH_CHECK();
         return CME_OK;
     }

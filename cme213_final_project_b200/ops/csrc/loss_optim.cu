@@ -464,7 +464,8 @@ __global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
         const float gj = to_f32<TG>(reinterpret_cast<const TG*>(a.grads)[e]) * gs;
         float mi = a.m[e], vi = a.v[e];
         adam_moments(a, gj, mi, vi);
-        const float p = a.master[e] * (RANGES && !adam_decays(a, e) ? 1.f : keep) - lr * (mi * ibc1) / (sqrtf(vi * ibc2) + a.eps);
+        const float decay = RANGES && !adam_decays(a, e) ? 1.f : keep;
+        const float p = a.master[e] * decay - lr * (mi * ibc1) / (sqrtf(vi * ibc2) + a.eps);
         a.m[e] = mi;
         a.v[e] = vi;
         a.master[e] = p;
@@ -588,8 +589,9 @@ CME_API int cme_adam(int grad_dtype, float* master, void* compute_bf16, const vo
         blocks = (n / 4 + 255) / 256;
         if (blocks > 148 * 16) blocks = 148 * 16;
         const bool ranges = weight_decay > 0.f && n_nodecay > 0;
-        auto kernel = grad_dtype == CME_BF16 ? (ranges ? adam_vec4_kernel<__nv_bfloat16, true> : adam_vec4_kernel<__nv_bfloat16, false>)
-                                             : (ranges ? adam_vec4_kernel<float, true> : adam_vec4_kernel<float, false>);
+        auto kernel = grad_dtype != CME_BF16 ? (ranges ? adam_vec4_kernel<float, true> : adam_vec4_kernel<float, false>)
+                      : ranges               ? adam_vec4_kernel<__nv_bfloat16, true>
+                                             : adam_vec4_kernel<__nv_bfloat16, false>;
         kernel<<<(int)blocks, 256, 0, st>>>(a);
     } else if (grad_dtype == CME_BF16) adam_kernel<__nv_bfloat16><<<(int)blocks, 256, 0, st>>>(a);
     else adam_kernel<float><<<(int)blocks, 256, 0, st>>>(a);
