@@ -97,7 +97,7 @@ class NativeEngine:
                         B=cfg.batch_size, act=ops.ACT[cfg.activation], causal=int(cfg.causal),
                         head_flat=int(cfg.head_layout == "flat"), tied=int(cfg.tied_embeddings),
                         final_ln=int(cfg.final_layernorm), fused_qkv=int(cfg.mode == "gpt"),
-                        allow_tf32=int(self.tf32), fuse_epilogues=int(run.epilogue_fusion and not self.tf32),
+                        allow_tf32=2 * self.tf32, fuse_epilogues=int(run.epilogue_fusion and not self.tf32),
                         ffn_lowp={"full": 0, "store": 1, "bf16": 2}[run.ffn_precision] if self.strict else 0,
                         ln_eps=cfg.ln_eps,
                         prob_eps=1e-9 if cfg.mode == "parity" else 0.0, dtype=ops.F32 if self.strict else ops.BF16,

@@ -167,8 +167,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bo
     stores it, backward multiplies by it).  ``dbias`` (a ``[N]`` tensor): receives the column sums of ``out`` --
     from the GEMM's own epilogue when the kernel that runs can produce them, else from a separate pass.
     fp32 operands: ``backend="simt"`` multiplies them exactly; the tcgen05 kernel takes them as tf32 (plain products
-    with fp32 output only) unless ``allow_tf32=False``.  With an operand stored along M or N, ``auto`` does so where K is
-    a multiple of four and those operands hold at most 32 MB; it multiplies the others exactly.
+    with fp32 output only) unless ``allow_tf32=False``.  With an operand stored along M or N it takes those with K a multiple
+    of four and such operands of at most 32 MB together, and ``auto`` multiplies the others exactly; ``allow_tf32=2`` lets it
+    take them all.
     """
     _cuda(a, b, out, bias, aux_out, aux_in, residual)
     batch = 1

@@ -49,7 +49,7 @@ struct CmeEngineDesc {
     int V, T, D, H, FF, L, B;
     int act;             // CME_ACT_RELU | CME_ACT_GELU
     int causal, head_flat, tied, final_ln, fused_qkv;
-    int allow_tf32;      // fp32 storage: plain products may run on the tensor cores with tf32 inputs
+    int allow_tf32;      // fp32 storage: plain products may run on the tensor cores with tf32 inputs (CmeGemm)
     int fuse_epilogues;  // 0: bias / activation / residual adds and the activation derivative run as separate kernels
                          // after plain products (the ablation the reference measures with CME213_LT_FUSION)
     int ffn_lowp;        // fp32 storage only.  1: the feed-forward activation is rounded to bf16 where it is stored (the

@@ -38,9 +38,9 @@ struct CmeGemm {
     int aux_deriv;                                        // aux tensors hold act'(pre-activation), see above
     float* colsum; int* colsum_slabs;                     // optional column sums of C (device scratch, host count)
     int allow_tf32;                                       // fp32 operands may be multiplied as tf32 (10-bit mantissa
-                                                          // inputs, fp32 accumulation): plain products with fp32 output
-                                                          // whose operands lie along K, or along M / N with K % 4 == 0
-                                                          // and within half of the workspace; all others are exact
+                                                          // inputs, fp32 accumulation), plain products with fp32 output:
+                                                          // 1: operands along K, or along M / N with K % 4 == 0 and within
+                                                          // half of the workspace; 2: all that the kernel reads; 0: none
 };
 
 int gemm_tcgen05_supported(const CmeGemm* g);

@@ -258,11 +258,12 @@ int gemm_tcgen05_supported(const CmeGemm* g) {
     if (tf32 && (!g->allow_tf32 || g->c_dtype != CME_F32 || g->bias || g->residual || g->aux_out || g->aux_in ||
                  g->act || g->dact || g->N % 4 || g->ldc % 4 || (g->batch > 1 && g->strideC % 4)))
         return 0;
-    // Which fp32 products run as tf32 shows in their results, so the line lies where it always lay: with an operand stored
-    // along M or N, K is a multiple of four and those operands take up to half of the workspace (a K-major copy of each had
-    // to fit there once).  The kernel reads the others as well, but they keep all 24 bits of their inputs on the CUDA cores:
-    // the weight gradients of a 9749 x 152 x 608 feed-forward block were 1.3 and 1.4 times as far from 64-bit sums as tf32.
-    if (tf32 && (g->a_trans || !g->b_trans)) {
+    // Which fp32 products run as tf32 shows in their results, so without the caller's word for all of them (allow_tf32 = 2) the
+    // line lies where it always lay: with an operand stored along M or N, K is a multiple of four and those operands take up
+    // to half of the workspace (a K-major copy of each had to fit there once).  The others keep all 24 bits of their inputs on
+    // the CUDA cores: as tf32 the weight gradients of a 9749 x 152 x 608 feed-forward block are 1.3 and 1.4 times as far from
+    // 64-bit sums, and 20 times as fast (8192 x 512 x 2048: 39 us for 788).
+    if (tf32 && g->allow_tf32 < 2 && (g->a_trans || !g->b_trans)) {
         const long long na = g->a_trans ? (long long)(g->strideA ? g->batch : 1) * g->M * g->K : 0;
         const long long nb = !g->b_trans ? (long long)(g->strideB ? g->batch : 1) * g->N * g->K : 0;
         if (g->K % 4 || !g->workspace || (na + nb) * 4 + 512 > g->workspace_bytes / 2) return 0;

@@ -247,8 +247,7 @@ def test_derivative_kept_by_forward_and_bias_gradient_in_the_epilogue(bn, M, N):
 @pytest.mark.parametrize("M,N,K,bn", [(128, 128, 64, 0), (256, 512, 256, 0), (384, 192, 320, 64), (1000, 520, 328, 128),
                                       (1024, 256, 4096, 0), (512, 768, 256, 512), (1024, 1024, 96, 256)])
 def test_tf32_products_on_fp32_storage(M, N, K, bn, a_trans, b_trans):
-    """fp32 operands multiplied as tf32 on the tcgen05 kernel (every tile shape, both storage orders of both operands
-    -- the tensor core takes tf32 operands K-major only, the launcher transposes the others into the workspace --
+    """fp32 operands multiplied as tf32 on the tcgen05 kernel (every tile shape, both storage orders of both operands,
     split-K through the workspace, ragged edges) against an fp64 product.  tf32 keeps 10 mantissa bits of each
     input: the tolerance is the reference's for its tensor-core backend on fp32 data (5e-3 of the output scale,
     FINAL_CLEAN_CODE_/tests/test_gemm.cu:28-105)."""

@@ -9,14 +9,14 @@ from cme213_final_project_b200 import ops
 F32 = torch.float32
 
 
-def _native_answer(M, N, K, a_trans, b_trans, batch=1, workspace_bytes=64 << 20):
+def _native_answer(M, N, K, a_trans, b_trans, batch=1, workspace_bytes=64 << 20, allow=1):
     """What the tensor-core kernel says to a product, without a device: 2 (shape not supported), or 1 once it looks for one."""
     lib = ops.host_lib()
     if lib is None or torch.cuda.is_available():
         pytest.skip("asks the native library without a device")
     g = ops.CmeGemm(M, N, K, batch, 1 << 20, M if a_trans else K, M * K if batch > 1 else 0, a_trans,
                     1 << 21, K if b_trans else N, N * K if batch > 1 else 0, b_trans, 1 << 22, N, M * N, ops.F32, ops.F32,
-                    0, 0, N, 0, 0, N, 0, 0, 0, 1 << 23 if workspace_bytes else 0, workspace_bytes, 0, 0, 0, 0, None, 1)
+                    0, 0, N, 0, 0, N, 0, 0, 0, 1 << 23 if workspace_bytes else 0, workspace_bytes, 0, 0, 0, 0, None, allow)
     return lib.cme_gemm(ctypes.byref(g), 1, None)
 
 
@@ -28,6 +28,8 @@ def _native_answer(M, N, K, a_trans, b_trans, batch=1, workspace_bytes=64 << 20)
     (64, 64, 64, 0, 1, 1, 0, True), (128, 128, 128, 1, 0, 200, 64 << 20, True), (128, 128, 128, 1, 0, 300, 64 << 20, False)])
 def test_which_products_are_taken(M, N, K, a_trans, b_trans, batch, ws, tf32):
     assert _native_answer(M, N, K, a_trans, b_trans, batch, ws) == (1 if tf32 else 2)
+    assert _native_answer(M, N, K, a_trans, b_trans, batch, ws, allow=2) == 1
+    assert _native_answer(M, N, K, a_trans, b_trans, batch, ws, allow=0) == 2
 
 
 @pytest.mark.parametrize("M,N,K,pair", [(8192, 768, 2304, True), (16384, 768, 768, True), (8192, 2048, 512, True), (16384, 3072, 768, True),
@@ -60,6 +62,7 @@ def test_other_products_keep_all_bits_of_their_inputs(M, N, K):
     assert _rel(ops.gemm(x, dy, a_trans=True), x.double().t() @ dy.double()) < 4 * K ** 0.5 * 2.0 ** -24
     with pytest.raises(ops.NativeError):
         ops.gemm(x, dy, a_trans=True, backend="tcgen05")
+    assert 2.0 ** -13 < _rel(ops.gemm(x, dy, a_trans=True, allow_tf32=2), x.double().t() @ dy.double()) < TF32_REL
 
 
 # tf32 keeps 11 bits of each input (10 stored), rounded or cut: 2^-10 relative each, independent over the sum
@@ -69,16 +72,18 @@ TF32_REL = 2.0 ** -10
 @pytest.mark.gpu
 @pytest.mark.parametrize("a_trans,b_trans", [(True, False), (False, False), (True, True)])
 @pytest.mark.parametrize("bn,splits", [(0, 0), (64, 1), (128, 2), (256, 3), (512, 1)])
-@pytest.mark.parametrize("M,N,K", [(256, 264, 36), (388, 516, 1000), (300, 192, 4092)])
+@pytest.mark.parametrize("M,N,K", [(256, 264, 33), (256, 264, 36), (388, 516, 1001), (300, 192, 4095)])
 def test_ragged_operands_along_m_or_n(M, N, K, bn, splits, a_trans, b_trans):
     """K that does not fill a 32-deep block, every tile width, split and accumulating, nothing written beside the result."""
     if splits > max(1, -(-K // 32) // 4):
         pytest.skip("too short to split")
+    if K % 4 and (b_trans or not a_trans):
+        pytest.skip("rows along K that are not whole 16-byte words")
     a, b = _rand((K, M) if a_trans else (M, K), 3), _rand((N, K) if b_trans else (K, N), 4)
     want = (a.double().t() if a_trans else a.double()) @ (b.double().t() if b_trans else b.double())
     big = torch.full((M * N + 2048,), 7.0, device="cuda")
     out = big[1024:1024 + M * N].view(M, N)
-    kw = dict(a_trans=a_trans, b_trans=b_trans, backend="tcgen05", force_bn=bn, force_splits=splits)
+    kw = dict(a_trans=a_trans, b_trans=b_trans, backend="tcgen05", force_bn=bn, force_splits=splits, allow_tf32=2)
     ops.gemm(a, b, out=out, **kw)
     assert ops.gemm_check_status() == 0
     assert _rel(out, want) < TF32_REL
