@@ -6,7 +6,7 @@
 // probabilities to the next product's operand without a trip through memory): a tcgen05 product would be a 128-row
 // tile half empty, and each of the chain's steps would add a tensor-memory round trip and a barrier.
 // Precision as in the paths it stands in for: scores, softmax, delta and all sums fp32, P and dS rounded to bf16 once.
-// 32 x 4 heads x 64 tokens: head size 128 in 5.0 us forward and 7.5 us backward, where the batched products took 23.6 us in
+// 32 x 4 heads x 64 tokens: head size 128 in 5.3 us forward and 7.5 us backward, where the batched products take 23.6 us in
 // three launches and 44 us in seven; head size 32 5.7 and 6.7 us inside a training step.
 #include "attention.h"
 

@@ -366,8 +366,7 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream) {
     }
     ep.status = g_status;
     // Partial rows are padded to whole 16-byte words where the workspace has room: they then leave by TMA stores and are
-    // read back four columns at a time also when N is odd, like the 65-column output head's weight gradient (with the
-    // cost table above: parity-h128 step 130.0 -> 127.7 us).
+    // read back four columns at a time also when N is odd, like the 65-column output head's weight gradient.
     const int n_pad = (g->N + 3) / 4 * 4;
     const int ldw = (long long)splits * g->batch * g->M * n_pad * 4 <= g->workspace_bytes &&
                             (reinterpret_cast<uintptr_t>(g->workspace) & 15) == 0 ? n_pad : g->N;

@@ -40,9 +40,10 @@ template <> __device__ __forceinline__ void unpack_raw<float>(const uint4& r, fl
 }
 template <> __device__ __forceinline__ void unpack_raw<__nv_bfloat16>(const uint4& r, float* f) { unpack8(r, f); }
 
-// Rows travel through a ring of shared-memory stages, LN_STAGES - 1 rows ahead of the row a warp works on.  A lane copies
-// exactly the 16-byte words it will read itself, so waiting for its own copies is all the synchronisation there is.
-// Registers alone kept one row in flight per warp, and the memory idle while its statistics were reduced.
+// Rows travel through a ring of shared-memory stages: all of its stages but one are ahead of the row a warp works on (three
+// stages; two in the backward of four vectors per lane).  A lane copies exactly the 16-byte words it will read itself, so
+// waiting for its own copies is all the synchronisation there is.  Registers alone keep one row in flight per warp, and the
+// memory idle while its statistics are reduced.
 constexpr int LN_STAGES = 3;
 // Row numbers are unsigned: the row fetched ahead of the last ones may lie beyond the largest int.
 constexpr unsigned row_ahead(unsigned row, unsigned step, int n) { return row + n * step; }
@@ -56,7 +57,7 @@ template <int N> __device__ __forceinline__ void ring_wait() { asm volatile("cp.
 
 // y = LN(a [+ b]) * gamma + beta; optionally writes r = a + b, mean and rstd.  Rows of at most 32 * NV 16-byte vectors, one
 // warp per row, the grid what is resident at once.  Bound by memory: 16384 x 768 bf16 from memory with the residual add and
-// its sum stored (101 MB) 18.7 us; with one row per warp and four vectors per lane whatever the row's length, 22.0 us.
+// its sum stored (101 MB) 18.7-19.5 us; with one row per warp and four vectors per lane whatever the row's length, 22.0 us.
 template <typename T, int NV>
 __global__ void __launch_bounds__(LN_WARPS * 32, NV <= 3 ? 3 : 2)
 ln_fwd_vec_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ r_out, const T* __restrict__ gamma,
@@ -239,7 +240,7 @@ ln_fwd_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ 
 // d(gamma) / d(beta) accumulate in registers over all rows of the warp; they reach the warp's shared-memory slice
 // (slot (i*W + j)*32 + lane: conflict-free, in the ring's place) once at the end.  The grid is sized to what is
 // resident at once, so every block runs the same number of rounds.  Bound by memory: 16384 x 768 bf16 with
-// a residual gradient (101 MB) took 24.4 us with the rows in registers, 20 us now; forward + backward call 50.2 -> 43.9 us.
+// a residual gradient (101 MB) takes 21.7 us, 24.4 us with the rows in registers instead of the ring.
 template <typename T, int NV>
 __global__ void __launch_bounds__(LN_WARPS * 32, 2)
 ln_bwd_vec_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
@@ -247,7 +248,7 @@ ln_bwd_vec_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __
                   T* __restrict__ dx, float* __restrict__ partial /*[gridDim.x][2][D]*/, int rows, int D) {
     constexpr int W = VecOf<T>::N, S = NV <= 3 ? LN_STAGES : 2;
     constexpr int SLOTS = NV * W * 32;
-    extern __shared__ uint4 ring[];   // [LN_WARPS][S][2 or 3][NV][32]; at the end [LN_WARPS][2][SLOTS] floats
+    extern __shared__ uint4 ring[];   // [LN_WARPS][S][3][NV][32] (x, dy, residual gradient); at the end [LN_WARPS][2][SLOTS] floats
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = D / W;
     const unsigned step = gridDim.x * LN_WARPS, n_rows = rows;
