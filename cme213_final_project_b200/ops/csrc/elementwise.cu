@@ -586,22 +586,34 @@ template <typename T, int NG>
 __global__ void __launch_bounds__(NG == 1 ? 256 : NG * 32)
 colsum_slabs_finalize_kernel(const float* __restrict__ partial, int slabs, int cols, T* dbias, int accumulate) {
     constexpr int NC = NG == 1 ? 256 : 32;         // columns per block
-    constexpr int NL = 4;                          // a thread's loads in flight
     __shared__ float sm[NG][33];
     pdl_wait();
     const int cx = threadIdx.x % NC, ry = threadIdx.x / NC;
     const int c = blockIdx.x * NC + cx;
     float s = 0.f;
     if (c < cols) {
-        float t[NL] = {0.f, 0.f, 0.f, 0.f};
-        for (int r = ry; r < slabs; r += NL * NG) {
-            float v[NL];
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+        int r = ry;
+        if constexpr (NG == 32) {                  // many rows: rounds without a test per load
+            for (; r + 3 * NG < slabs; r += 4 * NG) {
+                s0 += partial[(long long)r * cols + c];
+                s1 += partial[(long long)(r + NG) * cols + c];
+                s2 += partial[(long long)(r + 2 * NG) * cols + c];
+                s3 += partial[(long long)(r + 3 * NG) * cols + c];
+            }
+            for (; r < slabs; r += NG) s0 += partial[(long long)r * cols + c];
+        } else {                                   // few: the last round's loads are in flight together too
+            for (; r < slabs; r += 4 * NG) {
+                float v[4];
 #pragma unroll
-            for (int k = 0; k < NL; ++k) v[k] = r + k * NG < slabs ? partial[(long long)(r + k * NG) * cols + c] : 0.f;
-#pragma unroll
-            for (int k = 0; k < NL; ++k) t[k] += v[k];
+                for (int k = 0; k < 4; ++k) v[k] = r + k * NG < slabs ? partial[(long long)(r + k * NG) * cols + c] : 0.f;
+                s0 += v[0];
+                s1 += v[1];
+                s2 += v[2];
+                s3 += v[3];
+            }
         }
-        s = (t[0] + t[1]) + (t[2] + t[3]);
+        s = (s0 + s1) + (s2 + s3);
     }
     if (NG > 1) {
         sm[ry][cx] = s;
@@ -615,9 +627,9 @@ colsum_slabs_finalize_kernel(const float* __restrict__ partial, int slabs, int c
     }
 }
 // The time is that of a thread's chain of loads while the blocks fit the chip: 32 groups where 8 need more than three rounds
-// of loads (512 columns, us with 8 / 32 groups: 16 rows 1.3 / 1.5, 64 rows 1.5 / 1.6, 128 rows 1.7 / 1.7, 512 rows 3.6 / 2.6,
-// 2048 rows 11 / 6.1).  Beyond 32768 columns the blocks come in several waves and fewer groups pay for longer (50304
-// columns, 1 / 8 / 32 groups: 16 rows 1.9 / 2.8 / 6.8, 512 rows 78 / 17 / 19, 2048 rows 339 / 74 / 68).
+// of loads (512 columns, us with 8 / 32 groups: 16 rows 1.3 / 1.5, 64 rows 1.5 / 1.7, 128 rows 1.7 / 1.6, 512 rows 3.6 / 2.6,
+// 2048 rows 11 / 5.8).  Beyond 32768 columns the blocks come in several waves and fewer groups pay (50304 columns, 1 / 8 / 32
+// groups: 16 rows 1.9 / 2.8 / 6.8, 512 rows 39 / 17 / 27, 2048 rows 159 / 74 / 93).
 template <typename T>
 int colsum_finish(const float* partial, int slabs, int cols, T* dbias, int accumulate, cudaStream_t st) {
     auto run = [&](auto kernel, int columns, int threads) -> int {
@@ -628,7 +640,7 @@ int colsum_finish(const float* partial, int slabs, int cols, T* dbias, int accum
     };
     const bool wide = cols > 32768;
     if (wide && slabs <= 16) return run(colsum_slabs_finalize_kernel<T, 1>, 256, 256);
-    if (slabs <= (wide ? 512 : 96)) return run(colsum_slabs_finalize_kernel<T, 8>, 32, 256);
+    if (wide || slabs <= 96) return run(colsum_slabs_finalize_kernel<T, 8>, 32, 256);
     return run(colsum_slabs_finalize_kernel<T, 32>, 32, 1024);
 }
 

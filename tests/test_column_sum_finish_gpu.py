@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,cols", [(1, 1), (1, 300), (3, 33), (16, 257), (17, 257), (31, 65), (96, 100), (97, 100), (130, 31), (2049, 64),
-                                       (1, 50304), (200, 32768), (200, 32769), (513, 32800)])
+                                       (1, 50304), (200, 32768), (200, 32769), (513, 32800), (128, 40), (513, 40)])
 def test_partial_rows_are_added_up(dtype, rows, cols):
     from cme213_final_project_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(1)
