@@ -14,13 +14,13 @@ namespace {
 // takes the SM's shared memory four clocks, in which its schedulers issue sixteen multiply-adds.  So every product is
 // register-tiled.  Forward: a warp owns 16 whole rows, a lane 4 of them (ty + 4 i) and every eighth streamed row
 // (tx + 8 j), or 4 consecutive columns in 32 (tx * 4 + 32 g): 12 loads for 128 multiply-adds in a 4-deep step (two loads
-// per multiply-add before there were tiles, 10 for 64 with 2 rows per lane), the softmax needs shuffles among 8 lanes only
+// per multiply-add without tiles, 10 for 64 with 2 rows per lane), the softmax needs shuffles among 8 lanes only
 // and P never crosses a warp.  Backward: the warps form 4 groups of 16 rows x 2 halves -- of the streamed rows in the
 // score products, of the head's columns in the others -- so that a lane's 4-row tiles of two outputs fit its registers.
 // No load has a bank conflict, since a row's pitch is an odd number of 16-byte words.
 // The head size is padded with zeros to a multiple of 32 (template G = ceil(HD / 32)).
 // 32 x 4 heads x 64 tokens x head size 128, fp32, forward + backward call: 297 us without tiles, 58 us
-// with 2 rows per lane, 51 us now (its floor at the fp32 rate, 0.94 GFLOP at 74 TFLOP/s, is 13 us).
+// with 2 rows per lane, 52 us with 4 (its floor at the fp32 rate, 0.94 GFLOP at 74 TFLOP/s, is 13 us).
 constexpr int CT = 64;               // rows streamed per step
 constexpr int WR = 16;               // rows a warp owns
 constexpr int LR = WR / 4;           // rows a lane has of them
@@ -245,7 +245,7 @@ __global__ void attn_delta_kernel(const CmeAttn a) {
 // bf16, head size 64, 16-byte aligned rows: 8 lanes per row (one 128-bit load of each operand per lane), two rows per
 // lane so that four loads are in flight.  `clear`: 64 floats per row, set to zero in the same pass (the scratch the
 // backward adds its parts of dQ to), which saves a clearing pass between this kernel and the backward: 16 x 12
-// heads x 1024 tokens 12.9 us + a 9.5 us clear before, 12.8 us for both now.
+// heads x 1024 tokens 12.7 us for both, 12.9 + 9.5 us as two passes.
 __global__ void __launch_bounds__(256) attn_delta_hd64_kernel(const CmeAttn a, float* __restrict__ clear) {
     pdl_wait();
     const int rows = a.nb * a.nh * a.T, sub = threadIdx.x & 7;

@@ -42,8 +42,8 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ P, int splits, lo
 // Same, four consecutive columns per thread: 16-byte reads of every partial.  The partials' rows are N4 float4 long, which
 // may be padding beyond N; `vec`: C takes four columns at once (N, ldc, strideC multiples of 4, C aligned).  The index is
 // split with one 32-bit division (Index = unsigned, whenever the partials of one split fit): with 64-bit divisions the
-// kernel was bound by them, not by memory (two partials of 3072 x 768:
-// 10.9 -> 4.8 us; four of 2048 x 512: 9.0 -> 3.8 us).
+// kernel is bound by them, not by memory (two partials of 3072 x 768 4.8 us, 10.9 us with those; four of 2048 x 512 3.8 and
+// 9.0 us).
 template <typename Index>
 __global__ void __launch_bounds__(256)
 splitk_reduce_vec4_kernel(const float4* __restrict__ P, int splits, long long per_split4, void* Cout, int c_f32, int accumulate,

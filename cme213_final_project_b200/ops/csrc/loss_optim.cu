@@ -188,9 +188,9 @@ cross_entropy_bf16_reg_kernel(const __nv_bfloat16* __restrict__ logits, const in
 // Rows of at most WARPS * 32 * NV elements of any length, alignment and type, held in registers from their one read to
 // their one write: WARPS == 1 gives every warp a row (8 rows per block), else a block of WARPS warps shares one.
 // Character vocabularies are a few elements per lane: what bounds them is the latency of one row's chain of load,
-// maximum, exponentials, sum, store, so it is the number of rows in flight that counts -- a block per row left 191 of
-// 256 threads of a 65-symbol row without work and paid four block-wide synchronisations per row.
-// 16384 rows of 65 bf16 logits: 27.8 -> 5.3 us.
+// maximum, exponentials, sum, store, so it is the number of rows in flight that counts -- a block per row leaves 191 of
+// 256 threads of a 65-symbol row without work and pays four block-wide synchronisations per row.
+// 16384 rows of 65 bf16 logits: 5.3 us, 27.8 us with a block per row.
 // One exponential per element (the general kernel evaluates it once for the sum and again for the gradient).
 template <typename T, int NV, int WARPS>
 __global__ void __launch_bounds__(256)
@@ -256,7 +256,7 @@ cudaError_t ce_short(const void* logits, const int* targets, void* dlogits, floa
 }
 
 // out (+)= weight * sum(x[0..n)); single block, fixed order.  One block's time is its chain of loads, so each thread has
-// four 16-byte loads in flight where x is aligned (16384 row losses: 5.9 us with a 4-byte load per step, 2.5 us now).
+// four 16-byte loads in flight where x is aligned (16384 row losses: 2.3 us, 5.9 us with a 4-byte load per step).
 __global__ void __launch_bounds__(1024) reduce_scalar_kernel(const float* __restrict__ x, int n, float weight, float* out,
                                                              int accumulate) {
     __shared__ float scratch[32];
@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(256) normsq_partial_kernel(const T* __restrict
     if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
-// Same over whole 16-byte words, four in flight per thread: a 2-byte load per iteration left the sum of 124 M bf16
-// gradients waiting for its loads: 86 us, now about 60 (249 MB).
+// Same over whole 16-byte words, four in flight per thread: with a 2-byte load per iteration the sum of 124 M bf16
+// gradients waits for its loads (249 MB: 58 us, 86 us so).
 template <typename T>
 __global__ void __launch_bounds__(256) normsq_partial_vec_kernel(const T* __restrict__ grads, long long n, float* partial) {
     __shared__ float scratch[32];
