@@ -186,7 +186,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bo
     if out is None:
         shape = (batch, M, N) if (a.dim() == 3 or b.dim() == 3) else (M, N)
         out = torch.empty(shape, dtype=odt, device=a.device)
-    ws = workspace(device=a.device)
+    try:
+        ws = workspace(device=a.device)
+    except torch.OutOfMemoryError:        # a product that finds no room is not split
+        ws = None
     a3, b3 = a.dim() == 3, b.dim() == 3
     slabs = part = None
     if dbias is not None:
@@ -197,8 +200,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bo
                 b.data_ptr(), b2[1], b2[0] * b2[1] if b3 else 0, int(b_trans),
                 out.data_ptr(), N, M * N, _dt(out), _dt(a),
                 _a(bias), _a(residual), N, _a(aux_out), _a(aux_in), N,
-                ACT[act], ACT[dact], int(accumulate), ws.data_ptr(), ws.numel() * 4, force_bn, force_splits, int(aux_deriv),
-                _a(part), None if slabs is None else ctypes.pointer(slabs), int(allow_tf32))
+                ACT[act], ACT[dact], int(accumulate), _a(ws), 0 if ws is None else ws.numel() * 4, force_bn, force_splits,
+                int(aux_deriv), _a(part), None if slabs is None else ctypes.pointer(slabs), int(allow_tf32))
     _check(lib().cme_gemm(ctypes.byref(g), _GEMM_BACKENDS[backend], _st()))
     if dbias is not None:
         gemm.last_colsum_slabs = slabs.value          # 0: the epilogue did not sum (tests look at this)

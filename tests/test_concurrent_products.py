@@ -33,6 +33,26 @@ def test_calls_in_flight_have_scratch_of_their_own(monkeypatch):
     assert lo0 < hi0 <= lo1 < hi1
 
 
+def test_a_full_device_does_without_scratch(monkeypatch):
+    seen = []
+
+    class Lib:
+        @staticmethod
+        def cme_gemm(desc, backend, stream):
+            seen.append((desc._obj.workspace, desc._obj.workspace_bytes))
+            return 0
+
+    def full(*args, **kwargs):
+        raise torch.OutOfMemoryError("no memory left")
+
+    monkeypatch.setattr(ops, "lib", lambda: Lib)
+    monkeypatch.setattr(ops, "_cuda", lambda *t: None)
+    monkeypatch.setattr(ops, "_st", lambda: 0)
+    monkeypatch.setattr(ops, "workspace", full)
+    ops.gemm(torch.zeros(64, 512), torch.zeros(512, 64))
+    assert seen == [(None, 0)]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kw", [dict(), dict(force_splits=3), dict(backend="simt")])
 @pytest.mark.parametrize("M,N,K", [(2048, 512, 2048), (512, 2048, 2048), (1024, 512, 2048)])
