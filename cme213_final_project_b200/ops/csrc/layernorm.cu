@@ -406,22 +406,34 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __rest
 template <typename T, int NG>
 __global__ void __launch_bounds__(16 * NG)
 ln_bwd_finalize_kernel(const float* __restrict__ partial, int nblocks, int D, T* dgamma, T* dbeta, int accumulate) {
-    constexpr int NL = NG == 64 ? 10 : 4;                  // a thread's loads in flight: 640 partials, more than there are
     __shared__ float sm[NG][17];
     pdl_wait();
     const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;
     const int c = blockIdx.x * 16 + cx;
     float s = 0.f;
     if (c < 2 * D) {
-        float t[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int b = ry; b < nblocks; b += NL * NG) {
-            float v[NL];
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;      // independent chains: the loads of four blocks overlap
+        int b = ry;
+        if constexpr (NG == 64) {                          // many partials: rounds without a test per load
+            for (; b + 3 * NG < nblocks; b += 4 * NG) {
+                s0 += partial[(long long)b * 2 * D + c];
+                s1 += partial[(long long)(b + NG) * 2 * D + c];
+                s2 += partial[(long long)(b + 2 * NG) * 2 * D + c];
+                s3 += partial[(long long)(b + 3 * NG) * 2 * D + c];
+            }
+            for (; b < nblocks; b += NG) s0 += partial[(long long)b * 2 * D + c];
+        } else {                                           // few: the last round's loads are in flight together too
+            for (; b < nblocks; b += 4 * NG) {
+                float v[4];
 #pragma unroll
-            for (int k = 0; k < NL; ++k) v[k] = b + k * NG < nblocks ? partial[(long long)(b + k * NG) * 2 * D + c] : 0.f;
-#pragma unroll
-            for (int k = 0; k < NL; ++k) t[k % 4] += v[k];
+                for (int k = 0; k < 4; ++k) v[k] = b + k * NG < nblocks ? partial[(long long)(b + k * NG) * 2 * D + c] : 0.f;
+                s0 += v[0];
+                s1 += v[1];
+                s2 += v[2];
+                s3 += v[3];
+            }
         }
-        s = (t[0] + t[1]) + (t[2] + t[3]);
+        s = (s0 + s1) + (s2 + s3);
     }
     sm[ry][cx] = s;
     __syncthreads();
