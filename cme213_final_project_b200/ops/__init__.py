@@ -137,12 +137,28 @@ def _cuda(*ts) -> None:
             raise NativeError("native ops need contiguous CUDA tensors")
 
 
-def workspace(nbytes: int = 64 << 20, device="cuda") -> torch.Tensor:
-    """fp32 scratch for one product launched through the Python wrappers (the partial sums of a split reduction).
+_workspaces = {}
 
-    Taken anew for each call from torch's allocator, which hands freed memory out again on the same stream only: products
-    on several streams, or issued by several threads, never share it, and it goes back when the call has been issued."""
-    return torch.empty(nbytes // 4, dtype=torch.float32, device=device)
+
+def workspace(nbytes: int = 64 << 20) -> torch.Tensor:
+    """One fp32 scratch buffer per device that stays allocated, for callers of the C entry points who order its uses
+    themselves.  ``gemm`` does not use it."""
+    dev = torch.cuda.current_device()
+    w = _workspaces.get(dev)
+    if w is None or w.numel() * 4 < nbytes:
+        w = torch.empty(nbytes // 4, dtype=torch.float32, device="cuda")
+        _workspaces[dev] = w
+    return w
+
+
+def _scratch(device) -> Optional[torch.Tensor]:
+    """64 MB for the partial sums of one product, from torch's allocator, which hands freed memory out again on the same
+    stream only: products on several streams, or issued by several threads, never share it, and it goes back when the call
+    has been issued.  ``None`` where there is no room: the product then runs unsplit."""
+    try:
+        return torch.empty(16 << 20, dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
 
 
 # --------------------------------------------------------------------------------------------------
@@ -186,10 +202,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bo
     if out is None:
         shape = (batch, M, N) if (a.dim() == 3 or b.dim() == 3) else (M, N)
         out = torch.empty(shape, dtype=odt, device=a.device)
-    try:
-        ws = workspace(device=a.device)
-    except torch.OutOfMemoryError:        # a product that finds no room is not split
-        ws = None
+    ws = _scratch(a.device)
     a3, b3 = a.dim() == 3, b.dim() == 3
     slabs = part = None
     if dbias is not None:

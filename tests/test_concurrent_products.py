@@ -42,14 +42,19 @@ def test_a_full_device_does_without_scratch(monkeypatch):
             seen.append((desc._obj.workspace, desc._obj.workspace_bytes))
             return 0
 
-    def full(*args, **kwargs):
-        raise torch.OutOfMemoryError("no memory left")
+    a, b = torch.zeros(64, 512), torch.zeros(512, 64)
+    empty = torch.empty
+
+    def full(*size, **kwargs):
+        if size == (16 << 20,):
+            raise torch.OutOfMemoryError("no memory left")
+        return empty(*size, **kwargs)
 
     monkeypatch.setattr(ops, "lib", lambda: Lib)
     monkeypatch.setattr(ops, "_cuda", lambda *t: None)
     monkeypatch.setattr(ops, "_st", lambda: 0)
-    monkeypatch.setattr(ops, "workspace", full)
-    ops.gemm(torch.zeros(64, 512), torch.zeros(512, 64))
+    monkeypatch.setattr(torch, "empty", full)
+    ops.gemm(a, b)
     assert seen == [(None, 0)]
 
 
