@@ -6,17 +6,13 @@
 // with P, dP and dS materialised as [B*H, T, T] buffers, and four more batched GEMMs plus a dS kernel in
 // backward (FINAL_CLEAN_CODE_/src/kernels/attention.cu:138-200, 253-328).
 //
-// Forward, per CTA = one (batch, head) and 128 queries; 4 softmax warps (thread = query row) + 1 warp whose
+// Forward, per CTA = one (batch, head) and 128 queries, 64 keys at a time; 4 softmax warps (thread = query row) + 1 warp whose
 // lane 0 issues TMA loads and tcgen05.mma:
-//     S_j = Q K_j^T (TMEM) -> copied to registers (the tensor core starts S_{j+1} at once) -> online softmax with a
-//     lazily raised reference maximum; a quarter of the exponentials are a packed cubic on the FMA pipe, the rest go
-//     to the special-function unit -> P_j (bf16 pairs) written back to tensor memory with tcgen05.st
-//     -> O += P_j V_j with the A operand read from tensor memory (P never passes through shared memory; TMEM
-//     accumulator, rescaled in place only when the reference maximum is raised)
-// Backward, per CTA = one (batch, head) and 128 keys, looping over query blocks (thread = query row, so the
-// row's log-sum-exp and delta are two registers):
-//     S = Q_i K^T,  dP = dO_i V^T (TMEM)  ->  P, dS (bf16, shared, double buffered)
-//     dV += P^T dO_i,  dK += dS^T Q_i (A operand read transposed; TMEM accumulators),  dQ_i = dS K (TMEM).
+//     S_j = Q K_j^T (TMEM) -> registers -> online softmax with a lazily raised reference maximum
+//     -> P_j (bf16 pairs) written over S_j with tcgen05.st -> O += P_j V_j with the A operand read from tensor memory (P
+//     never passes through shared memory; TMEM accumulator, rescaled in place only when the reference maximum is raised)
+// Backward, per CTA = one (batch, head) and 128 keys, looping over query blocks:
+//     S, dP (TMEM)  ->  P, dS (bf16)  ->  dV += P^T dO_i,  dK += dS^T Q_i (TMEM accumulators),  dQ_i = dS K (TMEM).
 //     dQ_i gets a part from every key block that sees query block i.  The parts are added to an fp32 scratch with
 //     bulk reduce-adds in whatever order the CTAs arrive (fast; the last bits of dQ depend on the order), and
 //     either (dq_mode 0, the default) the launch clears the scratch first and a small kernel scales and casts the
@@ -28,9 +24,7 @@
 //     highest key block stores its part, each lower one adds its own when the tile's counter says it is its turn,
 //     and key block 0, whose turn is last, adds the sum to its part in registers, scales, casts and writes dQ --
 //     bit-reproducible, no clearing or conversion pass, but the chain of turns makes CTAs wait for one another
-//     (measured 0.32 ms against 0.25 ms per call at 16 x 12 heads x 1024 tokens).
-//     The scores of block i+1 are issued before the gradient MMAs of block i, so the arithmetic of block i+1
-//     overlaps them.
+//     (measured 0.32 ms against 0.25 ms per call at 16 x 12 heads x 1024 tokens).  dq_mode 1 and 2 have a kernel of their own.
 // Every mbarrier wait is bounded; on expiry the CTA flags the status word, frees TMEM and returns.
 #include "attention.h"
 #include "sm100_ptx.cuh"
@@ -71,24 +65,11 @@ __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* m, const vo
                  : "memory");
 }
 
-// 2^x for two values on the FMA and integer pipes (no special-function unit): x = n + f with n = round(x) taken from
-// the mantissa of x + 1.5 * 2^23, 2^f by a cubic on [-0.5, 0.5] (relative error 7.5e-5, far below bf16 resolution),
-// and n added into the exponent field.  x is clamped at -126 (masked scores arrive as -inf and come out as 1e-38).
-// The softmax loop sends part of its exponentials here so that the special-function unit, which takes 8 cycles per
-// warp instruction, is no longer what the loop waits for.
-__device__ __forceinline__ void ex2_poly2(float x0, float x1, float& y0, float& y1) {
-    const F32x2 x = f2_pack(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
-    const F32x2 t = f2_add(x, f2_splat(12582912.f));
-    const F32x2 n = f2_add(t, f2_splat(-12582912.f));
-    const F32x2 f = f2_fma(n, f2_splat(-1.f), x);
-    F32x2 q = f2_fma(f2_splat(0.05517165f), f, f2_splat(0.24261112f));
-    q = f2_fma(q, f, f2_splat(0.69326099f));
-    q = f2_fma(q, f, f2_splat(0.99992807f));
-    float t0, t1, q0, q1;
-    f2_unpack(t, t0, t1);
-    f2_unpack(q, q0, q1);
-    y0 = __uint_as_float(__float_as_uint(q0) + (__float_as_uint(t0) << 23));
-    y1 = __uint_as_float(__float_as_uint(q1) + (__float_as_uint(t1) << 23));
+// The largest of three in one instruction.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float y;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
 }
 
 // A descriptor whose start address is `bytes` further than that of `base` (the address field counts 16-byte
@@ -109,22 +90,26 @@ struct FwdParams {
 // ------------------------------------------------------------------------------------------------------
 // Forward
 // ------------------------------------------------------------------------------------------------------
-// shared: Q 16K | K[3] 48K | V[3] 48K | barriers      (P never passes through shared memory)
-constexpr int FWD_KV_STAGES = 3;           // a K / V tile is requested two blocks ahead of its use: its ~1200-clock
-                                           // latency no longer delays the next S product
-constexpr int FWD_SMEM = (1 + 2 * FWD_KV_STAGES) * TILE_BYTES + 128;   // two CTAs per SM: 2 x (this + 1 KB) <= 228 KB
+// What bounds it: the chain MMA -> TMEM load -> softmax -> TMEM store -> MMA of a tile (no pipe is busy for half of the time).
+// So a CTA is kept small enough for four on an SM: 128 queries, 64 keys at a time, P in the columns that its scores came
+// from, 128 TMEM columns, 64 score registers per thread; every scheduler then has four softmax warps of independent chains,
+// and a tile's start and end run under the others' work.  16 x 12 heads x 1024 tokens: causal 56 us, all keys 89 us (two CTAs
+// with 128 keys at a time 70 us causal; three with S_{j+1} made under softmax_j 57 and 87 us; a quarter of the exponentials as
+// a polynomial on the FMA pipe 58 and 91 us; the query tiles of a head side by side instead of the heavy ones first 73 us causal).
+// The tensor pipe runs the MMAs of one thread in the order they are issued, so S_{j+1} may follow P_j V_j into the same
+// columns without a wait, and the barrier that announces S_{j+1} also says that O is complete up to block j.
+// shared: Q 16K | K[2] 16K | V[2] 16K | barriers      (P never passes through shared memory)
+constexpr int FWD_BKV = 64;                // keys per step
+constexpr int FWD_KV_BYTES = FWD_BKV * HD * 2;
+constexpr int FWD_SMEM = TILE_BYTES + 4 * FWD_KV_BYTES + 128;
 constexpr int FWD_THREADS = 160;
-constexpr int FWD_TMEM_COLS = 256;         // S: [0,128)  O accumulator: [128,192)  P (bf16 pairs): [192,256)
-static_assert(2 * (FWD_SMEM + 1024) <= 228 * 1024, "two forward CTAs must fit one SM's shared memory");
-static_assert(128 + HD + BKV / 2 <= FWD_TMEM_COLS && 2 * FWD_TMEM_COLS <= 512,
-              "forward TMEM budget: S + O + P per CTA, two CTAs per SM");
-#ifndef CME_ATTN_FWD_POLY_PAIRS
-#define CME_ATTN_FWD_POLY_PAIRS 1
-#endif
-constexpr int FWD_POLY_PAIRS = CME_ATTN_FWD_POLY_PAIRS;   // of every 4 score pairs, how many take 2^x on the FMA pipe
+constexpr int FWD_CTAS_PER_SM = 4;
+constexpr int FWD_TMEM_COLS = 128;         // S, then P (bf16 pairs, 32 columns): [0,64)  O accumulator: [64,128)
+static_assert(FWD_CTAS_PER_SM * (FWD_SMEM + 1024) <= 228 * 1024, "the forward CTAs must fit one SM's shared memory");
+static_assert(FWD_BKV + HD <= FWD_TMEM_COLS && FWD_CTAS_PER_SM * FWD_TMEM_COLS <= 512, "forward TMEM budget: S + O per CTA");
 constexpr float RESCALE_THRESHOLD = 8.f;   // log2 units: the running maximum is only raised when it grows by > 2^8
 
-__global__ void __launch_bounds__(FWD_THREADS, 2)
+__global__ void __launch_bounds__(FWD_THREADS, FWD_CTAS_PER_SM)
 attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                    const FwdParams p) {
@@ -134,33 +119,29 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         return;
     }
     uint8_t* sQ = smem;
-    uint8_t* sK = sQ + TILE_BYTES;                            // FWD_KV_STAGES stages
-    uint8_t* sV = sK + FWD_KV_STAGES * TILE_BYTES;            // FWD_KV_STAGES stages
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + FWD_KV_STAGES * TILE_BYTES);
+    uint8_t* sK = sQ + TILE_BYTES;                            // 2 stages
+    uint8_t* sV = sK + 2 * FWD_KV_BYTES;                      // 2 stages
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * FWD_KV_BYTES);
     uint64_t* q_full = bars;                  // 1
-    uint64_t* kv_full = bars + 1;             // [3]
-    uint64_t* kv_empty = bars + 4;            // [3]
-    uint64_t* s_full = bars + 7;              // S ready for softmax
-    uint64_t* s_free = bars + 8;              // S copied to registers (128 arrivals): the next S may be issued
-    uint64_t* p_ready = bars + 9;             // P written to tensor memory, O rescaled (128 arrivals)
-    uint64_t* o_full = bars + 10;             // P V accumulated, P consumed
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+    uint64_t* k_full = bars + 1;              // [2]
+    uint64_t* v_full = bars + 3;              // [2]
+    uint64_t* s_full = bars + 5;              // phase j: S_j is ready and O is complete up to block j - 1
+    uint64_t* p_ready = bars + 6;             // S_j read, P_j written over it, O rescaled (128 arrivals)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qt = gridDim.x - 1 - blockIdx.x;               // heavy (late) causal tiles first
-    const int q0 = qt * BQ;
-    const int bh = blockIdx.y, b = bh / p.nh, h = bh % p.nh;
-    const int nkv = p.causal ? min((q0 + BQ + BKV - 1) / BKV, (p.T + BKV - 1) / BKV) : (p.T + BKV - 1) / BKV;
+    // the late (causal: heavy) query tiles of all heads first, so that the last wave is made of the light ones
+    const int q0 = (gridDim.y - 1 - blockIdx.y) * BQ;
+    const int bh = blockIdx.x, b = bh / p.nh, h = bh % p.nh;
+    const int nkv = cme_cdiv_dev(p.causal ? min(q0 + BQ, p.T) : p.T, FWD_BKV);
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         mbar_init(q_full, 1);
-        for (int s = 0; s < FWD_KV_STAGES; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1); }
         mbar_init(s_full, 1);
-        mbar_init(s_free, 128);
         mbar_init(p_ready, 128);
-        mbar_init(o_full, 1);
         fence_barrier_init();
     }
     if (warp == 4) { tmem_alloc(tmem_slot, FWD_TMEM_COLS); tmem_relinquish(); }
@@ -168,65 +149,56 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + 128, tmem_P = tmem_base + 128 + HD;
+    const uint32_t tmem_S = tmem_base, tmem_P = tmem_base, tmem_O = tmem_base + FWD_BKV;
     pdl_wait();        // barrier set-up and TMEM allocation above may overlap the tail of the previous kernel
 
     if (warp == 4) {
         if (lane == 0) {
             // ---------------- producer + MMA issuer (one thread) ----------------
-            constexpr uint32_t idesc_s = make_idesc(1, false, false, 128, 128);   // Q K^T: both K-major
-            constexpr uint32_t idesc_o = make_idesc(1, false, true, 128, HD);     // P V: V is MN-major
-            bool ok = true;
-            mbar_arrive_expect_tx(q_full, TILE_BYTES);
-            tma_load_4d(sQ, &tmQ, q_full, 0, q0, h, b);
-            auto load_kv = [&](int j) {
-                const int st = j % FWD_KV_STAGES;
-                mbar_arrive_expect_tx(&kv_full[st], 2 * TILE_BYTES);
-                tma_load_4d(sK + st * TILE_BYTES, &tmK, &kv_full[st], 0, j * BKV, h, b);
-                tma_load_4d(sV + st * TILE_BYTES, &tmV, &kv_full[st], 0, j * BKV, h, b);
+            constexpr uint32_t idesc_s = make_idesc(1, false, false, BQ, FWD_BKV);   // Q K^T: both K-major
+            constexpr uint32_t idesc_o = make_idesc(1, false, true, BQ, HD);         // P V: V is MN-major
+            auto load_k = [&](int j) {
+                mbar_arrive_expect_tx(&k_full[j & 1], FWD_KV_BYTES);
+                tma_load_4d(sK + (j & 1) * FWD_KV_BYTES, &tmK, &k_full[j & 1], 0, j * FWD_BKV, h, b);
+            };
+            auto load_v = [&](int j) {
+                mbar_arrive_expect_tx(&v_full[j & 1], FWD_KV_BYTES);
+                tma_load_4d(sV + (j & 1) * FWD_KV_BYTES, &tmV, &v_full[j & 1], 0, j * FWD_BKV, h, b);
             };
             const uint64_t dQ_ = make_smem_desc(smem_u32(sQ), 0, 1024);
             const uint64_t dK0 = make_smem_desc(smem_u32(sK), 0, 1024);
-            const uint64_t dV0 = make_smem_desc(smem_u32(sV), TILE_BYTES, 1024);
+            const uint64_t dV0 = make_smem_desc(smem_u32(sV), FWD_KV_BYTES, 1024);
             auto issue_s = [&](int j) {
-                const uint64_t kd = desc_add(dK0, (j % FWD_KV_STAGES) * TILE_BYTES);
+                const uint64_t kd = desc_add(dK0, (j & 1) * FWD_KV_BYTES);
 #pragma unroll
                 for (int k = 0; k < HD / 16; ++k)
                     mma_f16_ss(tmem_S, desc_add(dQ_, k * 32), desc_add(kd, k * 32), idesc_s, k > 0);
                 mma_commit(s_full);
             };
-            for (int j = 0; j < FWD_KV_STAGES && j < nkv; ++j) load_kv(j);
-            ok = mbar_wait(q_full, 0, abort_flag) && mbar_wait(&kv_full[0], 0, abort_flag);
+            mbar_arrive_expect_tx(q_full, TILE_BYTES);
+            tma_load_4d(sQ, &tmQ, q_full, 0, q0, h, b);
+            load_k(0);
+            load_v(0);
+            if (nkv > 1) { load_k(1); load_v(1); }
+            bool ok = mbar_wait(q_full, 0, abort_flag) && mbar_wait(&k_full[0], 0, abort_flag);
             if (ok) { tc_fence_after(); issue_s(0); }
             for (int j = 0; j < nkv && ok; ++j) {
-                const int st = j % FWD_KV_STAGES;
-                if (j >= 1 && j + 2 < nkv) {
-                    // the stage that block j - 1 used is refilled with block j + 2: its P V product was issued one
-                    // block ago, so this wait does not hold anything up
-                    if (!mbar_wait(&kv_empty[(j - 1) % FWD_KV_STAGES], ((j - 1) / FWD_KV_STAGES) & 1, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    load_kv(j + 2);
-                }
-                if (j + 1 < nkv) {
-                    // S_j sits in registers now: the tensor core computes S_{j+1} while softmax_j runs
-                    if (!mbar_wait(s_free, j & 1, abort_flag) ||
-                        !mbar_wait(&kv_full[(j + 1) % FWD_KV_STAGES], ((j + 1) / FWD_KV_STAGES) & 1, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    issue_s(j + 1);
-                }
                 if (!mbar_wait(p_ready, j & 1, abort_flag)) { ok = false; break; }
+                // S_j has been read, so its MMAs and with them those of P_{j-1} V_{j-1} are complete: refill their tiles
+                if (j + 2 < nkv) load_k(j + 2);
+                if (j >= 1 && j + 1 < nkv) load_v(j + 1);
+                if (!mbar_wait(&v_full[j & 1], (j >> 1) & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                const uint64_t vd = desc_add(dV0, st * TILE_BYTES);
+                const uint64_t vd = desc_add(dV0, (j & 1) * FWD_KV_BYTES);
 #pragma unroll
-                for (int k = 0; k < BKV / 16; ++k)       // A = P from tensor memory: 16 keys = 8 columns per step
+                for (int k = 0; k < FWD_BKV / 16; ++k)       // A = P from tensor memory: 16 keys = 8 columns per step
                     mma_f16_ts(tmem_O, tmem_P + k * 8, desc_add(vd, k * 2048), idesc_o, (j > 0 || k > 0));
-                mma_commit(o_full);
-                mma_commit(&kv_empty[st]);
+                if (j + 1 < nkv) {
+                    if (!mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag)) { ok = false; break; }
+                    issue_s(j + 1);
+                } else {
+                    mma_commit(s_full);                      // phase nkv: O is complete
+                }
             }
             if (!ok) for (int i = 0; i < 2000; ++i) __nanosleep(500);
         }
@@ -237,30 +209,32 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const uint32_t lane_addr = uint32_t(warp * 32) << 16;
         float m_ref = -INFINITY, l = 0.f;                 // reference maximum (log2 units) and running row sum
         bool ok = true;
-        for (int j = 0; j < nkv && ok; ++j) {
+        for (int j = 0; j < nkv; ++j) {
             if (!mbar_wait(s_full, j & 1, abort_flag)) { ok = false; break; }
             tc_fence_after();
-            uint32_t r[128];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) tmem_ld32(tmem_S + lane_addr + c * 32, r + c * 32);
+            uint32_t r[64];
+            tmem_ld32(tmem_S + lane_addr, r);
+            tmem_ld32(tmem_S + lane_addr + 32, r + 32);
             tmem_wait_ld();
-            tc_fence_before();
-            mbar_arrive(s_free);
-            const int k0 = j * BKV;
-            if ((k0 + BKV > p.T) || (p.causal && k0 + BKV - 1 > q0)) {        // diagonal or ragged block
+            const int k0 = j * FWD_BKV;
+            if ((k0 + FWD_BKV > p.T) || (p.causal && k0 + FWD_BKV - 1 > q0 + warp * 32)) {     // diagonal or ragged block
                 // keys [0, lim) of this block are visible to this row: one compare and one select per score
                 const int lim = min(p.T, p.causal ? q + 1 : p.T) - k0;
 #pragma unroll
-                for (int i = 0; i < 128; ++i) r[i] = i < lim ? r[i] : 0xff800000u;     // -inf
+                for (int i = 0; i < 64; ++i) r[i] = i < lim ? r[i] : 0xff800000u;     // -inf
             }
-            // eight independent chains (a single one would be 128 dependent operations long)
-            float mx8[8];
+            float mx4[4];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) mx8[c] = __uint_as_float(r[c]);
+            for (int c = 0; c < 4; ++c) mx4[c] = __uint_as_float(r[c]);
 #pragma unroll
-            for (int i = 8; i < 128; ++i) mx8[i & 7] = fmaxf(mx8[i & 7], __uint_as_float(r[i]));
-            float mx = fmaxf(fmaxf(fmaxf(mx8[0], mx8[1]), fmaxf(mx8[2], mx8[3])),
-                             fmaxf(fmaxf(mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7])));
+            for (int i = 4; i + 8 <= 64; i += 8) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    mx4[c] = max3(mx4[c], __uint_as_float(r[i + 2 * c]), __uint_as_float(r[i + 2 * c + 1]));
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(mx4[c], __uint_as_float(r[60 + c]));
+            float mx = fmaxf(max3(mx4[0], mx4[1], mx4[2]), mx4[3]);
             mx *= p.scale_log2;                            // scale > 0, so the maximum commutes with it
             // Raise the reference maximum only when it would grow by more than the threshold: the accumulated
             // output then needs a rescale, which is rare after the first blocks.
@@ -270,21 +244,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 alpha = (m_ref == -INFINITY) ? 0.f : ex2_approx(m_ref - mx);
                 m_ref = mx;
             }
-            if (j > 0) {
-                // the previous P V product must be complete before P is overwritten or O is rescaled
-                if (!mbar_wait(o_full, (j - 1) & 1, abort_flag)) { ok = false; break; }
-                tc_fence_after();
-                if (__any_sync(0xffffffffu, raise)) {
+            if (j > 0 && __any_sync(0xffffffffu, raise)) {
 #pragma unroll 1
-                    for (int c = 0; c < HD / 16; ++c) {       // 16 columns at a time: the score row stays in registers
-                        uint32_t o[16];
-                        tmem_ld16(tmem_O + lane_addr + c * 16, o);
-                        tmem_wait_ld();
+                for (int c = 0; c < HD / 8; ++c) {        // 8 columns at a time: the score row stays in registers
+                    uint32_t o[8];
+                    tmem_ld8(tmem_O + lane_addr + c * 8, o);
+                    tmem_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                        tmem_st16(tmem_O + lane_addr + c * 16, o);
-                    }
-                    tmem_wait_st();
+                    for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                    tmem_st8(tmem_O + lane_addr + c * 8, o);
                 }
                 l *= alpha;
             }
@@ -297,19 +265,12 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             // In passes over 32 keys, so that the 16 scale-and-shifts, then the 32 exponentials, then the sums and
             // stores are each a run of independent instructions (no exponential waits for its own operand or result)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < 2; ++c) {
                 float* x = reinterpret_cast<float*>(r + c * 32);
 #pragma unroll
                 for (int i = 0; i < 32; i += 2) f2_unpack(f2_fma(f2_pack(x[i], x[i + 1]), sc2, nm2), x[i], x[i + 1]);
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    if ((i & 7) < 2 * FWD_POLY_PAIRS) {
-                        ex2_poly2(x[i], x[i + 1], x[i], x[i + 1]);
-                    } else {
-                        x[i] = ex2_approx(x[i]);
-                        x[i + 1] = ex2_approx(x[i + 1]);
-                    }
-                }
+                for (int i = 0; i < 32; ++i) x[i] = ex2_approx(x[i]);
 #pragma unroll
                 for (int i = 0; i < 32; i += 2) sum2[(i >> 1) & 3] = f2_add(sum2[(i >> 1) & 3], f2_pack(x[i], x[i + 1]));
                 // 32 probabilities = 16 columns of bf16 pairs, straight into the A operand of the P V product
@@ -319,43 +280,36 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 tmem_st16(tmem_P + lane_addr + c * 16, pw);
             }
             tmem_wait_st();
-            {
-                float s0, s1;
-                f2_unpack(f2_add(f2_add(sum2[0], sum2[1]), f2_add(sum2[2], sum2[3])), s0, s1);
-                l += s0 + s1;
-            }
             tc_fence_before();
             mbar_arrive(p_ready);
+            float s0, s1;
+            f2_unpack(f2_add(f2_add(sum2[0], sum2[1]), f2_add(sum2[2], sum2[3])), s0, s1);
+            l += s0 + s1;
         }
-        if (ok && nkv > 0) {
-            if (mbar_wait(o_full, (nkv - 1) & 1, abort_flag)) {
-                tc_fence_after();
-                float o[HD];
+        if (ok && mbar_wait(s_full, nkv & 1, abort_flag)) {
+            tc_fence_after();
+            const float inv = l > 0.f ? 1.f / l : 0.f;
+            // stage this warp's 32 rows (every product is complete: the Q tile is free) and store them with one TMA
+            uint8_t* stage = sQ + warp * 4096;
 #pragma unroll
-                for (int c = 0; c < HD / 32; ++c) {
-                    uint32_t t[32];
-                    tmem_ld32(tmem_O + lane_addr + c * 32, t);
-                    tmem_wait_ld();
+            for (int c = 0; c < HD / 32; ++c) {
+                uint32_t t[32];
+                tmem_ld32(tmem_O + lane_addr + c * 32, t);
+                tmem_wait_ld();
+                float* o = reinterpret_cast<float*>(t);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) o[c * 32 + i] = __uint_as_float(t[i]);
-                }
-                const float inv = l > 0.f ? 1.f / l : 0.f;
+                for (int i = 0; i < 32; ++i) o[i] *= inv;
 #pragma unroll
-                for (int i = 0; i < HD; ++i) o[i] *= inv;
-                // stage this warp's 32 rows (every product is complete and no load is in flight: the first K stage is
-                // free) and store them with one TMA tile store
-                uint8_t* stage = sK + warp * 4096;
-#pragma unroll
-                for (int g = 0; g < 8; ++g) *reinterpret_cast<uint4*>(stage + swz(lane, g)) = pack8(o + g * 8);
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) {
-                    tma_store_4d(&tmO, stage, 0, q0 + warp * 32, h, b);
-                    tma_store_commit();
-                    tma_store_wait_read<0>();         // shared memory may go once the copy engine has read the tile
-                }
-                if (q < p.T) p.lse[(long long)bh * p.T + q] = (m_ref == -INFINITY) ? -INFINITY : (m_ref + log2f(l)) / LOG2E;
+                for (int g = 0; g < 4; ++g) *reinterpret_cast<uint4*>(stage + swz(lane, c * 4 + g)) = pack8(o + g * 8);
             }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                tma_store_4d(&tmO, stage, 0, q0 + warp * 32, h, b);
+                tma_store_commit();
+                tma_store_wait_read<0>();         // shared memory may go once the copy engine has read the tile
+            }
+            if (q < p.T) p.lse[(long long)bh * p.T + q] = (m_ref == -INFINITY) ? -INFINITY : (m_ref + log2f(l)) / LOG2E;
         }
     }
     tc_fence_before();
@@ -367,7 +321,325 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // ------------------------------------------------------------------------------------------------------
 // Backward
 // ------------------------------------------------------------------------------------------------------
+// CTA = one (batch, head) and 128 keys, walking over blocks of 64 queries; two CTAs per SM, so that the serial chain of one
+// (MMA -> TMEM load -> arithmetic -> MMA), its start and its end run under the other's work.  The scores are computed
+// transposed (thread = key row, columns = queries):
+//     S^T = K Q_i^T,  dP^T = V dO_i^T (TMEM)  ->  P^T, dS^T (bf16)
+//     dV += P^T dO_i,  dK += dS^T Q_i  with P^T and dS^T as A operands from TMEM, written over the scores they came from
+//     dQ_i = dS K, whose A operand is the copy of dS^T in shared memory read transposed; its accumulator takes dP^T's place
+// so P never passes through shared memory and 256 TMEM columns and 106 KB of shared memory are enough.
+// The parts that the key blocks contribute to dQ_i are added to an fp32 scratch by bulk reduce-adds in arrival order; the
+// launch clears the scratch beforehand and dq_convert_kernel scales and casts the sums.
+// What bounds it: the chain of a block (two round trips to the tensor pipe, about 6000 clocks, hidden by one other CTA only);
+// the tensor pipe is busy for 45 % of the time (a product of 64 columns takes as long as one of 128).
+// 16 x 12 heads x 1024 tokens, causal: 154 us; one CTA per SM with 128 queries at a time, P through shared memory: 179 us.
+// shared: K 16K | V 16K | Q[3] 24K | dO[2] 16K | dS^T 16K | dQ staging (fp32) 16K | row statistics[2] 1K | barriers
+constexpr int BWD_BQ = 64;                 // queries per step
+constexpr int BWD_Q_BYTES = BWD_BQ * HD * 2;
+constexpr int BWD_Q_STAGES = 3, BWD_DO_STAGES = 2;
+constexpr int BWD_STAT_FLOATS = 2 * BWD_BQ;           // -log-sum-exp (log2 units) and -delta of a block's queries
+constexpr int BWD_SMEM = 4 * TILE_BYTES + (BWD_Q_STAGES + BWD_DO_STAGES) * BWD_Q_BYTES + 2 * BWD_STAT_FLOATS * 4 + 128;
+constexpr int BWD_MMA_WARP = 8;            // warps 0..7 compute, warp 8 issues TMA loads and MMA,
+constexpr int BWD_STORE_WARP = 9;          // warp 9 issues the dQ reduce-adds
+constexpr int BWD_THREADS = 10 * 32;
+constexpr int BWD_TMEM_COLS = 256;         // S^T, then P^T and dS^T [0,64)   dP^T, then dQ [64,128)   dV [128,192)   dK [192,256)
+static_assert(2 * (BWD_SMEM + 1024) <= 228 * 1024, "two backward CTAs must fit one SM's shared memory");
+static_assert(2 * BWD_BQ + 2 * HD <= BWD_TMEM_COLS && 2 * BWD_TMEM_COLS <= 512, "backward TMEM budget, two CTAs per SM");
+
 struct BwdParams {
+    int T, nh, causal;
+    float scale, scale_log2;
+    const float* lse;
+    const float* delta;
+    __nv_bfloat16* dk; __nv_bfloat16* dv;
+    long long sb, sh, st;          // strides of dK / dV
+    int* status;
+};
+
+__global__ void __launch_bounds__(BWD_THREADS, 2)
+attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
+                   const __grid_constant__ CUtensorMap tmdQ, const BwdParams p) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    if (smem_u32(smem) & 1023u) {
+        if (threadIdx.x == 0 && p.status) atomicExch(p.status, CME_ERR_SHAPE);
+        return;
+    }
+    uint8_t* sK = smem;
+    uint8_t* sV = sK + TILE_BYTES;
+    uint8_t* sQ = sV + TILE_BYTES;
+    uint8_t* sdO = sQ + BWD_Q_STAGES * BWD_Q_BYTES;
+    uint8_t* sdS = sdO + BWD_DO_STAGES * BWD_Q_BYTES;     // [128 keys][64 queries = 128 B]
+    uint8_t* sdQ = sdS + TILE_BYTES;                      // [2 column atoms][64 query rows][128 B]
+    float* stats = reinterpret_cast<float*>(sdQ + TILE_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(stats + 2 * BWD_STAT_FLOATS);
+    uint64_t* kv_full = bars;
+    uint64_t* q_full = bars + 1;               // [3]
+    uint64_t* do_full = bars + 4;              // [2]
+    uint64_t* s_full = bars + 6;               // S^T and dP^T of a query block are in TMEM
+    uint64_t* p_ready = bars + 7;              // S^T, dP^T read; P^T, dS^T written; the next statistics stored (256 arrivals)
+    uint64_t* dq_full = bars + 8;              // dQ of a query block complete
+    uint64_t* dq_free = bars + 9;              // dQ in registers (256 arrivals): dP^T may overwrite it
+    uint64_t* in_free = bars + 10;             // dV, dK accumulated: the block's Q and dO tiles may be refilled
+    uint64_t* dqs_full = bars + 11;            // dQ staging written (256 arrivals)
+    uint64_t* dqs_free = bars + 12;            // dQ staging read by the reduce-add
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the key blocks that the most queries see (causal: the lowest) of all heads first
+    const int k0 = blockIdx.y * BKV;
+    const int bh = blockIdx.x, b = bh / p.nh, h = bh % p.nh;
+    const int q_begin = p.causal ? k0 : 0;
+    const int n_it = cme_cdiv_dev(p.T - q_begin, BWD_BQ);          // >= 1: k0 < T
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        mbar_init(kv_full, 1);
+        for (int s = 0; s < BWD_Q_STAGES; ++s) mbar_init(&q_full[s], 1);
+        for (int s = 0; s < BWD_DO_STAGES; ++s) mbar_init(&do_full[s], 1);
+        mbar_init(s_full, 1);
+        mbar_init(p_ready, 256);
+        mbar_init(dq_full, 1);
+        mbar_init(dq_free, 256);
+        mbar_init(in_free, 1);
+        mbar_init(dqs_full, 256);
+        mbar_init(dqs_free, 1);
+        fence_barrier_init();
+    }
+    if (warp == BWD_MMA_WARP) { tmem_alloc(tmem_slot, BWD_TMEM_COLS); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + BWD_BQ, tmem_dQ = tmem_dP, tmem_dV = tmem_base + 2 * BWD_BQ,
+                   tmem_dK = tmem_dV + HD;
+    pdl_wait();        // barrier set-up and TMEM allocation above may overlap the tail of the previous kernel
+
+    if (warp == BWD_MMA_WARP) {
+        if (lane == 0) {
+            constexpr uint32_t idesc_s = make_idesc(1, false, false, BKV, BWD_BQ);    // K Q^T, V dO^T
+            constexpr uint32_t idesc_t = make_idesc(1, false, true, BKV, HD);         // P^T dO, dS^T Q
+            constexpr uint32_t idesc_q = make_idesc(1, true, true, BWD_BQ, HD);       // dS K (A read transposed)
+            auto load_q = [&](int it) {
+                const int s = it % BWD_Q_STAGES;
+                mbar_arrive_expect_tx(&q_full[s], BWD_Q_BYTES);
+                tma_load_4d(sQ + s * BWD_Q_BYTES, &tmQ, &q_full[s], 0, q_begin + it * BWD_BQ, h, b);
+            };
+            auto load_do = [&](int it) {
+                const int s = it % BWD_DO_STAGES;
+                mbar_arrive_expect_tx(&do_full[s], BWD_Q_BYTES);
+                tma_load_4d(sdO + s * BWD_Q_BYTES, &tmdO, &do_full[s], 0, q_begin + it * BWD_BQ, h, b);
+            };
+            // descriptors are encoded once; per MMA only a byte offset is added
+            const uint64_t kK = make_smem_desc(smem_u32(sK), 0, 1024), vK = make_smem_desc(smem_u32(sV), 0, 1024);
+            const uint64_t kMN = make_smem_desc(smem_u32(sK), TILE_BYTES, 1024);
+            const uint64_t qK0 = make_smem_desc(smem_u32(sQ), 0, 1024), oK0 = make_smem_desc(smem_u32(sdO), 0, 1024);
+            const uint64_t qMN0 = make_smem_desc(smem_u32(sQ), BWD_Q_BYTES, 1024);
+            const uint64_t oMN0 = make_smem_desc(smem_u32(sdO), BWD_Q_BYTES, 1024);
+            const uint64_t sMN = make_smem_desc(smem_u32(sdS), TILE_BYTES, 1024);
+            auto issue_s = [&](int it) {
+                const uint64_t qd = desc_add(qK0, (it % BWD_Q_STAGES) * BWD_Q_BYTES);
+#pragma unroll
+                for (int k = 0; k < HD / 16; ++k)
+                    mma_f16_ss(tmem_S, desc_add(kK, k * 32), desc_add(qd, k * 32), idesc_s, k > 0);
+            };
+            auto issue_dp = [&](int it) {
+                const uint64_t od = desc_add(oK0, (it % BWD_DO_STAGES) * BWD_Q_BYTES);
+#pragma unroll
+                for (int k = 0; k < HD / 16; ++k)
+                    mma_f16_ss(tmem_dP, desc_add(vK, k * 32), desc_add(od, k * 32), idesc_s, k > 0);
+                mma_commit(s_full);
+            };
+            mbar_arrive_expect_tx(kv_full, 2 * TILE_BYTES);
+            tma_load_4d(sK, &tmK, kv_full, 0, k0, h, b);
+            load_q(0);
+            tma_load_4d(sV, &tmV, kv_full, 0, k0, h, b);
+            load_do(0);
+            for (int it = 1; it < BWD_Q_STAGES && it < n_it; ++it) load_q(it);
+            for (int it = 1; it < BWD_DO_STAGES && it < n_it; ++it) load_do(it);
+            bool ok = mbar_wait(kv_full, 0, abort_flag) && mbar_wait(&q_full[0], 0, abort_flag) &&
+                      mbar_wait(&do_full[0], 0, abort_flag);
+            if (ok) { tc_fence_after(); issue_s(0); issue_dp(0); }
+            for (int it = 0; it < n_it && ok; ++it) {
+                if (!mbar_wait(p_ready, it & 1, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                const uint64_t qd = desc_add(qMN0, (it % BWD_Q_STAGES) * BWD_Q_BYTES),
+                               od = desc_add(oMN0, (it % BWD_DO_STAGES) * BWD_Q_BYTES);
+                // dQ first: the warps read it out while the other products of this block run
+#pragma unroll
+                for (int k = 0; k < BKV / 16; ++k)        // reduction over the 128 keys of this CTA
+                    mma_f16_ss(tmem_dQ, desc_add(sMN, k * 2048), desc_add(kMN, k * 2048), idesc_q, k > 0);
+                mma_commit(dq_full);
+                const uint32_t acc = it > 0;
+#pragma unroll
+                for (int k = 0; k < BWD_BQ / 16; ++k)     // reduction over the 64 queries of this block
+                    mma_f16_ts(tmem_dV, tmem_S + (k >> 1) * 32 + (k & 1) * 8, desc_add(od, k * 2048), idesc_t, acc | (k > 0));
+#pragma unroll
+                for (int k = 0; k < BWD_BQ / 16; ++k)
+                    mma_f16_ts(tmem_dK, tmem_S + (k >> 1) * 32 + 16 + (k & 1) * 8, desc_add(qd, k * 2048), idesc_t, acc | (k > 0));
+                mma_commit(in_free);
+                if (it + 1 < n_it) {
+                    // S^T takes the place of P^T and dS^T once the products above have read them (the tensor pipe runs them
+                    // in this order); dP^T that of dQ once the warps have it in registers
+                    const int n = it + 1;
+                    if (!mbar_wait(&q_full[n % BWD_Q_STAGES], (n / BWD_Q_STAGES) & 1, abort_flag)) { ok = false; break; }
+                    issue_s(n);
+                    if (!mbar_wait(dq_free, it & 1, abort_flag) ||
+                        !mbar_wait(&do_full[n % BWD_DO_STAGES], (n / BWD_DO_STAGES) & 1, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
+                    issue_dp(n);
+                }
+                if (it + BWD_DO_STAGES < n_it) {
+                    if (!mbar_wait(in_free, it & 1, abort_flag)) { ok = false; break; }
+                    load_do(it + BWD_DO_STAGES);
+                    if (it + BWD_Q_STAGES < n_it) load_q(it + BWD_Q_STAGES);
+                }
+            }
+            if (!ok) for (int i = 0; i < 2000; ++i) __nanosleep(500);
+        }
+    } else if (warp == BWD_STORE_WARP) {
+        if (lane == 0) {
+            for (int it = 0; it < n_it; ++it) {
+                if (!mbar_wait(dqs_full, it & 1, abort_flag)) break;
+                const int q0 = q_begin + it * BWD_BQ;
+                tma_reduce_add_3d(&tmdQ, sdQ, 0, q0, bh);
+                tma_reduce_add_3d(&tmdQ, sdQ + TILE_BYTES / 2, 32, q0, bh);
+                tma_store_commit();
+                tma_store_wait_read<0>();
+                mbar_arrive(dqs_free);                  // the staging tile may be refilled
+            }
+            tma_store_wait<0>();
+        }
+    } else {
+        // ---------------- gradient warps: warp w owns TMEM lanes 32 (w & 3).. (key rows) and the 32 queries (w >> 2) of a
+        // block, so its P^T and dS^T go to columns that only it has read ----
+        const int quarter = warp & 3, cg = warp >> 2;
+        const int row = quarter * 32 + lane;            // TMEM lane: key row for S^T, dP^T, dV, dK
+        const int key = k0 + row;
+        const uint32_t lane_addr = uint32_t(quarter * 32) << 16;
+        const uint32_t tS = tmem_S + lane_addr + cg * 32;
+        // -lse and -delta of a block's queries are read by all threads as columns: 128 threads bring them to shared memory,
+        // one block ahead.  Queries beyond T get probability 2^-inf = 0.
+        auto stat = [&](int it) {
+            const int i = threadIdx.x & (BWD_BQ - 1), q = q_begin + it * BWD_BQ + i;
+            const long long at = (long long)bh * p.T + q;
+            if (threadIdx.x < BWD_BQ) return q < p.T ? -p.lse[at] * LOG2E : -INFINITY;
+            return q < p.T ? -p.delta[at] : 0.f;
+        };
+        if (threadIdx.x < BWD_STAT_FLOATS) stats[threadIdx.x] = stat(0);
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const F32x2 sc2 = f2_splat(p.scale_log2);
+        bool ok = true;
+        for (int it = 0; it < n_it; ++it) {
+            const int q0 = q_begin + it * BWD_BQ;
+            float next = 0.f;
+            const bool fetch = it + 1 < n_it && threadIdx.x < BWD_STAT_FLOATS;
+            if (fetch) next = stat(it + 1);
+            // the statistics were stored before the previous block's arrivals on p_ready (a phase that is complete)
+            if ((it > 0 && !mbar_wait(p_ready, (it - 1) & 1, abort_flag)) || !mbar_wait(s_full, it & 1, abort_flag)) {
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            uint32_t rs[32], rd[32];
+            tmem_ld32(tS, rs);
+            tmem_ld32(tmem_dP + lane_addr + cg * 32, rd);
+            tmem_wait_ld();
+            const bool need_mask = k0 + BKV > p.T || (p.causal && q0 < k0 + BKV);
+            // queries [lo, 32) of this thread's 32 see its key
+            const int lo = (key < p.T ? (p.causal ? key - q0 : 0) : BWD_BQ) - cg * 32;
+            const float4* st = reinterpret_cast<const float4*>(stats + (it & 1) * BWD_STAT_FLOATS + cg * 32);
+            // scale-and-shift, dP - delta and the product on packed pairs (one instruction per two queries)
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                float pr[8], ds[8];
+#pragma unroll
+                for (int i = 0; i < 8; i += 4) {
+                    const float4 nl = st[(g * 8 + i) / 4], nd = st[(BWD_BQ + g * 8 + i) / 4];
+                    const float* s = reinterpret_cast<const float*>(rs + g * 8 + i);
+                    const float* d = reinterpret_cast<const float*>(rd + g * 8 + i);
+                    f2_unpack(f2_fma(f2_pack(s[0], s[1]), sc2, f2_pack(nl.x, nl.y)), pr[i], pr[i + 1]);
+                    f2_unpack(f2_fma(f2_pack(s[2], s[3]), sc2, f2_pack(nl.z, nl.w)), pr[i + 2], pr[i + 3]);
+                    f2_unpack(f2_add(f2_pack(d[0], d[1]), f2_pack(nd.x, nd.y)), ds[i], ds[i + 1]);
+                    f2_unpack(f2_add(f2_pack(d[2], d[3]), f2_pack(nd.z, nd.w)), ds[i + 2], ds[i + 3]);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) pr[i] = ex2_approx(pr[i]);
+                if (need_mask) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) pr[i] = g * 8 + i >= lo ? pr[i] : 0.f;
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) f2_unpack(f2_mul(f2_pack(pr[i], pr[i + 1]), f2_pack(ds[i], ds[i + 1])), ds[i], ds[i + 1]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {           // the packed pairs take the registers of the scores they came from
+                    rs[g * 4 + i] = f2_to_bf2(pr[2 * i], pr[2 * i + 1]);
+                    rd[g * 4 + i] = f2_to_bf2(ds[2 * i], ds[2 * i + 1]);
+                }
+                *reinterpret_cast<uint4*>(sdS + swz(row, cg * 4 + g)) =
+                    make_uint4(rd[g * 4], rd[g * 4 + 1], rd[g * 4 + 2], rd[g * 4 + 3]);
+            }
+            tmem_st16(tS, rs);
+            tmem_st16(tS + 16, rd);
+            if (fetch) stats[((it + 1) & 1) * BWD_STAT_FLOATS + threadIdx.x] = next;
+            tmem_wait_st();
+            tc_fence_before();
+            fence_proxy_async();                        // dS^T
+            mbar_arrive(p_ready);
+            // dQ: 64 query rows in lanes 0..15 of each quarter; this warp takes 16 rows x 32 columns to the staging tile
+            // (swizzled for TMA), from where the store warp adds it to the global scratch
+            if (!mbar_wait(dq_full, it & 1, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            uint32_t t[32];
+            tmem_ld32(tmem_dQ + lane_addr + cg * 32, t);
+            tmem_wait_ld();
+            tc_fence_before();
+            mbar_arrive(dq_free);
+            if (it > 0 && !mbar_wait(dqs_free, (it - 1) & 1, abort_flag)) { ok = false; break; }
+            if (lane < 16) {
+                uint8_t* atom = sdQ + cg * (TILE_BYTES / 2);
+#pragma unroll
+                for (int g = 0; g < 8; ++g)
+                    *reinterpret_cast<uint4*>(atom + swz(quarter * 16 + lane, g)) =
+                        make_uint4(t[4 * g], t[4 * g + 1], t[4 * g + 2], t[4 * g + 3]);
+            }
+            fence_proxy_async();
+            mbar_arrive(dqs_full);
+        }
+        // dV, dK of this key block: this warp's 32 columns (64 bytes = two full sectors per row) straight from registers
+        if (ok && mbar_wait(in_free, (n_it - 1) & 1, abort_flag)) {
+            tc_fence_after();
+            const long long off = (long long)b * p.sb + (long long)h * p.sh + (long long)key * p.st + cg * 32;
+            uint32_t t[32];
+            tmem_ld32(tmem_dV + lane_addr + cg * 32, t);
+            tmem_wait_ld();
+            if (key < p.T) {
+#pragma unroll
+                for (int g = 0; g < 4; ++g)
+                    *reinterpret_cast<uint4*>(p.dv + off + g * 8) = pack8(reinterpret_cast<const float*>(t) + g * 8);
+            }
+            tmem_ld32(tmem_dK + lane_addr + cg * 32, t);
+            tmem_wait_ld();
+            if (key < p.T) {
+                float* v = reinterpret_cast<float*>(t);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[i] *= p.scale;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) *reinterpret_cast<uint4*>(p.dk + off + g * 8) = pack8(v + g * 8);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, CME_ERR_TIMEOUT);
+    if (warp == BWD_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, BWD_TMEM_COLS); }
+}
+
+// ------------------------------------------------------------------------------------------------------
+// Backward with dQ finished inside the kernel (dq_mode 1 and 2)
+// ------------------------------------------------------------------------------------------------------
+struct FinParams {
     int T, nh, causal;
     float scale, scale_log2;
     const float* lse;
@@ -378,8 +650,7 @@ struct BwdParams {
     int* status;
     int* dq_sem;                   // [nb*nh, query blocks] contribution counters (zero between launches); null in mode 0
     __nv_bfloat16* dq;             // final dQ (modes 1 and 2)
-    int dq_mode;                   // 0: unordered adds into a scratch the launch cleared, converted by dq_convert_kernel
-                                   // 1: ordered adds, key block 0 finishes   2: unordered adds, the last part's CTA finishes
+    int ordered;                   // 1: ordered adds, key block 0 finishes   0: unordered adds, the last part's CTA finishes
 };
 
 // Bounded wait until *sem >= want (acquire).  Lane 0 of the calling warp polls; the warp then synchronises.
@@ -401,21 +672,21 @@ __device__ __forceinline__ bool sem_wait_warp(const int* sem, int want, volatile
 }
 
 // shared: K 16K | V 16K | Q[2] 32K | dO[2] 32K | P 32K | dS[2] 64K | dQ staging (fp32) 32K | barriers   (one CTA per SM)
-constexpr int BWD_SMEM = 14 * TILE_BYTES + 512;     // tiles | barriers, flags and the finishing warp's ring
-constexpr int BWD_MMA_WARP = 16;           // warps 0..15 compute, warp 16 issues TMA loads and MMA,
-constexpr int BWD_STORE_WARP = 17;         // warp 17 issues the dQ reduce-stores
-constexpr int BWD_FINISH_WARP = 18;        // warp 18 (mode 2) converts the dQ tiles whose last part this CTA added
-constexpr int BWD_THREADS = 19 * 32;
+constexpr int FIN_SMEM = 14 * TILE_BYTES + 512;     // tiles | barriers, flags and the finishing warp's ring
+constexpr int FIN_MMA_WARP = 16;           // warps 0..15 compute, warp 16 issues TMA loads and MMA,
+constexpr int FIN_STORE_WARP = 17;         // warp 17 issues the dQ reduce-stores
+constexpr int FIN_CONVERT_WARP = 18;        // warp 18 (mode 2) converts the dQ tiles whose last part this CTA added
+constexpr int FIN_THREADS = 19 * 32;
 constexpr int FIN_RING = CME_ATTN_FINISH_MAX_QBLOCKS;   // a CTA hands over at most one tile per query block
-constexpr int BWD_TMEM_COLS = 512;     // S [0,128) dP [128,256) dV [256,320) dK [320,384) dQ [384,448)
+constexpr int FIN_TMEM_COLS = 512;     // S [0,128) dP [128,256) dV [256,320) dK [320,384) dQ [384,448)
 static_assert(12 * 8 + 4 + 4 + 4 + FIN_RING * 4 <= 512, "barriers, flags and ring exceed their block");
-static_assert(BWD_SMEM <= 227 * 1024, "backward shared-memory carve-up exceeds what one CTA may have");
-static_assert(2 * 128 + 3 * HD <= BWD_TMEM_COLS, "backward TMEM budget: S, dP, dV, dK, dQ");
+static_assert(FIN_SMEM <= 227 * 1024, "backward shared-memory carve-up exceeds what one CTA may have");
+static_assert(2 * 128 + 3 * HD <= FIN_TMEM_COLS, "backward TMEM budget: S, dP, dV, dK, dQ");
 
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+__global__ void __launch_bounds__(FIN_THREADS, 1)
+attn_bwd_finish_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
-                   const __grid_constant__ CUtensorMap tmdQ, const BwdParams p) {
+                   const __grid_constant__ CUtensorMap tmdQ, const FinParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     if (smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0 && p.status) atomicExch(p.status, CME_ERR_SHAPE);
@@ -450,7 +721,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // above its own, which are then resident or finished.  Unordered form: the key blocks with the most query blocks
     // (the lowest) first.
     const int nkb = gridDim.x;
-    const bool ordered = p.dq_mode == 1, finish_last = p.dq_mode == 2;
+    const bool ordered = p.ordered != 0, finish_last = !ordered;
     const int kb = ordered ? nkb - 1 - (int)blockIdx.x : (int)blockIdx.x, k0 = kb * BKV;
     const int bh = blockIdx.y, b = bh / p.nh, h = bh % p.nh;
     const int nq = (p.T + BQ - 1) / BQ;
@@ -479,7 +750,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_init(s_free, 512);
         fence_barrier_init();
     }
-    if (warp == BWD_MMA_WARP) { tmem_alloc(tmem_slot, BWD_TMEM_COLS); tmem_relinquish(); }
+    if (warp == FIN_MMA_WARP) { tmem_alloc(tmem_slot, FIN_TMEM_COLS); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -487,7 +758,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + 128, tmem_dV = tmem_base + 256,
                    tmem_dK = tmem_base + 320, tmem_dQ = tmem_base + 384;
 
-    if (warp == BWD_MMA_WARP) {
+    if (warp == FIN_MMA_WARP) {
         if (lane == 0) {
             constexpr uint32_t idesc_s = make_idesc(1, false, false, 128, 128);    // Q K^T, dO V^T
             constexpr uint32_t idesc_t = make_idesc(1, true, true, 128, HD);       // P^T dO, dS^T Q (A read transposed)
@@ -566,7 +837,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             }
             if (!ok) for (int i = 0; i < 2000; ++i) __nanosleep(500);
         }
-    } else if (warp == BWD_STORE_WARP) {
+    } else if (warp == FIN_STORE_WARP) {
         // ---------------- dQ store issuer: moves each staged 128 x 64 fp32 tile into the global scratch.  Ordered form:
         // when it is this key block's turn -- a plain tile store if it is the first part, else a bulk reduce-add --
         // and the tile's counter is raised once the write has completed.  Key block 0 does not come through here.
@@ -622,7 +893,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             tma_store_wait<0>();
             if (finish_last) { __threadfence_block(); *fin_count = -1 - *fin_count; }
         }
-    } else if (warp == BWD_FINISH_WARP) {
+    } else if (warp == FIN_CONVERT_WARP) {
         // ---------------- finishing warp (mode 2): every part of a handed-over tile is in the scratch; scale and cast the
         // sums to dQ, and leave zeros behind for the next launch.  A tile is 128 x 64 fp32 = 32 KB of contiguous scratch.
         if (finish_last && n_it > 0) {
@@ -824,7 +1095,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // for the next launch
     if (ordered && kb == 0 && (int)threadIdx.x < n_it) p.dq_sem[(long long)bh * nq + i_begin + threadIdx.x] = 0;
     if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, CME_ERR_TIMEOUT);
-    if (warp == BWD_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, BWD_TMEM_COLS); }
+    if (warp == FIN_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, FIN_TMEM_COLS); }
 }
 
 // dq[b, h, t, :] = scale * acc[b * nh + h, t, :] (bf16, strided destination).  One thread per 8 elements, one (batch, head)
@@ -878,13 +1149,13 @@ int make_map4(CUtensorMap* out, const void* base, int T, int nh, int nb, long lo
     return CME_OK;
 }
 
-// fp32 map over the dQ accumulator [nbh, T, 64]: box (32 columns = 128 bytes, 128 rows, 1), 128-byte swizzle.
-int make_map_dq(CUtensorMap* out, const void* base, int T, int nbh) {
+// fp32 map over the dQ accumulator [nbh, T, 64]: box (32 columns = 128 bytes, rows, 1), 128-byte swizzle.
+int make_map_dq(CUtensorMap* out, const void* base, int T, int nbh, int rows) {
     EncodeTiledFn enc = encoder();
     CME_REQUIRE(enc != nullptr, CME_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[3] = {(cuuint64_t)HD, (cuuint64_t)T, (cuuint64_t)nbh};
     cuuint64_t strides[2] = {(cuuint64_t)HD * 4, (cuuint64_t)T * HD * 4};
-    cuuint32_t box[3] = {32, 128, 1};
+    cuuint32_t box[3] = {32, (cuuint32_t)rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -918,8 +1189,8 @@ int attention_tc_fwd(const CmeAttn* a, cudaStream_t st) {
     CUtensorMap mq, mk, mv, mo;
     int rc;
     if ((rc = make_map4(&mq, a->q, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
-    if ((rc = make_map4(&mk, a->k, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
-    if ((rc = make_map4(&mv, a->v, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
+    if ((rc = make_map4(&mk, a->k, a->T, a->nh, a->nb, a->st, a->sh, a->sb, FWD_BKV))) return rc;
+    if ((rc = make_map4(&mv, a->v, a->T, a->nh, a->nb, a->st, a->sh, a->sb, FWD_BKV))) return rc;
     if ((rc = make_map4(&mo, a->o, a->T, a->nh, a->nb, a->ost, a->osh, a->osb, 32))) return rc;
     static bool attr[CME_MAX_DEVICES] = {};               // function attributes are per device
     int dev = 0;
@@ -929,7 +1200,7 @@ int attention_tc_fwd(const CmeAttn* a, cudaStream_t st) {
         attr[dev % CME_MAX_DEVICES] = true;
     }
     FwdParams p{a->T, a->nh, a->causal, a->scale * LOG2E, a->lse, g_attn_status};
-    dim3 grid(cme_cdiv(a->T, BQ), a->nb * a->nh);
+    dim3 grid(a->nb * a->nh, cme_cdiv(a->T, BQ));
     CME_CUDA(cme_launch_dependent(attn_fwd_tc_kernel, grid, dim3(FWD_THREADS), (size_t)FWD_SMEM, st, mq, mk, mv, mo, p));
     CME_LAUNCH_CHECK();
     return CME_OK;
@@ -959,26 +1230,35 @@ int attention_tc_bwd(const CmeAttn* a, cudaStream_t st) {
     // delta, and in the same pass over the rows the zeros that the dQ parts are added to
     if ((rc = attention_delta_launch(a, st, a->dq_mode == 0 && !a->dq_accum_clean ? a->dq_accum : nullptr))) return rc;
     CUtensorMap mq, mk, mv, mdo, mdq;
-    if ((rc = make_map4(&mq, a->q, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
+    const bool finish = a->dq_mode != 0;           // dQ is completed inside the kernel
+    const int qrows = finish ? BQ : BWD_BQ;
+    if ((rc = make_map4(&mq, a->q, a->T, a->nh, a->nb, a->st, a->sh, a->sb, qrows))) return rc;
     if ((rc = make_map4(&mk, a->k, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
     if ((rc = make_map4(&mv, a->v, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
-    if ((rc = make_map4(&mdo, a->d_o, a->T, a->nh, a->nb, a->ost, a->osh, a->osb, 128))) return rc;
-    if ((rc = make_map_dq(&mdq, a->dq_accum, a->T, a->nb * a->nh))) return rc;
-    const int mode = a->dq_mode;
+    if ((rc = make_map4(&mdo, a->d_o, a->T, a->nh, a->nb, a->ost, a->osh, a->osb, qrows))) return rc;
+    if ((rc = make_map_dq(&mdq, a->dq_accum, a->T, a->nb * a->nh, qrows))) return rc;
     static bool attr[CME_MAX_DEVICES] = {};               // function attributes are per device
     int dev = 0;
     CME_CUDA(cudaGetDevice(&dev));
     if (!attr[dev % CME_MAX_DEVICES]) {
         CME_CUDA(cudaFuncSetAttribute(attn_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM));
+        CME_CUDA(cudaFuncSetAttribute(attn_bwd_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FIN_SMEM));
         attr[dev % CME_MAX_DEVICES] = true;
     }
-    BwdParams p{a->T, a->nh, a->causal, a->scale, a->scale * LOG2E, a->lse, a->delta, a->dq_accum,
-                (__nv_bfloat16*)a->dk, (__nv_bfloat16*)a->dv, a->sb, a->sh, a->st, g_attn_status, a->dq_sem,
-                (__nv_bfloat16*)a->dq, mode};
-    dim3 grid(cme_cdiv(a->T, BKV), a->nb * a->nh);
-    attn_bwd_tc_kernel<<<grid, BWD_THREADS, BWD_SMEM, st>>>(mq, mk, mv, mdo, mdq, p);
+    if (finish) {
+        FinParams p{a->T, a->nh, a->causal, a->scale, a->scale * LOG2E, a->lse, a->delta, a->dq_accum,
+                    (__nv_bfloat16*)a->dk, (__nv_bfloat16*)a->dv, a->sb, a->sh, a->st, g_attn_status, a->dq_sem,
+                    (__nv_bfloat16*)a->dq, a->dq_mode == 1};
+        dim3 grid(cme_cdiv(a->T, BKV), a->nb * a->nh);
+        attn_bwd_finish_kernel<<<grid, FIN_THREADS, FIN_SMEM, st>>>(mq, mk, mv, mdo, mdq, p);
+        CME_LAUNCH_CHECK();
+        return CME_OK;
+    }
+    BwdParams p{a->T, a->nh, a->causal, a->scale, a->scale * LOG2E, a->lse, a->delta, (__nv_bfloat16*)a->dk,
+                (__nv_bfloat16*)a->dv, a->sb, a->sh, a->st, g_attn_status};
+    CME_CUDA(cme_launch_dependent(attn_bwd_tc_kernel, dim3(a->nb * a->nh, cme_cdiv(a->T, BKV)), dim3(BWD_THREADS), (size_t)BWD_SMEM,
+                                  st, mq, mk, mv, mdo, mdq, p));
     CME_LAUNCH_CHECK();
-    if (mode != 0) return CME_OK;                  // dQ was completed inside the kernel
     CME_CUDA(cme_launch_dependent(dq_convert_kernel, dim3(cme_cdiv(a->T, 32), a->nb * a->nh), dim3(256), 0, st,
                                   (const float*)a->dq_accum, (__nv_bfloat16*)a->dq, a->T, a->nh, a->sb, a->sh, a->st,
                                   a->scale));

@@ -1,0 +1,40 @@
+"""The flash kernels (head size 64) at the edges of their 64- and 128-row blocks, against float64 PyTorch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# P, dS and every result are rounded to 8 bits (2^-9 relative at most each); two full roundings bound the 2-norm, and twice
+# that the gradients, whose products carry the rounding of dS as well
+BF16_REL = 2 * 2.0 ** -8
+
+
+def _reference(q, k, v, do, causal):
+    leaves = [t.double().requires_grad_(True) for t in (q, k, v)]
+    s = leaves[0] @ leaves[1].transpose(1, 2) / 8
+    if causal:
+        s = s.masked_fill(torch.ones(s.shape[1:], dtype=torch.bool, device=s.device).triu(1), float("-inf"))
+    out = torch.softmax(s, -1) @ leaves[2]
+    return out.detach(), torch.logsumexp(s, -1).detach(), torch.autograd.grad(out, leaves, do.double())
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("T", [1, 63, 64, 65, 127, 128, 129, 191, 192, 193, 257, 520])
+def test_every_remainder_of_a_block(T, causal):
+    from cme213_final_project_b200 import ops
+    H = 5
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q, k, v, do = (torch.randn(T, H * 64, generator=g, device="cuda").to(torch.bfloat16) for _ in range(4))
+    out, lse = ops.attention_fwd(q, k, v, 1, H, T, "split", causal, backend="tc")
+    runs = {m: ops.attention_bwd(q, k, v, out, lse, do, 1, H, T, "split", causal, backend="tc", dq_mode=m) for m in (0, 1)}
+    assert ops.attention_check_status() == 0
+    heads = [t.reshape(T, H, 64).transpose(0, 1) for t in (q, k, v, do)]
+    ref, ref_lse, ref_grads = _reference(*heads, causal)
+    back = lambda t: t.transpose(0, 1).reshape(T, H * 64)                    # noqa: E731
+    assert ((out.double() - back(ref)).norm() / ref.norm()).item() < BF16_REL
+    assert (lse.double() - ref_lse.reshape(-1)).abs().max().item() < 1e-4
+    for grads in runs.values():
+        for got, want in zip(grads, ref_grads):
+            err = (got.double() - back(want)).norm().item()
+            # one visible key: dS = P (dP - delta) cancels to rounding noise, compare with dO's size
+            assert err < (2 * BF16_REL * want.norm().item() if T > 1 else 2.0 ** -4)
