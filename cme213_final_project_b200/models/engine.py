@@ -205,11 +205,14 @@ class NativeEngine:
         """Enqueue the forward pass; the mean loss lands in ``self.loss_dev`` (no host sync)."""
         self._tokens = tokens
         gs = (1.0 / self.cfg.tokens_per_step) if grad_scale is None else grad_scale
+        self._forward(tokens, targets, self.loss_dev, loss_weight, accumulate_loss, gs)
+        return self.loss_dev
+
+    def _forward(self, tokens, targets, loss_dev, loss_weight: float, accumulate_loss: bool, gs: float) -> None:
         with torch.cuda.device(self.device):
             ops._check(self.lib.cme_engine_forward(
-                self._h, ops._p(tokens), ops._p(targets), ops._p(self.loss_dev), ctypes.c_float(loss_weight),
+                self._h, ops._p(tokens), ops._p(targets), ops._p(loss_dev), ctypes.c_float(loss_weight),
                 int(accumulate_loss), ctypes.c_float(gs), ops._stream()))
-        return self.loss_dev
 
     def backward(self, bucket_callback: Optional[Callable[[Bucket], None]] = None,
                  buckets: Optional[Sequence[Bucket]] = None, scale: float = 1.0, accumulate: bool = False) -> None:
@@ -282,18 +285,20 @@ class NativeEngine:
         accum = len(tokens)
         gs = 1.0 / (self.cfg.tokens_per_step * accum)
         for i, (x, y) in enumerate(zip(tokens, targets)):
-            self.forward(x, y, loss_weight=1.0 / accum, accumulate_loss=i > 0, grad_scale=gs)
             last = i == accum - 1
-            if last:
-                self._publish_loss()
+            self._tokens = x
+            self._forward(x, y, None, 1.0 / accum, i > 0, gs)
+            self._loss(1.0 / accum, i > 0, publish=last)
             self.backward(bucket_callback if last else None, buckets if last else None, accumulate=i > 0)
 
-    def _publish_loss(self) -> None:
-        """Enqueue (capturable) one single-thread kernel that bumps the sequence number and writes the loss, then the
-        sequence number, into pinned host memory: the host sees the new number only after the loss has landed."""
+    def _loss(self, loss_weight: float, accumulate_loss: bool, publish: bool) -> None:
+        """Enqueue (capturable) the mean of the row losses that ``_forward`` left and, with ``publish``, one single-thread
+        kernel that bumps the sequence number and writes the loss, then the sequence number, into pinned host memory: the host
+        sees the new number only after the loss has landed.  Both run beside the backward pass, which has to follow."""
         with torch.cuda.device(self.device):
-            ops._check(self.lib.cme_publish_loss(ops._p(self.loss_dev), ops._p(self.seq_dev), self._loss_host_dev,
-                                                 self._seq_host_dev, ops._stream()))
+            ops._check(self.lib.cme_engine_loss(self._h, ops._p(self.loss_dev), ctypes.c_float(loss_weight), int(accumulate_loss),
+                                                ops._p(self.seq_dev if publish else None), self._loss_host_dev,
+                                                self._seq_host_dev, ops._stream()))
 
     def read_loss(self) -> float:
         return float(self.loss_dev.item())

@@ -42,6 +42,8 @@ int cme_cross_entropy(int, const void*, const int*, void*, float*, float*, int, 
 int cme_attention_fwd(const CmeAttn*, int, void*);
 int cme_attention_bwd(const CmeAttn*, int, void*);
 int cme_gemm(const CmeGemm*, int, void*);
+int cme_loss_mean(const float*, int, float, float*, int, void*);
+int cme_publish_loss(const float*, int*, void*, void*, void*);
 int cme_cast(int, const void*, int, void*, long long, void*);
 }
 
@@ -105,12 +107,20 @@ struct Engine {
     void* attn_ws; long long attn_ws_bytes;
     void* gemm_ws; long long gemm_ws_bytes;
     void* gemm_ws_side; long long gemm_ws_side_bytes;     // split-K partials of the products on the second stream
+    void* gemm_ws_side2; long long gemm_ws_side2_bytes;   // the same for the third stream
     float* col_scratch_side;
     float* slab_scratch;                                   // [ceil(BT / 32)][FF] column sums left by a GEMM epilogue
     char *lp_x = nullptr, *lp_h = nullptr, *lp_w = nullptr;  // bf16 copies for ffn_lowp: [BT, D], [BT, FF], [D, FF]
     // second stream for the weight-gradient work (null: everything on the caller's stream)
     cudaStream_t side = nullptr;
     std::vector<cudaEvent_t> ev;                           // [L + 1][8]: four "inputs ready" + four "done" per layer
+    // third stream: half of the weight-gradient work where a product is too short to fill the GPU (`two_sides`), and what
+    // nothing in the step waits for (the mean loss and its publication)
+    cudaStream_t side2 = nullptr;
+    bool two_sides = false;
+    cudaEvent_t ev_aux[4] = {};      // [0] fork of forward's side work  [1] padded output weights ready  [2] row losses
+                                     // ready  [3] side2's work done
+    bool loss_pending = false;       // side2 holds work that backward's end has to wait for
 
     char* P(long long off) const { return params + off * (long long)es; }
     char* G(long long off) const { return grads + off * (long long)es; }
@@ -177,6 +187,9 @@ size_t carve(Engine& e, char* base) {
     const long long side_ws = 8ll * (long long)D * (long long)widest * 4ll;
     e.gemm_ws_side_bytes = side_ws > (64ll << 20) ? side_ws : (64ll << 20);
     e.gemm_ws_side = take((size_t)e.gemm_ws_side_bytes);
+    // the third stream's products are short (two_sides), or there are none
+    e.gemm_ws_side2_bytes = e.two_sides ? 16ll * (long long)D * (long long)widest * 4ll : 0;
+    e.gemm_ws_side2 = e.two_sides ? take((size_t)e.gemm_ws_side2_bytes) : nullptr;
     e.slab_scratch = (float*)take((size_t)((BT + 31) / 32) * widest * 4);
     e.col_scratch_side = (float*)take((size_t)(cme_colsum_splits((int)BT, (int)D) + cme_colsum_splits((int)BT, (int)FF)) *
                                       widest * 4);
@@ -203,10 +216,30 @@ int gemm(const Engine& e, cudaStream_t st, int M, int N, int K, const void* A, l
     g.act = act; g.dact = dact; g.accumulate = accumulate;
     g.aux_deriv = aux_deriv; g.colsum = colsum; g.colsum_slabs = colsum_slabs;
     g.allow_tf32 = e.d.allow_tf32;
-    const bool on_side = e.side != nullptr && st == e.side;
-    g.workspace = on_side ? e.gemm_ws_side : e.gemm_ws;
-    g.workspace_bytes = on_side ? e.gemm_ws_side_bytes : e.gemm_ws_bytes;
+    const bool on_side = e.side != nullptr && st == e.side, on_side2 = e.side2 != nullptr && st == e.side2;
+    g.workspace = on_side ? e.gemm_ws_side : on_side2 ? e.gemm_ws_side2 : e.gemm_ws;
+    g.workspace_bytes = on_side ? e.gemm_ws_side_bytes : on_side2 ? e.gemm_ws_side2_bytes : e.gemm_ws_bytes;
     return cme_gemm(&g, e.d.gemm_backend, st);
+}
+
+// C = sum of three products A_i B_i^T whose operands lie planeA / planeB elements apart (d ln1 from the planes of dQ, dK, dV):
+// one reduction over the planes where the tensor-core kernel takes it, else three products that accumulate.
+int gemm_planes(const Engine& e, cudaStream_t st, int M, int N, int K, const char* A, long long lda, long long planeA,
+                const char* B, long long ldb, long long planeB, void* C, long long ldc) {
+    CmeGemm g{};
+    g.M = M; g.N = N; g.K = K; g.batch = 1;
+    g.A = A; g.lda = lda;
+    g.B = B; g.ldb = ldb; g.b_trans = 1;
+    g.C = C; g.ldc = ldc; g.c_dtype = e.d.dtype; g.ab_dtype = e.d.dtype;
+    g.workspace = e.gemm_ws; g.workspace_bytes = e.gemm_ws_bytes;
+    if (e.d.dtype == CME_BF16 && e.d.gemm_backend != 2 && planeA % 8 == 0 && planeB % 8 == 0 && gemm_tcgen05_supported(&g))
+        return gemm_tcgen05_launch(&g, st, 3, planeA, planeB);
+    for (int i = 0; i < 3; ++i) {
+        const int rc = gemm(e, st, M, N, K, A + i * planeA * (long long)e.es, lda, 0, B + i * planeB * (long long)e.es, ldb, 1, C,
+                            ldc, i > 0);
+        if (rc) return rc;
+    }
+    return CME_OK;
 }
 
 // A plain product of bf16 operands with an fp32 result (the reduced-precision feed-forward experiment).
@@ -300,6 +333,9 @@ CME_API int cme_engine_create(const CmeEngineDesc* desc, const CmeLayerSlots* la
     e->BH = desc->B * desc->H;
     e->ls.assign(layers, layers + desc->L);
     e->gs = *globals;
+    // A weight gradient of up to 10 GFLOP (7 us of the whole GPU) is latency: a few tiles, each for longer than that.  Step of the
+    // parity models, one / two streams: hidden 128 106-111 / 94-101 us, 256 and 512 no difference, 512 with 64 sequences 261 / 254.
+    e->two_sides = desc->dtype == CME_BF16 && desc->fuse_epilogues != 0 && 2.0 * e->BT * desc->D * desc->FF <= 1e10;
     e->ws_bytes = carve(*e, nullptr);
     *out = e;
     return CME_OK;
@@ -325,7 +361,9 @@ CME_API void cme_engine_destroy(void* h) {
     for (cudaEvent_t v : e->ev) cudaEventDestroy(v);
     for (cudaEvent_t v : e->ev_dq) if (v) cudaEventDestroy(v);
     for (cudaEvent_t v : e->ev_ln) cudaEventDestroy(v);
+    for (cudaEvent_t v : e->ev_aux) if (v) cudaEventDestroy(v);
     if (e->side) cudaStreamDestroy(e->side);
+    if (e->side2) cudaStreamDestroy(e->side2);
     delete e;
 }
 
@@ -335,6 +373,8 @@ CME_API int cme_engine_set_overlap(void* h, int on) {
     Engine* e = static_cast<Engine*>(h);
     if (on && !e->side) {
         CME_CUDA(cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking));
+        CME_CUDA(cudaStreamCreateWithFlags(&e->side2, cudaStreamNonBlocking));
+        for (cudaEvent_t& v : e->ev_aux) CME_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
         e->ev.resize((size_t)(e->d.L + 1) * 8);
         for (cudaEvent_t& v : e->ev) CME_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
         for (cudaEvent_t& v : e->ev_dq) CME_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
@@ -342,6 +382,11 @@ CME_API int cme_engine_set_overlap(void* h, int on) {
         for (cudaEvent_t& v : e->ev_ln) CME_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
     } else if (!on && e->side) {
         CME_CUDA(cudaStreamSynchronize(e->side));
+        CME_CUDA(cudaStreamSynchronize(e->side2));
+        for (cudaEvent_t& v : e->ev_aux) { cudaEventDestroy(v); v = nullptr; }
+        CME_CUDA(cudaStreamDestroy(e->side2));
+        e->side2 = nullptr;
+        e->loss_pending = false;
         for (cudaEvent_t v : e->ev) cudaEventDestroy(v);
         for (cudaEvent_t& v : e->ev_dq) { cudaEventDestroy(v); v = nullptr; }
         for (cudaEvent_t v : e->ev_ln) cudaEventDestroy(v);
@@ -363,6 +408,8 @@ CME_API int cme_engine_fence(void* h, void* stream, void* target) {
     CME_CUDA(cudaStreamWaitEvent((cudaStream_t)target, v, 0));
     if (e->side) {
         CME_CUDA(cudaEventRecord(v, e->side));
+        CME_CUDA(cudaStreamWaitEvent((cudaStream_t)target, v, 0));
+        CME_CUDA(cudaEventRecord(v, e->side2));
         CME_CUDA(cudaStreamWaitEvent((cudaStream_t)target, v, 0));
     }
     CME_CUDA(cudaEventDestroy(v));           // released once the recorded work has completed
@@ -392,6 +439,17 @@ CME_API int cme_engine_forward(void* h, const int* tokens, const int* targets, f
     CME_REQUIRE(e.ws != nullptr, CME_ERR_SHAPE, "engine: not bound");
     const int BT = e.BT, D = d.D, FF = d.FF, V = d.V, dt = d.dtype;
     const bool fused = d.fuse_epilogues != 0;
+    if (e.wout_pad) {
+        // the padded copy of the output weights is needed at the end of forward: made beside it where there is a second stream
+        cudaStream_t cs = e.side ? e.side : st;
+        if (e.side) {
+            CME_CUDA(cudaEventRecord(e.ev_aux[0], st));
+            CME_CUDA(cudaStreamWaitEvent(cs, e.ev_aux[0], 0));
+        }
+        CME_CUDA(cudaMemcpy2DAsync(e.wout_pad, (size_t)e.VL * e.es, e.P(e.gs.Wout), (size_t)V * e.es, (size_t)V * e.es, D,
+                                   cudaMemcpyDeviceToDevice, cs));
+        if (e.side) CME_CUDA(cudaEventRecord(e.ev_aux[1], cs));
+    }
     TRY(cme_embedding_fwd(dt, tokens, e.P(e.gs.tok), e.P(e.gs.pos), e.x[0], BT, d.T, D, V, st));
     for (int l = 0; l < d.L; ++l) {
         const CmeLayerSlots& s = e.ls[l];
@@ -459,8 +517,7 @@ CME_API int cme_engine_forward(void* h, const int* tokens, const int* targets, f
     if (d.tied) {
         TRY(gemm(e, st, BT, V, D, xlast, D, 0, e.P(e.gs.tok), D, 1, e.logits, e.VL));
     } else if (e.wout_pad) {
-        CME_CUDA(cudaMemcpy2DAsync(e.wout_pad, (size_t)e.VL * e.es, e.P(e.gs.Wout), (size_t)V * e.es, (size_t)V * e.es, D,
-                                   cudaMemcpyDeviceToDevice, st));
+        if (e.side) CME_CUDA(cudaStreamWaitEvent(st, e.ev_aux[1], 0));
         TRY(gemm(e, st, BT, V, D, xlast, D, 0, e.wout_pad, e.VL, 0, e.logits, e.VL));
     } else {
         TRY(gemm(e, st, BT, V, D, xlast, D, 0, e.P(e.gs.Wout), V, 0, e.logits, e.VL));
@@ -469,6 +526,22 @@ CME_API int cme_engine_forward(void* h, const int* tokens, const int* targets, f
         TRY(cme_cross_entropy(dt, e.logits, targets, e.logits, e.losses, loss_out, BT, V, e.VL, grad_scale, d.prob_eps,
                               loss_weight, accumulate_loss, st));
     return CME_OK;
+}
+
+// After a forward that left the mean loss out (loss_out null): *loss_out (+)= loss_weight * mean of the row losses, and the
+// loss published to the host.  Nothing else in a step waits for either, so they run on the third stream where there is one,
+// and cme_engine_backward, which has to follow, makes `stream` wait for them at its end.
+CME_API int cme_engine_loss(void* h, float* loss_out, float loss_weight, int accumulate_loss, int* seq, void* host_loss_dev,
+                            void* host_seq_dev, void* stream) {
+    Engine& e = *static_cast<Engine*>(h);
+    cudaStream_t st = (cudaStream_t)stream, ls = e.side2 ? e.side2 : st;
+    if (e.side2) {
+        CME_CUDA(cudaEventRecord(e.ev_aux[2], st));
+        CME_CUDA(cudaStreamWaitEvent(ls, e.ev_aux[2], 0));
+        e.loss_pending = true;
+    }
+    TRY(cme_loss_mean(e.losses, e.BT, loss_weight, loss_out, accumulate_loss, ls));
+    return seq ? cme_publish_loss(loss_out, seq, host_loss_dev, host_seq_dev, ls) : CME_OK;
 }
 
 // Backward from d(logits) left in the logits buffer by forward.  accumulate != 0 adds into the gradient
@@ -485,7 +558,9 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
     const CmeEngineDesc& d = e.d;
     cudaStream_t st = (cudaStream_t)stream;
     const bool ov = e.side != nullptr;
-    cudaStream_t ws = ov ? e.side : st;                     // stream of the weight-gradient work
+    cudaStream_t ws = ov ? e.side : st;                     // stream of the weight-gradient work,
+    cudaStream_t ws2 = ov && e.two_sides ? e.side2 : ws;    // and of that of W2 and Wo
+    auto of = [&](int slot, int k) { return slot < d.L && (k & 1) == 0 ? ws2 : ws; };
     const int BT = e.BT, D = d.D, FF = d.FF, V = d.V, dt = d.dtype;
     int bucket = 0;
     auto emit = [&]() { if (bucket_ready) bucket_ready(user, bucket); ++bucket; };
@@ -494,12 +569,12 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
     auto ready = [&](int slot, int k) -> int {              // side work may start: its inputs are enqueued on `st`
         if (!ov) return CME_OK;
         CME_CUDA(cudaEventRecord(evt(slot, k), st));
-        CME_CUDA(cudaStreamWaitEvent(ws, evt(slot, k), 0));
+        CME_CUDA(cudaStreamWaitEvent(of(slot, k), evt(slot, k), 0));
         return CME_OK;
     };
     auto done = [&](int slot, int k) -> int {               // marks the end of a piece of side work
         if (!ov) return CME_OK;
-        CME_CUDA(cudaEventRecord(evt(slot, 4 + k), ws));
+        CME_CUDA(cudaEventRecord(evt(slot, 4 + k), of(slot, k)));
         return CME_OK;
     };
     auto need = [&](int slot, int k) -> int {               // `st` is about to overwrite what that piece reads
@@ -508,6 +583,7 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
         return CME_OK;
     };
     float* col_s = ov ? e.col_scratch_side : e.col_scratch;
+    float* col_s2 = ws2 != ws ? e.col_scratch : col_s;      // (two_sides: nothing on `st` uses it)
     // LayerNorm backward at `site` (2 l + 1: LN2 of block l, 2 l: LN1, 2 L: final): dx on `st`; the sums of the
     // per-block partial d(gamma) / d(beta) follow on the second stream when there is one
     auto ln_bwd = [&](int site, const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
@@ -586,8 +662,8 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
                 TRY(cme_dact_colsum(dt, e.dff, aux, e.dff, e.G(s.b1), e.col_scratch, BT, FF, d.act, accumulate, st));
                 db1_done = true;
             }
-            TRY(gemm(e, ws, FF, D, BT, a.ffact, FF, 1, dx, D, 0, e.G(s.W2), D, accumulate));
-            TRY(cme_dact_colsum(dt, dx, nullptr, nullptr, e.G(s.b2), col_s, BT, D, 0, accumulate, ws));
+            TRY(gemm(e, ws2, FF, D, BT, a.ffact, FF, 1, dx, D, 0, e.G(s.W2), D, accumulate));
+            TRY(cme_dact_colsum(dt, dx, nullptr, nullptr, e.G(s.b2), col_s2, BT, D, 0, accumulate, ws2));
             TRY(done(l, 0));
             emit();
             // ---- FFN1:  ff_pre = ln2 @ W1 + b1   (e.dff now holds d ff_pre)
@@ -607,7 +683,7 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
         // ---- attention output projection:  x_mid = x + attn @ Wo
         TRY(ready(l, 2));                                                   // d x_mid exists
         TRY(gemm(e, st, BT, D, D, dx, D, 0, e.P(s.Wo), D, 1, e.dattn, D));
-        TRY(gemm(e, ws, D, D, BT, a.attn, D, 1, dx, D, 0, e.G(s.Wo), D, accumulate));
+        TRY(gemm(e, ws2, D, D, BT, a.attn, D, 1, dx, D, 0, e.G(s.Wo), D, accumulate));
         TRY(done(l, 2));
         emit();
         // ---- attention
@@ -640,9 +716,7 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
             TRY(gemm(e, st, BT, D, 3 * D, e.dqkv, 3 * D, 0, e.P(s.Wqkv), 3 * D, 1, e.dln, D));
             TRY(gemm(e, ws, D, 3 * D, BT, a.ln1, D, 1, e.dqkv, 3 * D, 0, e.G(s.Wqkv), 3 * D, accumulate));
         } else {
-            const long long pl = (long long)BT * D * e.es, wm = (long long)D * D * e.es;
-            for (int i = 0; i < 3; ++i)
-                TRY(gemm(e, st, BT, D, D, e.dqkv + i * pl, D, 0, e.P(s.Wq) + i * wm, D, 1, e.dln, D, i > 0));
+            TRY(gemm_planes(e, st, BT, D, D, e.dqkv, D, (long long)BT * D, e.P(s.Wq), D, (long long)D * D, e.dln, D));
             TRY(gemm(e, ws, D, D, BT, a.ln1, D, 1, e.dqkv, D, 0, e.G(s.Wq), D, accumulate, nullptr, 0, nullptr, 0,
                      nullptr, 0, nullptr, 0, 3, 0, (long long)BT * D, (long long)D * D));
         }
@@ -661,6 +735,10 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
         cudaEvent_t fin = evt(d.L, 5);
         CME_CUDA(cudaEventRecord(fin, ws));
         CME_CUDA(cudaStreamWaitEvent(st, fin, 0));
+        if (ws2 != ws) {                                    // (the loss published there does not hold the scatter up)
+            CME_CUDA(cudaStreamWaitEvent(st, evt(0, 4), 0));
+            CME_CUDA(cudaStreamWaitEvent(st, evt(0, 6), 0));
+        }
     }
     // the two tables are independent: the position table's sums run on the second stream beside the token scatter,
     // and join before the last bucket is handed over
@@ -675,6 +753,11 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
     } else {
         TRY(cme_embedding_bwd(dt, tokens, dx, e.G(e.gs.tok), nullptr, BT, d.T, D, V, (d.tied || accumulate) ? 1 : 0, st));
         TRY(cme_embedding_bwd(dt, tokens, dx, nullptr, e.G(e.gs.pos), BT, d.T, D, V, accumulate, st));
+    }
+    if (e.loss_pending) {
+        CME_CUDA(cudaEventRecord(e.ev_aux[3], e.side2));
+        CME_CUDA(cudaStreamWaitEvent(st, e.ev_aux[3], 0));
+        e.loss_pending = false;
     }
     emit();
     return CME_OK;

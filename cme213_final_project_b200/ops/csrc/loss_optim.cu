@@ -327,7 +327,10 @@ __global__ void __launch_bounds__(256) normsq_partial_vec_kernel(const T* __rest
     if (threadIdx.x == 0) partial[blockIdx.x] = t;
 }
 
-__global__ void step_inc_kernel(int* step) { *step += 1; }
+__global__ void step_inc_kernel(int* step) {
+    pdl_wait();
+    *step += 1;
+}
 
 struct AdamArgs {
     float* master; __nv_bfloat16* compute; const void* grads; float* m; float* v;
@@ -360,6 +363,7 @@ __device__ __forceinline__ void adam_moments(const AdamArgs& a, float g, float& 
 
 template <typename TG>
 __global__ void __launch_bounds__(256) adam_kernel(const AdamArgs a) {
+    pdl_wait();
     const int t = *a.step;
     const float lr = *a.lr;
     const float bc1 = 1.f - powf(a.beta1, (float)t), bc2 = 1.f - powf(a.beta2, (float)t);
@@ -392,6 +396,7 @@ constexpr int ADAM_LIST = 512;             // ranges that a block keeps in share
 // 6.54 TB/s copy (574 and 575 us with accesses marked as streaming, which pay at 10 M only, 46 for 49 us).
 template <typename TG, bool RANGES>
 __global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
+    pdl_wait();
     const int t = *a.step;
     const float lr = *a.lr;
     const float bc1 = 1.f - powf(a.beta1, (float)t), bc2 = 1.f - powf(a.beta2, (float)t);
@@ -475,6 +480,15 @@ __global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
 
 }  // namespace
 
+// *loss_out (+)= loss_weight * mean(losses).
+CME_API int cme_loss_mean(const float* losses, int rows, float loss_weight, float* loss_out, int accumulate_loss, void* stream) {
+    CME_REQUIRE(rows > 0, CME_ERR_SHAPE, "loss_mean: empty input");
+    CME_CUDA(cme_launch_dependent(reduce_scalar_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, losses, rows,
+                                  loss_weight / (float)rows, loss_out, accumulate_loss));
+    CME_LAUNCH_CHECK();
+    return CME_OK;
+}
+
 // Per-row loss and gradient, then *loss_out (+)= loss_weight * mean(losses).
 // prob_eps > 0 selects the reference's form  -log(p + eps), p = e / (sum + eps);  0 the exact log-softmax.
 CME_API int cme_cross_entropy(int dtype, const void* logits, const int* targets, void* dlogits, float* losses,
@@ -511,12 +525,7 @@ CME_API int cme_cross_entropy(int dtype, const void* logits, const int* targets,
         cross_entropy_kernel<float><<<rows, CE_THREADS, 0, st>>>((const float*)logits, targets, (float*)dlogits, losses,
                                                                  V, ld, grad_scale, prob_eps);
     CME_LAUNCH_CHECK();
-    if (loss_out) {
-        CME_CUDA(cme_launch_dependent(reduce_scalar_kernel, dim3(1), dim3(1024), 0, st, (const float*)losses, rows,
-                                      loss_weight / (float)rows, loss_out, accumulate_loss));
-        CME_LAUNCH_CHECK();
-    }
-    return CME_OK;
+    return loss_out ? cme_loss_mean(losses, rows, loss_weight, loss_out, accumulate_loss, stream) : CME_OK;
 }
 
 // *out = sum(g^2) over n elements; `partial` holds 1024 floats.
@@ -564,7 +573,7 @@ CME_API int cme_publish_loss(const float* loss, int* seq, void* host_loss_dev, v
 }
 
 CME_API int cme_step_inc(int* step, void* stream) {
-    step_inc_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(step);
+    CME_CUDA(cme_launch_dependent(step_inc_kernel, dim3(1), dim3(1), 0, (cudaStream_t)stream, step));
     CME_LAUNCH_CHECK();
     return CME_OK;
 }
@@ -592,9 +601,11 @@ CME_API int cme_adam(int grad_dtype, float* master, void* compute_bf16, const vo
         auto kernel = grad_dtype != CME_BF16 ? (ranges ? adam_vec4_kernel<float, true> : adam_vec4_kernel<float, false>)
                       : ranges               ? adam_vec4_kernel<__nv_bfloat16, true>
                                              : adam_vec4_kernel<__nv_bfloat16, false>;
-        kernel<<<(int)blocks, 256, 0, st>>>(a);
-    } else if (grad_dtype == CME_BF16) adam_kernel<__nv_bfloat16><<<(int)blocks, 256, 0, st>>>(a);
-    else adam_kernel<float><<<(int)blocks, 256, 0, st>>>(a);
+        CME_CUDA(cme_launch_dependent(kernel, dim3((int)blocks), dim3(256), 0, st, a));
+    } else {
+        CME_CUDA(cme_launch_dependent(grad_dtype == CME_BF16 ? adam_kernel<__nv_bfloat16> : adam_kernel<float>,
+                                      dim3((int)blocks), dim3(256), 0, st, a));
+    }
     CME_LAUNCH_CHECK();
     return CME_OK;
 }

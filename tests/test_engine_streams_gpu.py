@@ -1,0 +1,59 @@
+"""The engine's extra streams (weight gradients, mean loss, padded output weights) against the same step on one stream, and the
+one reduction over the planes of dQ, dK, dV at inner sizes that end inside a block of 64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(hidden, batch, overlap):
+    from cme213_final_project_b200.config import ModelConfig, OptimConfig, RunConfig
+    from cme213_final_project_b200.models.engine import NativeEngine
+    # GELU: no pre-activation that rounding takes across zero switches a gradient on or off
+    cfg = ModelConfig(vocab_size=65, seq_len=32, hidden=hidden, heads=4, ff=2 * hidden, batch_size=batch, activation="gelu")
+    eng = NativeEngine(cfg, OptimConfig(), RunConfig(), device="cuda", seed=3)
+    eng.set_overlap(overlap)
+    # weights of the size that keeps a layer's output at its input's: with the small uniform start the softmax is flat, and
+    # what reaches d ln1 through it is a difference of nearly equal sums, all rounding
+    g = torch.Generator().manual_seed(7)
+    flat = torch.zeros(eng.layout.total)
+    for s in eng.layout.specs:
+        v = torch.randn(s.numel, generator=g) * {"weight": hidden ** -0.5, "embed": 1.0}.get(s.kind, 0.1)
+        flat[s.offset:s.offset + s.numel] = v + (1.0 if s.kind == "ln_gamma" else 0.0)
+    eng.set_params(flat.to(torch.bfloat16).float())
+    return eng, cfg
+
+
+def _batches(cfg, n):
+    g = torch.Generator().manual_seed(5)
+    draw = lambda: torch.randint(0, 65, (cfg.tokens_per_step,), generator=g, dtype=torch.int32).cuda()      # noqa: E731
+    return [draw() for _ in range(n)], [draw() for _ in range(n)]
+
+
+@pytest.mark.parametrize("micro", [1, 3])
+@pytest.mark.parametrize("hidden", [32, 64, 96, 200, 256])
+def test_streams_and_planes_give_the_step_of_one_stream(hidden, micro):
+    from cme213_final_project_b200.config import OptimConfig
+    from cme213_final_project_b200.models.reference import ReferenceModel
+    runs = []
+    for overlap in (False, True, True):
+        eng, cfg = _engine(hidden, 8, overlap)
+        xs, ys = _batches(cfg, micro)
+        for _ in range(3):
+            eng.train_step(xs, ys)
+        runs.append((eng.grads.clone(), eng.loss_dev.clone()))
+    for g, loss in runs[1:]:
+        assert torch.equal(g, runs[0][0]) and torch.equal(loss, runs[0][1])
+    ref = ReferenceModel(cfg, OptimConfig(), device="cpu", dtype=torch.float64, seed=3, layout=eng.layout)
+    ref.params.data.copy_(eng.master.cpu())
+    want = torch.zeros(eng.layout.total, dtype=torch.float64)
+    for x, y in zip(xs, ys):
+        ref.zero_grad()
+        ref.forward(x.cpu(), y.cpu())
+        ref.backward()
+        want += ref.grads.double() / micro
+    for name in ("ln1_gamma", "ln1_beta", "tok_embed", "pos_embed"):          # what d ln1 goes into
+        s = eng.layout.by_name[name]
+        sl = slice(s.offset, s.offset + s.numel)
+        # a handful of bf16 roundings (2^-9 each) of values that enter as sums of the same size
+        assert ((eng.grads[sl].cpu().double() - want[sl]).norm() / want[sl].norm()).item() < 3e-2
