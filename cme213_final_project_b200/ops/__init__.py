@@ -2,7 +2,8 @@
 
 The library has a plain C ABI (pointers, sizes, a stream handle) and is loaded with ``ctypes``; every
 wrapper here takes ``torch`` tensors, checks them, passes ``data_ptr()`` and the current CUDA stream, and
-raises :class:`NativeError` with the library's message when a call fails.  There is no PyTorch fallback
+raises :class:`NativeError` with the library's message when a call fails.  The wrappers of the short operations do these
+steps in a compiled module (``csrc/wrappers.cpp``): their calls are bound by the host.  There is no PyTorch fallback
 behind these functions: on a GPU machine a missing library is an error, not a silent slow path.
 
 The op list mirrors the reference's kernel header (``FINAL_CLEAN_CODE_/include/kernels.h:6-138``).
@@ -56,8 +57,12 @@ _PROTOTYPES = {
     "cme_colsum_splits": "ii", "cme_dact_colsum": "ivvvvviiiiv", "cme_scale": "ivlfv", "cme_cast": "ivivlv",
     "cme_add": "ivvvlv", "cme_relu_bwd": "ivvvlv", "cme_init_uniform": "ivlfuv", "cme_embedding_fwd": "ivvvviiiiv",
     "cme_embedding_bwd": "ivvvviiiiiv", "cme_cross_entropy": "ivvvvviilfffiv", "cme_grad_normsq": "ivlvvv",
-    "cme_adam": "ivvvvvlvvvffffffviv", "cme_attention_fwd": "viv", "cme_attention_bwd": "viv",
+    "cme_adam": "ivvvvvlvvvffffffviv", "cme_attention_fwd": "viv", "cme_attention_bwd": "viv", "cme_attention_path": "vii",
 }
+# Entry points that the compiled wrappers call.
+_WRAPPED = ("cme_last_error", "cme_cross_entropy", "cme_attention_fwd", "cme_attention_bwd", "cme_attention_path",
+            "cme_attention_gemm_ws_bytes", "cme_layernorm_fwd", "cme_layernorm_bwd_blocks", "cme_layernorm_bwd",
+            "cme_bias_act_residual", "cme_colsum_splits", "cme_dact_colsum", "cme_embedding_fwd", "cme_embedding_bwd")
 _CTYPES = {"v": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float, "u": ctypes.c_uint}
 
 
@@ -92,6 +97,23 @@ def lib() -> ctypes.CDLL:
     if l is None:
         raise NativeError(f"native library not found at {LIB_PATH}; run `python -m cme213_final_project_b200.ops.build`")
     return l
+
+
+_wrappers_bound = None
+
+
+def _native():
+    """The compiled wrappers, calling the library that :func:`lib` has loaded."""
+    global _wrappers_bound
+    if _wrappers_bound is None:
+        l = lib()
+        try:
+            from . import _wrappers
+        except ImportError as e:
+            raise NativeError(f"compiled wrappers not usable ({e}); run `python -m cme213_final_project_b200.ops.build`") from e
+        _wrappers.bind(NativeError, {n: ctypes.cast(getattr(l, n), ctypes.c_void_p).value for n in _WRAPPED})
+        _wrappers_bound = _wrappers
+    return _wrappers_bound
 
 
 def available() -> bool:
@@ -238,29 +260,12 @@ def gemm_check_status() -> int:
 def layernorm_fwd(x, gamma, beta, eps: float = 1e-5, residual=None, save_sum: bool = False):
     """``y = LN(x [+ residual])``.  Returns ``(y, mean, rstd, summed)`` where ``summed`` is
     ``x + residual`` when ``save_sum`` (the fused residual + LayerNorm forward) else ``None``."""
-    _cuda(x, gamma, beta, residual)
-    rows, D = x.numel() // x.shape[-1], x.shape[-1]
-    y = torch.empty_like(x)
-    mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-    rstd = torch.empty_like(mean)
-    r = torch.empty_like(x) if (save_sum and residual is not None) else None
-    _check(lib().cme_layernorm_fwd(_dt(x), _a(x), _a(residual), _a(r), _a(gamma), _a(beta), _a(y), _a(mean), _a(rstd),
-                                   rows, D, eps, _st()))
-    return y, mean, rstd, r
+    return _native().layernorm_fwd(x, gamma, beta, eps, residual, save_sum)
 
 
 def layernorm_bwd(dy, x, gamma, mean, rstd, dres=None, dgamma=None, dbeta=None, accumulate: bool = False):
     """Returns ``(dx, dgamma, dbeta)``; ``dx`` includes ``+ dres`` when given (fused residual-gradient add)."""
-    _cuda(dy, x, gamma, mean, rstd, dres, dgamma, dbeta)
-    rows, D = x.numel() // x.shape[-1], x.shape[-1]
-    dx = torch.empty_like(x)
-    if dgamma is None:
-        dgamma, dbeta, accumulate = torch.empty_like(gamma), torch.empty_like(gamma), False
-    nb = lib().cme_layernorm_bwd_blocks(rows)
-    scratch = torch.empty(nb * 2 * D, dtype=torch.float32, device=x.device)
-    _check(lib().cme_layernorm_bwd(_dt(x), _a(dy), _a(x), _a(gamma), _a(mean), _a(rstd), _a(dres), _a(dx), _a(dgamma),
-                                   _a(dbeta), _a(scratch), rows, D, int(accumulate), _st()))
-    return dx, dgamma, dbeta
+    return _native().layernorm_bwd(dy, x, gamma, mean, rstd, dres, dgamma, dbeta, accumulate)
 
 
 # --------------------------------------------------------------------------------------------------
@@ -268,28 +273,12 @@ def layernorm_bwd(dy, x, gamma, mean, rstd, dres=None, dgamma=None, dbeta=None, 
 # --------------------------------------------------------------------------------------------------
 def bias_act_residual(x, bias=None, act=None, residual=None, save_pre: bool = False):
     """``out = act(x + bias) + residual``; returns ``(out, pre)`` with ``pre = x + bias`` if ``save_pre``."""
-    _cuda(x, bias, residual)
-    cols = x.shape[-1]
-    rows = x.numel() // cols
-    out = torch.empty_like(x)
-    pre = torch.empty_like(x) if save_pre else None
-    _check(lib().cme_bias_act_residual(_dt(x), _a(x), _a(bias), _a(residual), _a(pre), _a(out), rows, cols, ACT[act],
-                                       _st()))
-    return out, pre
+    return _native().bias_act_residual(x, bias, ACT[act], residual, save_pre)
 
 
 def dact_colsum(dout, pre=None, act=None, want_g: bool = True, dbias=None, accumulate: bool = False):
     """``g = dout * act'(pre)`` and ``dbias (+)= g.sum(0)`` — the fused activation-backward + bias-backward."""
-    _cuda(dout, pre, dbias)
-    cols = dout.shape[-1]
-    rows = dout.numel() // cols
-    g = torch.empty_like(dout) if (want_g and pre is not None) else None
-    if dbias is None:
-        dbias, accumulate = torch.empty(cols, dtype=dout.dtype, device=dout.device), False
-    scratch = torch.empty(lib().cme_colsum_splits(rows, cols) * cols, dtype=torch.float32, device=dout.device)
-    _check(lib().cme_dact_colsum(_dt(dout), _a(dout), _a(pre), _a(g), _a(dbias), _a(scratch), rows, cols, ACT[act],
-                                 int(accumulate), _st()))
-    return g, dbias
+    return _native().dact_colsum(dout, pre, ACT[act], want_g, dbias, accumulate)
 
 
 def scale_(x, s: float):
@@ -329,22 +318,11 @@ def init_uniform_(out, scale: float, seed: int):
 # Embedding
 # --------------------------------------------------------------------------------------------------
 def embedding_fwd(tokens, tok, pos):
-    _cuda(tokens, tok, pos)
-    BT, (V, D), T = tokens.numel(), tok.shape, pos.shape[0]
-    out = torch.empty(BT, D, dtype=tok.dtype, device=tok.device)
-    _check(lib().cme_embedding_fwd(_dt(tok), _a(tokens), _a(tok), _a(pos), _a(out), BT, T, D, V, _st()))
-    return out
+    return _native().embedding_fwd(tokens, tok, pos)
 
 
 def embedding_bwd(tokens, dout, V: int, T: int, dtok=None, dpos=None, accumulate: bool = False):
-    _cuda(tokens, dout, dtok, dpos)
-    BT, D = dout.shape
-    if dtok is None:
-        dtok, dpos, accumulate = (torch.empty(V, D, dtype=dout.dtype, device=dout.device),
-                                  torch.empty(T, D, dtype=dout.dtype, device=dout.device), False)
-    _check(lib().cme_embedding_bwd(_dt(dout), _a(tokens), _a(dout), _a(dtok), _a(dpos), BT, T, D, V, int(accumulate),
-                                   _st()))
-    return dtok, dpos
+    return _native().embedding_bwd(tokens, dout, V, T, dtok, dpos, accumulate)
 
 
 # --------------------------------------------------------------------------------------------------
@@ -353,15 +331,7 @@ def embedding_bwd(tokens, dout, V: int, T: int, dtok=None, dpos=None, accumulate
 def cross_entropy(logits, targets, grad_scale: Optional[float] = None, prob_eps: float = 0.0, inplace: bool = False):
     """Returns ``(mean loss [1] fp32, dlogits, per-row losses)``; ``dlogits = (softmax - onehot) * grad_scale``
     (default ``1/rows``).  ``prob_eps = 1e-9`` reproduces the reference's ``-log(p + 1e-9)`` form."""
-    _cuda(logits, targets)
-    rows, V = logits.shape
-    dl = logits if inplace else torch.empty_like(logits)
-    losses = torch.empty(rows, dtype=torch.float32, device=logits.device)
-    loss = torch.empty(1, dtype=torch.float32, device=logits.device)
-    gs = 1.0 / rows if grad_scale is None else grad_scale
-    _check(lib().cme_cross_entropy(_dt(logits), _a(logits), _a(targets), _a(dl), _a(losses), _a(loss), rows, V,
-                                   V, gs, prob_eps, 1.0, 0, _st()))
-    return loss, dl, losses
+    return _native().cross_entropy(logits, targets, grad_scale, prob_eps, inplace)
 
 
 def grad_normsq(g):
@@ -422,13 +392,7 @@ def attention_fwd(q, k, v, B: int, H: int, T: int, layout: str = "split", causal
                   backend: str = "auto"):
     """``q, k, v``: ``[B*T, D]``.  ``layout="flat"`` views each as ``[B*H, T, HD]`` without a transpose (the
     reference's head layout); ``"split"`` is the standard ``[B, T, H, HD]`` split.  Returns ``(out, lse)``."""
-    _cuda(q, k, v)
-    a = _attn_desc(q, B, H, T, layout, causal)
-    out = torch.empty_like(q)
-    lse = torch.empty(B * H * T, dtype=torch.float32, device=q.device)
-    a.q, a.k, a.v, a.o, a.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr()
-    _check(lib().cme_attention_fwd(ctypes.byref(a), _BACKENDS[backend], _st()))
-    return out, lse
+    return _native().attention_fwd(q, k, v, B, H, T, layout == "flat", int(causal), _BACKENDS[backend])
 
 
 def attention_bwd(q, k, v, out, lse, dout, B: int, H: int, T: int, layout: str = "split", causal: bool = False,
@@ -441,25 +405,11 @@ def attention_bwd(q, k, v, out, lse, dout, B: int, H: int, T: int, layout: str =
     large shapes).  ``scratch`` = (fp32 tensor of ``q.numel()``
     zeros, int32 tensor of ``B * H * ceil(T / 128)`` zeros) lets calls share the buffers; modes 1 and 2 leave both
     zero again."""
-    _cuda(q, k, v, out, lse, dout)
-    a = _attn_desc(q, B, H, T, layout, causal)
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    delta = torch.empty_like(lse)
     if dq_mode is None:
         dq_mode = 1 if ordered_dq else 0
-    if scratch is not None:
-        acc, sem = scratch
-    else:
-        # mode 0 clears the scratch itself and counts nothing; the other modes start from zeros
-        make = torch.zeros if dq_mode else torch.empty
-        acc = make(q.numel(), dtype=torch.float32, device=q.device)
-        sem = make(B * H * ((T + 127) // 128), dtype=torch.int32, device=q.device)
-    a.q, a.k, a.v, a.o, a.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr()
-    a.d_o, a.dq, a.dk, a.dv = dout.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    a.delta, a.dq_accum = delta.data_ptr(), acc.data_ptr()
-    a.dq_sem, a.dq_mode = sem.data_ptr(), int(dq_mode)
-    _check(lib().cme_attention_bwd(ctypes.byref(a), _BACKENDS[backend], _st()))
-    return dq, dk, dv
+    acc, sem = (None, None) if scratch is None else scratch
+    return _native().attention_bwd(q, k, v, out, lse, dout, B, H, T, layout == "flat", int(causal), _BACKENDS[backend], int(dq_mode),
+                                   acc, sem)
 
 
 def launch_count() -> int:

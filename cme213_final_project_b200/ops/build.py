@@ -4,7 +4,8 @@ shared object with a C ABI (``libcme213_b200.so`` next to this file).
 The reference builds with a Makefile (``FINAL_CLEAN_CODE_/Makefile``: ``-arch=sm_75``, every source through
 ``nvcc``, separate object files, per-thread default stream).  Here: one arch (``sm_100a``), objects cached
 by source hash under ``build/`` next to the sources, parallel compile, no link-time dependency on the
-driver library (the tensor-map encoder is looked up at run time).
+driver library (the tensor-map encoder is looked up at run time).  The compiled Python wrappers (``csrc/wrappers.cpp``) become
+a module of their own (``_wrappers.so``), against torch's headers.
 """
 from __future__ import annotations
 
@@ -20,6 +21,7 @@ from typing import List
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OUT = HERE / "libcme213_b200.so"
+WRAPPERS = HERE / "_wrappers.so"
 BUILD = HERE / "build"
 
 NVCC_FLAGS = [
@@ -41,6 +43,31 @@ def _digest(src: Path, headers: List[Path]) -> str:
     for p in [src] + headers:
         h.update(p.read_bytes())
     return h.hexdigest()[:16]
+
+
+def _build_wrappers(verbose: bool, force: bool) -> None:
+    """The extension module, rebuilt when its sources, this Python or torch change."""
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    src, key = CSRC / "wrappers.cpp", BUILD / "wrappers.key"
+    h = hashlib.sha256(f"{sys.version} {torch.__version__}".encode())
+    for p in (src, CSRC / "attention_desc.h"):
+        h.update(p.read_bytes())
+    if not force and WRAPPERS.exists() and key.exists() and key.read_text() == h.hexdigest():
+        return
+    cuda = Path(_nvcc()).resolve().parent.parent / "include"
+    cmd = [os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", str(root / "include"),
+           "-I", str(root / "include/torch/csrc/api/include"), "-I", str(cuda), "-I", sysconfig.get_paths()["include"], str(src),
+           "-o", str(WRAPPERS), "-L", str(root / "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"compiling wrappers.cpp failed:\n{r.stdout}\n{r.stderr}")
+    key.write_text(h.hexdigest())
+    if verbose:
+        print(f"[build] built {WRAPPERS}", file=sys.stderr)
 
 
 def build(verbose: bool = False, force: bool = False) -> Path:
@@ -81,6 +108,7 @@ def build(verbose: bool = False, force: bool = False) -> Path:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
         if verbose:
             print(f"[build] linked {OUT}", file=sys.stderr)
+    _build_wrappers(verbose, force)
     return OUT
 
 

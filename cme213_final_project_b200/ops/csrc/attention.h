@@ -10,35 +10,7 @@
 // strides (osb, osh, ost), because a fused [B*T, 3D] projection buffer has a different row pitch than O.
 #pragma once
 #include "common.h"
-
-struct CmeAttn {
-    int nb, nh, T, HD;
-    long long sb, sh, st;        // strides of Q / K / V / dQ / dK / dV
-    long long osb, osh, ost;     // strides of O / dO
-    int causal;
-    float scale;                 // 1 / sqrt(HD)
-    int dtype;                   // CME_BF16 or CME_F32
-    const void* q; const void* k; const void* v;
-    void* o;                     // forward output / backward input
-    float* lse;                  // [nb*nh, T] log-sum-exp of scaled scores (saved by forward)
-    // backward only
-    const void* d_o; void* dq; void* dk; void* dv;
-    float* delta;                // [nb*nh, T] scratch: rowsum(dO * O)
-    float* dq_accum;             // fp32 scratch [nb*nh*T*HD] for the tcgen05 backward (may be null)
-    void* ws; long long ws_bytes;    // scratch of attention_gemm_ws_bytes() for the batched-GEMM path (may be null)
-    int* dq_sem;                 // [nb*nh * ceil(T / 128)] ints, zero before the first launch (the kernel leaves them zero);
-                                 // needed by dq_mode 1 and 2
-    int dq_mode;                 // how the tcgen05 backward completes dQ from the key blocks' parts:
-                                 //   0  the launch clears dq_accum, the parts are added in arrival order, a second kernel
-                                 //      scales and casts the sums
-                                 //   1  the parts are added in a fixed order (bit-reproducible); key block 0 finishes
-                                 //   2  arrival order; the CTA whose part comes last scales, casts and writes zeros back:
-                                 //      dq_accum must be zero before the first launch and is zero after every launch
-    int dq_accum_clean;          // dq_mode 0: non-zero = the caller has cleared dq_accum itself (e.g. on another stream,
-                                 // ahead of time); the launch then skips its own clear
-};
-
-constexpr int CME_ATTN_FINISH_MAX_QBLOCKS = 64;      // dq_mode 2: query blocks (of 128 rows) per sequence
+#include "attention_desc.h"
 
 int attention_simt_fwd(const CmeAttn* a, cudaStream_t st);
 int attention_simt_bwd(const CmeAttn* a, cudaStream_t st);

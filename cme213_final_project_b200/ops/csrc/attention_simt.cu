@@ -524,28 +524,41 @@ int attention_takes_short(const CmeAttn* a, int bwd) {
 
 // backend: 0 auto (one-launch kernel up to 64 tokens, else fused tensor-core kernel, else batched-GEMM path, else SIMT),
 //          1 fused tensor-core only, 2 SIMT only, 3 batched-GEMM path only
+// The path of a call with that backend (CmeAttnPath).
+CME_API int cme_attention_path(const CmeAttn* a, int backend, int bwd) {
+    if (backend == 0 && attention_takes_short(a, bwd)) return CME_ATTN_PATH_SHORT;
+    if ((backend == 0 || backend == 1) && attention_tc_supported(a)) return CME_ATTN_PATH_TC;
+    if ((backend == 0 || backend == 3) && attention_gemm_supported(a)) return CME_ATTN_PATH_GEMM;
+    return CME_ATTN_PATH_SIMT;
+}
+static int check_path(int backend, int path) {
+    CME_REQUIRE(backend != 1 || path == CME_ATTN_PATH_TC, CME_ERR_SHAPE, "attention shape not supported by the tensor-core kernel");
+    CME_REQUIRE(backend != 3 || path == CME_ATTN_PATH_GEMM, CME_ERR_SHAPE, "attention shape not supported by the batched-GEMM path");
+    return CME_OK;
+}
 CME_API int cme_attention_fwd(const CmeAttn* a, int backend, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
-    if (backend == 0 && attention_takes_short(a, 0)) return attention_short_fwd(a, st);
-    if ((backend == 0 || backend == 1) && attention_tc_supported(a)) return attention_tc_fwd(a, st);
-    CME_REQUIRE(backend != 1, CME_ERR_SHAPE, "attention shape not supported by the tensor-core kernel");
-    if ((backend == 0 || backend == 3) && attention_gemm_supported(a)) return attention_gemm_fwd(a, st);
-    CME_REQUIRE(backend != 3, CME_ERR_SHAPE, "attention shape not supported by the batched-GEMM path");
-    return attention_simt_fwd(a, st);
+    const int path = cme_attention_path(a, backend, 0), rc = check_path(backend, path);
+    if (rc) return rc;
+    switch (path) {
+        case CME_ATTN_PATH_SHORT: return attention_short_fwd(a, st);
+        case CME_ATTN_PATH_TC: return attention_tc_fwd(a, st);
+        case CME_ATTN_PATH_GEMM: return attention_gemm_fwd(a, st);
+        default: return attention_simt_fwd(a, st);
+    }
 }
 CME_API int cme_attention_bwd(const CmeAttn* a, int backend, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
-    if (backend == 0 && attention_takes_short(a, 1)) {
-        if (attention_tc_supported(a)) {           // the same calls are refused as without this kernel
-            const int rc = attention_tc_check_bwd(a);
-            if (rc) return rc;
-        }
-        return attention_short_bwd(a, st);
+    const int path = cme_attention_path(a, backend, 1);
+    int rc = check_path(backend, path);
+    // the same calls are refused as without the one-launch kernel
+    if (!rc && path == CME_ATTN_PATH_SHORT && attention_tc_supported(a)) rc = attention_tc_check_bwd(a);
+    if (rc) return rc;
+    switch (path) {
+        case CME_ATTN_PATH_SHORT: return attention_short_bwd(a, st);
+        case CME_ATTN_PATH_TC: return attention_tc_bwd(a, st);
+        case CME_ATTN_PATH_GEMM: return attention_gemm_bwd(a, st);
+        default: return attention_simt_bwd(a, st);
     }
-    if ((backend == 0 || backend == 1) && attention_tc_supported(a)) return attention_tc_bwd(a, st);
-    CME_REQUIRE(backend != 1, CME_ERR_SHAPE, "attention shape not supported by the tensor-core kernel");
-    if ((backend == 0 || backend == 3) && attention_gemm_supported(a)) return attention_gemm_bwd(a, st);
-    CME_REQUIRE(backend != 3, CME_ERR_SHAPE, "attention shape not supported by the batched-GEMM path");
-    return attention_simt_bwd(a, st);
 }
 CME_API long long cme_attention_gemm_ws_bytes(int nb, int T) { return attention_gemm_ws_bytes(nb, T); }
