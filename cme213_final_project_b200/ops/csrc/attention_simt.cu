@@ -12,15 +12,15 @@ namespace {
 
 // What bounds these kernels is the fp32 multiply-add rate and, next to it, shared-memory reads: a 16-byte load per lane
 // takes the SM's shared memory four clocks, in which its schedulers issue sixteen multiply-adds.  So every product is
-// register-tiled.  Forward: a warp owns 16 whole rows, a lane 4 of them (ty + 4 i) and every eighth streamed row
-// (tx + 8 j), or 4 consecutive columns in 32 (tx * 4 + 32 g): 12 loads for 128 multiply-adds in a 4-deep step (two loads
-// per multiply-add without tiles, 10 for 64 with 2 rows per lane), the softmax needs shuffles among 8 lanes only
-// and P never crosses a warp.  Backward: the warps form 4 groups of 16 rows x 2 halves -- of the streamed rows in the
-// score products, of the head's columns in the others -- so that a lane's 4-row tiles of two outputs fit its registers.
-// No load has a bank conflict, since a row's pitch is an odd number of 16-byte words.
+// register-tiled.  The warps form groups of 16 rows x 2 halves -- of the streamed rows in the score products, of the head's
+// columns in the others; a lane has 4 of the rows (ty + 4 i) and every eighth streamed row of its half (tx + 8 j), or VW
+// consecutive columns in 8 VW, so that a lane's 4-row tiles of two outputs fit its registers.  No load has a bank conflict,
+// since a row's pitch is an odd number of 16-byte words.  Multiply-adds are packed pairs, fp32 tiles arrive by asynchronous
+// copies, all of a block's at once, the ones that the second product needs under the first.
 // The head size is padded with zeros to a multiple of 32 (template G = ceil(HD / 32)).
-// 32 x 4 heads x 64 tokens x head size 128, fp32, forward + backward call: 297 us without tiles, 58 us
-// with 2 rows per lane, 52 us with 4 (its floor at the fp32 rate, 0.94 GFLOP at 74 TFLOP/s, is 13 us).
+// 32 x 4 heads x 64 tokens x head size 128, fp32, forward + backward: 13 + 27.6 us, 18 + 31 us with a warp for whole rows of the
+// forward, single multiply-adds and tiles loaded through registers one after the other (floor of both at the fp32 rate, 0.94 GFLOP
+// at 74 TFLOP/s: 13 us).  64 query rows a block instead of 32 in the forward: 12.8 us, no different.
 constexpr int CT = 64;               // rows streamed per step
 constexpr int WR = 16;               // rows a warp owns
 constexpr int LR = WR / 4;           // rows a lane has of them
@@ -51,11 +51,10 @@ template <> __device__ __forceinline__ void st4<__nv_bfloat16>(__nv_bfloat16* p,
     *reinterpret_cast<uint2*>(p) = make_uint2(f2_to_bf2(v[0], v[1]), f2_to_bf2(v[2], v[3]));
 }
 
-// Rows [r0, r0 + NR) of a [T_, HD] operand to shared memory as fp32 times `mul`, zeros beyond T_ and HD.  `vec`: every
+// Rows [r0, r0 + NR) of a [T_, HD] operand to shared memory as fp32, zeros beyond T_ and HD.  `vec`: every
 // row starts on a boundary of four elements and HD is a multiple of four.
 template <typename T, int G, int NR, int NT>
-__device__ __forceinline__ void load_rows(float* dst, const T* src, long long st, int r0, int T_, int HD, float mul,
-                                          bool vec) {
+__device__ __forceinline__ void load_rows(float* dst, const T* src, long long st, int r0, int T_, int HD, bool vec) {
     static_assert(NR * 8 * G % NT == 0, "whole rounds");
 #pragma unroll 8
     for (int k = 0; k < NR * 8 * G / NT; ++k) {
@@ -71,16 +70,44 @@ __device__ __forceinline__ void load_rows(float* dst, const T* src, long long st
                 if (c + 2 < HD) v.z = to_f32<T>(p[2]);
                 if (c + 3 < HD) v.w = to_f32<T>(p[3]);
             }
-            v.x *= mul; v.y *= mul; v.z *= mul; v.w *= mul;
         }
         *reinterpret_cast<float4*>(dst + r * Pitch<G>::P + c) = v;
     }
 }
 
-// s[i][j] += A[ty + 4 i] . B[tx + 8 j]
+// The same as they are, fp32 in whole 16-byte words by asynchronous copies: all of a block's tiles are on their way at once,
+// where the registers of a thread hold eight words (80 rounds of its loads for the forward's 80 KB and 64 threads).  Other
+// types and alignments are loaded at once.  Complete after copies_wait by every thread and a barrier.
+template <typename T, int G, int NR, int NT>
+__device__ __forceinline__ void copy_rows(float* dst, const T* src, long long st, int r0, int T_, int HD, bool vec) {
+    if (sizeof(T) == 4 && vec) {
+        const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+#pragma unroll
+        for (int k = 0; k < NR * 8 * G / NT; ++k) {
+            const int i = threadIdx.x + k * NT, r = i / (8 * G), c = (i % (8 * G)) * 4;
+            const bool in = r0 + r < T_ && c < HD;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + (uint32_t)(r * Pitch<G>::P + c) * 4u),
+                         "l"(in ? src + (long long)(r0 + r) * st + c : src), "r"(in ? 16 : 0)
+                         : "memory");
+        }
+    } else {
+        load_rows<T, G, NR, NT>(dst, src, st, r0, T_, HD, vec);
+    }
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// All but the last N committed groups of this thread have arrived.
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// s[i][j] = A[ty + 4 i] . B[tx + 8 j].  Packed pairs: the even and the odd elements are summed apart, two multiply-adds per
+// instruction, so that a scheduler with one or two warps has issue slots left for their loads.
 template <int G, int NJ>
 __device__ __forceinline__ void dot_rows(const float* A, const float* B, int ty, int tx, float (&s)[LR][NJ]) {
     constexpr int P = Pitch<G>::P;
+    F32x2 t[LR][NJ];
+#pragma unroll
+    for (int i = 0; i < LR; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) t[i][j] = f2_splat(0.f);
 #pragma unroll 2
     for (int d = 0; d < 32 * G; d += 4) {
         float4 a[LR];
@@ -91,7 +118,17 @@ __device__ __forceinline__ void dot_rows(const float* A, const float* B, int ty,
             const float4 b = *reinterpret_cast<const float4*>(B + (tx + 8 * j) * P + d);
 #pragma unroll
             for (int i = 0; i < LR; ++i)
-                s[i][j] = fmaf(a[i].w, b.w, fmaf(a[i].z, b.z, fmaf(a[i].y, b.y, fmaf(a[i].x, b.x, s[i][j]))));
+                t[i][j] = f2_fma(f2_pack(a[i].z, a[i].w), f2_pack(b.z, b.w),
+                                 f2_fma(f2_pack(a[i].x, a[i].y), f2_pack(b.x, b.y), t[i][j]));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < LR; ++i) {
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            float even, odd;
+            f2_unpack(t[i][j], even, odd);
+            s[i][j] = even + odd;
         }
     }
 }
@@ -133,7 +170,9 @@ __device__ __forceinline__ void weighted_rows(const float* W, const float* B, fl
 #pragma unroll
                 for (int i = 0; i < LR; ++i)
 #pragma unroll
-                    for (int c = 0; c < VW; ++c) o[i][k][c] = fmaf(w[i][jj], b[c], o[i][k][c]);
+                    for (int c = 0; c < VW; c += 2)
+                        f2_unpack(f2_fma(f2_splat(w[i][jj]), f2_pack(b[c], b[c + 1]), f2_pack(o[i][k][c], o[i][k][c + 1])),
+                                  o[i][k][c], o[i][k][c + 1]);
             }
         }
     }
@@ -152,79 +191,99 @@ __device__ __forceinline__ void store_cols(T* row, int c, int HD, const float* v
 }
 
 template <typename T, int G, int NW>
-__global__ void __launch_bounds__(NW * 32) attn_fwd_kernel(const CmeAttn a, const bool vec) {
-    constexpr int P = Pitch<G>::P, RT = NW * WR, NT = NW * 32;
+__global__ void __launch_bounds__(NW * 64) attn_fwd_kernel(const CmeAttn a, const bool vec) {
+    constexpr int P = Pitch<G>::P, RT = NW * WR, NT = NW * 64;
+    // a lane's columns: VW at half * 16 G + tx * VW, then every 8 VW
+    constexpr int VW = G % 2 == 0 ? 4 : 2, NK = 2 * G / VW;
     extern __shared__ __align__(16) float sm[];
     float* sQ = sm;                    // [RT][P]
     float* sK = sQ + RT * P;           // [CT][P]
     float* sV = sK + CT * P;           // [CT][P]
     float* sP = sV + CT * P;           // [RT][SP]
+    __shared__ float sM[2][RT], sL[2][RT];     // the halves' row maxima and sums
     pdl_wait();
     const int bh = blockIdx.y, q0 = blockIdx.x * RT, HD = a.HD;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3;
+    const int w0 = (warp % NW) * WR, half = warp / NW, c0 = half * 16 * G + tx * VW;
     const long long base = head_base(a, bh);
-    load_rows<T, G, RT, NT>(sQ, (const T*)a.q + base, a.st, q0, a.T, HD, a.scale, vec);
-    float m[LR], l[LR], o[LR][G][4];
+    copy_rows<T, G, RT, NT>(sQ, (const T*)a.q + base, a.st, q0, a.T, HD, vec);
+    float m[LR], l[LR], o[LR][NK][VW];
 #pragma unroll
     for (int i = 0; i < LR; ++i) {
         m[i] = -INFINITY;
         l[i] = 0.f;
 #pragma unroll
-        for (int g = 0; g < G; ++g)
+        for (int g = 0; g < NK; ++g)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) o[i][g][c] = 0.f;
+            for (int c = 0; c < VW; ++c) o[i][g][c] = 0.f;
     }
     const int kend = a.causal ? min(a.T, q0 + RT) : a.T;
-    float* wP = sP + warp * WR * SP;
+    float* wP = sP + (w0 + ty) * SP;
     for (int k0 = 0; k0 < kend; k0 += CT) {
         __syncthreads();
-        load_rows<T, G, CT, NT>(sK, (const T*)a.k + base, a.st, k0, a.T, HD, 1.f, vec);
-        load_rows<T, G, CT, NT>(sV, (const T*)a.v + base, a.st, k0, a.T, HD, 1.f, vec);
+        copy_rows<T, G, CT, NT>(sK, (const T*)a.k + base, a.st, k0, a.T, HD, vec);
+        copies_commit();
+        copy_rows<T, G, CT, NT>(sV, (const T*)a.v + base, a.st, k0, a.T, HD, vec);
+        copies_commit();
+        copies_wait<1>();
         __syncthreads();
-        float s[LR][8] = {};
-        dot_rows<G, 8>(sQ + warp * WR * P, sK, ty, tx, s);
+        float s[LR][4];
+        dot_rows<G, 4>(sQ + w0 * P, sK + half * 32 * P, ty, tx, s);
 #pragma unroll
         for (int i = 0; i < LR; ++i) {
-            const int q = q0 + warp * WR + ty + 4 * i;
+            const int row = w0 + ty + 4 * i, q = q0 + row;
             float mx = -INFINITY;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int k = k0 + tx + 8 * j;
-                if (!(k < a.T && (!a.causal || k <= q))) s[i][j] = -INFINITY;
+            for (int j = 0; j < 4; ++j) {
+                const int k = k0 + half * 32 + tx + 8 * j;
+                s[i][j] = k < a.T && (!a.causal || k <= q) ? s[i][j] * a.scale : -INFINITY;
                 mx = fmaxf(mx, s[i][j]);
             }
 #pragma unroll
             for (int off = 1; off < 8; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-            const float mnew = fmaxf(m[i], mx);
+            if (tx == 0) sM[half][row] = mx;
+        }
+        __syncthreads();                           // the other half of these rows' scores is another warp's
+        float alpha[LR];
+#pragma unroll
+        for (int i = 0; i < LR; ++i) {
+            const int row = w0 + ty + 4 * i;
+            const float mnew = fmaxf(m[i], fmaxf(sM[0][row], sM[1][row]));
             float sum = 0.f;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < 4; ++j) {
                 const float p = (mnew == -INFINITY) ? 0.f : __expf(s[i][j] - mnew);
-                wP[(ty + 4 * i) * SP + tx + 8 * j] = p;
+                wP[4 * i * SP + half * 32 + tx + 8 * j] = p;
                 sum += p;
             }
 #pragma unroll
             for (int off = 1; off < 8; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-            const float alpha = (m[i] == -INFINITY) ? 0.f : __expf(m[i] - mnew);
-            l[i] = l[i] * alpha + sum;
+            if (tx == 0) sL[half][row] = sum;
+            alpha[i] = (m[i] == -INFINITY) ? 0.f : __expf(m[i] - mnew);
             m[i] = mnew;
-#pragma unroll
-            for (int g = 0; g < G; ++g)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) o[i][g][c] *= alpha;
         }
-        __syncwarp();
-        weighted_rows<G, 4, G, SP, 1>(wP + ty * SP, sV + tx * 4, o);
+        copies_wait<0>();
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < LR; ++i) {
+            const int row = w0 + ty + 4 * i;
+            l[i] = l[i] * alpha[i] + (sL[0][row] + sL[1][row]);
+#pragma unroll
+            for (int g = 0; g < NK; ++g)
+#pragma unroll
+                for (int c = 0; c < VW; ++c) o[i][g][c] *= alpha[i];
+        }
+        weighted_rows<G, VW, NK, SP, 1>(wP, sV + c0, o);
     }
 #pragma unroll
     for (int i = 0; i < LR; ++i) {
-        const int q = q0 + warp * WR + ty + 4 * i;
+        const int q = q0 + w0 + ty + 4 * i;
         if (q < a.T) {
             const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
             T* out = (T*)a.o + head_base_o(a, bh) + (long long)q * a.ost;
 #pragma unroll
-            for (int g = 0; g < G; ++g) store_cols<T, 4>(out, tx * 4 + 32 * g, HD, o[i][g], inv, vec);
-            if (tx == 0 && a.lse) a.lse[(long long)bh * a.T + q] = m[i] + logf(l[i]);
+            for (int g = 0; g < NK; ++g) store_cols<T, VW>(out, c0 + 8 * VW * g, HD, o[i][g], inv, vec);
+            if (half == 0 && tx == 0 && a.lse) a.lse[(long long)bh * a.T + q] = m[i] + logf(l[i]);
         }
     }
 }
@@ -283,9 +342,11 @@ __global__ void __launch_bounds__(256) attn_delta_hd64_kernel(const CmeAttn a, f
     }
 }
 
-// delta[r] = sum_d dO[r][d] * O[r][d] for the rows whose dO tile has just been staged, one warp per row.
+// delta[r] = sum_d dO[r][d] * O[r][d] for the rows whose dO tile has just been staged, one warp per row.  `sO`: the same rows of
+// O in shared memory, or null.
 template <typename T, int G>
-__device__ __forceinline__ void delta_rows(float* dst, const float* sdO, const T* o, long long ost, int r0, int T_, int HD) {
+__device__ __forceinline__ void delta_rows(float* dst, const float* sdO, const float* sO, const T* o, long long ost, int r0, int T_,
+                                           int HD) {
     constexpr int NW = BWD_THREADS / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -296,7 +357,8 @@ __device__ __forceinline__ void delta_rows(float* dst, const float* sdO, const T
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 const int d = lane + 32 * g;
-                if (d < HD) s = fmaf(sdO[r * Pitch<G>::P + d], to_f32<T>(o[(long long)(r0 + r) * ost + d]), s);
+                const int at = r * Pitch<G>::P + d;
+                if (d < HD) s = fmaf(sdO[at], sO ? sO[at] : to_f32<T>(o[(long long)(r0 + r) * ost + d]), s);
             }
         }
         s = warp_sum(s);
@@ -309,6 +371,8 @@ __device__ __forceinline__ void delta_rows(float* dst, const float* sdO, const T
 //                  seven of the split form.
 // blockIdx.z == 1: the block owns 64 queries and streams keys:    dQ = scale * sum_j dS_ij K_j
 // Both kinds run in one launch, and delta = rowsum(dO * O) is made from the staged rows instead of by a kernel before.
+// Whether O is staged beside dO: fp32 heads wide enough for one block per SM anyway.
+template <typename T, int G> __host__ __device__ constexpr bool bwd_stages_o() { return sizeof(T) == 4 && G >= 3; }
 template <typename T, int G>
 __global__ void __launch_bounds__(BWD_THREADS) attn_bwd_kernel(const CmeAttn a, const bool vec) {
     constexpr int P = Pitch<G>::P, NT = BWD_THREADS, RT = BWD_ROWS;
@@ -323,6 +387,7 @@ __global__ void __launch_bounds__(BWD_THREADS) attn_bwd_kernel(const CmeAttn a, 
     float* sP = sD + CT * P;           // [RT][SP] P (own row, streamed row)
     float* sS = sP + RT * SP;          // [RT][SP] dS
     float* sDl = sS + RT * SP;         // [CT] delta of the queries in shared memory
+    float* sO = bwd_stages_o<T, G>() ? sDl + CT : nullptr;        // O of the rows whose delta is made
     pdl_wait();
     const bool kv = blockIdx.z == 0;
     const int bh = blockIdx.y, r0 = blockIdx.x * RT, HD = a.HD;
@@ -332,8 +397,12 @@ __global__ void __launch_bounds__(BWD_THREADS) attn_bwd_kernel(const CmeAttn a, 
     const T* q = (const T*)a.q + base; const T* k = (const T*)a.k + base; const T* v = (const T*)a.v + base;
     const T* d_o = (const T*)a.d_o + obase; const T* o = (const T*)a.o + obase;
     const float* lse = a.lse + (long long)bh * a.T;
-    load_rows<T, G, RT, NT>(sA, kv ? k : q, a.st, r0, a.T, HD, 1.f, vec);
-    load_rows<T, G, RT, NT>(sB, kv ? v : d_o, kv ? a.st : a.ost, r0, a.T, HD, 1.f, vec);
+    copy_rows<T, G, RT, NT>(sA, kv ? k : q, a.st, r0, a.T, HD, vec);
+    if (!kv) {
+        copy_rows<T, G, RT, NT>(sB, d_o, a.ost, r0, a.T, HD, vec);
+        if (sO) copy_rows<T, G, RT, NT>(sO, o, a.ost, r0, a.T, HD, vec);
+        copies_commit();
+    }
     float acc1[LR][NK][VW], acc2[LR][NK][VW];
 #pragma unroll
     for (int i = 0; i < LR; ++i)
@@ -342,20 +411,28 @@ __global__ void __launch_bounds__(BWD_THREADS) attn_bwd_kernel(const CmeAttn a, 
 #pragma unroll
             for (int c = 0; c < VW; ++c) { acc1[i][g][c] = 0.f; acc2[i][g][c] = 0.f; }
     if (!kv) {
+        copies_wait<0>();
         __syncthreads();
-        delta_rows<T, G>(sDl, sB, o, a.ost, r0, a.T, HD);
+        delta_rows<T, G>(sDl, sB, sO, o, a.ost, r0, a.T, HD);
     }
     // causal: queries see keys <= their index.  dQ blocks stop early; dK / dV blocks start late.
     const int s_begin = (kv && a.causal) ? r0 : 0;
     const int s_end = (!kv && a.causal) ? min(a.T, r0 + RT) : a.T;
     for (int s0 = s_begin; s0 < s_end; s0 += CT) {
         __syncthreads();
-        load_rows<T, G, CT, NT>(sC, kv ? q : k, a.st, s0, a.T, HD, 1.f, vec);
-        load_rows<T, G, CT, NT>(sD, kv ? d_o : v, kv ? a.ost : a.st, s0, a.T, HD, 1.f, vec);
+        copy_rows<T, G, CT, NT>(sC, kv ? q : k, a.st, s0, a.T, HD, vec);
+        copies_commit();
+        if (kv && s0 == s_begin) copy_rows<T, G, RT, NT>(sB, v, a.st, r0, a.T, HD, vec);
+        copy_rows<T, G, CT, NT>(sD, kv ? d_o : v, kv ? a.ost : a.st, s0, a.T, HD, vec);
+        if (kv && sO) copy_rows<T, G, CT, NT>(sO, o, a.ost, s0, a.T, HD, vec);
+        copies_commit();
+        copies_wait<1>();                          // the tiles of the first product; the others arrive meanwhile
         __syncthreads();
-        if (kv) delta_rows<T, G>(sDl, sD, o, a.ost, s0, a.T, HD);
-        float s[LR][4] = {}, dp[LR][4] = {};
+        float s[LR][4], dp[LR][4];
         dot_rows<G, 4>(sA + w0 * P, sC + half * 32 * P, ty, tx, s);
+        copies_wait<0>();
+        __syncthreads();
+        if (kv) delta_rows<T, G>(sDl, sD, sO, o, a.ost, s0, a.T, HD);
         dot_rows<G, 4>(sB + w0 * P, sD + half * 32 * P, ty, tx, dp);
         if (kv) __syncthreads();                   // delta is written by all warps
 #pragma unroll
@@ -441,14 +518,14 @@ template <typename T, int G, int NW> int fwd_launch(const CmeAttn* a, cudaStream
     auto k = attn_fwd_kernel<T, G, NW>;
     int rc = allow_smem(k, smem);
     if (rc) return rc;
-    CME_CUDA(cme_launch_dependent(k, dim3(cme_cdiv(a->T, RT), a->nb * a->nh), dim3(NW * 32), smem, st, *a,
+    CME_CUDA(cme_launch_dependent(k, dim3(cme_cdiv(a->T, RT), a->nb * a->nh), dim3(NW * 64), smem, st, *a,
                                   rows_vectorisable(a, false)));
     CME_LAUNCH_CHECK();
     return CME_OK;
 }
 template <typename T, int G> int bwd_launch(const CmeAttn* a, cudaStream_t st) {
     constexpr int P = Pitch<G>::P, RT = BWD_ROWS;
-    constexpr size_t smem = (4 * RT * P + 2 * RT * SP + CT) * sizeof(float);
+    constexpr size_t smem = ((bwd_stages_o<T, G>() ? 5 : 4) * RT * P + 2 * RT * SP + CT) * sizeof(float);
     static_assert(smem <= 227 * 1024, "one block's shared memory");
     auto k = attn_bwd_kernel<T, G>;
     int rc = allow_smem(k, smem);
