@@ -27,10 +27,17 @@ class GraphedStep:
         self.static_y = torch.zeros(accum, tokens_per_step, dtype=torch.int32, device=device)
         self.captured_launches = 0
 
+    def _stage(self, dx: torch.Tensor, x: torch.Tensor, dy: torch.Tensor, y: torch.Tensor) -> None:
+        if all(t.device == dx.device and t.dtype == torch.int32 and t.is_contiguous() and t.shape == dx.shape for t in (x, y)):
+            from . import ops
+            ops._check(ops.lib().cme_copy_pair_i32(ops._a(dx), ops._a(x), ops._a(dy), ops._a(y), dx.numel(), ops._st()))
+            return
+        dx.copy_(x, non_blocking=True)                  # host batches, other types
+        dy.copy_(y, non_blocking=True)
+
     def __call__(self, tokens: Sequence[torch.Tensor], targets: Sequence[torch.Tensor]) -> None:
         for i, (x, y) in enumerate(zip(tokens, targets)):
-            self.static_x[i].copy_(x, non_blocking=True)
-            self.static_y[i].copy_(y, non_blocking=True)
+            self._stage(self.static_x[i], x, self.static_y[i], y)
         xs = [self.static_x[i] for i in range(self.static_x.shape[0])]
         ys = [self.static_y[i] for i in range(self.static_y.shape[0])]
         self.calls += 1

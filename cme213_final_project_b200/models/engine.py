@@ -258,17 +258,24 @@ class NativeEngine:
             self.set_lr(lr)
         self.step_count += 1
         with torch.cuda.device(self.device):
-            ops._check(self.lib.cme_step_inc(ops._p(self.step_dev), ops._stream()))
-            normsq = None
+            nodecay = self.nodecay if o.weight_decay > 0 else None
             if o.clip_norm > 0:
-                ops._check(self.lib.cme_grad_normsq(ops._dt(self.grads), ops._p(self.grads),
-                                                    ctypes.c_longlong(self.grads.numel()), ops._p(self._norm_partial),
-                                                    ops._p(self.normsq), ops._stream()))
-                normsq = self.normsq
+                # two launches: the kernel that squares the gradients also counts the step, the update adds up its partial sums
+                ops._check(self.lib.cme_grad_normsq_partials(
+                    ops._dt(self.grads), ops._p(self.grads), ctypes.c_longlong(self.grads.numel()), ops._p(self._norm_partial),
+                    ops._p(self.step_dev), ops._stream()))
+                ops._check(self.lib.cme_adam_partials(
+                    ops._dt(self.grads), ops._p(self.master), ops._p(None if self.strict else self.params), ops._p(self.grads),
+                    ops._p(self.adam_m), ops._p(self.adam_v), ctypes.c_longlong(self.master.numel()), ops._p(self.step_dev),
+                    ops._p(self.lr_dev), ops._p(self._norm_partial), *map(ctypes.c_float, (o.beta1, o.beta2, o.eps, o.weight_decay,
+                                                                                          grad_scale, o.clip_norm)),
+                    ops._p(nodecay), 0 if nodecay is None else nodecay.shape[0], self._norm_partial.numel(), ops._p(self.normsq),
+                    ops._stream()))
+                return
+            ops._check(self.lib.cme_step_inc(ops._p(self.step_dev), ops._stream()))
             ops.adam_step(self.master, self.grads, self.adam_m, self.adam_v, self.step_dev, self.lr_dev,
-                          compute=None if self.strict else self.params, normsq=normsq, beta1=o.beta1, beta2=o.beta2,
-                          eps=o.eps, weight_decay=o.weight_decay, grad_scale=grad_scale, clip_norm=o.clip_norm,
-                          nodecay=self.nodecay if o.weight_decay > 0 else None)
+                          compute=None if self.strict else self.params, beta1=o.beta1, beta2=o.beta2, eps=o.eps,
+                          weight_decay=o.weight_decay, grad_scale=grad_scale, nodecay=nodecay)
 
     def train_step(self, tokens: Sequence[torch.Tensor], targets: Sequence[torch.Tensor],
                    bucket_callback=None, buckets=None) -> None:

@@ -57,7 +57,7 @@ _PROTOTYPES = {
     "cme_colsum_splits": "ii", "cme_dact_colsum": "ivvvvviiiiv", "cme_scale": "ivlfv", "cme_cast": "ivivlv",
     "cme_add": "ivvvlv", "cme_relu_bwd": "ivvvlv", "cme_init_uniform": "ivlfuv", "cme_embedding_fwd": "ivvvviiiiv",
     "cme_embedding_bwd": "ivvvviiiiiv", "cme_cross_entropy": "ivvvvviilfffiv", "cme_grad_normsq": "ivlvvv",
-    "cme_adam": "ivvvvvlvvvffffffviv", "cme_attention_fwd": "viv", "cme_attention_bwd": "viv", "cme_attention_path": "vii",
+    "cme_adam": "ivvvvvlvvvffffffviv", "cme_copy_pair_i32": "vvvvlv", "cme_attention_fwd": "viv", "cme_attention_bwd": "viv", "cme_attention_path": "vii",
 }
 # Entry points that the compiled wrappers call.
 _WRAPPED = ("cme_last_error", "cme_cross_entropy", "cme_attention_fwd", "cme_attention_bwd", "cme_attention_path",

@@ -47,6 +47,24 @@ CME_API int cme_copy_d2d(void* dst, const void* src, long long bytes, void* stre
     return CME_OK;
 }
 
+// Two int32 arrays of one length in one launch (a step's tokens and targets; as two copies they are two nodes of 1.5 us in
+// front of every replayed step, with a gap behind each).
+static __global__ void __launch_bounds__(256) copy_pair_kernel(int* __restrict__ d0, const int* __restrict__ s0, int* __restrict__ d1,
+                                                               const int* __restrict__ s1, long long n) {
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < 2 * n; i += step) {
+        if (i < n) d0[i] = s0[i];
+        else d1[i - n] = s1[i - n];
+    }
+}
+CME_API int cme_copy_pair_i32(int* d0, const int* s0, int* d1, const int* s1, long long n, void* stream) {
+    if (n <= 0) return CME_OK;
+    const long long blocks = (2 * n + 255) / 256;
+    copy_pair_kernel<<<(int)(blocks < 1184 ? blocks : 1184), 256, 0, (cudaStream_t)stream>>>(d0, s0, d1, s1, n);
+    CME_LAUNCH_CHECK();
+    return CME_OK;
+}
+
 // Number of kernels this library has launched (or captured into a graph) in this process.
 CME_API long long cme_launch_count() { return g_cme_launches; }
 

@@ -280,9 +280,12 @@ __global__ void __launch_bounds__(1024) reduce_scalar_kernel(const float* __rest
     if (threadIdx.x == 0) *out = (accumulate ? *out : 0.f) + s * weight;
 }
 
+constexpr int NORM_PARTIALS = 1024;
+
 template <typename T>
-__global__ void __launch_bounds__(256) normsq_partial_kernel(const T* __restrict__ g, long long n, float* partial) {
+__global__ void __launch_bounds__(256) normsq_partial_kernel(const T* __restrict__ g, long long n, float* partial, int* count) {
     __shared__ float scratch[32];
+    if (count && blockIdx.x == 0 && threadIdx.x == 0) *count += 1;
     float s = 0.f;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float v = to_f32<T>(g[i]);
@@ -295,12 +298,13 @@ __global__ void __launch_bounds__(256) normsq_partial_kernel(const T* __restrict
 // Same over whole 16-byte words, four in flight per thread: with a 2-byte load per iteration the sum of 124 M bf16
 // gradients waits for its loads (249 MB: 58 us, 86 us so).
 template <typename T>
-__global__ void __launch_bounds__(256) normsq_partial_vec_kernel(const T* __restrict__ grads, long long n, float* partial) {
+__global__ void __launch_bounds__(256) normsq_partial_vec_kernel(const T* __restrict__ grads, long long n, float* partial, int* count) {
     __shared__ float scratch[32];
     constexpr int W = 16 / sizeof(T);
     const uint4* g = reinterpret_cast<const uint4*>(grads);
     const long long nvec = n / W;
     pdl_wait();
+    if (count && blockIdx.x == 0 && threadIdx.x == 0) *count += 1;
     float s[4] = {0.f, 0.f, 0.f, 0.f};
     const long long step = (long long)gridDim.x * blockDim.x;
     auto add = [&](const uint4& u, float& t) {
@@ -338,7 +342,24 @@ struct AdamArgs {
     const int* step; const float* lr; const float* normsq;
     float beta1, beta2, eps, weight_decay, grad_scale, clip_norm;
     const long long* nodecay; int n_nodecay;      // sorted [start, end) pairs exempt from weight decay
+    int n_norm; float* norm_out;                  // > 1: `normsq` holds that many partial sums; their total goes to norm_out
 };
+
+// The gradient's scale.  Partial sums of the squared norm are added by every block (1024 of them: a few loads from L2 and two
+// barriers, against a kernel of its own in front of this one).
+__device__ __forceinline__ float adam_grad_scale(const AdamArgs& a, float* scratch) {
+    if (!a.normsq || a.clip_norm <= 0.f) return a.grad_scale;
+    float sq = 0.f;
+    if (a.n_norm > 1) {
+        for (int i = threadIdx.x; i < a.n_norm; i += blockDim.x) sq += a.normsq[i];
+        sq = block_sum(sq, scratch);
+        if (a.norm_out && blockIdx.x == 0 && threadIdx.x == 0) *a.norm_out = sq;
+    } else {
+        sq = *a.normsq;
+    }
+    const float norm = sqrtf(sq) * a.grad_scale;
+    return norm > a.clip_norm ? a.grad_scale * (a.clip_norm / norm) : a.grad_scale;
+}
 
 // The first of `n` sorted no-decay ranges, from `lo` on, with end > i (n if there is none).
 __device__ __forceinline__ int adam_range_at(const long long* ranges, int n, int lo, long long i) {
@@ -367,11 +388,8 @@ __global__ void __launch_bounds__(256) adam_kernel(const AdamArgs a) {
     const int t = *a.step;
     const float lr = *a.lr;
     const float bc1 = 1.f - powf(a.beta1, (float)t), bc2 = 1.f - powf(a.beta2, (float)t);
-    float gs = a.grad_scale;
-    if (a.normsq && a.clip_norm > 0.f) {
-        const float norm = sqrtf(*a.normsq) * a.grad_scale;
-        if (norm > a.clip_norm) gs *= a.clip_norm / norm;
-    }
+    __shared__ float scratch[32];
+    const float gs = adam_grad_scale(a, scratch);
     const TG* grads = reinterpret_cast<const TG*>(a.grads);
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (long long)gridDim.x * blockDim.x) {
         const float g = to_f32<TG>(grads[i]) * gs;
@@ -401,11 +419,8 @@ __global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
     const float lr = *a.lr;
     const float bc1 = 1.f - powf(a.beta1, (float)t), bc2 = 1.f - powf(a.beta2, (float)t);
     const float ibc1 = 1.f / bc1, ibc2 = 1.f / bc2;
-    float gs = a.grad_scale;
-    if (a.normsq && a.clip_norm > 0.f) {
-        const float norm = sqrtf(*a.normsq) * a.grad_scale;
-        if (norm > a.clip_norm) gs *= a.clip_norm / norm;
-    }
+    __shared__ float scratch[32];
+    const float gs = adam_grad_scale(a, scratch);
     const long long nv = a.n >> 2;
     // The no-decay range at or after the element at hand stays in registers; where it is over, the next one is searched for
     // in a copy of the list in shared memory.  From global memory that is a chain of dependent loads: all of the list where
@@ -528,22 +543,30 @@ CME_API int cme_cross_entropy(int dtype, const void* logits, const int* targets,
     return loss_out ? cme_loss_mean(losses, rows, loss_weight, loss_out, accumulate_loss, stream) : CME_OK;
 }
 
-// *out = sum(g^2) over n elements; `partial` holds 1024 floats.
-CME_API int cme_grad_normsq(int dtype, const void* g, long long n, float* partial, float* out, void* stream) {
+// partial[0 .. 1024) = sums whose total is sum(g^2) over n elements; *step (or null) is incremented on the way.
+CME_API int cme_grad_normsq_partials(int dtype, const void* g, long long n, float* partial, int* step, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     const bool bf = dtype == CME_BF16;
     if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
-        CME_CUDA(bf ? cme_launch_dependent(normsq_partial_vec_kernel<__nv_bfloat16>, dim3(1024), dim3(256), 0, st,
-                                           (const __nv_bfloat16*)g, n, partial)
-                    : cme_launch_dependent(normsq_partial_vec_kernel<float>, dim3(1024), dim3(256), 0, st, (const float*)g, n,
-                                           partial));
+        CME_CUDA(bf ? cme_launch_dependent(normsq_partial_vec_kernel<__nv_bfloat16>, dim3(NORM_PARTIALS), dim3(256), 0, st,
+                                           (const __nv_bfloat16*)g, n, partial, step)
+                    : cme_launch_dependent(normsq_partial_vec_kernel<float>, dim3(NORM_PARTIALS), dim3(256), 0, st, (const float*)g, n,
+                                           partial, step));
     } else if (bf) {
-        normsq_partial_kernel<__nv_bfloat16><<<1024, 256, 0, st>>>((const __nv_bfloat16*)g, n, partial);
+        normsq_partial_kernel<__nv_bfloat16><<<NORM_PARTIALS, 256, 0, st>>>((const __nv_bfloat16*)g, n, partial, step);
     } else {
-        normsq_partial_kernel<float><<<1024, 256, 0, st>>>((const float*)g, n, partial);
+        normsq_partial_kernel<float><<<NORM_PARTIALS, 256, 0, st>>>((const float*)g, n, partial, step);
     }
     CME_LAUNCH_CHECK();
-    CME_CUDA(cme_launch_dependent(reduce_scalar_kernel, dim3(1), dim3(1024), 0, st, (const float*)partial, 1024, 1.f, out, 0));
+    return CME_OK;
+}
+
+// *out = sum(g^2) over n elements; `partial` holds 1024 floats.
+CME_API int cme_grad_normsq(int dtype, const void* g, long long n, float* partial, float* out, void* stream) {
+    const int rc = cme_grad_normsq_partials(dtype, g, n, partial, nullptr, stream);
+    if (rc) return rc;
+    CME_CUDA(cme_launch_dependent(reduce_scalar_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, (const float*)partial,
+                                  NORM_PARTIALS, 1.f, out, 0));
     CME_LAUNCH_CHECK();
     return CME_OK;
 }
@@ -581,14 +604,15 @@ CME_API int cme_step_inc(int* step, void* stream) {
 // Adam / AdamW over [0, n).  `step` (already incremented), `lr` and `normsq` live in device memory.
 // g_eff = grad * grad_scale * min(1, clip_norm / (sqrt(normsq) * grad_scale)); decoupled weight decay
 // except inside the `nodecay` ranges; writes the fp32 master and, if given, its bf16 copy.
-CME_API int cme_adam(int grad_dtype, float* master, void* compute_bf16, const void* grads, float* m, float* v,
-                     long long n, const int* step, const float* lr, const float* normsq, float beta1, float beta2,
-                     float eps, float weight_decay, float grad_scale, float clip_norm, const long long* nodecay,
-                     int n_nodecay, void* stream) {
+// n_norm > 1: `normsq` holds that many partial sums (cme_grad_normsq_partials: 1024); their total goes to norm_out (or null).
+CME_API int cme_adam_partials(int grad_dtype, float* master, void* compute_bf16, const void* grads, float* m, float* v,
+                              long long n, const int* step, const float* lr, const float* normsq, float beta1, float beta2,
+                              float eps, float weight_decay, float grad_scale, float clip_norm, const long long* nodecay,
+                              int n_nodecay, int n_norm, float* norm_out, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if (n <= 0) return CME_OK;
     AdamArgs a{master, (__nv_bfloat16*)compute_bf16, grads, m, v, n, step, lr, normsq, beta1, beta2, eps,
-               weight_decay, grad_scale, clip_norm, nodecay, n_nodecay};
+               weight_decay, grad_scale, clip_norm, nodecay, n_nodecay, n_norm, norm_out};
     long long blocks = (n + 255) / 256;
     if (blocks > 148 * 8) blocks = 148 * 8;
     auto al = [](const void* p, int b) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & (b - 1)) == 0; };
@@ -608,4 +632,12 @@ CME_API int cme_adam(int grad_dtype, float* master, void* compute_bf16, const vo
     }
     CME_LAUNCH_CHECK();
     return CME_OK;
+}
+
+CME_API int cme_adam(int grad_dtype, float* master, void* compute_bf16, const void* grads, float* m, float* v,
+                     long long n, const int* step, const float* lr, const float* normsq, float beta1, float beta2,
+                     float eps, float weight_decay, float grad_scale, float clip_norm, const long long* nodecay,
+                     int n_nodecay, void* stream) {
+    return cme_adam_partials(grad_dtype, master, compute_bf16, grads, m, v, n, step, lr, normsq, beta1, beta2, eps, weight_decay,
+                             grad_scale, clip_norm, nodecay, n_nodecay, 1, nullptr, stream);
 }
