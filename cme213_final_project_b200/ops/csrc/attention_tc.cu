@@ -93,11 +93,11 @@ struct FwdParams {
 // What bounds it: the chain MMA -> TMEM load -> softmax -> TMEM store -> MMA of a tile (no pipe is busy for half of the time).
 // So a CTA is kept small enough for four on an SM: 128 queries, 64 keys at a time, P in the columns that its scores came
 // from, 128 TMEM columns, 64 score registers per thread; every scheduler then has four softmax warps of independent chains,
-// and a tile's start and end run under the others' work.  16 x 12 heads x 1024 tokens: causal 56 us, all keys 89 us (two CTAs
-// with 128 keys at a time 70 us causal; three with S_{j+1} made under softmax_j 57 and 87 us; a quarter of the exponentials as
-// a polynomial on the FMA pipe 58 and 91 us; the query tiles of a head side by side instead of the heavy ones first 73 us causal).
-// The tensor pipe runs the MMAs of one thread in the order they are issued, so S_{j+1} may follow P_j V_j into the same
-// columns without a wait, and the barrier that announces S_{j+1} also says that O is complete up to block j.
+// and a tile's start and end run under the others' work.  16 x 12 heads x 1024 tokens: causal 58 us, all keys 91 us.
+// S_{j+1} goes to the columns that P_j V_j reads its A operand from.  PTX orders two MMAs of a thread only if they accumulate in
+// the same place, so S_{j+1} is issued once a barrier says that P_j V_j is complete.  Measured without that wait, when this form
+// took 57 and 89 us: two CTAs with 128 keys at a time 70 us causal; three with S_{j+1} made under softmax_j 57 and 87 us; a quarter
+// of the exponentials as a polynomial on the FMA pipe 58 and 91 us; the query tiles of a head side by side 73 us causal.
 // shared: Q 16K | K[2] 16K | V[2] 16K | barriers      (P never passes through shared memory)
 constexpr int FWD_BKV = 64;                // keys per step
 constexpr int FWD_KV_BYTES = FWD_BKV * HD * 2;
@@ -127,7 +127,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint64_t* v_full = bars + 3;              // [2]
     uint64_t* s_full = bars + 5;              // phase j: S_j is ready and O is complete up to block j - 1
     uint64_t* p_ready = bars + 6;             // S_j read, P_j written over it, O rescaled (128 arrivals)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
+    uint64_t* p_free = bars + 7;              // P_j V_j complete: S_{j+1} may take the columns of P_j
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -142,6 +143,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int s = 0; s < 2; ++s) { mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1); }
         mbar_init(s_full, 1);
         mbar_init(p_ready, 128);
+        mbar_init(p_free, 1);
         fence_barrier_init();
     }
     if (warp == 4) { tmem_alloc(tmem_slot, FWD_TMEM_COLS); tmem_relinquish(); }
@@ -194,7 +196,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 for (int k = 0; k < FWD_BKV / 16; ++k)       // A = P from tensor memory: 16 keys = 8 columns per step
                     mma_f16_ts(tmem_O, tmem_P + k * 8, desc_add(vd, k * 2048), idesc_o, (j > 0 || k > 0));
                 if (j + 1 < nkv) {
-                    if (!mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag)) { ok = false; break; }
+                    mma_commit(p_free);
+                    if (!mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag) ||
+                        !mbar_wait(p_free, j & 1, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
                     issue_s(j + 1);
                 } else {
                     mma_commit(s_full);                      // phase nkv: O is complete
@@ -332,7 +337,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // launch clears the scratch beforehand and dq_convert_kernel scales and casts the sums.
 // What bounds it: the chain of a block (two round trips to the tensor pipe, about 6000 clocks, hidden by one other CTA only);
 // the tensor pipe is busy for 45 % of the time (a product of 64 columns takes as long as one of 128).
-// 16 x 12 heads x 1024 tokens, causal: 154 us; one CTA per SM with 128 queries at a time, P through shared memory: 179 us.
+// 16 x 12 heads x 1024 tokens, causal: 157 us; one CTA per SM with 128 queries at a time, P through shared memory: 179 us.
 // shared: K 16K | V 16K | Q[3] 24K | dO[2] 16K | dS^T 16K | dQ staging (fp32) 16K | row statistics[2] 1K | barriers
 constexpr int BWD_BQ = 64;                 // queries per step
 constexpr int BWD_Q_BYTES = BWD_BQ * HD * 2;
@@ -449,7 +454,6 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
                 for (int k = 0; k < HD / 16; ++k)
                     mma_f16_ss(tmem_dP, desc_add(vK, k * 32), desc_add(od, k * 32), idesc_s, k > 0);
-                mma_commit(s_full);
             };
             mbar_arrive_expect_tx(kv_full, 2 * TILE_BYTES);
             tma_load_4d(sK, &tmK, kv_full, 0, k0, h, b);
@@ -460,7 +464,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             for (int it = 1; it < BWD_DO_STAGES && it < n_it; ++it) load_do(it);
             bool ok = mbar_wait(kv_full, 0, abort_flag) && mbar_wait(&q_full[0], 0, abort_flag) &&
                       mbar_wait(&do_full[0], 0, abort_flag);
-            if (ok) { tc_fence_after(); issue_s(0); issue_dp(0); }
+            if (ok) { tc_fence_after(); issue_s(0); issue_dp(0); mma_commit(s_full); }
             for (int it = 0; it < n_it && ok; ++it) {
                 if (!mbar_wait(p_ready, it & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
@@ -480,19 +484,20 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     mma_f16_ts(tmem_dK, tmem_S + (k >> 1) * 32 + 16 + (k & 1) * 8, desc_add(qd, k * 2048), idesc_t, acc | (k > 0));
                 mma_commit(in_free);
                 if (it + 1 < n_it) {
-                    // S^T takes the place of P^T and dS^T once the products above have read them (the tensor pipe runs them
-                    // in this order); dP^T that of dQ once the warps have it in registers
+                    // dP^T takes the place of dQ once the warps have it in registers; S^T that of P^T and dS^T once a barrier says
+                    // that the products above, which read them, are complete (PTX orders MMAs of a thread only if they accumulate
+                    // in the same place).  S^T second: what it waits for runs beside dP^T (first: 3 us of 183 more)
                     const int n = it + 1;
-                    if (!mbar_wait(&q_full[n % BWD_Q_STAGES], (n / BWD_Q_STAGES) & 1, abort_flag)) { ok = false; break; }
-                    issue_s(n);
                     if (!mbar_wait(dq_free, it & 1, abort_flag) ||
                         !mbar_wait(&do_full[n % BWD_DO_STAGES], (n / BWD_DO_STAGES) & 1, abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     issue_dp(n);
-                }
-                if (it + BWD_DO_STAGES < n_it) {
-                    if (!mbar_wait(in_free, it & 1, abort_flag)) { ok = false; break; }
-                    load_do(it + BWD_DO_STAGES);
+                    if (!mbar_wait(&q_full[n % BWD_Q_STAGES], (n / BWD_Q_STAGES) & 1, abort_flag) ||
+                        !mbar_wait(in_free, it & 1, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
+                    issue_s(n);
+                    mma_commit(s_full);
+                    if (it + BWD_DO_STAGES < n_it) load_do(it + BWD_DO_STAGES);
                     if (it + BWD_Q_STAGES < n_it) load_q(it + BWD_Q_STAGES);
                 }
             }
