@@ -551,6 +551,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             tmem_ld32(tS, rs);
             tmem_ld32(tmem_dP + lane_addr + cg * 32, rd);
             tmem_wait_ld();
+            if (q0 + BWD_BQ > p.T) {
+                // the rows of Q beyond T are zeros, and 0 k is NaN where an element of the key is infinite: 0, so that the
+                // statistics' -inf decides
+                const int hi = p.T - q0 - cg * 32;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) rs[i] = i < hi ? rs[i] : 0u;
+            }
             const bool need_mask = k0 + BKV > p.T || (p.causal && q0 < k0 + BKV);
             // queries [lo, 32) of this thread's 32 see its key
             const int lo = (key < p.T ? (p.causal ? key - q0 : 0) : BWD_BQ) - cg * 32;

@@ -56,3 +56,28 @@ def test_the_same_call_gives_the_same_bits(T, causal):
     assert ops.attention_check_status() == 0
     for run in runs[1:]:
         assert all(torch.equal(a, b) for a, b in zip(run, runs[0]))
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("T", [65, 96, 130, 200, 256])
+def test_a_key_that_an_infinite_element_hides(T, causal):
+    """Every score of the key is -inf, so it gets no weight and no gradient; the rows of the last block beyond T are zeros, and
+    0 x inf must not reach the gradients either."""
+    from cme213_final_project_b200 import ops
+    H, j = 3, T // 2
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q, k, v, do = (torch.randn(T, H, 64, generator=g, device="cuda").to(torch.bfloat16) for _ in range(4))
+    q[:, :, 3] = q[:, :, 3].abs() + 0.5
+    k[j, :, 3] = float("-inf")
+    flat = [t.reshape(T, H * 64) for t in (q, k, v, do)]
+    out, lse = ops.attention_fwd(*flat[:3], 1, H, T, "split", causal, backend="tc")
+    ref, ref_lse, ref_grads = _reference(*(t.transpose(0, 1) for t in (q, k, v, do)), causal)
+    rel = lambda a, b: ((a.double().reshape(T, H, 64).transpose(0, 1) - b).norm() / b.norm()).item()          # noqa: E731
+    assert rel(out, ref) < BF16_REL and (lse.double() - ref_lse.reshape(-1)).abs().max().item() < 1e-4
+    seen = torch.arange(64, device="cuda") != 3             # dQ = dS K is NaN in the element's column, as it has to be
+    for mode in (0, 1, 2):
+        dq, dk, dv = ops.attention_bwd(*flat[:3], out, lse, flat[3], 1, H, T, "split", causal, backend="tc", dq_mode=mode)
+        assert rel(dk, ref_grads[1]) < 2 * BF16_REL and rel(dv, ref_grads[2]) < 2 * BF16_REL
+        dq = dq.double().reshape(T, H, 64).transpose(0, 1)[..., seen]
+        assert ((dq - ref_grads[0][..., seen]).norm() / ref_grads[0][..., seen].norm()).item() < 2 * BF16_REL
+        assert dv.reshape(T, H, 64)[j].abs().max().item() == 0 and dk.reshape(T, H, 64)[j].abs().max().item() == 0
