@@ -138,8 +138,8 @@ class NativeEngine:
         self.overlap_wgrad = bool(on)
 
     def fence(self, target: "torch.cuda.Stream") -> None:
-        """Make ``target`` wait for everything backward has enqueued so far, on the current stream and on the
-        engine's second stream: call it from a bucket callback before reading the bucket on ``target``."""
+        """Make ``target`` wait for the gradients that backward has enqueued so far, on the current stream and on the
+        engine's own: call it from a bucket callback before reading the bucket on ``target``."""
         ops._check(self.lib.cme_engine_fence(self._h, ops._stream(), ctypes.c_void_p(target.cuda_stream)))
 
     def rebind(self, params: torch.Tensor, grads: torch.Tensor) -> None:

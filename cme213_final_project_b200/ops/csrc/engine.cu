@@ -121,6 +121,7 @@ struct Engine {
     cudaEvent_t ev_aux[4] = {};      // [0] fork of forward's side work  [1] padded output weights ready  [2] row losses
                                      // ready  [3] side2's work done
     bool loss_pending = false;       // side2 holds work that backward's end has to wait for
+    bool side2_grads = false;        // side2 holds gradient products that backward has not joined yet
 
     char* P(long long off) const { return params + off * (long long)es; }
     char* G(long long off) const { return grads + off * (long long)es; }
@@ -398,8 +399,10 @@ CME_API int cme_engine_set_overlap(void* h, int on) {
     return CME_OK;
 }
 
-// Makes `target` wait for everything enqueued so far on `stream` and on the engine's second stream: what a
-// gradient-synchronisation stream needs before it may read a bucket that backward has just completed.
+// Makes `target` wait for everything enqueued so far on `stream` and for the gradient products on the engine's other streams:
+// what a gradient-synchronisation stream needs before it may read a bucket that backward has just completed.  The third stream
+// counts only between its first product of a backward pass and the join: at other times it holds the loss at most, which no bucket
+// needs, and under capture it need not be part of the graph, where waiting for it is an error.
 CME_API int cme_engine_fence(void* h, void* stream, void* target) {
     Engine* e = static_cast<Engine*>(h);
     cudaEvent_t v;
@@ -409,8 +412,10 @@ CME_API int cme_engine_fence(void* h, void* stream, void* target) {
     if (e->side) {
         CME_CUDA(cudaEventRecord(v, e->side));
         CME_CUDA(cudaStreamWaitEvent((cudaStream_t)target, v, 0));
-        CME_CUDA(cudaEventRecord(v, e->side2));
-        CME_CUDA(cudaStreamWaitEvent((cudaStream_t)target, v, 0));
+        if (e->side2_grads) {
+            CME_CUDA(cudaEventRecord(v, e->side2));
+            CME_CUDA(cudaStreamWaitEvent((cudaStream_t)target, v, 0));
+        }
     }
     CME_CUDA(cudaEventDestroy(v));           // released once the recorded work has completed
     return CME_OK;
@@ -558,6 +563,7 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
     const CmeEngineDesc& d = e.d;
     cudaStream_t st = (cudaStream_t)stream;
     const bool ov = e.side != nullptr;
+    e.side2_grads = false;
     cudaStream_t ws = ov ? e.side : st;                     // stream of the weight-gradient work,
     cudaStream_t ws2 = ov && e.two_sides ? e.side2 : ws;    // and of that of W2 and Wo
     auto of = [&](int slot, int k) { return slot < d.L && (k & 1) == 0 ? ws2 : ws; };
@@ -570,6 +576,7 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
         if (!ov) return CME_OK;
         CME_CUDA(cudaEventRecord(evt(slot, k), st));
         CME_CUDA(cudaStreamWaitEvent(of(slot, k), evt(slot, k), 0));
+        if (of(slot, k) == e.side2) e.side2_grads = true;
         return CME_OK;
     };
     auto done = [&](int slot, int k) -> int {               // marks the end of a piece of side work
@@ -738,6 +745,7 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
         if (ws2 != ws) {                                    // (the loss published there does not hold the scatter up)
             CME_CUDA(cudaStreamWaitEvent(st, evt(0, 4), 0));
             CME_CUDA(cudaStreamWaitEvent(st, evt(0, 6), 0));
+            e.side2_grads = false;
         }
     }
     // the two tables are independent: the position table's sums run on the second stream beside the token scatter,

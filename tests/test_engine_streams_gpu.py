@@ -57,3 +57,40 @@ def test_streams_and_planes_give_the_step_of_one_stream(hidden, micro):
         sl = slice(s.offset, s.offset + s.numel)
         # a handful of bf16 roundings (2^-9 each) of values that enter as sums of the same size
         assert ((eng.grads[sl].cpu().double() - want[sl]).norm() / want[sl].norm()).item() < 3e-2
+
+
+@pytest.mark.parametrize("hidden,batch", [(256, 8), (512, 304)])
+def test_fences_of_a_captured_backward(hidden, batch):
+    """Buckets that another stream reads behind a fence, captured as ``forward`` + ``backward``: the third stream is no part of the
+    graph before its first product, or at all where a weight gradient is more than 10 GFLOP (the second size)."""
+    eng, cfg = _engine(hidden, batch, True)
+    (x,), (y,) = _batches(cfg, 1)
+    buckets = eng.layout.coalesced_buckets(1)
+    reader, copy, errors = torch.cuda.Stream(), torch.empty_like(eng.grads), []
+
+    def ready(b):
+        try:
+            eng.fence(reader)
+            with torch.cuda.stream(reader):
+                copy[b.start:b.end].copy_(eng.grads[b.start:b.end])
+        except Exception as e:                              # (an exception does not leave the native call)
+            errors.append(e)
+
+    def step():
+        eng.forward(x, y)
+        eng.backward(ready, buckets)
+        torch.cuda.current_stream().wait_stream(reader)
+
+    step()
+    torch.cuda.synchronize()
+    assert len(buckets) > 2 and torch.equal(copy, eng.grads)
+    want = copy.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    assert not errors
+    for _ in range(3):
+        copy.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(copy, want)
