@@ -28,9 +28,11 @@ class GraphedStep:
         self.captured_launches = 0
 
     def _stage(self, dx: torch.Tensor, x: torch.Tensor, dy: torch.Tensor, y: torch.Tensor) -> None:
-        if all(t.device == dx.device and t.dtype == torch.int32 and t.is_contiguous() and t.shape == dx.shape for t in (x, y)):
+        if dx.is_cuda and all(t.device == dx.device and t.dtype == torch.int32 and t.is_contiguous() and t.shape == dx.shape
+                              for t in (x, y)):
             from . import ops
-            ops._check(ops.lib().cme_copy_pair_i32(ops._a(dx), ops._a(x), ops._a(dy), ops._a(y), dx.numel(), ops._st()))
+            with torch.cuda.device(dx.device):
+                ops._check(ops.lib().cme_copy_pair_i32(ops._a(dx), ops._a(x), ops._a(dy), ops._a(y), dx.numel(), ops._st()))
             return
         dx.copy_(x, non_blocking=True)                  # host batches, other types
         dy.copy_(y, non_blocking=True)
