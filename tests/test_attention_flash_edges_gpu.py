@@ -81,3 +81,23 @@ def test_a_key_that_an_infinite_element_hides(T, causal):
         dq = dq.double().reshape(T, H, 64).transpose(0, 1)[..., seen]
         assert ((dq - ref_grads[0][..., seen]).norm() / ref_grads[0][..., seen].norm()).item() < 2 * BF16_REL
         assert dv.reshape(T, H, 64)[j].abs().max().item() == 0 and dk.reshape(T, H, 64)[j].abs().max().item() == 0
+
+
+def test_probability_of_the_largest_of_128_keys_is_exact():
+    """The second block of 64 keys holds a row's largest score, less than the rescaling threshold above the first block's: the
+    probability is 1 at the reference maximum only, and anything else is rounded to 8 bits before it is multiplied with V."""
+    from cme213_final_project_b200 import ops
+    H, T = 3, 128
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k = (torch.zeros(T, H, 64, device="cuda") for _ in range(2))
+    v = torch.randn(T, H, 64, generator=g, device="cuda")
+    q[..., 0] = 3 + 2.3 * torch.rand(T, H, generator=g, device="cuda")       # scores 3 to 5.3, log2 4.3 to 7.6, of key 100,
+    k[..., 0], k[5, :, 0], k[100, :, 0] = -64, 0, 8                          # 0 of key 5, -24 and less of the others
+    q, k, v = (t.to(torch.bfloat16).reshape(T, H * 64) for t in (q, k, v))
+    out, _ = ops.attention_fwd(q, k, v, 1, H, T, "split", False, backend="tc")
+    heads = [t.reshape(T, H, 64).transpose(0, 1) for t in (q, k, v)]
+    ref, _, _ = _reference(*heads, torch.zeros_like(heads[0]), False)
+    rounding = ((ref.to(torch.bfloat16).double() - ref).norm() / ref.norm()).item()
+    err = ((out.reshape(T, H, 64).transpose(0, 1).double() - ref).norm() / ref.norm()).item()
+    # the result is rounded, and the probability of key 5 (a weight of 5 % at most); rounding that of key 100 too gives 1.4
+    assert err < 1.1 * rounding
