@@ -115,9 +115,10 @@ struct Engine {
     cudaStream_t side = nullptr;
     std::vector<cudaEvent_t> ev;                           // [L + 1][8]: four "inputs ready" + four "done" per layer
     // third stream: half of the weight-gradient work where a product is too short to fill the GPU (`two_sides`), and what
-    // nothing in the step waits for (the mean loss and its publication)
+    // nothing in the step waits for (the mean loss and its publication, where `loss_aside`)
     cudaStream_t side2 = nullptr;
     bool two_sides = false;
+    bool loss_aside = false;
     cudaEvent_t ev_aux[4] = {};      // [0] fork of forward's side work  [1] padded output weights ready  [2] row losses
                                      // ready  [3] side2's work done
     bool loss_pending = false;       // side2 holds work that backward's end has to wait for
@@ -337,6 +338,10 @@ CME_API int cme_engine_create(const CmeEngineDesc* desc, const CmeLayerSlots* la
     // A weight gradient of up to 10 GFLOP (7 us of the whole GPU) is latency: a few tiles, each for longer than that.  Step of the
     // parity models, one / two streams: hidden 128 106-111 / 94-101 us, 256 and 512 no difference, 512 with 64 sequences 261 / 254.
     e->two_sides = desc->dtype == CME_BF16 && desc->fuse_epilogues != 0 && 2.0 * e->BT * desc->D * desc->FF <= 1e10;
+    // Beside the chain the loss starts when the head's products, which are enqueued at the same time, leave room: behind them where
+    // they fill the GPU.  A step's loss reaches the host of a GPT-2 small model (1270 GFLOP each) after 5.9-6.0 ms from the chain, after
+    // 6.7 ms from beside it; the 6 us that it takes on the chain are nothing there, and 2-6 % of the parity models' steps.
+    e->loss_aside = 2.0 * e->BT * desc->D * desc->V <= 1e10;
     e->ws_bytes = carve(*e, nullptr);
     *out = e;
     return CME_OK;
@@ -534,13 +539,14 @@ CME_API int cme_engine_forward(void* h, const int* tokens, const int* targets, f
 }
 
 // After a forward that left the mean loss out (loss_out null): *loss_out (+)= loss_weight * mean of the row losses, and the
-// loss published to the host.  Nothing else in a step waits for either, so they run on the third stream where there is one,
-// and cme_engine_backward, which has to follow, makes `stream` wait for them at its end.
+// loss published to the host.  Nothing else in a step waits for either, so they run on the third stream (`loss_aside`), and
+// cme_engine_backward, which has to follow, makes `stream` wait for them at its end.
 CME_API int cme_engine_loss(void* h, float* loss_out, float loss_weight, int accumulate_loss, int* seq, void* host_loss_dev,
                             void* host_seq_dev, void* stream) {
     Engine& e = *static_cast<Engine*>(h);
-    cudaStream_t st = (cudaStream_t)stream, ls = e.side2 ? e.side2 : st;
-    if (e.side2) {
+    const bool aside = e.side2 && e.loss_aside;
+    cudaStream_t st = (cudaStream_t)stream, ls = aside ? e.side2 : st;
+    if (aside) {
         CME_CUDA(cudaEventRecord(e.ev_aux[2], st));
         CME_CUDA(cudaStreamWaitEvent(ls, e.ev_aux[2], 0));
         e.loss_pending = true;

@@ -6,11 +6,11 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _engine(hidden, batch, overlap):
+def _engine(hidden, batch, overlap, vocab=65):
     from cme213_final_project_b200.config import ModelConfig, OptimConfig, RunConfig
     from cme213_final_project_b200.models.engine import NativeEngine
     # GELU: no pre-activation that rounding takes across zero switches a gradient on or off
-    cfg = ModelConfig(vocab_size=65, seq_len=32, hidden=hidden, heads=4, ff=2 * hidden, batch_size=batch, activation="gelu")
+    cfg = ModelConfig(vocab_size=vocab, seq_len=32, hidden=hidden, heads=4, ff=2 * hidden, batch_size=batch, activation="gelu")
     eng = NativeEngine(cfg, OptimConfig(), RunConfig(), device="cuda", seed=3)
     eng.set_overlap(overlap)
     # weights of the size that keeps a layer's output at its input's: with the small uniform start the softmax is flat, and
@@ -94,3 +94,21 @@ def test_fences_of_a_captured_backward(hidden, batch):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(copy, want)
+
+
+@pytest.mark.parametrize("vocab", [65, 4096, 12288])
+def test_loss_beside_short_and_before_long_products_of_the_head(vocab):
+    """The mean loss and its publication run beside the backward pass or, where the head's products are more than 10 GFLOP (the
+    largest vocabulary), before it: the same loss, whichever way it is read, and the same gradients."""
+    runs = []
+    for overlap in (False, True):
+        eng, cfg = _engine(256, 64, overlap, vocab)
+        xs, ys = _batches(cfg, 3)
+        seen = []
+        for i in range(3):
+            eng.seq_expected += 1
+            eng.train_step(xs[:i + 1], ys[:i + 1])          # one to three micro-batches
+            seen.append(eng.wait_loss())
+            assert seen[-1] == eng.read_loss()
+        runs.append((seen, eng.grads.clone()))
+    assert runs[0][0] == runs[1][0] and torch.equal(runs[0][1], runs[1][1])
