@@ -335,9 +335,15 @@ CME_API int cme_engine_create(const CmeEngineDesc* desc, const CmeLayerSlots* la
     e->BH = desc->B * desc->H;
     e->ls.assign(layers, layers + desc->L);
     e->gs = *globals;
-    // A weight gradient of up to 10 GFLOP (7 us of the whole GPU) is latency: a few tiles, each for longer than that.  Step of the
-    // parity models, one / two streams: hidden 128 106-111 / 94-101 us, 256 and 512 no difference, 512 with 64 sequences 261 / 254.
-    e->two_sides = desc->dtype == CME_BF16 && desc->fuse_epilogues != 0 && 2.0 * e->BT * desc->D * desc->FF <= 1e10;
+    // A weight gradient of up to 10 GFLOP (7 us of the whole GPU) is latency: a few tiles, each for longer than that.  Half of them on
+    // a stream of their own pays where the chain leaves SMs idle beside them: with the one-launch attention (up to 64 tokens), or in
+    // models so small that the chain does everywhere.  Flash attention fills the GPU, and then they only take its SMs.  Step in us,
+    // one / two streams of weight gradients.  64 tokens: parity hidden 128 108 / 97, 256 129.5 / 127, 512 240 / 240.5, 512 with 64
+    // and 96 sequences 253 / 247 and 315 / 305; GPT of 2.4, 4.3, 9.7 GFLOP 992 / 981, 861 / 827, 1035 / 1044.  128 and 256 tokens: 0.3,
+    // 0.6, 1.1, 1.2 GFLOP 543 / 530, 330 / 321, 480 / 472, 532 / 532; 1.7, 2.1, 2.4, 4.3, 9.7 GFLOP 637 / 640, 655 / 678, 384 / 389.5,
+    // 1240 / 1267, 1632 / 1663.
+    e->two_sides = desc->dtype == CME_BF16 && desc->fuse_epilogues != 0 &&
+                   2.0 * e->BT * desc->D * desc->FF <= (desc->T <= 64 ? 1e10 : 1.5e9);
     // Beside the chain the loss starts when the head's products, which are enqueued at the same time, leave room: behind them where
     // they fill the GPU.  A step's loss reaches the host of a GPT-2 small model (1270 GFLOP each) after 5.9-6.0 ms from the chain, after
     // 6.7 ms from beside it; the 6 us that it takes on the chain are nothing there, and 2-6 % of the parity models' steps.
