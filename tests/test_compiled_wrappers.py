@@ -1,4 +1,5 @@
 """The compiled wrappers refuse what the Python statements before them refused, and give the same objects back."""
+import numpy as np
 import pytest
 import torch
 
@@ -58,21 +59,52 @@ def test_objects_that_the_caller_passed_come_back():
         ops.embedding_bwd(i, x, 4, 3)                       # 8 tokens are not whole sequences of 3
 
 
+@pytest.fixture
+def poisoned():
+    """Every tensor that torch allocates starts as NaN, the largest number where it holds whole ones (torch's own debugging aid)."""
+    torch.use_deterministic_algorithms(True)
+    assert torch.empty(1000, device="cuda").isnan().all() and (torch.empty(1000, dtype=torch.uint8, device="cuda") == 255).all()
+    yield
+    torch.use_deterministic_algorithms(False)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("T,HD,layout,dtype", [(64, 64, "split", torch.bfloat16), (64, 128, "flat", torch.bfloat16), (96, 64, "split", torch.bfloat16),
                                                (96, 128, "flat", torch.bfloat16), (64, 128, "split", torch.bfloat16), (64, 64, "flat", torch.float32)])
-def test_each_attention_path_gets_its_scratch(T, HD, layout, dtype):
-    """Every path of the dispatch, with scratch that earlier calls left full of NaN."""
+def test_each_attention_path_gets_its_scratch(poisoned, T, HD, layout, dtype):
+    """Every path of the dispatch and every way to complete dQ, with results and scratch in memory full of NaN: what a kernel reads
+    it, or the wrapper, has written."""
     B, H = 2, 4
     g = torch.Generator(device="cuda").manual_seed(1)
     q, k, v, do = (torch.randn(B * T, H * HD, generator=g, device="cuda").to(dtype) for _ in range(4))
     want = ops.attention_fwd(q, k, v, B, H, T, layout, True, backend="simt")
     want_grads = ops.attention_bwd(q, k, v, *want, do, B, H, T, layout, True, backend="simt")
-    for _ in range(2):
-        torch.full((8 << 20,), float("nan"), device="cuda")
+    for mode in (0, 1, 2):
         out, lse = ops.attention_fwd(q, k, v, B, H, T, layout, True)
-        grads = ops.attention_bwd(q, k, v, out, lse, do, B, H, T, layout, True)
+        grads = ops.attention_bwd(q, k, v, out, lse, do, B, H, T, layout, True, dq_mode=mode)
         # bf16: P, dS and the results rounded to 8 bits on either side
         tol = 2.0 ** -6 if dtype == torch.bfloat16 else 1e-5
         for a, b in zip((out, lse) + tuple(grads), want + tuple(want_grads)):
             assert ((a.float() - b.float()).norm() / b.float().norm()).item() < tol
+    scratch = torch.empty(q.numel(), device="cuda"), torch.empty(B * H * ((T + 127) // 128), dtype=torch.int32, device="cuda")
+    grads = ops.attention_bwd(q, k, v, out, lse, do, B, H, T, layout, True, scratch=scratch)
+    assert all(t.isfinite().all() for t in grads)           # (mode 0 clears the accumulator that it is given)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("yes,no", [(np.bool_(True), np.bool_(False)), (1.0, 0.0), (np.int64(1), 0)])
+def test_flags_are_what_counts_as_true(yes, no):
+    g = torch.Generator(device="cuda").manual_seed(2)
+    q, k, v, do = (torch.randn(40, 64, generator=g, device="cuda").to(torch.bfloat16) for _ in range(4))
+    for flag, plain in ((yes, True), (no, False)):
+        out, lse = ops.attention_fwd(q, k, v, 1, 1, 40, causal=flag)
+        want, want_lse = ops.attention_fwd(q, k, v, 1, 1, 40, causal=plain)
+        assert torch.equal(out, want) and torch.equal(lse, want_lse)
+        for a, b in zip(ops.attention_bwd(q, k, v, out, lse, do, 1, 1, 40, causal=flag),
+                        ops.attention_bwd(q, k, v, out, lse, do, 1, 1, 40, causal=plain)):
+            assert torch.equal(a, b)
+        sums = [torch.ones(64, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+        ops.dact_colsum(do, dbias=sums[0], accumulate=flag)
+        ops.dact_colsum(do, dbias=sums[1], accumulate=plain)
+        assert torch.equal(*sums)
+        assert (ops.bias_act_residual(q, save_pre=flag)[1] is None) == (not plain)

@@ -27,5 +27,24 @@ def test_product_flags(monkeypatch, yes, no):
 
 
 @pytest.mark.parametrize("causal,want", [(np.bool_(True), 1), (np.bool_(False), 0), (1.0, 1), (0, 0)])
-def test_attention_flag(causal, want):
-    assert ops._attn_desc(torch.zeros(8, 64), 1, 1, 8, "split", causal).causal == want
+def test_attention_flag(monkeypatch, causal, want):
+    seen = []
+
+    class Native:
+        @staticmethod
+        def attention_fwd(*args):
+            seen.append(args[3:])
+            return None, None
+
+        @staticmethod
+        def attention_bwd(*args):
+            seen.append(args[6:])
+            return None, None, None
+
+    monkeypatch.setattr(ops, "_native", lambda: Native)
+    x = torch.zeros(8, 64)
+    ops.attention_fwd(x, x, x, 1, 1, 8, "split", causal)
+    ops.attention_bwd(x, x, x, x, x, x, 1, 1, 8, "flat", causal, ordered_dq=True)
+    # B, H, T, flat, causal, backend and, backward, the way dQ is completed and the caller's scratch
+    assert seen == [(1, 1, 8, False, want, 0), (1, 1, 8, True, want, 0, 1, None, None)]
+    assert all(type(args[4]) is int for args in seen)
