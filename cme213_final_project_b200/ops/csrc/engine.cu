@@ -224,26 +224,6 @@ int gemm(const Engine& e, cudaStream_t st, int M, int N, int K, const void* A, l
     return cme_gemm(&g, e.d.gemm_backend, st);
 }
 
-// C = sum of three products A_i B_i^T whose operands lie planeA / planeB elements apart (d ln1 from the planes of dQ, dK, dV):
-// one reduction over the planes where the tensor-core kernel takes it, else three products that accumulate.
-int gemm_planes(const Engine& e, cudaStream_t st, int M, int N, int K, const char* A, long long lda, long long planeA,
-                const char* B, long long ldb, long long planeB, void* C, long long ldc) {
-    CmeGemm g{};
-    g.M = M; g.N = N; g.K = K; g.batch = 1;
-    g.A = A; g.lda = lda;
-    g.B = B; g.ldb = ldb; g.b_trans = 1;
-    g.C = C; g.ldc = ldc; g.c_dtype = e.d.dtype; g.ab_dtype = e.d.dtype;
-    g.workspace = e.gemm_ws; g.workspace_bytes = e.gemm_ws_bytes;
-    if (e.d.dtype == CME_BF16 && e.d.gemm_backend != 2 && planeA % 8 == 0 && planeB % 8 == 0 && gemm_tcgen05_supported(&g))
-        return gemm_tcgen05_launch(&g, st, 3, planeA, planeB);
-    for (int i = 0; i < 3; ++i) {
-        const int rc = gemm(e, st, M, N, K, A + i * planeA * (long long)e.es, lda, 0, B + i * planeB * (long long)e.es, ldb, 1, C,
-                            ldc, i > 0);
-        if (rc) return rc;
-    }
-    return CME_OK;
-}
-
 // A plain product of bf16 operands with an fp32 result (the reduced-precision feed-forward experiment).
 int gemm_lp(const Engine& e, cudaStream_t st, int M, int N, int K, const void* A, long long lda, int a_trans,
             const void* B, long long ldb, int b_trans, void* C, long long ldc, int accumulate = 0) {
@@ -338,8 +318,8 @@ CME_API int cme_engine_create(const CmeEngineDesc* desc, const CmeLayerSlots* la
     // A weight gradient of up to 10 GFLOP (7 us of the whole GPU) is latency: a few tiles, each for longer than that.  Half of them on
     // a stream of their own pays where the chain leaves SMs idle beside them: with the one-launch attention (up to 64 tokens), or in
     // models so small that the chain does everywhere.  Flash attention fills the GPU, and then they only take its SMs.  Step in us,
-    // one / two streams of weight gradients.  64 tokens: parity hidden 128 108 / 97, 256 129.5 / 127, 512 240 / 240.5, 512 with 64
-    // and 96 sequences 253 / 247 and 315 / 305; GPT of 2.4, 4.3, 9.7 GFLOP 992 / 981, 861 / 827, 1035 / 1044.  128 and 256 tokens: 0.3,
+    // one / two streams of weight gradients.  64 tokens: parity hidden 128 108 / 103, 256 138 / 134, 512 249 / 250, 512 with 64
+    // and 96 sequences 262 / 257.5 and 333 / 328; GPT of 2.4, 4.3, 9.7 GFLOP 992 / 981, 861 / 827, 1035 / 1044.  128 and 256 tokens: 0.3,
     // 0.6, 1.1, 1.2 GFLOP 543 / 530, 330 / 321, 480 / 472, 532 / 532; 1.7, 2.1, 2.4, 4.3, 9.7 GFLOP 637 / 640, 655 / 678, 384 / 389.5,
     // 1240 / 1267, 1632 / 1663.
     e->two_sides = desc->dtype == CME_BF16 && desc->fuse_epilogues != 0 &&
@@ -735,7 +715,9 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
             TRY(gemm(e, st, BT, D, 3 * D, e.dqkv, 3 * D, 0, e.P(s.Wqkv), 3 * D, 1, e.dln, D));
             TRY(gemm(e, ws, D, 3 * D, BT, a.ln1, D, 1, e.dqkv, 3 * D, 0, e.G(s.Wqkv), 3 * D, accumulate));
         } else {
-            TRY(gemm_planes(e, st, BT, D, D, e.dqkv, D, (long long)BT * D, e.P(s.Wq), D, (long long)D * D, e.dln, D));
+            const long long pl = (long long)BT * D * e.es, wm = (long long)D * D * e.es;
+            for (int i = 0; i < 3; ++i)
+                TRY(gemm(e, st, BT, D, D, e.dqkv + i * pl, D, 0, e.P(s.Wq) + i * wm, D, 1, e.dln, D, i > 0));
             TRY(gemm(e, ws, D, D, BT, a.ln1, D, 1, e.dqkv, D, 0, e.G(s.Wq), D, accumulate, nullptr, 0, nullptr, 0,
                      nullptr, 0, nullptr, 0, 3, 0, (long long)BT * D, (long long)D * D));
         }

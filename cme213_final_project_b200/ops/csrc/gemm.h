@@ -44,6 +44,5 @@ struct CmeGemm {
 };
 
 int gemm_tcgen05_supported(const CmeGemm* g);
-// planes > 1 (batch 1): C (+)= sum of `planes` products whose operands lie planeA / planeB elements apart, as one reduction.
-int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream, int planes = 1, long long planeA = 0, long long planeB = 0);
+int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream);
 int gemm_simt_launch(const CmeGemm* g, cudaStream_t stream);

@@ -284,7 +284,7 @@ int gemm_tcgen05_supported(const CmeGemm* g) {
     return 1;
 }
 
-int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream, int planes, long long planeA, long long planeB) {
+int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream) {
     CME_REQUIRE(gemm_tcgen05_supported(g), CME_ERR_SHAPE, "gemm shape/alignment not supported by the tcgen05 kernel");
     CmeDeviceState* ds;
     {
@@ -300,12 +300,11 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream, int planes, long 
     const bool tf32 = g->ab_dtype == CME_F32;
     const int BK = tf32 ? 32 : 64;                            // K elements per 128-byte k-block
     int tiles_m = cme_cdiv(g->M, BM);
-    const int kb_per_plane = cme_cdiv(g->K, BK), num_kb = planes * kb_per_plane;
-    CME_REQUIRE(planes == 1 || (g->batch == 1 && planeA % 8 == 0 && planeB % 8 == 0), CME_ERR_SHAPE, "gemm: operand planes");
+    const int num_kb = cme_cdiv(g->K, BK);
     const bool plain_epi = !g->bias && !g->residual && !g->aux_out && !g->act && !g->dact;
     int bn = 0, splits = 0;
     bool pair = false;
-    plan_tiles(g->M, g->N, planes > 1 ? num_kb * BK : g->K, g->batch, plain_epi, g->workspace ? g->workspace_bytes : 0, g_num_sms, g_max_pairs,
+    plan_tiles(g->M, g->N, g->K, g->batch, plain_epi, g->workspace ? g->workspace_bytes : 0, g_num_sms, g_max_pairs,
                g->force_bn, g->force_splits, &bn, &pair, &splits, BK, (g->a_trans != 0) + (g->b_trans == 0));
     // A tf32 product that accumulates into C goes through the fp32 workspace like a split-K product (one "split"
     // is then added to C by the reduction kernel): the tf32 kernel variants only store.
@@ -330,25 +329,21 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream, int planes, long 
     int kb_per = cme_cdiv(num_kb, splits);
     splits = cme_cdiv(num_kb, kb_per);
 
-    // the third coordinate of the operands' tensor maps: the batch, or the planes of one reduction
-    const int za = planes > 1 ? planes : g->strideA ? g->batch : 1, zb = planes > 1 ? planes : g->strideB ? g->batch : 1;
-    const long long sza = planes > 1 ? planeA : g->strideA, szb = planes > 1 ? planeB : g->strideB;
     CUtensorMap ta, tb;
     int rc;
     // A: K-major -> map (K, M), box (64, 128); MN-major -> map (M, K), box (64, 64)
-    if (!g->a_trans) rc = make_tmap(&ta, g->A, g->K, g->M, g->lda, za, sza, BM, tf32, tf32);
-    else             rc = make_tmap(&ta, g->A, g->M, g->K, g->lda, za, sza, BK, tf32, tf32, true);
+    if (!g->a_trans) rc = make_tmap(&ta, g->A, g->K, g->M, g->lda, g->strideA ? g->batch : 1, g->strideA, BM, tf32, tf32);
+    else             rc = make_tmap(&ta, g->A, g->M, g->K, g->lda, g->strideA ? g->batch : 1, g->strideA, BK, tf32, tf32, true);
     if (rc) return rc;
     // B: stored [N, K] (b_trans) is K-major -> map (K, N), box (64, bn); stored [K, N] -> map (N, K), box (64, 64)
-    if (g->b_trans) rc = make_tmap(&tb, g->B, g->K, g->N, g->ldb, zb, szb,
+    if (g->b_trans) rc = make_tmap(&tb, g->B, g->K, g->N, g->ldb, g->strideB ? g->batch : 1, g->strideB,
                                    pair ? bn / 2 : bn, tf32, tf32);
-    else            rc = make_tmap(&tb, g->B, g->N, g->K, g->ldb, zb, szb, BK, tf32, tf32, true);
+    else            rc = make_tmap(&tb, g->B, g->N, g->K, g->ldb, g->strideB ? g->batch : 1, g->strideB, BK, tf32, tf32, true);
     if (rc) return rc;
 
     EpiParams ep{};
     ep.M = g->M; ep.N = g->N; ep.K = g->K; ep.batch = g->batch;
     ep.tiles_m = tiles_m; ep.tiles_n = tiles_n; ep.splits = splits; ep.kb_per_split = kb_per; ep.num_kb = num_kb;
-    ep.kb_per_plane = kb_per_plane;
     ep.a_batched = g->strideA != 0 && g->batch > 1; ep.b_batched = g->strideB != 0 && g->batch > 1;
     {
         // Tile order by estimated DRAM traffic.  The CTAs that run together walk K at about the same pace, so the

@@ -98,7 +98,6 @@ template <int BN, bool PAIR, bool SIMPLE, int SPEC = -1> struct Cfg {
 struct EpiParams {
     int M, N, K, batch;
     int tiles_m, tiles_n, splits, kb_per_split, num_kb;
-    int kb_per_plane;              // k-blocks of one operand plane: num_kb unless the reduction runs over several planes
     int stream_aux;                // the auxiliary tensors (activation derivative written by forward, read once by backward)
                                    // go through L2 with the evict-first policy
     int n_fast;                    // tile order: 0 = consecutive tiles walk down M (share a B stripe), 1 = across N (share A rows)
@@ -437,11 +436,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const int n0 = tn * BN + int(cta_rank) * C::BN_LOCAL;
                 const int kb0 = split * p.kb_per_split;
                 const int kb1 = min(kb0 + p.kb_per_split, p.num_kb);
-                // (several planes: only with batch 1)
-                int plane = kb0 / p.kb_per_plane, kp = kb0 - plane * p.kb_per_plane;
-                for (int kb = kb0; kb < kb1; ++kb, ++kp) {
-                    if (kp == p.kb_per_plane) { kp = 0; ++plane; }
-                    const int za = p.a_batched ? bidx : plane, zb = p.b_batched ? bidx : plane;
+                const int za = p.a_batched ? bidx : 0, zb = p.b_batched ? bidx : 0;
+                for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
                     uint8_t* sA = smem + stage * C::STAGE_BYTES;
                     uint8_t* sB = sA + A_TILE_BYTES;
@@ -450,34 +446,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * C::STAGE_BYTES);
                         const uint32_t fb = mapa_u32(&full_bar[stage], 0);
                         if (!A_MN) {
-                            tma_load_3d_pair(sA, &tmA, fb, kp * BK, m0, za);
+                            tma_load_3d_pair(sA, &tmA, fb, kb * BK, m0, za);
                         } else {
 #pragma unroll
                             for (int j = 0; j < BM / GW; ++j)
-                                tma_load_3d_pair(sA + j * GROUP_BYTES, &tmA, fb, m0 + j * GW, kp * BK, za);
+                                tma_load_3d_pair(sA + j * GROUP_BYTES, &tmA, fb, m0 + j * GW, kb * BK, za);
                         }
                         if (!B_MN) {
-                            tma_load_3d_pair(sB, &tmB, fb, kp * BK, n0, zb);
+                            tma_load_3d_pair(sB, &tmB, fb, kb * BK, n0, zb);
                         } else {
 #pragma unroll
                             for (int j = 0; j < C::BN_LOCAL / GW; ++j)
-                                tma_load_3d_pair(sB + j * GROUP_BYTES, &tmB, fb, n0 + j * GW, kp * BK, zb);
+                                tma_load_3d_pair(sB + j * GROUP_BYTES, &tmB, fb, n0 + j * GW, kb * BK, zb);
                         }
                     } else {
                         mbar_arrive_expect_tx(&full_bar[stage], C::STAGE_BYTES);
                         if (!A_MN) {
-                            tma_load_3d(sA, &tmA, &full_bar[stage], kp * BK, m0, za);
+                            tma_load_3d(sA, &tmA, &full_bar[stage], kb * BK, m0, za);
                         } else {
 #pragma unroll
                             for (int j = 0; j < BM / GW; ++j)
-                                tma_load_3d(sA + j * GROUP_BYTES, &tmA, &full_bar[stage], m0 + j * GW, kp * BK, za);
+                                tma_load_3d(sA + j * GROUP_BYTES, &tmA, &full_bar[stage], m0 + j * GW, kb * BK, za);
                         }
                         if (!B_MN) {
-                            tma_load_3d(sB, &tmB, &full_bar[stage], kp * BK, n0, zb);
+                            tma_load_3d(sB, &tmB, &full_bar[stage], kb * BK, n0, zb);
                         } else {
 #pragma unroll
                             for (int j = 0; j < BN / GW; ++j)
-                                tma_load_3d(sB + j * GROUP_BYTES, &tmB, &full_bar[stage], n0 + j * GW, kp * BK, zb);
+                                tma_load_3d(sB + j * GROUP_BYTES, &tmB, &full_bar[stage], n0 + j * GW, kb * BK, zb);
                         }
                     }
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }

@@ -1,5 +1,4 @@
-"""The engine's extra streams (weight gradients, mean loss, padded output weights) against the same step on one stream, and the
-one reduction over the planes of dQ, dK, dV at inner sizes that end inside a block of 64."""
+"""The engine's extra streams (weight gradients, mean loss, padded output weights) against the same step on one stream."""
 import pytest
 import torch
 
@@ -32,7 +31,7 @@ def _batches(cfg, n):
 
 @pytest.mark.parametrize("micro", [1, 3])
 @pytest.mark.parametrize("hidden", [32, 64, 96, 200, 256])
-def test_streams_and_planes_give_the_step_of_one_stream(hidden, micro):
+def test_streams_give_the_step_of_one_stream(hidden, micro):
     from cme213_final_project_b200.config import OptimConfig
     from cme213_final_project_b200.models.reference import ReferenceModel
     runs = []
