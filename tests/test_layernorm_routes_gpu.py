@@ -58,3 +58,28 @@ def test_operands_off_a_vector_boundary(dtype, rows, D):
     a = [t.clone() for t in (y, x, gamma, res)]
     want_dx, want_dg, want_db = ops.layernorm_bwd(a[0], a[1], a[2], mean, rstd, dres=a[3])
     assert _close(dx, want_dx.double(), dtype) and _close(dg, want_dg.double(), dtype) and _close(db, want_db.double(), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,D", [(300, 64), (300, 520), (300, 768), (8193, 768), (20001, 384)])
+def test_order_of_a_row_sum(dtype, rows, D):
+    """The mean bit for bit: a lane adds the elements of its 16-byte vectors (lane, lane + 32, ...) one after the other, then the
+    32 lanes are added in pairs at distances 16, 8, 4, 2, 1.  A whole model's later bits hang on this order."""
+    from cme213_final_project_b200 import ops
+    if D % (16 // dtype.itemsize) or D > 32 * 4 * (16 // dtype.itemsize):
+        pytest.skip("rows that the vector kernels do not take")
+    x, _, gamma, beta = _inputs(rows, D, dtype, 3)
+    _, mean, _, _ = ops.layernorm_fwd(x, gamma, beta)
+    w = 16 // dtype.itemsize
+    n = -(-D // (32 * w))
+    v = torch.zeros(rows, n * 32 * w, device="cuda")
+    v[:, :D] = x.float()                                    # (adding zeros changes nothing)
+    v = v.view(rows, n, 32, w)
+    lanes = torch.zeros(rows, 32, device="cuda")
+    for i in range(n):
+        for j in range(w):
+            lanes = lanes + v[:, i, :, j]
+    at = torch.arange(32, device="cuda")
+    for distance in (16, 8, 4, 2, 1):
+        lanes = lanes + lanes[:, at ^ distance]
+    assert torch.equal(mean, lanes[:, 0] / torch.full_like(mean, D))       # (by a number, torch multiplies by its reciprocal)
