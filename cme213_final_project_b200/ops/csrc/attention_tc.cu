@@ -18,13 +18,14 @@
 //     either (dq_mode 0, the default) the launch clears the scratch first and a small kernel scales and casts the
 //     sums afterwards, or (dq_mode 2) a counter per tile tells the CTA whose part arrived last to do that itself --
 //     a spare warp converts the tile and writes zeros back, so no clearing or conversion pass runs; the query
-//     blocks are then walked downwards so that the finishing work spreads over the CTAs.  Still slower at large shapes
-//     (about 0.05 ms per call at 16 x 12 heads x 1024 tokens: every reduce-add has to complete before its part is
-//     counted in, and one warp converts a 32 KB tile).  Deterministic form (dq_mode 1): the
+//     blocks are then walked downwards so that the finishing work spreads over the CTAs.  Still slower: every reduce-add
+//     has to complete before its part is counted in, and one warp converts a 32 KB tile.  Deterministic form (dq_mode 1): the
 //     highest key block stores its part, each lower one adds its own when the tile's counter says it is its turn,
 //     and key block 0, whose turn is last, adds the sum to its part in registers, scales, casts and writes dQ --
-//     bit-reproducible, no clearing or conversion pass, but the chain of turns makes CTAs wait for one another
-//     (measured 0.32 ms against 0.25 ms per call at 16 x 12 heads x 1024 tokens).  dq_mode 1 and 2 have a kernel of their own.
+//     bit-reproducible, no clearing or conversion pass, but the chain of turns makes CTAs wait for one another.  Whole backward in
+//     modes 0 / 1 / 2: 16 x 12 heads x 1024 tokens 183 / 283 / 279 us causal, 290 / 500 / 389 all keys; 64 x 6 x 256 causal
+//     58 / 78 / 107.
+// Grids that fill the GPU take small CTAs, several to an SM; others, and the backward's modes 1 and 2, 128 x 128 blocks.
 // Every mbarrier wait is bounded; on expiry the CTA flags the status word, frees TMEM and returns.
 #include "attention.h"
 #include "sm100_ptx.cuh"
@@ -325,6 +326,252 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     __syncthreads();
     if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, CME_ERR_TIMEOUT);
     if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem_base, FWD_TMEM_COLS); }
+}
+
+// ------------------------------------------------------------------------------------------------------
+// Forward of grids that leave the small CTAs above without neighbours (fwd_wide)
+// ------------------------------------------------------------------------------------------------------
+// 128 keys per step in a CTA of which two fit an SM: S_j is copied to registers, the tensor core makes S_{j+1} while softmax_j runs, and P
+// has columns of its own.  Alone on its SM, a CTA gets through its keys in 0.6 of the time that the small one takes.
+// shared: Q 16K | K[3] 48K | V[3] 48K | barriers      (P never passes through shared memory)
+constexpr int FWD_WIDE_STAGES = 3;           // a K / V tile is requested two blocks ahead of its use: its ~1200-clock
+                                           // latency no longer delays the next S product
+constexpr int FWD_WIDE_SMEM = (1 + 2 * FWD_WIDE_STAGES) * TILE_BYTES + 128;   // two CTAs per SM: 2 x (this + 1 KB) <= 228 KB
+constexpr int FWD_WIDE_TMEM_COLS = 256;         // S: [0,128)  O accumulator: [128,192)  P (bf16 pairs): [192,256)
+static_assert(2 * (FWD_WIDE_SMEM + 1024) <= 228 * 1024, "two forward CTAs must fit one SM's shared memory");
+static_assert(128 + HD + BKV / 2 <= FWD_WIDE_TMEM_COLS && 2 * FWD_WIDE_TMEM_COLS <= 512,
+              "forward TMEM budget: S + O + P per CTA, two CTAs per SM");
+
+__global__ void __launch_bounds__(FWD_THREADS, 2)
+attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FwdParams p) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    if (smem_u32(smem) & 1023u) {             // swizzled tiles need a 1024-byte aligned base
+        if (threadIdx.x == 0 && p.status) atomicExch(p.status, CME_ERR_SHAPE);
+        return;
+    }
+    uint8_t* sQ = smem;
+    uint8_t* sK = sQ + TILE_BYTES;                            // FWD_WIDE_STAGES stages
+    uint8_t* sV = sK + FWD_WIDE_STAGES * TILE_BYTES;            // FWD_WIDE_STAGES stages
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + FWD_WIDE_STAGES * TILE_BYTES);
+    uint64_t* q_full = bars;                  // 1
+    uint64_t* kv_full = bars + 1;             // [3]
+    uint64_t* kv_empty = bars + 4;            // [3]
+    uint64_t* s_full = bars + 7;              // S ready for softmax
+    uint64_t* s_free = bars + 8;              // S copied to registers (128 arrivals): the next S may be issued
+    uint64_t* p_ready = bars + 9;             // P written to tensor memory, O rescaled (128 arrivals)
+    uint64_t* o_full = bars + 10;             // P V accumulated, P consumed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int qt = gridDim.x - 1 - blockIdx.x;               // heavy (late) causal tiles first
+    const int q0 = qt * BQ;
+    const int bh = blockIdx.y, b = bh / p.nh, h = bh % p.nh;
+    const int nkv = p.causal ? min((q0 + BQ + BKV - 1) / BKV, (p.T + BKV - 1) / BKV) : (p.T + BKV - 1) / BKV;
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        mbar_init(q_full, 1);
+        for (int s = 0; s < FWD_WIDE_STAGES; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
+        mbar_init(s_full, 1);
+        mbar_init(s_free, 128);
+        mbar_init(p_ready, 128);
+        mbar_init(o_full, 1);
+        fence_barrier_init();
+    }
+    if (warp == 4) { tmem_alloc(tmem_slot, FWD_WIDE_TMEM_COLS); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + 128, tmem_P = tmem_base + 128 + HD;
+    pdl_wait();        // barrier set-up and TMEM allocation above may overlap the tail of the previous kernel
+
+    if (warp == 4) {
+        if (lane == 0) {
+            // ---------------- producer + MMA issuer (one thread) ----------------
+            constexpr uint32_t idesc_s = make_idesc(1, false, false, 128, 128);   // Q K^T: both K-major
+            constexpr uint32_t idesc_o = make_idesc(1, false, true, 128, HD);     // P V: V is MN-major
+            bool ok = true;
+            mbar_arrive_expect_tx(q_full, TILE_BYTES);
+            tma_load_4d(sQ, &tmQ, q_full, 0, q0, h, b);
+            auto load_kv = [&](int j) {
+                const int st = j % FWD_WIDE_STAGES;
+                mbar_arrive_expect_tx(&kv_full[st], 2 * TILE_BYTES);
+                tma_load_4d(sK + st * TILE_BYTES, &tmK, &kv_full[st], 0, j * BKV, h, b);
+                tma_load_4d(sV + st * TILE_BYTES, &tmV, &kv_full[st], 0, j * BKV, h, b);
+            };
+            const uint64_t dQ_ = make_smem_desc(smem_u32(sQ), 0, 1024);
+            const uint64_t dK0 = make_smem_desc(smem_u32(sK), 0, 1024);
+            const uint64_t dV0 = make_smem_desc(smem_u32(sV), TILE_BYTES, 1024);
+            auto issue_s = [&](int j) {
+                const uint64_t kd = desc_add(dK0, (j % FWD_WIDE_STAGES) * TILE_BYTES);
+#pragma unroll
+                for (int k = 0; k < HD / 16; ++k)
+                    mma_f16_ss(tmem_S, desc_add(dQ_, k * 32), desc_add(kd, k * 32), idesc_s, k > 0);
+                mma_commit(s_full);
+            };
+            for (int j = 0; j < FWD_WIDE_STAGES && j < nkv; ++j) load_kv(j);
+            ok = mbar_wait(q_full, 0, abort_flag) && mbar_wait(&kv_full[0], 0, abort_flag);
+            if (ok) { tc_fence_after(); issue_s(0); }
+            for (int j = 0; j < nkv && ok; ++j) {
+                const int st = j % FWD_WIDE_STAGES;
+                if (j >= 1 && j + 2 < nkv) {
+                    // the stage that block j - 1 used is refilled with block j + 2: its P V product was issued one
+                    // block ago, so this wait does not hold anything up
+                    if (!mbar_wait(&kv_empty[(j - 1) % FWD_WIDE_STAGES], ((j - 1) / FWD_WIDE_STAGES) & 1, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    load_kv(j + 2);
+                }
+                if (j + 1 < nkv) {
+                    // S_j sits in registers now: the tensor core computes S_{j+1} while softmax_j runs
+                    if (!mbar_wait(s_free, j & 1, abort_flag) ||
+                        !mbar_wait(&kv_full[(j + 1) % FWD_WIDE_STAGES], ((j + 1) / FWD_WIDE_STAGES) & 1, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    issue_s(j + 1);
+                }
+                if (!mbar_wait(p_ready, j & 1, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                const uint64_t vd = desc_add(dV0, st * TILE_BYTES);
+#pragma unroll
+                for (int k = 0; k < BKV / 16; ++k)       // A = P from tensor memory: 16 keys = 8 columns per step
+                    mma_f16_ts(tmem_O, tmem_P + k * 8, desc_add(vd, k * 2048), idesc_o, (j > 0 || k > 0));
+                mma_commit(o_full);
+                mma_commit(&kv_empty[st]);
+            }
+            if (!ok) for (int i = 0; i < 2000; ++i) __nanosleep(500);
+        }
+    } else {
+        // ---------------- softmax warps: thread = query row ----------------
+        const int row = warp * 32 + lane;                 // 0..127 == TMEM lane
+        const int q = q0 + row;
+        const uint32_t lane_addr = uint32_t(warp * 32) << 16;
+        float m_ref = -INFINITY, l = 0.f;                 // reference maximum (log2 units) and running row sum
+        bool ok = true;
+        for (int j = 0; j < nkv && ok; ++j) {
+            if (!mbar_wait(s_full, j & 1, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            uint32_t r[128];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) tmem_ld32(tmem_S + lane_addr + c * 32, r + c * 32);
+            tmem_wait_ld();
+            tc_fence_before();
+            mbar_arrive(s_free);
+            const int k0 = j * BKV;
+            if ((k0 + BKV > p.T) || (p.causal && k0 + BKV - 1 > q0)) {        // diagonal or ragged block
+                // keys [0, lim) of this block are visible to this row: one compare and one select per score
+                const int lim = min(p.T, p.causal ? q + 1 : p.T) - k0;
+#pragma unroll
+                for (int i = 0; i < 128; ++i) r[i] = i < lim ? r[i] : 0xff800000u;     // -inf
+            }
+            // eight independent chains (a single one would be 128 dependent operations long)
+            float mx8[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) mx8[c] = __uint_as_float(r[c]);
+#pragma unroll
+            for (int i = 8; i < 128; ++i) mx8[i & 7] = fmaxf(mx8[i & 7], __uint_as_float(r[i]));
+            float mx = fmaxf(fmaxf(fmaxf(mx8[0], mx8[1]), fmaxf(mx8[2], mx8[3])),
+                             fmaxf(fmaxf(mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7])));
+            mx *= p.scale_log2;                            // scale > 0, so the maximum commutes with it
+            // Raise the reference maximum only when it would grow by more than the threshold: the accumulated
+            // output then needs a rescale, which is rare after the first blocks.
+            const bool raise = (j == 0) ? true : (mx > m_ref + RESCALE_THRESHOLD);
+            float alpha = 1.f;
+            if (raise) {
+                alpha = (m_ref == -INFINITY) ? 0.f : ex2_approx(m_ref - mx);
+                m_ref = mx;
+            }
+            if (j > 0) {
+                // the previous P V product must be complete before P is overwritten or O is rescaled
+                if (!mbar_wait(o_full, (j - 1) & 1, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                if (__any_sync(0xffffffffu, raise)) {
+#pragma unroll 1
+                    for (int c = 0; c < HD / 16; ++c) {       // 16 columns at a time: the score row stays in registers
+                        uint32_t o[16];
+                        tmem_ld16(tmem_O + lane_addr + c * 16, o);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st16(tmem_O + lane_addr + c * 16, o);
+                    }
+                    tmem_wait_st();
+                }
+                l *= alpha;
+            }
+            const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
+            // scale-and-shift and the row sum on packed pairs (one instruction per two keys); four independent chains
+            const F32x2 sc2 = f2_splat(p.scale_log2), nm2 = f2_splat(-m_use);
+            F32x2 sum2[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) sum2[c] = f2_splat(0.f);
+            // In passes over 32 keys, so that the 16 scale-and-shifts, then the 32 exponentials, then the sums and
+            // stores are each a run of independent instructions (no exponential waits for its own operand or result)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float* x = reinterpret_cast<float*>(r + c * 32);
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) f2_unpack(f2_fma(f2_pack(x[i], x[i + 1]), sc2, nm2), x[i], x[i + 1]);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) x[i] = ex2_approx(x[i]);
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) sum2[(i >> 1) & 3] = f2_add(sum2[(i >> 1) & 3], f2_pack(x[i], x[i + 1]));
+                // 32 probabilities = 16 columns of bf16 pairs, straight into the A operand of the P V product
+                uint32_t pw[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) pw[i] = f2_to_bf2(x[2 * i], x[2 * i + 1]);
+                tmem_st16(tmem_P + lane_addr + c * 16, pw);
+            }
+            tmem_wait_st();
+            {
+                float s0, s1;
+                f2_unpack(f2_add(f2_add(sum2[0], sum2[1]), f2_add(sum2[2], sum2[3])), s0, s1);
+                l += s0 + s1;
+            }
+            tc_fence_before();
+            mbar_arrive(p_ready);
+        }
+        if (ok && nkv > 0) {
+            if (mbar_wait(o_full, (nkv - 1) & 1, abort_flag)) {
+                tc_fence_after();
+                float o[HD];
+#pragma unroll
+                for (int c = 0; c < HD / 32; ++c) {
+                    uint32_t t[32];
+                    tmem_ld32(tmem_O + lane_addr + c * 32, t);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) o[c * 32 + i] = __uint_as_float(t[i]);
+                }
+                const float inv = l > 0.f ? 1.f / l : 0.f;
+#pragma unroll
+                for (int i = 0; i < HD; ++i) o[i] *= inv;
+                // stage this warp's 32 rows (every product is complete and no load is in flight: the first K stage is
+                // free) and store them with one TMA tile store
+                uint8_t* stage = sK + warp * 4096;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) *reinterpret_cast<uint4*>(stage + swz(lane, g)) = pack8(o + g * 8);
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_4d(&tmO, stage, 0, q0 + warp * 32, h, b);
+                    tma_store_commit();
+                    tma_store_wait_read<0>();         // shared memory may go once the copy engine has read the tile
+                }
+                if (q < p.T) p.lse[(long long)bh * p.T + q] = (m_ref == -INFINITY) ? -INFINITY : (m_ref + log2f(l)) / LOG2E;
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, CME_ERR_TIMEOUT);
+    if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem_base, FWD_WIDE_TMEM_COLS); }
 }
 
 // ------------------------------------------------------------------------------------------------------
@@ -653,9 +900,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 }
 
 // ------------------------------------------------------------------------------------------------------
-// Backward with dQ finished inside the kernel (dq_mode 1 and 2)
+// Backward with 128 x 128 blocks and one CTA per SM: where dQ is finished inside the kernel (dq_mode 1 and 2), and for grids that leave
+// the small CTAs above without neighbours (bwd_wide)
 // ------------------------------------------------------------------------------------------------------
-struct FinParams {
+struct BwdWideParams {
     int T, nh, causal;
     float scale, scale_log2;
     const float* lse;
@@ -666,7 +914,8 @@ struct FinParams {
     int* status;
     int* dq_sem;                   // [nb*nh, query blocks] contribution counters (zero between launches); null in mode 0
     __nv_bfloat16* dq;             // final dQ (modes 1 and 2)
-    int ordered;                   // 1: ordered adds, key block 0 finishes   0: unordered adds, the last part's CTA finishes
+    int dq_mode;                   // 0: unordered adds into a scratch the launch cleared, converted by dq_convert_kernel
+                                   // 1: ordered adds, key block 0 finishes   2: unordered adds, the last part's CTA finishes
 };
 
 // Bounded wait until *sem >= want (acquire).  Lane 0 of the calling warp polls; the warp then synchronises.
@@ -688,21 +937,21 @@ __device__ __forceinline__ bool sem_wait_warp(const int* sem, int want, volatile
 }
 
 // shared: K 16K | V 16K | Q[2] 32K | dO[2] 32K | P 32K | dS[2] 64K | dQ staging (fp32) 32K | barriers   (one CTA per SM)
-constexpr int FIN_SMEM = 14 * TILE_BYTES + 512;     // tiles | barriers, flags and the finishing warp's ring
-constexpr int FIN_MMA_WARP = 16;           // warps 0..15 compute, warp 16 issues TMA loads and MMA,
-constexpr int FIN_STORE_WARP = 17;         // warp 17 issues the dQ reduce-stores
-constexpr int FIN_CONVERT_WARP = 18;        // warp 18 (mode 2) converts the dQ tiles whose last part this CTA added
-constexpr int FIN_THREADS = 19 * 32;
+constexpr int BWD_WIDE_SMEM = 14 * TILE_BYTES + 512;     // tiles | barriers, flags and the finishing warp's ring
+constexpr int BWD_WIDE_MMA_WARP = 16;           // warps 0..15 compute, warp 16 issues TMA loads and MMA,
+constexpr int BWD_WIDE_STORE_WARP = 17;         // warp 17 issues the dQ reduce-stores
+constexpr int BWD_WIDE_CONVERT_WARP = 18;        // warp 18 (mode 2) converts the dQ tiles whose last part this CTA added
+constexpr int BWD_WIDE_THREADS = 19 * 32;
 constexpr int FIN_RING = CME_ATTN_FINISH_MAX_QBLOCKS;   // a CTA hands over at most one tile per query block
-constexpr int FIN_TMEM_COLS = 512;     // S [0,128) dP [128,256) dV [256,320) dK [320,384) dQ [384,448)
+constexpr int BWD_WIDE_TMEM_COLS = 512;     // S [0,128) dP [128,256) dV [256,320) dK [320,384) dQ [384,448)
 static_assert(12 * 8 + 4 + 4 + 4 + FIN_RING * 4 <= 512, "barriers, flags and ring exceed their block");
-static_assert(FIN_SMEM <= 227 * 1024, "backward shared-memory carve-up exceeds what one CTA may have");
-static_assert(2 * 128 + 3 * HD <= FIN_TMEM_COLS, "backward TMEM budget: S, dP, dV, dK, dQ");
+static_assert(BWD_WIDE_SMEM <= 227 * 1024, "backward shared-memory carve-up exceeds what one CTA may have");
+static_assert(2 * 128 + 3 * HD <= BWD_WIDE_TMEM_COLS, "backward TMEM budget: S, dP, dV, dK, dQ");
 
-__global__ void __launch_bounds__(FIN_THREADS, 1)
-attn_bwd_finish_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+__global__ void __launch_bounds__(BWD_WIDE_THREADS, 1)
+attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
-                   const __grid_constant__ CUtensorMap tmdQ, const FinParams p) {
+                   const __grid_constant__ CUtensorMap tmdQ, const BwdWideParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     if (smem_u32(smem) & 1023u) {
         if (threadIdx.x == 0 && p.status) atomicExch(p.status, CME_ERR_SHAPE);
@@ -737,7 +986,7 @@ attn_bwd_finish_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // above its own, which are then resident or finished.  Unordered form: the key blocks with the most query blocks
     // (the lowest) first.
     const int nkb = gridDim.x;
-    const bool ordered = p.ordered != 0, finish_last = !ordered;
+    const bool ordered = p.dq_mode == 1, finish_last = p.dq_mode == 2;
     const int kb = ordered ? nkb - 1 - (int)blockIdx.x : (int)blockIdx.x, k0 = kb * BKV;
     const int bh = blockIdx.y, b = bh / p.nh, h = bh % p.nh;
     const int nq = (p.T + BQ - 1) / BQ;
@@ -766,7 +1015,7 @@ attn_bwd_finish_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         mbar_init(s_free, 512);
         fence_barrier_init();
     }
-    if (warp == FIN_MMA_WARP) { tmem_alloc(tmem_slot, FIN_TMEM_COLS); tmem_relinquish(); }
+    if (warp == BWD_WIDE_MMA_WARP) { tmem_alloc(tmem_slot, BWD_WIDE_TMEM_COLS); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -774,7 +1023,7 @@ attn_bwd_finish_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + 128, tmem_dV = tmem_base + 256,
                    tmem_dK = tmem_base + 320, tmem_dQ = tmem_base + 384;
 
-    if (warp == FIN_MMA_WARP) {
+    if (warp == BWD_WIDE_MMA_WARP) {
         if (lane == 0) {
             constexpr uint32_t idesc_s = make_idesc(1, false, false, 128, 128);    // Q K^T, dO V^T
             constexpr uint32_t idesc_t = make_idesc(1, true, true, 128, HD);       // P^T dO, dS^T Q (A read transposed)
@@ -853,7 +1102,7 @@ attn_bwd_finish_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             }
             if (!ok) for (int i = 0; i < 2000; ++i) __nanosleep(500);
         }
-    } else if (warp == FIN_STORE_WARP) {
+    } else if (warp == BWD_WIDE_STORE_WARP) {
         // ---------------- dQ store issuer: moves each staged 128 x 64 fp32 tile into the global scratch.  Ordered form:
         // when it is this key block's turn -- a plain tile store if it is the first part, else a bulk reduce-add --
         // and the tile's counter is raised once the write has completed.  Key block 0 does not come through here.
@@ -909,7 +1158,7 @@ attn_bwd_finish_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             tma_store_wait<0>();
             if (finish_last) { __threadfence_block(); *fin_count = -1 - *fin_count; }
         }
-    } else if (warp == FIN_CONVERT_WARP) {
+    } else if (warp == BWD_WIDE_CONVERT_WARP) {
         // ---------------- finishing warp (mode 2): every part of a handed-over tile is in the scratch; scale and cast the
         // sums to dQ, and leave zeros behind for the next launch.  A tile is 128 x 64 fp32 = 32 KB of contiguous scratch.
         if (finish_last && n_it > 0) {
@@ -1111,7 +1360,7 @@ attn_bwd_finish_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // for the next launch
     if (ordered && kb == 0 && (int)threadIdx.x < n_it) p.dq_sem[(long long)bh * nq + i_begin + threadIdx.x] = 0;
     if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, CME_ERR_TIMEOUT);
-    if (warp == FIN_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, FIN_TMEM_COLS); }
+    if (warp == BWD_WIDE_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, BWD_WIDE_TMEM_COLS); }
 }
 
 // dq[b, h, t, :] = scale * acc[b * nh + h, t, :] (bf16, strided destination).  One thread per 8 elements, one (batch, head)
@@ -1197,27 +1446,67 @@ int attention_tc_supported(const CmeAttn* a) {
     return 1;
 }
 
+// Which kernel a call takes, by how it fills the SMs.  ctas: 128-row tiles of all heads; the small CTAs share an SM by four (forward)
+// or two (backward), the wide ones by two or one.  Times in us, wide / small, heads x tokens.
+//
+// Forward.  Up to two tiles per SM the small CTAs run without enough neighbours: 16 x 1024 14.1 / 26.1 causal, 24 x 582 11.1 / 18.0,
+// 128 x 256 8.8 / 9.7, 192 x 128 6.5 / 7.3 (with 129 to 192 tokens up to one: 64 x 192 7.4 / 7.9, 96 x 192 8.8 / 7.9).  Beyond, causal
+// calls take the small ones (192 x 256 14.0 / 11.0, 96 x 1024 40 / 32.6) but for long sequences just beyond (48 x 1024 23.5 / 27.4;
+// 64 x 1024 30.1 / 28.6).  With all keys both do a full GPU's work at one rate, and what counts is the last wave: to six tiles per SM
+// the wide ones (64 x 1024 33.8 / 37.2, 96 x 1024 49.8 / 57.7, 128 x 582 33.7 / 37.5; 192 x 582 49 / 43), then where that of the small
+// ones would be a quarter full (160 x 1024 81 / 86).
+bool fwd_wide(long long ctas, int T, bool causal, int sms) {
+    if (T > 128 && T <= 192) return ctas <= sms;
+    if (ctas <= 2ll * sms) return true;
+    if (causal) return (T > 512 && 5 * ctas <= 13ll * sms) || (T > 768 && ctas <= 3ll * sms);
+    const long long last = ctas % (4ll * sms);
+    return (T > 512 && ctas <= 6ll * sms) || (T > 768 && ctas > 8ll * sms && last > 0 && last <= sms);
+}
+// Backward.  One tile per SM: 16 x 1024 24.1 / 38.9, 24 x 582 17.0 / 25.9, 64 x 256 10.2 / 13.1, 128 x 128 8.5 / 9.0.  Two per SM: the small
+// ones win (96 x 256 17.1 / 15.2, all keys 24 x 1024 47.6 / 46.2), causal not beyond 448 tokens (24 and 32 x 1024 35.0 / 41.3 and 41.7 / 42.7,
+// 48 x 582 28.3 / 28.7), since the wide CTAs of light tiles make room for others.  With all keys and an odd number, the small ones' last
+// wave is half empty: three 48 x 1024 71 / 86, 64 x 582 48 / 55, 192 x 256 28.8 / 30.2, but 192 x 192 26.8 / 22.4; five 80 x 1024 121 / 126, 128 x
+// 582 82 / 83.  Else the small ones (causal 48 x 1024 53 / 48, 96 x 1024 93 / 80.5; all keys 96 x 1024 148 / 132, 128 x 1024 178 / 173).
+bool bwd_wide(long long ctas, int T, bool causal, int sms) {
+    const long long waves = (ctas + sms - 1) / sms;
+    if (causal) return waves <= 1 || (waves == 2 && T > 448);
+    return waves <= 1 || (waves == 3 && T > 192) || (waves == 5 && T > 512);
+}
+CME_API int cme_attention_tc_wide(int heads, int T, int causal, int bwd, int num_sms) {
+    const long long ctas = (long long)heads * cme_cdiv(T, BQ);
+    return bwd ? bwd_wide(ctas, T, causal != 0, num_sms) : fwd_wide(ctas, T, causal != 0, num_sms);
+}
+
 int attention_tc_fwd(const CmeAttn* a, cudaStream_t st) {
     CME_REQUIRE(attention_tc_supported(a), CME_ERR_SHAPE, "attention: shape not supported by the tensor-core kernel");
     CME_REQUIRE(a->lse != nullptr, CME_ERR_SHAPE, "attention: lse buffer is required");
     int* const g_attn_status = cme_attn_status_ptr();
     CME_REQUIRE(g_attn_status != nullptr, CME_ERR_CUDA, "attention: device state unavailable");
     CUtensorMap mq, mk, mv, mo;
-    int rc;
+    int rc, sms;
+    if ((rc = cme_num_sms(&sms))) return rc;
+    const bool wide = cme_attention_tc_wide(a->nb * a->nh, a->T, a->causal, 0, sms) != 0;
+    const int krows = wide ? BKV : FWD_BKV;
     if ((rc = make_map4(&mq, a->q, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
-    if ((rc = make_map4(&mk, a->k, a->T, a->nh, a->nb, a->st, a->sh, a->sb, FWD_BKV))) return rc;
-    if ((rc = make_map4(&mv, a->v, a->T, a->nh, a->nb, a->st, a->sh, a->sb, FWD_BKV))) return rc;
+    if ((rc = make_map4(&mk, a->k, a->T, a->nh, a->nb, a->st, a->sh, a->sb, krows))) return rc;
+    if ((rc = make_map4(&mv, a->v, a->T, a->nh, a->nb, a->st, a->sh, a->sb, krows))) return rc;
     if ((rc = make_map4(&mo, a->o, a->T, a->nh, a->nb, a->ost, a->osh, a->osb, 32))) return rc;
     static bool attr[CME_MAX_DEVICES] = {};               // function attributes are per device
     int dev = 0;
     CME_CUDA(cudaGetDevice(&dev));
     if (!attr[dev % CME_MAX_DEVICES]) {
         CME_CUDA(cudaFuncSetAttribute(attn_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM));
+        CME_CUDA(cudaFuncSetAttribute(attn_fwd_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_WIDE_SMEM));
         attr[dev % CME_MAX_DEVICES] = true;
     }
     FwdParams p{a->T, a->nh, a->causal, a->scale * LOG2E, a->lse, g_attn_status};
-    dim3 grid(a->nb * a->nh, cme_cdiv(a->T, BQ));
-    CME_CUDA(cme_launch_dependent(attn_fwd_tc_kernel, grid, dim3(FWD_THREADS), (size_t)FWD_SMEM, st, mq, mk, mv, mo, p));
+    const int tiles = cme_cdiv(a->T, BQ), heads = a->nb * a->nh;
+    if (wide)
+        CME_CUDA(cme_launch_dependent(attn_fwd_wide_kernel, dim3(tiles, heads), dim3(FWD_THREADS), (size_t)FWD_WIDE_SMEM, st, mq, mk,
+                                      mv, mo, p));
+    else
+        CME_CUDA(cme_launch_dependent(attn_fwd_tc_kernel, dim3(heads, tiles), dim3(FWD_THREADS), (size_t)FWD_SMEM, st, mq, mk, mv, mo,
+                                      p));
     CME_LAUNCH_CHECK();
     return CME_OK;
 }
@@ -1246,8 +1535,11 @@ int attention_tc_bwd(const CmeAttn* a, cudaStream_t st) {
     // delta, and in the same pass over the rows the zeros that the dQ parts are added to
     if ((rc = attention_delta_launch(a, st, a->dq_mode == 0 && !a->dq_accum_clean ? a->dq_accum : nullptr))) return rc;
     CUtensorMap mq, mk, mv, mdo, mdq;
+    int sms;
+    if ((rc = cme_num_sms(&sms))) return rc;
     const bool finish = a->dq_mode != 0;           // dQ is completed inside the kernel
-    const int qrows = finish ? BQ : BWD_BQ;
+    const bool wide = finish || cme_attention_tc_wide(a->nb * a->nh, a->T, a->causal, 1, sms) != 0;
+    const int qrows = wide ? BQ : BWD_BQ;
     if ((rc = make_map4(&mq, a->q, a->T, a->nh, a->nb, a->st, a->sh, a->sb, qrows))) return rc;
     if ((rc = make_map4(&mk, a->k, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
     if ((rc = make_map4(&mv, a->v, a->T, a->nh, a->nb, a->st, a->sh, a->sb, 128))) return rc;
@@ -1258,23 +1550,24 @@ int attention_tc_bwd(const CmeAttn* a, cudaStream_t st) {
     CME_CUDA(cudaGetDevice(&dev));
     if (!attr[dev % CME_MAX_DEVICES]) {
         CME_CUDA(cudaFuncSetAttribute(attn_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM));
-        CME_CUDA(cudaFuncSetAttribute(attn_bwd_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FIN_SMEM));
+        CME_CUDA(cudaFuncSetAttribute(attn_bwd_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_WIDE_SMEM));
         attr[dev % CME_MAX_DEVICES] = true;
     }
-    if (finish) {
-        FinParams p{a->T, a->nh, a->causal, a->scale, a->scale * LOG2E, a->lse, a->delta, a->dq_accum,
-                    (__nv_bfloat16*)a->dk, (__nv_bfloat16*)a->dv, a->sb, a->sh, a->st, g_attn_status, a->dq_sem,
-                    (__nv_bfloat16*)a->dq, a->dq_mode == 1};
+    if (wide) {
+        BwdWideParams p{a->T, a->nh, a->causal, a->scale, a->scale * LOG2E, a->lse, a->delta, a->dq_accum,
+                        (__nv_bfloat16*)a->dk, (__nv_bfloat16*)a->dv, a->sb, a->sh, a->st, g_attn_status, a->dq_sem,
+                        (__nv_bfloat16*)a->dq, a->dq_mode};
         dim3 grid(cme_cdiv(a->T, BKV), a->nb * a->nh);
-        attn_bwd_finish_kernel<<<grid, FIN_THREADS, FIN_SMEM, st>>>(mq, mk, mv, mdo, mdq, p);
+        attn_bwd_wide_kernel<<<grid, BWD_WIDE_THREADS, BWD_WIDE_SMEM, st>>>(mq, mk, mv, mdo, mdq, p);
         CME_LAUNCH_CHECK();
-        return CME_OK;
+        if (finish) return CME_OK;
+    } else {
+        BwdParams p{a->T, a->nh, a->causal, a->scale, a->scale * LOG2E, a->lse, a->delta, (__nv_bfloat16*)a->dk,
+                    (__nv_bfloat16*)a->dv, a->sb, a->sh, a->st, g_attn_status};
+        CME_CUDA(cme_launch_dependent(attn_bwd_tc_kernel, dim3(a->nb * a->nh, cme_cdiv(a->T, BKV)), dim3(BWD_THREADS),
+                                      (size_t)BWD_SMEM, st, mq, mk, mv, mdo, mdq, p));
+        CME_LAUNCH_CHECK();
     }
-    BwdParams p{a->T, a->nh, a->causal, a->scale, a->scale * LOG2E, a->lse, a->delta, (__nv_bfloat16*)a->dk,
-                (__nv_bfloat16*)a->dv, a->sb, a->sh, a->st, g_attn_status};
-    CME_CUDA(cme_launch_dependent(attn_bwd_tc_kernel, dim3(a->nb * a->nh, cme_cdiv(a->T, BKV)), dim3(BWD_THREADS), (size_t)BWD_SMEM,
-                                  st, mq, mk, mv, mdo, mdq, p));
-    CME_LAUNCH_CHECK();
     CME_CUDA(cme_launch_dependent(dq_convert_kernel, dim3(cme_cdiv(a->T, 32), a->nb * a->nh), dim3(256), 0, st,
                                   (const float*)a->dq_accum, (__nv_bfloat16*)a->dq, a->T, a->nh, a->sb, a->sh, a->st,
                                   a->scale));
