@@ -49,15 +49,13 @@ class CmeGemm(ctypes.Structure):
     ]
 
 
-# Argument types of the entry points that the wrappers below call: with them declared, addresses and sizes go over as
+# Argument types of the entry points that are called from Python by address: with them declared, addresses and sizes go over as
 # plain Python numbers (no wrapper object per argument).  v: address, i: int, l: long long, f: float, u: unsigned.
 _PROTOTYPES = {
-    "cme_gemm": "viv", "cme_colsum_slabs_finalize": "iviiviv", "cme_layernorm_fwd": "ivvvvvvvviifv",
-    "cme_layernorm_bwd_blocks": "i", "cme_layernorm_bwd": "ivvvvvvvvvviiiv", "cme_bias_act_residual": "ivvvvvliiv",
-    "cme_colsum_splits": "ii", "cme_dact_colsum": "ivvvvviiiiv", "cme_scale": "ivlfv", "cme_cast": "ivivlv",
+    "cme_gemm": "viv", "cme_colsum_slabs_finalize": "iviiviv", "cme_scale": "ivlfv", "cme_cast": "ivivlv",
     "cme_add": "ivvvlv", "cme_relu_bwd": "ivvvlv", "cme_init_uniform": "ivlfuv", "cme_embedding_fwd": "ivvvviiiiv",
-    "cme_embedding_bwd": "ivvvviiiiiv", "cme_cross_entropy": "ivvvvviilfffiv", "cme_grad_normsq": "ivlvvv",
-    "cme_adam": "ivvvvvlvvvffffffviv", "cme_copy_pair_i32": "vvvvlv", "cme_attention_fwd": "viv", "cme_attention_bwd": "viv", "cme_attention_path": "vii",
+    "cme_embedding_bwd": "ivvvviiiiiv", "cme_grad_normsq": "ivlvvv", "cme_adam": "ivvvvvlvvvffffffviv",
+    "cme_copy_pair_i32": "vvvvlv", "cme_attention_fwd": "viv", "cme_attention_bwd": "viv",
 }
 # Entry points that the compiled wrappers call.
 _WRAPPED = ("cme_last_error", "cme_cross_entropy", "cme_attention_fwd", "cme_attention_bwd", "cme_attention_path",
@@ -375,6 +373,8 @@ _BACKENDS = {"auto": 0, "tc": 1, "simt": 2, "gemm": 3}
 
 
 def _attn_desc(q, B, H, T, layout, causal):
+    """The descriptor for those who call the C entry points themselves, with strides and buffers of their own; ``attention_fwd`` and
+    ``attention_bwd`` fill theirs in compiled code."""
     D = q.shape[-1]
     HD = D // H
     nb, nh, sb, sh, st = (B * H, 1, T * HD, 0, HD) if layout == "flat" else (B, H, T * D, HD, D)
