@@ -262,7 +262,7 @@ ln_fwd_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ 
 // with a residual gradient (101 MB) takes 20.1 us on packed pairs, 21.2 us one element at a time, 24.4 us with the rows in
 // registers instead of the ring.
 template <typename T, int NV>
-__global__ void __launch_bounds__(LN_WARPS * 32, 2)
+__global__ void __launch_bounds__(LN_WARPS * 32, NV == 1 ? 4 : 2)
 ln_bwd_vec_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                   const float* __restrict__ mean, const float* __restrict__ rstd, const T* __restrict__ dres,
                   T* __restrict__ dx, float* __restrict__ partial /*[gridDim.x][2][D]*/, int rows, int D) {
@@ -584,8 +584,7 @@ int ln_bwd_vec_launch(const T* dy, const T* x, const T* g, const float* mean, co
         if (rc) return rc;
         res = n;
     }
-    int nb = even_grid(rows, res);
-    if (nb > max_blocks) nb = max_blocks;
+    const int nb = even_grid(rows, res < max_blocks ? res : max_blocks);     // (the blocks' sums have room for max_blocks)
     CME_CUDA(cme_launch_dependent(k, dim3(nb), dim3(LN_WARPS * 32), smem, st, dy, x, g, mean, rstd, dres, dx, scratch, rows,
                                   D));
     *used_blocks = nb;
