@@ -76,7 +76,7 @@ __device__ __forceinline__ void load_rows(float* dst, const T* src, long long st
 }
 
 // The same as they are, fp32 in whole 16-byte words by asynchronous copies: all of a block's tiles are on their way at once,
-// where the registers of a thread hold eight words (80 rounds of its loads for the forward's 80 KB and 64 threads).  Other
+// where the registers of a thread hold eight words (40 rounds of its loads for the forward's 80 KB and 128 threads).  Other
 // types and alignments are loaded at once.  Complete after copies_wait by every thread and a barrier.
 template <typename T, int G, int NR, int NT>
 __device__ __forceinline__ void copy_rows(float* dst, const T* src, long long st, int r0, int T_, int HD, bool vec) {
@@ -190,8 +190,12 @@ __device__ __forceinline__ void store_cols(T* row, int c, int HD, const float* v
         if (c + k < HD) row[c + k] = from_f32<T>(t[k]);
 }
 
+// Blocks per SM that the registers have to leave room for: what shared memory takes (G = 1: five of seven, at 72 registers it spills).
+// Left to itself the compiler gave the bf16 backward of two groups 162 registers and with them one block per SM for two (64 heads x 128
+// tokens, head size 64: 51 us, 40 so), and the forwards of three and four groups fewer than there is room for.
+template <int G, int NW> constexpr int fwd_blocks_per_sm() { return G == 1 ? (NW == 1 ? 8 : 5) : G == 2 ? (NW == 1 ? 5 : 4) : G == 3 ? 3 : 2; }
 template <typename T, int G, int NW>
-__global__ void __launch_bounds__(NW * 64) attn_fwd_kernel(const CmeAttn a, const bool vec) {
+__global__ void __launch_bounds__(NW * 64, fwd_blocks_per_sm<G, NW>()) attn_fwd_kernel(const CmeAttn a, const bool vec) {
     constexpr int P = Pitch<G>::P, RT = NW * WR, NT = NW * 64;
     // a lane's columns: VW at half * 16 G + tx * VW, then every 8 VW
     constexpr int VW = G % 2 == 0 ? 4 : 2, NK = 2 * G / VW;
@@ -374,7 +378,7 @@ __device__ __forceinline__ void delta_rows(float* dst, const float* sdO, const f
 // Whether O is staged beside dO: fp32 heads wide enough for one block per SM anyway.
 template <typename T, int G> __host__ __device__ constexpr bool bwd_stages_o() { return sizeof(T) == 4 && G >= 3; }
 template <typename T, int G>
-__global__ void __launch_bounds__(BWD_THREADS) attn_bwd_kernel(const CmeAttn a, const bool vec) {
+__global__ void __launch_bounds__(BWD_THREADS, G <= 2 ? 2 : 1) attn_bwd_kernel(const CmeAttn a, const bool vec) {
     constexpr int P = Pitch<G>::P, NT = BWD_THREADS, RT = BWD_ROWS;
     // a lane's columns: VW at half * 16 G + tx * VW, then every 8 VW
     constexpr int VW = G % 2 == 0 ? 4 : 2, NK = 2 * G / VW;
