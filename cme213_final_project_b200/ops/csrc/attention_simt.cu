@@ -193,7 +193,9 @@ __device__ __forceinline__ void store_cols(T* row, int c, int HD, const float* v
 // Blocks per SM that the registers have to leave room for: what shared memory takes (G = 1: five of seven, at 72 registers it spills).
 // Left to itself the compiler gave the bf16 backward of two groups 162 registers and with them one block per SM for two (64 heads x 128
 // tokens, head size 64: 51 us, 40 so), and the forwards of three and four groups fewer than there is room for.
-template <int G, int NW> constexpr int fwd_blocks_per_sm() { return G == 1 ? (NW == 1 ? 8 : 5) : G == 2 ? (NW == 1 ? 5 : 4) : G == 3 ? 3 : 2; }
+template <int G, int NW> constexpr int fwd_blocks_per_sm() {
+    return G == 1 ? (NW == 1 ? 8 : 5) : G == 2 ? (NW == 1 ? 5 : 4) : G == 3 ? 3 : 2;
+}
 template <typename T, int G, int NW>
 __global__ void __launch_bounds__(NW * 64, fwd_blocks_per_sm<G, NW>()) attn_fwd_kernel(const CmeAttn a, const bool vec) {
     constexpr int P = Pitch<G>::P, RT = NW * WR, NT = NW * 64;

@@ -1462,11 +1462,12 @@ bool fwd_wide(long long ctas, int T, bool causal, int sms) {
     const long long last = ctas % (4ll * sms);
     return (T > 512 && ctas <= 6ll * sms) || (T > 768 && ctas > 8ll * sms && last > 0 && last <= sms);
 }
-// Backward.  One tile per SM: 16 x 1024 24.1 / 38.9, 24 x 582 17.0 / 25.9, 64 x 256 10.2 / 13.1, 128 x 128 8.5 / 9.0.  Two per SM: the small
-// ones win (96 x 256 17.1 / 15.2, all keys 24 x 1024 47.6 / 46.2), causal not beyond 448 tokens (24 and 32 x 1024 35.0 / 41.3 and 41.7 / 42.7,
-// 48 x 582 28.3 / 28.7), since the wide CTAs of light tiles make room for others.  With all keys and an odd number, the small ones' last
-// wave is half empty: three 48 x 1024 71 / 86, 64 x 582 48 / 55, 192 x 256 28.8 / 30.2, but 192 x 192 26.8 / 22.4; five 80 x 1024 121 / 126, 128 x
-// 582 82 / 83.  Else the small ones (causal 48 x 1024 53 / 48, 96 x 1024 93 / 80.5; all keys 96 x 1024 148 / 132, 128 x 1024 178 / 173).
+// Backward.  One tile per SM: 16 x 1024 24.1 / 38.9, 24 x 582 17.0 / 25.9, 64 x 256 10.2 / 13.1, 128 x 128 8.5 / 9.0.  Two per SM: the
+// small ones win (96 x 256 17.1 / 15.2, all keys 24 x 1024 47.6 / 46.2), causal not beyond 448 tokens (24 and 32 x 1024 35.0 / 41.3 and
+// 41.7 / 42.7, 48 x 582 28.3 / 28.7), since the wide CTAs of light tiles make room for others.  With all keys and an odd number, the small
+// ones' last wave is half empty: three 48 x 1024 71 / 86, 64 x 582 48 / 55, 192 x 256 28.8 / 30.2, but 192 x 192 26.8 / 22.4; five 80 x 1024
+// 121 / 126, 128 x 582 82 / 83.  Else the small ones (causal 48 x 1024 53 / 48, 96 x 1024 93 / 80.5; all keys 96 x 1024 148 / 132,
+// 128 x 1024 178 / 173).
 bool bwd_wide(long long ctas, int T, bool causal, int sms) {
     const long long waves = (ctas + sms - 1) / sms;
     if (causal) return waves <= 1 || (waves == 2 && T > 448);
