@@ -9,8 +9,8 @@
 // gradients are bit-reproducible.
 //
 // Structure per CTA (192 threads -- 320 with eight epilogue warps for the arithmetic-heavy epilogues; 1 CTA per SM):
-//   warp 0      one lane issues TMA tile loads into a ring of shared-memory stages
-//   warp 1      allocates TMEM; one lane issues tcgen05.mma (128 x BN x 16 per instruction)
+//   warp 0      one elected lane issues TMA tile loads into a ring of shared-memory stages
+//   warp 1      allocates TMEM; one elected lane issues tcgen05.mma (128 x BN x 16 per instruction)
 //   warps 2..5  epilogue: tcgen05.ld of their 32-lane quarter of the accumulator, fused epilogue, stores
 //   (warps 6..9  a second epilogue set on the same four quarters, taking every other 64-column chunk)
 // Operands may be K-major or MN-major in global memory; MN-major tiles are fetched as 64-wide column
@@ -384,7 +384,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(in_bar + C::EPI_WARPS * C::NB);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // a uniform value
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
@@ -423,7 +423,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     if (warp == 0) {
         // ------------------------------- TMA producer -------------------------------
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -486,9 +486,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else if (warp == 1) {
         // ------------------------------- MMA issuer ---------------------------------
-        if (lane == 0 && cta_rank == 0) {
+        if (cta_rank == 0 && elect_one()) {
             constexpr uint32_t idesc = make_idesc(C::TF32 ? 2 /*tf32*/ : 1 /*bf16*/, A_MN, B_MN, BMT, BN);
             constexpr int KROWS = MMA_K_BYTES / C::ES;      // k-rows one MMA consumes of an MN-major tile: 16 or 8
+            auto operand_desc = [](bool mn, uint32_t at) {
+                return !mn ? make_smem_desc(at, 0, 1024)
+                           : C::TF32 ? make_smem_desc_mn32(at, GROUP_BYTES) : make_smem_desc(at, GROUP_BYTES, 1024);
+            };
+            const uint64_t descA = operand_desc(A_MN, smem_u32(smem)), descB = operand_desc(B_MN, smem_u32(smem) + A_TILE_BYTES);
             int stage = 0;
             uint32_t phase = 0;
             int it = 0;
@@ -503,21 +508,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (!mbar_wait(&tempty_bar[buf], acc_phase ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + buf * BN;
+                uint32_t accf = 0;
                 for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t sA = smem_u32(smem + stage * C::STAGE_BYTES);
-                    const uint32_t sB = sA + A_TILE_BYTES;
+                    const uint32_t at = (uint32_t)(stage * C::STAGE_BYTES) >> 4;
 #pragma unroll
                     for (int k = 0; k < BK_BYTES / MMA_K_BYTES; ++k) {
                         // K-major: step 32 bytes (16 bf16 / 8 tf32 elements) inside the 128-byte row.
                         // MN-major: step KROWS k-rows of 128 bytes; column groups are GROUP_BYTES apart.
-                        auto mn_desc = [](uint32_t at) {
-                            return C::TF32 ? make_smem_desc_mn32(at, GROUP_BYTES) : make_smem_desc(at, GROUP_BYTES, 1024);
-                        };
-                        const uint64_t da = A_MN ? mn_desc(sA + k * KROWS * 128) : make_smem_desc(sA + k * MMA_K_BYTES, 0, 1024);
-                        const uint64_t db = B_MN ? mn_desc(sB + k * KROWS * 128) : make_smem_desc(sB + k * MMA_K_BYTES, 0, 1024);
-                        const uint32_t accf = (kb > kb0 || k > 0) ? 1u : 0u;
+                        const uint64_t da = desc_at(descA, at + ((A_MN ? k * KROWS * 128 : k * MMA_K_BYTES) >> 4));
+                        const uint64_t db = desc_at(descB, at + ((B_MN ? k * KROWS * 128 : k * MMA_K_BYTES) >> 4));
                         if constexpr (C::TF32) {
                             if constexpr (PAIR) mma_tf32_ss_pair(tmem_d, da, db, idesc, accf);
                             else                mma_tf32_ss(tmem_d, da, db, idesc, accf);
@@ -525,6 +526,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             if constexpr (PAIR) mma_f16_ss_pair(tmem_d, da, db, idesc, accf);
                             else                mma_f16_ss(tmem_d, da, db, idesc, accf);
                         }
+                        accf = 1;
                     }
                     // stage is free (in both CTAs of a pair) once these MMAs have read it
                     if constexpr (PAIR) mma_commit_pair(&empty_bar[stage], 3); else mma_commit(&empty_bar[stage]);
