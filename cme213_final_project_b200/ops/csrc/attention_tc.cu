@@ -94,7 +94,8 @@ struct FwdParams {
 // What bounds it: the chain MMA -> TMEM load -> softmax -> TMEM store -> MMA of a tile (no pipe is busy for half of the time).
 // So a CTA is kept small enough for four on an SM: 128 queries, 64 keys at a time, P in the columns that its scores came
 // from, 128 TMEM columns, 64 score registers per thread; every scheduler then has four softmax warps of independent chains,
-// and a tile's start and end run under the others' work.  16 x 12 heads x 1024 tokens: causal 59 us, all keys 93 us.
+// and a tile's start and end run under the others' work.  16 x 12 heads x 1024 tokens: causal 51.4 us, all keys 82.6 us (59.7 and
+// 93.4 with an issuing thread that the compiler did not know to be alone, see elect_one).
 // S_{j+1} goes to the columns that P_j V_j reads its A operand from.  PTX orders two MMAs of a thread only if they accumulate in
 // the same place, so S_{j+1} is issued once a barrier says that P_j V_j is complete.  Measured without that wait, when this form
 // took 57 and 89 us: two CTAs with 128 keys at a time 70 us causal; three with S_{j+1} made under softmax_j 57 and 87 us; a quarter
@@ -136,7 +137,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // the late (causal: heavy) query tiles of all heads first, so that the last wave is made of the light ones
     const int q0 = (gridDim.y - 1 - blockIdx.y) * BQ;
     const int bh = blockIdx.x, b = bh / p.nh, h = bh % p.nh;
@@ -160,7 +161,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     pdl_wait();        // barrier set-up and TMEM allocation above may overlap the tail of the previous kernel
 
     if (warp == 4) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---------------- producer + MMA issuer (one thread) ----------------
             constexpr uint32_t idesc_s = make_idesc(1, false, false, BQ, FWD_BKV);   // Q K^T: both K-major
             constexpr uint32_t idesc_o = make_idesc(1, false, true, BQ, HD);         // P V: V is MN-major
@@ -389,7 +390,7 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     pdl_wait();        // barrier set-up and TMEM allocation above may overlap the tail of the previous kernel
 
     if (warp == 4) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---------------- producer + MMA issuer (one thread) ----------------
             constexpr uint32_t idesc_s = make_idesc(1, false, false, 128, 128);   // Q K^T: both K-major
             constexpr uint32_t idesc_o = make_idesc(1, false, true, 128, HD);     // P V: V is MN-major
@@ -588,7 +589,8 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // launch clears the scratch beforehand and dq_convert_kernel scales and casts the sums.
 // What bounds it: the chain of a block (two round trips to the tensor pipe, about 6000 clocks, hidden by one other CTA only);
 // the tensor pipe is busy for 45 % of the time (a product of 64 columns takes as long as one of 128).
-// 16 x 12 heads x 1024 tokens, causal: 157 us; one CTA per SM with 128 queries at a time, P through shared memory: 179 us.
+// 16 x 12 heads x 1024 tokens: causal 135 us, all keys 229 us (157 and 265 with an issuing thread that the compiler did not know to
+// be alone, see elect_one).
 // shared: K 16K | V 16K | Q[3] 24K | dO[2] 16K | dS^T 16K | dQ staging (fp32) 16K | row statistics[2] 1K | barriers
 constexpr int BWD_BQ = 64;                 // queries per step
 constexpr int BWD_Q_BYTES = BWD_BQ * HD * 2;
@@ -642,7 +644,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // the key blocks that the most queries see (causal: the lowest) of all heads first
     const int k0 = blockIdx.y * BKV;
     const int bh = blockIdx.x, b = bh / p.nh, h = bh % p.nh;
@@ -673,7 +675,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     pdl_wait();        // barrier set-up and TMEM allocation above may overlap the tail of the previous kernel
 
     if (warp == BWD_MMA_WARP) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_s = make_idesc(1, false, false, BKV, BWD_BQ);    // K Q^T, V dO^T
             constexpr uint32_t idesc_t = make_idesc(1, false, true, BKV, HD);         // P^T dO, dS^T Q
             constexpr uint32_t idesc_q = make_idesc(1, true, true, BWD_BQ, HD);       // dS K (A read transposed)
@@ -755,7 +757,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             if (!ok) for (int i = 0; i < 2000; ++i) __nanosleep(500);
         }
     } else if (warp == BWD_STORE_WARP) {
-        if (lane == 0) {
+        if (elect_one()) {
             for (int it = 0; it < n_it; ++it) {
                 if (!mbar_wait(dqs_full, it & 1, abort_flag)) break;
                 const int q0 = q_begin + it * BWD_BQ;
@@ -981,7 +983,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                                                // has ended after n tiles
     volatile int* fin_ring = abort_flag + 2;   // [FIN_RING] query-block indices
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // Ordered form: higher key blocks are dispatched first, so a CTA only ever waits for the dQ parts of key blocks
     // above its own, which are then resident or finished.  Unordered form: the key blocks with the most query blocks
     // (the lowest) first.
@@ -1024,7 +1026,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                    tmem_dK = tmem_base + 320, tmem_dQ = tmem_base + 384;
 
     if (warp == BWD_WIDE_MMA_WARP) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_s = make_idesc(1, false, false, 128, 128);    // Q K^T, dO V^T
             constexpr uint32_t idesc_t = make_idesc(1, true, true, 128, HD);       // P^T dO, dS^T Q (A read transposed)
             constexpr uint32_t idesc_q = make_idesc(1, false, true, 128, HD);      // dS K
@@ -1106,7 +1108,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         // ---------------- dQ store issuer: moves each staged 128 x 64 fp32 tile into the global scratch.  Ordered form:
         // when it is this key block's turn -- a plain tile store if it is the first part, else a bulk reduce-add --
         // and the tile's counter is raised once the write has completed.  Key block 0 does not come through here.
-        if (lane == 0 && !(ordered && kb == 0)) {
+        if (!(ordered && kb == 0) && elect_one()) {
             for (int f = 0; f < n_it; ++f) {
                 if (!mbar_wait(dqs_full, f & 1, abort_flag)) break;
                 const int qi = qblock(f), q0 = qi * BQ;
