@@ -406,8 +406,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         else                { tmem_alloc(tmem_slot, C::TMEM_COLS); tmem_relinquish(); }
     }
     tc_fence_before();
+    __syncthreads();
     // In a pair, the peer's barriers and TMEM must exist before anything is signalled across.
-    if constexpr (PAIR) cluster_sync_all(); else __syncthreads();
+    if constexpr (PAIR) cluster_sync_relaxed();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t cta_rank = PAIR ? cluster_ctarank() : 0u;
@@ -850,13 +851,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             // input copies may still be in flight: give them time to land before shared memory is released
             for (int i = 0; i < 2000; ++i) __nanosleep(500);
         }
-        if (p.tma_store && lane == 0) tma_store_wait<0>();   // stores complete before shared memory goes away
+        if (p.tma_store && lane == 0) tma_store_wait_read<0>();   // shared memory may go once the copy engine has read it
     }
 
     __syncwarp();
     tc_fence_before();
     // A pair leaves together: neither CTA may exit while the other can still signal its barriers or read its tiles.
-    if constexpr (PAIR) cluster_sync_all(); else __syncthreads();
+    __syncthreads();
+    if constexpr (PAIR) cluster_sync_relaxed();
     if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, CME_ERR_TIMEOUT);
     if (warp == 1) {
         tc_fence_after();

@@ -193,11 +193,15 @@ __device__ __forceinline__ uint32_t mapa_u32(const void* p, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(p)), "r"(rank));
     return out;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+// Meeting points of the cluster's threads that order no memory.  What must be seen across is ordered by its own means (barrier
+// words by fence_barrier_init, tensor memory by the tcgen05 fences); a release at cluster scope waits for all of the thread's earlier
+// stores, 1000-2000 clocks.
+__device__ __forceinline__ void cluster_sync_relaxed() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
+// An arrival on another CTA's barrier, with the default release at CTA scope, for the same reason.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Both CTAs of the pair call these with the same warp index and the same shared-memory slot offset.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_slot, uint32_t cols) {
