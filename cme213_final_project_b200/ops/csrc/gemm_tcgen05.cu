@@ -365,6 +365,9 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream) {
         ep.stream_aux = (stream_aux && g->aux_deriv && (g->act == CME_ACT_GELU || g->dact == CME_ACT_GELU)) ? 1 : 0;
     }
     ep.status = g_status;
+    ep.div_fast.set(ep.n_fast ? tiles_n : tiles_m);
+    ep.div_mn.set(tiles_m * tiles_n);
+    ep.div_batch.set(g->batch);
     // Partial rows are padded to whole 16-byte words where the workspace has room: they then leave by TMA stores and are
     // read back four columns at a time also when N is odd, like the 65-column output head's weight gradient.
     const int n_pad = (g->N + 3) / 4 * 4;

@@ -95,8 +95,29 @@ template <int BN, bool PAIR, bool SIMPLE, int SPEC = -1> struct Cfg {
     static_assert(BAR_BYTES >= (2 * 8 + 4 + EPI_WARPS * NB) * 8 + 8, "barrier block too small");
 };
 
+// Division of 0 <= n < 2^31 by a divisor that the host knows: a multiplication and a shift (Granlund and Montgomery's method)
+// instead of about 100 clocks for each of the six divisions that take a tile's index apart.
+struct FastDiv {
+    uint32_t d, mul, shift;
+    __host__ void set(uint32_t divisor) {
+        d = divisor;
+        shift = 0;
+        while ((1ull << shift) < d) ++shift;
+        mul = (uint32_t)(((1ull << 32) * ((1ull << shift) - d)) / d + 1);
+    }
+    __host__ __device__ __forceinline__ int div(int n) const {
+#ifdef __CUDA_ARCH__
+        return (int)((__umulhi(mul, (uint32_t)n) + (uint32_t)n) >> shift);
+#else
+        return (int)((((unsigned long long)mul * (uint32_t)n >> 32) + (uint32_t)n) >> shift);
+#endif
+    }
+    __host__ __device__ __forceinline__ int mod(int n) const { return n - div(n) * (int)d; }
+};
+
 struct EpiParams {
     int M, N, K, batch;
+    FastDiv div_fast, div_mn, div_batch;       // by the tiles of the direction that runs fastest, by tiles_m * tiles_n, by batch
     int tiles_m, tiles_n, splits, kb_per_split, num_kb;
     int stream_aux;                // the auxiliary tensors (activation derivative written by forward, read once by backward)
                                    // go through L2 with the evict-first policy
@@ -119,8 +140,9 @@ struct EpiParams {
 // they share in L2: walking down M they share a stripe of B and every row block of A is fetched once per column block;
 // walking across N they share rows of A.  The launcher picks the order with the smaller DRAM traffic.
 __device__ __forceinline__ void tile_mn(const EpiParams& p, int mn, int& tm, int& tn) {
-    if (p.n_fast) { tn = mn % p.tiles_n; tm = mn / p.tiles_n; }
-    else          { tm = mn % p.tiles_m; tn = mn / p.tiles_m; }
+    const int slow = p.div_fast.div(mn), fast = mn - slow * (int)p.div_fast.d;
+    if (p.n_fast) { tn = fast; tm = slow; }
+    else          { tm = fast; tn = slow; }
 }
 
 __device__ __forceinline__ void epilogue_chunk(const EpiParams& p, float* acc, long long row_off_c,
@@ -386,31 +408,35 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // a uniform value
 
-    if (threadIdx.x == 0) {
-        *abort_flag = 0;
-        for (int s = 0; s < C::STAGES; ++s) {
-            mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
+    if (warp == 0) {
+        if (elect_one()) {
+            *abort_flag = 0;
+            for (int s = 0; s < C::STAGES; ++s) {
+                mbar_init(&full_bar[s], 1);
+                mbar_init(&empty_bar[s], 1);
+            }
+            for (int b = 0; b < 2; ++b) {
+                mbar_init(&tfull_bar[b], 1);
+                mbar_init(&tempty_bar[b], (PAIR ? 2 : 1) * C::EPI_WARPS);   // one arrival per epilogue warp (of both CTAs)
+            }
+            for (int b = 0; b < C::EPI_WARPS * C::NB; ++b) mbar_init(&in_bar[b], 1);
+            fence_barrier_init();
+            prefetch_tmap(&tmA);
+            prefetch_tmap(&tmB);
         }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&tfull_bar[b], 1);
-            mbar_init(&tempty_bar[b], (PAIR ? 2 : 1) * C::EPI_WARPS);   // one arrival per epilogue warp (of both CTAs)
-        }
-        for (int b = 0; b < C::EPI_WARPS * C::NB; ++b) mbar_init(&in_bar[b], 1);
-        fence_barrier_init();
-        prefetch_tmap(&tmA);
-        prefetch_tmap(&tmB);
+        __syncwarp();
     }
     if (warp == 1) {
         if constexpr (PAIR) { tmem_alloc_pair(tmem_slot, C::TMEM_COLS); tmem_relinquish_pair(); }
         else                { tmem_alloc(tmem_slot, C::TMEM_COLS); tmem_relinquish(); }
     }
     tc_fence_before();
-    __syncthreads();
-    // In a pair, the peer's barriers and TMEM must exist before anything is signalled across.
+    // Warp 0 has what its loads need, the barriers; it does not wait for the TMEM allocation, so that takes place under the first
+    // loads.  In a pair, the peer's barriers and TMEM must exist before anything is signalled across.
+    if (PAIR || warp != 0) named_bar_sync(1, C::THREADS); else named_bar_arrive(1, C::THREADS);
     if constexpr (PAIR) cluster_sync_relaxed();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = PAIR || warp != 0 ? *tmem_slot : 0u;
     const uint32_t cta_rank = PAIR ? cluster_ctarank() : 0u;
     const int tile0 = PAIR ? int(blockIdx.x >> 1) : int(blockIdx.x);
     const int tile_step = PAIR ? int(gridDim.x >> 1) : int(gridDim.x);
@@ -421,6 +447,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     const int tiles_mn = p.tiles_m * p.tiles_n;
     const int total_tiles = tiles_mn * p.batch * p.splits;
+    bool tmem_free = false;                                  // warp 1: the allocation has been given back
 
     if (warp == 0) {
         // ------------------------------- TMA producer -------------------------------
@@ -429,8 +456,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             uint32_t phase = 0;
             bool ok = true;
             for (int tile = tile0; tile < total_tiles && ok; tile += tile_step) {
-                const int mn = tile % tiles_mn, rest = tile / tiles_mn;
-                const int bidx = rest % p.batch, split = rest / p.batch;
+                const int rest = p.div_mn.div(tile), mn = tile - rest * tiles_mn;
+                const int split = p.div_batch.div(rest), bidx = rest - split * p.batch;
                 int tm, tn;
                 tile_mn(p, mn, tm, tn);
                 const int m0 = tm * BMT + int(cta_rank) * BM;
@@ -500,8 +527,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int it = 0;
             bool ok = true;
             for (int tile = tile0; tile < total_tiles && ok; tile += tile_step, ++it) {
-                const int rest = tile / tiles_mn;
-                const int split = rest / p.batch;
+                const int split = p.div_batch.div(p.div_mn.div(tile));
                 const int kb0 = split * p.kb_per_split;
                 const int kb1 = min(kb0 + p.kb_per_split, p.num_kb);
                 const int buf = it & 1;
@@ -537,6 +563,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     if constexpr (PAIR) mma_commit_pair(&tfull_bar[buf], 3); else mma_commit(&tfull_bar[buf]);
                 }
             }
+            if (!PAIR && ok) {                          // the accumulators of the last two tiles have been read
+                tmem_free = true;
+                for (int i = it > 1 ? it - 2 : 0; i < it; ++i)
+                    tmem_free = tmem_free && mbar_wait(&tempty_bar[i & 1], (i >> 1) & 1, abort_flag);
+            }
+        }
+        // freed under the last tile's stores, not after them (256 clocks); a pair's CTAs free theirs together
+        if constexpr (!PAIR) {
+            tmem_free = __any_sync(0xffffffffu, tmem_free);
+            if (tmem_free) { tc_fence_after(); tmem_dealloc(tmem_base, C::TMEM_COLS); }
         }
     } else {
         // ------------------------------- epilogue -----------------------------------
@@ -575,7 +611,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         auto fetch_next = [&]() {
             int fmn = 0, fn0 = 0, fm_blk = 0;
             while (f_tile < total_tiles) {              // next tile that has a chunk for this warp set
-                fmn = f_tile % tiles_mn;
+                fmn = p.div_mn.mod(f_tile);
                 int ftm, ftn;
                 tile_mn(p, fmn, ftm, ftn);
                 fn0 = ftn * BN;
@@ -587,7 +623,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 f_tile += tile_step;
             }
             if (f_tile >= total_tiles) return;
-            const int fb = (f_tile / tiles_mn) % p.batch;
+            const int fb = p.div_batch.mod(p.div_mn.div(f_tile));
             const int fm0 = fm_blk * BMT + int(cta_rank) * BM + quarter * 32;
             if (lane == 0) {
                 const uint32_t b = f_cnt % C::NB;
@@ -608,7 +644,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         auto bias_fetch = [&](int t) {                  // this lane's 8 bias values of tile t (zeros past N)
             float b8[8];
             int btm, btn;
-            tile_mn(p, t % tiles_mn, btm, btn);
+            tile_mn(p, p.div_mn.mod(t), btm, btn);
             const int tn0 = btn * BN;
             load8_guard(p.bias, tn0 + lane * 8, p.N, true, b8);
             return pack8(b8);
@@ -618,8 +654,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             __syncwarp();
         }
         for (int tile = tile0; tile < total_tiles && ok; tile += tile_step, ++it) {
-            const int mn = tile % tiles_mn, rest = tile / tiles_mn;
-            const int bidx = rest % p.batch, split = rest / p.batch;
+            const int rest = p.div_mn.div(tile), mn = tile - rest * tiles_mn;
+            const int split = p.div_batch.div(rest), bidx = rest - split * p.batch;
             int etm, etn;
             tile_mn(p, mn, etm, etn);
             const int m0 = etm * BMT + int(cta_rank) * BM, n0 = etn * BN;
@@ -860,7 +896,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncthreads();
     if constexpr (PAIR) cluster_sync_relaxed();
     if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, CME_ERR_TIMEOUT);
-    if (warp == 1) {
+    if (warp == 1 && !tmem_free) {
         tc_fence_after();
         if constexpr (PAIR) tmem_dealloc_pair(tmem_base, C::TMEM_COLS); else tmem_dealloc(tmem_base, C::TMEM_COLS);
     }

@@ -74,6 +74,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     return false;
 }
 
+// Named barrier of `threads` threads (whole warps): wait for all of them, or only be counted.
+__device__ __forceinline__ void named_bar_sync(int id, int threads) {
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_bar_arrive(int id, int threads) {
+    asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 // ---------------------------------------------------------------------------------------------
 // TMA (cp.async.bulk.tensor), tile mode, no multicast
 // ---------------------------------------------------------------------------------------------
