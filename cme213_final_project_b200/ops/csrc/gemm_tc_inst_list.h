@@ -81,6 +81,26 @@ CME_GEMM_TC_EXTERN(256, false, false, SPEC_TF32)
 CME_GEMM_TC_EXTERN(256, false, true, SPEC_TF32)
 #endif
 
+#if CME_GEMM_TC_GROUP == -1 || CME_GEMM_TC_GROUP == 12     // CTA pair, 192 columns: plain and run-time epilogues
+CME_GEMM_TC_EXTERN(192, true, true, -1)
+CME_GEMM_TC_EXTERN(192, false, true, -1)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_F32)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_ACC)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_BIAS)
+#endif
+#if CME_GEMM_TC_GROUP == -1 || CME_GEMM_TC_GROUP == 13     // CTA pair, 192 columns: compile-time epilogues
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_RES)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_BIAS_RES)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_BIAS_RELU)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_DRELU_COLSUM)
+#endif
+#if CME_GEMM_TC_GROUP == -1 || CME_GEMM_TC_GROUP == 14
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_BIAS_GELU_AUXD)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_DMUL_COLSUM)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_DMUL)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_DRELU)
+#endif
+
 #ifdef CME_GEMM_TC_GROUP_DEFAULTED
 #undef CME_GEMM_TC_GROUP
 #undef CME_GEMM_TC_GROUP_DEFAULTED

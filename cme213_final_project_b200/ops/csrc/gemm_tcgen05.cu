@@ -172,54 +172,77 @@ CME_API int cme_gemm_status_word(int** out) {
     return CME_OK;
 }
 
-// Tile shape and K splits for a product: minimise  waves x k-blocks per unit x cost(tile)  (+ fixed per-tile and
-// per-split overheads), with measured clocks per 16-deep MMA step for each tile shape.  Pure host arithmetic.
-//   force_bn: 0 = choose; 64 / 128 / 256 = tile width on one CTA; 512 = the 256 x 256 tile on a CTA pair
+// How the operands of a product lie in memory, as far as the time of their loads depends on it.
+struct OperandLayout {
+    bool a_mn, b_mn;               // stored along M / N instead of along K
+    long long a_pitch, b_pitch;    // bytes from row to row
+};
+
+// Tile shape and K splits for a product: the smallest estimated time.  Pure host arithmetic.
+//   force_bn: 0 = choose; 64 / 128 / 256 = tile width on one CTA; 512 / 384 = the 256 x 256 / 256 x 192 tile on a CTA pair
 //   force_splits: 0 = choose.  Split-K needs the plain epilogue, a workspace for the fp32 partials and at least
 //   four 64-deep k-blocks per split.
+// The estimate, in us: a start that depends on the tile (launch, first loads, last stores), then for every wave of tiles a time per
+// tile and one per 128-byte k-block.  A k-block takes what its tile needs alone (issuing its MMAs, or the tensor pipe's rate), or as
+// long as L2 takes to deliver the k-blocks of all SMs that load: 22 TB/s.  Rows that do not start on 128-byte lines cost up to 1.4
+// times that, on odd 16-byte pieces twice.  Constants: least squares over 33000 products (1400 shapes of 128-50304 x 128-50304 x
+// 128-50304, every tile, 1-16 splits).  The plan is then 0.75 % slower than the best one on average (2.5-3 % with the constants
+// from before the k-blocks got faster), at most 1.2 times.
 static void plan_tiles(int M, int N, int K, int batch, bool plain_epi, long long workspace_bytes, int num_sms,
                        int max_pairs, int force_bn, int force_splits, int* bn_out, bool* pair_out, int* splits_out,
-                       int bk = 64, int mn_operands = 0) {
+                       const OperandLayout& at, int bk = 64) {
     const int num_kb = cme_cdiv(K, bk);
     int bn = force_bn, splits = force_splits;
     bool pair = false;
-    if (bn == 512) { bn = 256; pair = true; }
+    if (bn == 512 || bn == 384) { bn /= 2; pair = true; }
     if (!bn || !splits) {
+        struct Tile { int bn; bool pair; double kblock[2], unit[2], start[2]; };          // [bf16, tf32]
+        static const Tile tiles[5] = {{256, true, {0.268, 0.279}, {1.01, 1.31}, {3.58, 4.01}},
+                                      {256, false, {0.305, 0.305}, {0.98, 1.57}, {3.18, 3.21}},
+                                      {128, false, {0.190, 0.182}, {0.42, 0.56}, {2.96, 3.37}},
+                                      {64, false, {0.147, 0.151}, {0.22, 0.33}, {2.75, 3.05}},
+                                      {192, true, {0.232, 0.0}, {0.80, 0.0}, {3.39, 0.0}}};
+        const int t32 = bk == 32;
+        const double l2_bytes = t32 ? 21.5e6 : 22.2e6;       // per us, all SMs together
+        // shares of the operands whose rows leave the 128-byte lines (along K, along M / N) or the 32-byte sectors, and what they
+        // add to the time of a k-block alone (k) and to that of L2 (l)
+        static const double line_k[2][2] = {{0.21, 0.40}, {0.21, 0.07}}, line_l[2][2] = {{0.17, 0.165}, {0.255, 0.11}};
+        static const double sector_l[2] = {0.82, 0.20};
         double best = 1e30;
         int best_bn = 128, best_s = 1;
         bool best_pair = false;
-        const int bns[4] = {256, 256, 128, 64};
-        // Clocks per MMA step (32 bytes of K) and SM, from sweeps over tile widths and splits.  With one tile per SM a
-        // 128-byte k-block takes about 550 clocks whatever the tile's width (2048 x 512 x 2048 bf16, 32 k-blocks: 13.1 us
-        // at 64 and at 128 columns, 13.9 us at 256, base 3.3-4 us): the ring's round trip to L2, not the tensor pipe, sets
-        // it, so narrow tiles buy no time per k-block, and splitting K over idle SMs does.  With every SM loading, 256
-        // columns on one CTA come near the 64 bytes per clock that an SM takes in (192 by that rate, 168 fits the sweeps).
-        // tf32 operands stored along M or N arrive as 32-column groups, two to four times as many copies per k-block.  With
-        // both along K the pair tile has to win where it can fill the SMs: over 130 products it is then 0.5 % off the best
-        // forced plan on average, 2.6 % with the single CTA's 150 (8192 x 768 x 2304 60.9 us as planned then, 52.0 on pairs).
-        const double b16[4] = {136.0, 168.0, 138.0, 140.0};
-        const double t32[4] = {mn_operands ? 150.0 + 35.0 * mn_operands : 140.0, 150.0 + 65.0 * mn_operands,
-                               150.0 + 30.0 * mn_operands, 145.0 + 15.0 * mn_operands};
-        const double* cost = bk == 32 ? t32 : b16;
-        const double pair_start = 2000.0;            // cluster launch and the pair's handshakes, once per CTA
-        for (int i = 0; i < 4; ++i) {
-            const bool pr = i == 0;
+        for (int i = 0; i < 5; ++i) {
+            const Tile& t = tiles[i];
+            const bool pr = t.pair;
+            if (t.bn == 192 && t32) continue;
             if (pr && (max_pairs <= 0 || M <= BM)) continue;
-            if (force_bn && (force_bn == 512 ? !pr : (pr || bns[i] != force_bn))) continue;
-            if (bns[i] > 64 && N <= bns[i] / 2) continue;            // tile mostly padding
-            const long long t = (long long)cme_cdiv(M, pr ? 2 * BM : BM) * cme_cdiv(N, bns[i]) * batch;
+            if (force_bn && force_bn != (pr ? 2 : 1) * t.bn) continue;
+            if (t.bn > 64 && N <= t.bn / 2) continue;                // tile mostly padding
+            const long long count = (long long)cme_cdiv(M, pr ? 2 * BM : BM) * cme_cdiv(N, t.bn) * batch;
             const int slots = pr ? max_pairs : num_sms;
+            // bytes that an SM loads per k-block (half of a 192-column tile stored along N arrives as two groups of 64)
+            const double a_bytes = BM * BK_BYTES;
+            const double b_bytes = BK_BYTES * (!pr ? t.bn : t.bn == 192 && !at.b_mn ? 96 : 128);
+            double more_k = 1.0, more_l = 1.0;
+            auto operand = [&](bool mn, long long pitch, double share) {
+                if (pitch % 128) { more_k += share * line_k[t32][mn]; more_l += share * line_l[t32][mn]; }
+                if (pitch % 32) more_l += share * sector_l[t32];
+            };
+            operand(at.a_mn, at.a_pitch, a_bytes / (a_bytes + b_bytes));
+            operand(at.b_mn, at.b_pitch, b_bytes / (a_bytes + b_bytes));
+            const double alone = t.kblock[t32] * more_k * (t32 ? 1.0 + 0.034 * ((int)at.a_mn + (int)at.b_mn) : 1.0);
             for (int s = 1; s <= 16; ++s) {
                 if (force_splits && s != force_splits) continue;
                 if (s > 1 && (!plain_epi || num_kb / s < 4 || (long long)s * batch * M * N * 4 > workspace_bytes)) break;
-                const long long units = t * s;
+                const int kb = cme_cdiv(num_kb, s), parts = cme_cdiv(num_kb, kb);
+                const long long units = count * parts;
                 const double waves = (double)((units + slots - 1) / slots);
-                const double kb = (double)cme_cdiv(num_kb, s);
-                // 4 MMAs per k-block; epilogue / pipeline fill ~ 6 k-blocks of the widest tile per unit;
-                // a split adds one fp32 write + read of the output per split
-                double est = waves * ((kb + 2.0) * 4.0 * cost[i] + 6.0 * 4.0 * bns[i] / 2.0) + (pr ? pair_start : 0.0);
-                if (s > 1) est += 6000.0 + (double)s * M * N * batch / num_sms / 16.0;   // + one more launch
-                if (est < best) { best = est; best_bn = bns[i]; best_s = s; best_pair = pr; }
+                const double loading = (double)(units < slots ? units : slots) * (pr ? 2 : 1);
+                const double shared = (a_bytes + b_bytes) * more_l * loading / l2_bytes;
+                double est = t.start[t32] + waves * (kb * (alone > shared ? alone : shared) + t.unit[t32]);
+                // the reduction's launch, the partials written and read
+                if (parts > 1) est += (t32 ? 1.65 : 2.17) + (double)parts * M * N * batch * (t32 ? 5.5e-7 : 5.9e-7);
+                if (est < best) { best = est; best_bn = t.bn; best_s = s; best_pair = pr; }
             }
         }
         if (!bn) { bn = best_bn; pair = best_pair; }
@@ -228,15 +251,15 @@ static void plan_tiles(int M, int N, int K, int batch, bool plain_epi, long long
     *bn_out = bn; *pair_out = pair; *splits_out = splits;
 }
 
-// The plan the launcher would choose, without a device: `num_sms` SMs, `max_pairs` co-resident CTA pairs (0 = no
-// cluster launches).  out = {tile width, pair (0/1), splits}.
+// The plan the launcher would choose for operands stored along K, without a device: `num_sms` SMs, `max_pairs` co-resident CTA
+// pairs (0 = no cluster launches).  out = {tile width, pair (0/1), splits}.
 CME_API int cme_gemm_plan(int M, int N, int K, int batch, int plain_epilogue, long long workspace_bytes, int num_sms,
                           int max_pairs, int force_bn, int force_splits, int* out) {
     CME_REQUIRE(M > 0 && N > 0 && K > 0 && batch > 0 && num_sms > 0, CME_ERR_SHAPE, "gemm plan: empty problem");
     int bn = 0, splits = 0;
     bool pair = false;
     plan_tiles(M, N, K, batch, plain_epilogue != 0, workspace_bytes, num_sms, max_pairs, force_bn, force_splits, &bn,
-               &pair, &splits);
+               &pair, &splits, {false, false, K * 2ll, K * 2ll});
     out[0] = bn; out[1] = pair ? 1 : 0; out[2] = splits;
     return CME_OK;
 }
@@ -246,7 +269,9 @@ CME_API int cme_gemm_plan_tf32(int M, int N, int K, int mn_operands, long long w
                                int* out) {
     CME_REQUIRE(M > 0 && N > 0 && K > 0 && num_sms > 0, CME_ERR_SHAPE, "gemm plan: empty problem");
     bool pair = false;
-    plan_tiles(M, N, K, 1, true, workspace_bytes, num_sms, max_pairs, 0, 0, &out[0], &pair, &out[2], 32, mn_operands);
+    const bool a_mn = mn_operands > 1, b_mn = mn_operands > 0;
+    plan_tiles(M, N, K, 1, true, workspace_bytes, num_sms, max_pairs, 0, 0, &out[0], &pair, &out[2],
+               {a_mn, b_mn, (a_mn ? M : K) * 4ll, (b_mn ? N : K) * 4ll}, 32);
     out[1] = pair ? 1 : 0;
     return CME_OK;
 }
@@ -305,14 +330,16 @@ int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream) {
     int bn = 0, splits = 0;
     bool pair = false;
     plan_tiles(g->M, g->N, g->K, g->batch, plain_epi, g->workspace ? g->workspace_bytes : 0, g_num_sms, g_max_pairs,
-               g->force_bn, g->force_splits, &bn, &pair, &splits, BK, (g->a_trans != 0) + (g->b_trans == 0));
+               g->force_bn, g->force_splits, &bn, &pair, &splits,
+               {g->a_trans != 0, g->b_trans == 0, g->lda * (tf32 ? 4 : 2), g->ldb * (tf32 ? 4 : 2)}, BK);
     // A tf32 product that accumulates into C goes through the fp32 workspace like a split-K product (one "split"
     // is then added to C by the reduction kernel): the tf32 kernel variants only store.
     const bool via_ws = splits > 1 || (tf32 && g->accumulate);
     if (tf32 && g->accumulate)
         CME_REQUIRE(g->workspace && (long long)splits * g->batch * g->M * g->N * 4 <= g->workspace_bytes, CME_ERR_LIMIT,
                     "tf32 accumulate needs an fp32 workspace of M x N");
-    CME_REQUIRE(bn == 64 || bn == 128 || bn == 256, CME_ERR_SHAPE, "tile width must be 64, 128, 256 or 512 (pair)");
+    CME_REQUIRE(bn == 64 || bn == 128 || bn == 256 || (bn == 192 && pair && !tf32), CME_ERR_SHAPE,
+                "tile width must be 64, 128, 256, 512 (pair) or, in bf16, 384 (pair, 192 columns)");
     CME_REQUIRE(!pair || g_max_pairs > 0, CME_ERR_SHAPE, "CTA-pair tiles are not available on this device");
     if (pair) tiles_m = cme_cdiv(g->M, 2 * BM);
     static const bool trace = getenv("CME213_GEMM_TRACE") != nullptr;

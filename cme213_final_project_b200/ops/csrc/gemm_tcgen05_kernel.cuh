@@ -43,7 +43,8 @@ constexpr int NUM_THREADS_WIDE = 320;     // ... + 8 epilogue warps (two per sch
 
 // PAIR: two CTAs of a cluster share one 256 x BN tile.  Each stages 128 rows of A and BN/2 columns of B, the
 // leader issues cta_group::2 MMAs, and each holds its own 128 accumulator rows.  Per SM that is 2/3 of the
-// shared-memory fill traffic of a 128 x 256 tile for the same tensor work.
+// shared-memory fill traffic of a 128 x 256 tile for the same tensor work.  BN is 256, or 192 where that wastes fewer columns
+// or fills the last wave better (plan_tiles).
 // Epilogue shared memory: per epilogue warp a ring of NB buffers of 32 rows x 128 bytes.  A buffer receives the
 // warp's slice of the epilogue's input operand by TMA (residual, activation input of a derivative, or the old C),
 // is overwritten in place with the result and is then the source of the TMA store.  While the main loops keep
@@ -66,9 +67,12 @@ template <int BN, bool PAIR, bool SIMPLE, int SPEC = -1> struct Cfg {
     static constexpr int ES = TF32 ? 4 : 2;                   // operand element size
     static constexpr int BK = BK_BYTES / ES;                  // K elements per k-block
     static constexpr int GW = 128 / ES;                       // elements per 128-byte row of an MN-major operand tile
-    static constexpr int B_TILE_BYTES = BN_LOCAL * BK_BYTES;
+    // MN-major operands arrive in whole groups of GW columns: half of a 192-column tile is one group and a half
+    static constexpr int B_GROUPS = (BN_LOCAL + GW - 1) / GW;
+    static constexpr int B_TILE_BYTES = B_GROUPS * GW * BK_BYTES;
+    static constexpr int load_bytes(bool b_mn) { return A_TILE_BYTES + (b_mn ? B_TILE_BYTES : BN_LOCAL * BK_BYTES); }
     static constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
-    static constexpr int TMEM_COLS = (2 * BN < 32) ? 32 : 2 * BN;
+    static constexpr int TMEM_COLS = 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
     // Compile-time variants with a TMA-fed input or a second (pre-activation) output run eight epilogue warps, two
     // per warp scheduler, each set taking every other 64-column chunk: their dependent chains (TMEM load, shared
     // memory, MUFU) then overlap instead of leaving the scheduler idle.  Two buffers per warp there; three for the
@@ -391,7 +395,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     using S = Spec<SPEC>;
     constexpr int BK = C::BK, GW = C::GW;
     constexpr int GROUP_BYTES = BK * 128;           // one GW-wide column group of an MN-major tile: BK rows of 128 bytes
-    static_assert(!PAIR || BN == 256, "CTA pairs use 256-wide tiles");
+    static_assert(PAIR ? BN == 256 || BN == 192 : BN == 64 || BN == 128 || BN == 256, "tile widths");
     static_assert(!SIMPLE || SPEC < 0, "the plain epilogue has no compile-time variants");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -471,7 +475,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     uint8_t* sB = sA + A_TILE_BYTES;
                     if constexpr (PAIR) {
                         // both CTAs' bytes are credited to the leader's barrier, which its MMA thread waits on
-                        if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * C::STAGE_BYTES);
+                        if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2 * C::load_bytes(B_MN));
                         const uint32_t fb = mapa_u32(&full_bar[stage], 0);
                         if (!A_MN) {
                             tma_load_3d_pair(sA, &tmA, fb, kb * BK, m0, za);
@@ -484,7 +488,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             tma_load_3d_pair(sB, &tmB, fb, kb * BK, n0, zb);
                         } else {
 #pragma unroll
-                            for (int j = 0; j < C::BN_LOCAL / GW; ++j)
+                            for (int j = 0; j < C::B_GROUPS; ++j)
                                 tma_load_3d_pair(sB + j * GROUP_BYTES, &tmB, fb, n0 + j * GW, kb * BK, zb);
                         }
                     } else {
@@ -594,7 +598,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // Ring of this warp's epilogue buffers and the cursor of the input prefetch (fused bf16 epilogues only).  The
         // cursor runs over (tile, 64-column chunk) in the order the warp will consume them, NB - 1 chunks ahead, and
         // crosses tile boundaries, so the first chunks of a tile are already in flight while its main loop runs.
-        constexpr int ESETS = C::EPI_WARPS / 4;         // warp sets; set s takes the chunks c with c % ESETS == s
+        constexpr int ESETS = C::EPI_WARPS / 4;         // warp sets; each takes every ESETS-th chunk
         const int eset = (warp - 2) >> 2;
         const int wslot = eset * 4 + quarter;
         uint8_t* ring = staging + wslot * C::WARP_RING_BYTES;
@@ -606,7 +610,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const bool ring_epi = !SIMPLE && (SPEC >= 0 ? !S::c_f32(p) : (p.tma_store && !p.c_f32));
         const int in_kind = ring_epi ? S::in_kind(p) : 0;
         uint32_t slot = 0;                              // ring buffers handed out so far
-        int f_tile = tile0, f_c = eset;
+        // An odd number of chunks alternates between the sets from tile to tile, so that both do the same work.
+        constexpr bool ALTERNATE = ESETS == 2 && (BN / 64) % 2 == 1;
+        auto first_chunk = [&](int i) { return ALTERNATE ? (eset + i) & 1 : eset; };
+        int f_tile = tile0, f_it = 0, f_c = first_chunk(0);
         uint32_t f_cnt = 0;
         auto fetch_next = [&]() {
             int fmn = 0, fn0 = 0, fm_blk = 0;
@@ -619,7 +626,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 int nchf = (p.N - fn0 + 63) / 64;
                 nchf = nchf < BN / 64 ? nchf : BN / 64;
                 if (f_c < nchf) break;
-                f_c = eset;
+                f_c = first_chunk(++f_it);
                 f_tile += tile_step;
             }
             if (f_tile >= total_tiles) return;
@@ -771,7 +778,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 __nv_bfloat16* Xrow = (S::aux_out(p) && !aux_ring) ? reinterpret_cast<__nv_bfloat16*>(p.aux_out) + offa
                                                                    : nullptr;
 #pragma unroll 1
-                for (int c2 = eset; c2 < BN / 64; c2 += ESETS) {
+                for (int c2 = first_chunk(it); c2 < BN / 64; c2 += ESETS) {
                     const int n = n0 + c2 * 64;
                     if (n >= p.N) break;
                     uint8_t* sbC = ring + (slot % C::NB) * 4096;
