@@ -94,8 +94,9 @@ struct FwdParams {
 // What bounds it: the chain MMA -> TMEM load -> softmax -> TMEM store -> MMA of a tile (no pipe is busy for half of the time).
 // So a CTA is kept small enough for four on an SM: 128 queries, 64 keys at a time, P in the columns that its scores came
 // from, 128 TMEM columns, 64 score registers per thread; every scheduler then has four softmax warps of independent chains,
-// and a tile's start and end run under the others' work.  16 x 12 heads x 1024 tokens: causal 51.4 us, all keys 82.6 us (59.7 and
-// 93.4 with an issuing thread that the compiler did not know to be alone, see elect_one).
+// and a tile's start and end run under the others' work.  16 x 12 heads x 1024 tokens: causal 50.4 us, all keys 80.7 us.  Of the
+// 2340 clocks of a block the exponentials take 512 at the least (MUFU), alone; four CTAs in their loops would keep it busy, but a CTA
+// spends 5000 clocks starting and ending, so 2.75 are in their loops on average.
 // S_{j+1} goes to the columns that P_j V_j reads its A operand from.  PTX orders two MMAs of a thread only if they accumulate in
 // the same place, so S_{j+1} is issued once a barrier says that P_j V_j is complete.  Measured without that wait, when this form
 // took 57 and 89 us: two CTAs with 128 keys at a time 70 us causal; three with S_{j+1} made under softmax_j 57 and 87 us; a quarter
@@ -143,7 +144,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int bh = blockIdx.x, b = bh / p.nh, h = bh % p.nh;
     const int nkv = cme_cdiv_dev(p.causal ? min(q0 + BQ, p.T) : p.T, FWD_BKV);
 
-    if (threadIdx.x == 0) {
+    auto load_k = [&](int j) {
+        mbar_arrive_expect_tx(&k_full[j & 1], FWD_KV_BYTES);
+        tma_load_4d(sK + (j & 1) * FWD_KV_BYTES, &tmK, &k_full[j & 1], 0, j * FWD_BKV, h, b);
+    };
+    auto load_v = [&](int j) {
+        mbar_arrive_expect_tx(&v_full[j & 1], FWD_KV_BYTES);
+        tma_load_4d(sV + (j & 1) * FWD_KV_BYTES, &tmV, &v_full[j & 1], 0, j * FWD_BKV, h, b);
+    };
+    if (warp == 4 && elect_one()) {
         *abort_flag = 0;
         mbar_init(q_full, 1);
         for (int s = 0; s < 2; ++s) { mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1); }
@@ -151,8 +160,14 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_init(p_ready, 128);
         mbar_init(p_free, 1);
         fence_barrier_init();
+        pdl_wait();                                // the first loads run under the TMEM allocation
+        mbar_arrive_expect_tx(q_full, TILE_BYTES);
+        tma_load_4d(sQ, &tmQ, q_full, 0, q0, h, b);
+        load_k(0);
+        load_v(0);
+        if (nkv > 1) { load_k(1); load_v(1); }
     }
-    if (warp == 4) { tmem_alloc(tmem_slot, FWD_TMEM_COLS); tmem_relinquish(); }
+    if (warp == 0) { tmem_alloc(tmem_slot, FWD_TMEM_COLS); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -165,14 +180,6 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             // ---------------- producer + MMA issuer (one thread) ----------------
             constexpr uint32_t idesc_s = make_idesc(1, false, false, BQ, FWD_BKV);   // Q K^T: both K-major
             constexpr uint32_t idesc_o = make_idesc(1, false, true, BQ, HD);         // P V: V is MN-major
-            auto load_k = [&](int j) {
-                mbar_arrive_expect_tx(&k_full[j & 1], FWD_KV_BYTES);
-                tma_load_4d(sK + (j & 1) * FWD_KV_BYTES, &tmK, &k_full[j & 1], 0, j * FWD_BKV, h, b);
-            };
-            auto load_v = [&](int j) {
-                mbar_arrive_expect_tx(&v_full[j & 1], FWD_KV_BYTES);
-                tma_load_4d(sV + (j & 1) * FWD_KV_BYTES, &tmV, &v_full[j & 1], 0, j * FWD_BKV, h, b);
-            };
             const uint64_t dQ_ = make_smem_desc(smem_u32(sQ), 0, 1024);
             const uint64_t dK0 = make_smem_desc(smem_u32(sK), 0, 1024);
             const uint64_t dV0 = make_smem_desc(smem_u32(sV), FWD_KV_BYTES, 1024);
@@ -183,18 +190,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     mma_f16_ss(tmem_S, desc_add(dQ_, k * 32), desc_add(kd, k * 32), idesc_s, k > 0);
                 mma_commit(s_full);
             };
-            mbar_arrive_expect_tx(q_full, TILE_BYTES);
-            tma_load_4d(sQ, &tmQ, q_full, 0, q0, h, b);
-            load_k(0);
-            load_v(0);
-            if (nkv > 1) { load_k(1); load_v(1); }
             bool ok = mbar_wait(q_full, 0, abort_flag) && mbar_wait(&k_full[0], 0, abort_flag);
             if (ok) { tc_fence_after(); issue_s(0); }
             for (int j = 0; j < nkv && ok; ++j) {
                 if (!mbar_wait(p_ready, j & 1, abort_flag)) { ok = false; break; }
-                // S_j has been read, so its MMAs and with them those of P_{j-1} V_{j-1} are complete: refill their tiles
-                if (j + 2 < nkv) load_k(j + 2);
-                if (j >= 1 && j + 1 < nkv) load_v(j + 1);
                 if (!mbar_wait(&v_full[j & 1], (j >> 1) & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint64_t vd = desc_add(dV0, (j & 1) * FWD_KV_BYTES);
@@ -203,6 +202,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     mma_f16_ts(tmem_O, tmem_P + k * 8, desc_add(vd, k * 2048), idesc_o, (j > 0 || k > 0));
                 if (j + 1 < nkv) {
                     mma_commit(p_free);
+                    // S_j has been read, so its MMAs and with them those of P_{j-1} V_{j-1} are complete: refill their tiles while
+                    // the product just issued runs
+                    if (j + 2 < nkv) load_k(j + 2);
+                    if (j >= 1) load_v(j + 1);
                     if (!mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag) ||
                         !mbar_wait(p_free, j & 1, abort_flag)) { ok = false; break; }
                     tc_fence_after();
@@ -326,7 +329,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tc_fence_before();
     __syncthreads();
     if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, CME_ERR_TIMEOUT);
-    if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem_base, FWD_TMEM_COLS); }
+    if (warp == 0) { tc_fence_after(); tmem_dealloc(tmem_base, FWD_TMEM_COLS); }
 }
 
 // ------------------------------------------------------------------------------------------------------
@@ -587,16 +590,18 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // so P never passes through shared memory and 256 TMEM columns and 106 KB of shared memory are enough.
 // The parts that the key blocks contribute to dQ_i are added to an fp32 scratch by bulk reduce-adds in arrival order; the
 // launch clears the scratch beforehand and dq_convert_kernel scales and casts the sums.
-// What bounds it: the chain of a block (two round trips to the tensor pipe, about 6000 clocks, hidden by one other CTA only);
-// the tensor pipe is busy for 45 % of the time (a product of 64 columns takes as long as one of 128).
-// 16 x 12 heads x 1024 tokens: causal 135 us, all keys 229 us (157 and 265 with an issuing thread that the compiler did not know to
-// be alone, see elect_one).
-// shared: K 16K | V 16K | Q[3] 24K | dO[2] 16K | dS^T 16K | dQ staging (fp32) 16K | row statistics[2] 1K | barriers
+// What bounds it: the chain of a block (two round trips to the tensor pipe, 3450 clocks, hidden by one other CTA only): 1500 from S^T
+// to dS^T, the same until the next S^T.  The tensor pipe is busy for 41 % of the time, issue slots 31 %.
+// 16 x 12 heads x 1024 tokens: causal 129 us, all keys 209 us (135 and 229 with dP^T made before S^T, arithmetic on the statistics as
+// they are loaded, and reduce-adds awaited after each block).
+// dS^T and the fp32 staging of the dQ that is made from it share a buffer, of which there are two: a block's tile is stored once
+// the reduce-adds of two blocks ago have been read.
+// shared: K 16K | V 16K | Q[3] 24K | dO[2] 16K | dS^T, then dQ staging [2] 32K | row statistics[2] 1K | barriers
 constexpr int BWD_BQ = 64;                 // queries per step
 constexpr int BWD_Q_BYTES = BWD_BQ * HD * 2;
 constexpr int BWD_Q_STAGES = 3, BWD_DO_STAGES = 2;
 constexpr int BWD_STAT_FLOATS = 2 * BWD_BQ;           // -log-sum-exp (log2 units) and -delta of a block's queries
-constexpr int BWD_SMEM = 4 * TILE_BYTES + (BWD_Q_STAGES + BWD_DO_STAGES) * BWD_Q_BYTES + 2 * BWD_STAT_FLOATS * 4 + 128;
+constexpr int BWD_SMEM = 4 * TILE_BYTES + (BWD_Q_STAGES + BWD_DO_STAGES) * BWD_Q_BYTES + 2 * BWD_STAT_FLOATS * 4 + 192;
 constexpr int BWD_MMA_WARP = 8;            // warps 0..7 compute, warp 8 issues TMA loads and MMA,
 constexpr int BWD_STORE_WARP = 9;          // warp 9 issues the dQ reduce-adds
 constexpr int BWD_THREADS = 10 * 32;
@@ -627,21 +632,22 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint8_t* sV = sK + TILE_BYTES;
     uint8_t* sQ = sV + TILE_BYTES;
     uint8_t* sdO = sQ + BWD_Q_STAGES * BWD_Q_BYTES;
-    uint8_t* sdS = sdO + BWD_DO_STAGES * BWD_Q_BYTES;     // [128 keys][64 queries = 128 B]
-    uint8_t* sdQ = sdS + TILE_BYTES;                      // [2 column atoms][64 query rows][128 B]
-    float* stats = reinterpret_cast<float*>(sdQ + TILE_BYTES);
+    uint8_t* sX = sdO + BWD_DO_STAGES * BWD_Q_BYTES;      // [2 buffers]: dS^T [128 keys][64 queries = 128 B], then
+                                                          // dQ [2 column atoms][64 query rows][128 B]
+    float* stats = reinterpret_cast<float*>(sX + 2 * TILE_BYTES);
     uint64_t* bars = reinterpret_cast<uint64_t*>(stats + 2 * BWD_STAT_FLOATS);
     uint64_t* kv_full = bars;
     uint64_t* q_full = bars + 1;               // [3]
     uint64_t* do_full = bars + 4;              // [2]
-    uint64_t* s_full = bars + 6;               // S^T and dP^T of a query block are in TMEM
-    uint64_t* p_ready = bars + 7;              // S^T, dP^T read; P^T, dS^T written; the next statistics stored (256 arrivals)
-    uint64_t* dq_full = bars + 8;              // dQ of a query block complete
-    uint64_t* dq_free = bars + 9;              // dQ in registers (256 arrivals): dP^T may overwrite it
-    uint64_t* in_free = bars + 10;             // dV, dK accumulated: the block's Q and dO tiles may be refilled
-    uint64_t* dqs_full = bars + 11;            // dQ staging written (256 arrivals)
-    uint64_t* dqs_free = bars + 12;            // dQ staging read by the reduce-add
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+    uint64_t* s_full = bars + 6;               // S^T of a query block is in TMEM
+    uint64_t* dp_full = bars + 7;              // dP^T too
+    uint64_t* p_ready = bars + 8;              // S^T, dP^T read; P^T, dS^T written; the next statistics stored (256 arrivals)
+    uint64_t* dq_full = bars + 9;              // dQ of a query block complete
+    uint64_t* dq_free = bars + 10;             // dQ in registers (256 arrivals): dP^T may overwrite it
+    uint64_t* in_free = bars + 11;             // dV, dK accumulated: P^T and dS^T, the block's Q and dO tiles may be overwritten
+    uint64_t* dqs_full = bars + 12;            // [2] dQ staging written (256 arrivals)
+    uint64_t* dqs_free = bars + 14;            // [2] dQ staging read by the reduce-add
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -651,21 +657,39 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int q_begin = p.causal ? k0 : 0;
     const int n_it = cme_cdiv_dev(p.T - q_begin, BWD_BQ);          // >= 1: k0 < T
 
-    if (threadIdx.x == 0) {
+    auto load_q = [&](int it) {
+        const int s = it % BWD_Q_STAGES;
+        mbar_arrive_expect_tx(&q_full[s], BWD_Q_BYTES);
+        tma_load_4d(sQ + s * BWD_Q_BYTES, &tmQ, &q_full[s], 0, q_begin + it * BWD_BQ, h, b);
+    };
+    auto load_do = [&](int it) {
+        const int s = it % BWD_DO_STAGES;
+        mbar_arrive_expect_tx(&do_full[s], BWD_Q_BYTES);
+        tma_load_4d(sdO + s * BWD_Q_BYTES, &tmdO, &do_full[s], 0, q_begin + it * BWD_BQ, h, b);
+    };
+    if (warp == BWD_MMA_WARP && elect_one()) {
         *abort_flag = 0;
         mbar_init(kv_full, 1);
         for (int s = 0; s < BWD_Q_STAGES; ++s) mbar_init(&q_full[s], 1);
         for (int s = 0; s < BWD_DO_STAGES; ++s) mbar_init(&do_full[s], 1);
         mbar_init(s_full, 1);
+        mbar_init(dp_full, 1);
         mbar_init(p_ready, 256);
         mbar_init(dq_full, 1);
         mbar_init(dq_free, 256);
         mbar_init(in_free, 1);
-        mbar_init(dqs_full, 256);
-        mbar_init(dqs_free, 1);
+        for (int s = 0; s < 2; ++s) { mbar_init(&dqs_full[s], 256); mbar_init(&dqs_free[s], 1); }
         fence_barrier_init();
+        pdl_wait();                                // the first loads run under the TMEM allocation
+        mbar_arrive_expect_tx(kv_full, 2 * TILE_BYTES);
+        tma_load_4d(sK, &tmK, kv_full, 0, k0, h, b);
+        load_q(0);
+        tma_load_4d(sV, &tmV, kv_full, 0, k0, h, b);
+        load_do(0);
+        for (int it = 1; it < BWD_Q_STAGES && it < n_it; ++it) load_q(it);
+        for (int it = 1; it < BWD_DO_STAGES && it < n_it; ++it) load_do(it);
     }
-    if (warp == BWD_MMA_WARP) { tmem_alloc(tmem_slot, BWD_TMEM_COLS); tmem_relinquish(); }
+    if (warp == BWD_STORE_WARP) { tmem_alloc(tmem_slot, BWD_TMEM_COLS); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -679,23 +703,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             constexpr uint32_t idesc_s = make_idesc(1, false, false, BKV, BWD_BQ);    // K Q^T, V dO^T
             constexpr uint32_t idesc_t = make_idesc(1, false, true, BKV, HD);         // P^T dO, dS^T Q
             constexpr uint32_t idesc_q = make_idesc(1, true, true, BWD_BQ, HD);       // dS K (A read transposed)
-            auto load_q = [&](int it) {
-                const int s = it % BWD_Q_STAGES;
-                mbar_arrive_expect_tx(&q_full[s], BWD_Q_BYTES);
-                tma_load_4d(sQ + s * BWD_Q_BYTES, &tmQ, &q_full[s], 0, q_begin + it * BWD_BQ, h, b);
-            };
-            auto load_do = [&](int it) {
-                const int s = it % BWD_DO_STAGES;
-                mbar_arrive_expect_tx(&do_full[s], BWD_Q_BYTES);
-                tma_load_4d(sdO + s * BWD_Q_BYTES, &tmdO, &do_full[s], 0, q_begin + it * BWD_BQ, h, b);
-            };
             // descriptors are encoded once; per MMA only a byte offset is added
             const uint64_t kK = make_smem_desc(smem_u32(sK), 0, 1024), vK = make_smem_desc(smem_u32(sV), 0, 1024);
             const uint64_t kMN = make_smem_desc(smem_u32(sK), TILE_BYTES, 1024);
             const uint64_t qK0 = make_smem_desc(smem_u32(sQ), 0, 1024), oK0 = make_smem_desc(smem_u32(sdO), 0, 1024);
             const uint64_t qMN0 = make_smem_desc(smem_u32(sQ), BWD_Q_BYTES, 1024);
             const uint64_t oMN0 = make_smem_desc(smem_u32(sdO), BWD_Q_BYTES, 1024);
-            const uint64_t sMN = make_smem_desc(smem_u32(sdS), TILE_BYTES, 1024);
+            const uint64_t sMN = make_smem_desc(smem_u32(sX), TILE_BYTES, 1024);
             auto issue_s = [&](int it) {
                 const uint64_t qd = desc_add(qK0, (it % BWD_Q_STAGES) * BWD_Q_BYTES);
 #pragma unroll
@@ -708,25 +722,18 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 for (int k = 0; k < HD / 16; ++k)
                     mma_f16_ss(tmem_dP, desc_add(vK, k * 32), desc_add(od, k * 32), idesc_s, k > 0);
             };
-            mbar_arrive_expect_tx(kv_full, 2 * TILE_BYTES);
-            tma_load_4d(sK, &tmK, kv_full, 0, k0, h, b);
-            load_q(0);
-            tma_load_4d(sV, &tmV, kv_full, 0, k0, h, b);
-            load_do(0);
-            for (int it = 1; it < BWD_Q_STAGES && it < n_it; ++it) load_q(it);
-            for (int it = 1; it < BWD_DO_STAGES && it < n_it; ++it) load_do(it);
             bool ok = mbar_wait(kv_full, 0, abort_flag) && mbar_wait(&q_full[0], 0, abort_flag) &&
                       mbar_wait(&do_full[0], 0, abort_flag);
-            if (ok) { tc_fence_after(); issue_s(0); issue_dp(0); mma_commit(s_full); }
+            if (ok) { tc_fence_after(); issue_s(0); mma_commit(s_full); issue_dp(0); mma_commit(dp_full); }
             for (int it = 0; it < n_it && ok; ++it) {
                 if (!mbar_wait(p_ready, it & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint64_t qd = desc_add(qMN0, (it % BWD_Q_STAGES) * BWD_Q_BYTES),
-                               od = desc_add(oMN0, (it % BWD_DO_STAGES) * BWD_Q_BYTES);
+                               od = desc_add(oMN0, (it % BWD_DO_STAGES) * BWD_Q_BYTES), sd = desc_add(sMN, (it & 1) * TILE_BYTES);
                 // dQ first: the warps read it out while the other products of this block run
 #pragma unroll
                 for (int k = 0; k < BKV / 16; ++k)        // reduction over the 128 keys of this CTA
-                    mma_f16_ss(tmem_dQ, desc_add(sMN, k * 2048), desc_add(kMN, k * 2048), idesc_q, k > 0);
+                    mma_f16_ss(tmem_dQ, desc_add(sd, k * 2048), desc_add(kMN, k * 2048), idesc_q, k > 0);
                 mma_commit(dq_full);
                 const uint32_t acc = it > 0;
 #pragma unroll
@@ -737,19 +744,20 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     mma_f16_ts(tmem_dK, tmem_S + (k >> 1) * 32 + 16 + (k & 1) * 8, desc_add(qd, k * 2048), idesc_t, acc | (k > 0));
                 mma_commit(in_free);
                 if (it + 1 < n_it) {
-                    // dP^T takes the place of dQ once the warps have it in registers; S^T that of P^T and dS^T once a barrier says
-                    // that the products above, which read them, are complete (PTX orders MMAs of a thread only if they accumulate
-                    // in the same place).  S^T second: what it waits for runs beside dP^T (first: 3 us of 183 more)
+                    // S^T takes the place of P^T and dS^T once a barrier says that the products above, which read them, are complete
+                    // (PTX orders MMAs of a thread only if they accumulate in the same place): before the warps have dQ in
+                    // registers, so that their exponentials run while dP^T, which takes its place, is made.
                     const int n = it + 1;
-                    if (!mbar_wait(dq_free, it & 1, abort_flag) ||
-                        !mbar_wait(&do_full[n % BWD_DO_STAGES], (n / BWD_DO_STAGES) & 1, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    issue_dp(n);
                     if (!mbar_wait(&q_full[n % BWD_Q_STAGES], (n / BWD_Q_STAGES) & 1, abort_flag) ||
                         !mbar_wait(in_free, it & 1, abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     issue_s(n);
                     mma_commit(s_full);
+                    if (!mbar_wait(&do_full[n % BWD_DO_STAGES], (n / BWD_DO_STAGES) & 1, abort_flag) ||
+                        !mbar_wait(dq_free, it & 1, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
+                    issue_dp(n);
+                    mma_commit(dp_full);
                     if (it + BWD_DO_STAGES < n_it) load_do(it + BWD_DO_STAGES);
                     if (it + BWD_Q_STAGES < n_it) load_q(it + BWD_Q_STAGES);
                 }
@@ -759,15 +767,15 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     } else if (warp == BWD_STORE_WARP) {
         if (elect_one()) {
             for (int it = 0; it < n_it; ++it) {
-                if (!mbar_wait(dqs_full, it & 1, abort_flag)) break;
+                if (!mbar_wait(&dqs_full[it & 1], (it >> 1) & 1, abort_flag)) break;
                 const int q0 = q_begin + it * BWD_BQ;
-                tma_reduce_add_3d(&tmdQ, sdQ, 0, q0, bh);
-                tma_reduce_add_3d(&tmdQ, sdQ + TILE_BYTES / 2, 32, q0, bh);
+                const uint8_t* tile = sX + (it & 1) * TILE_BYTES;
+                tma_reduce_add_3d(&tmdQ, tile, 0, q0, bh);
+                tma_reduce_add_3d(&tmdQ, tile + TILE_BYTES / 2, 32, q0, bh);
                 tma_store_commit();
                 tma_store_wait_read<0>();
-                mbar_arrive(dqs_free);                  // the staging tile may be refilled
+                mbar_arrive(&dqs_free[it & 1]);         // the buffer may be refilled; no shared memory is read after the last wait
             }
-            tma_store_wait<0>();
         }
     } else {
         // ---------------- gradient warps: warp w owns TMEM lanes 32 (w & 3).. (key rows) and the 32 queries (w >> 2) of a
@@ -779,13 +787,17 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const uint32_t tS = tmem_S + lane_addr + cg * 32;
         // -lse and -delta of a block's queries are read by all threads as columns: 128 threads bring them to shared memory,
         // one block ahead.  Queries beyond T get probability 2^-inf = 0.
-        auto stat = [&](int it) {
-            const int i = threadIdx.x & (BWD_BQ - 1), q = q_begin + it * BWD_BQ + i;
-            const long long at = (long long)bh * p.T + q;
-            if (threadIdx.x < BWD_BQ) return q < p.T ? -p.lse[at] * LOG2E : -INFINITY;
-            return q < p.T ? -p.delta[at] : 0.f;
+        // The loaded value is not touched before it is stored: arithmetic on it here would wait for the load (800 clocks of every
+        // block for these warps, and with them for all).
+        const bool is_lse = threadIdx.x < BWD_BQ;
+        const float* stat_src = (is_lse ? p.lse : p.delta) + (long long)bh * p.T;
+        auto stat_q = [&](int it) { return q_begin + it * BWD_BQ + (int)(threadIdx.x & (BWD_BQ - 1)); };
+        auto stat_load = [&](int it) { const int q = stat_q(it); return q < p.T ? stat_src[q] : 0.f; };
+        auto stat_store = [&](int it, float v) {
+            const float x = is_lse ? (stat_q(it) < p.T ? -v * LOG2E : -INFINITY) : -v;
+            stats[(it & 1) * BWD_STAT_FLOATS + threadIdx.x] = x;
         };
-        if (threadIdx.x < BWD_STAT_FLOATS) stats[threadIdx.x] = stat(0);
+        if (threadIdx.x < BWD_STAT_FLOATS) stat_store(0, stat_load(0));
         asm volatile("bar.sync 1, 256;" ::: "memory");
         const F32x2 sc2 = f2_splat(p.scale_log2);
         bool ok = true;
@@ -793,7 +805,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             const int q0 = q_begin + it * BWD_BQ;
             float next = 0.f;
             const bool fetch = it + 1 < n_it && threadIdx.x < BWD_STAT_FLOATS;
-            if (fetch) next = stat(it + 1);
+            if (fetch) next = stat_load(it + 1);
             // the statistics were stored before the previous block's arrivals on p_ready (a phase that is complete)
             if ((it > 0 && !mbar_wait(p_ready, (it - 1) & 1, abort_flag)) || !mbar_wait(s_full, it & 1, abort_flag)) {
                 ok = false;
@@ -802,7 +814,6 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             tc_fence_after();
             uint32_t rs[32], rd[32];
             tmem_ld32(tS, rs);
-            tmem_ld32(tmem_dP + lane_addr + cg * 32, rd);
             tmem_wait_ld();
             if (q0 + BWD_BQ > p.T) {
                 // the rows of Q beyond T are zeros, and 0 k is NaN where an element of the key is infinite: 0, so that the
@@ -811,43 +822,52 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
                 for (int i = 0; i < 32; ++i) rs[i] = i < hi ? rs[i] : 0u;
             }
-            const bool need_mask = k0 + BKV > p.T || (p.causal && q0 < k0 + BKV);
-            // queries [lo, 32) of this thread's 32 see its key
-            const int lo = (key < p.T ? (p.causal ? key - q0 : 0) : BWD_BQ) - cg * 32;
             const float4* st = reinterpret_cast<const float4*>(stats + (it & 1) * BWD_STAT_FLOATS + cg * 32);
+            float* pr = reinterpret_cast<float*>(rs);
             // scale-and-shift, dP - delta and the product on packed pairs (one instruction per two queries)
 #pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const float4 nl = st[i / 4];
+                f2_unpack(f2_fma(f2_pack(pr[i], pr[i + 1]), sc2, f2_pack(nl.x, nl.y)), pr[i], pr[i + 1]);
+                f2_unpack(f2_fma(f2_pack(pr[i + 2], pr[i + 3]), sc2, f2_pack(nl.z, nl.w)), pr[i + 2], pr[i + 3]);
+            }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) pr[i] = ex2_approx(pr[i]);
+            if (k0 + BKV > p.T || (p.causal && q0 < k0 + BKV)) {
+                // queries [lo, 32) of this thread's 32 see its key
+                const int lo = (key < p.T ? (p.causal ? key - q0 : 0) : BWD_BQ) - cg * 32;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) pr[i] = i >= lo ? pr[i] : 0.f;
+            }
+            if (!mbar_wait(dp_full, it & 1, abort_flag) ||
+                (it >= 2 && !mbar_wait(&dqs_free[it & 1], ((it >> 1) - 1) & 1, abort_flag))) { ok = false; break; }
+            tc_fence_after();
+            tmem_ld32(tmem_dP + lane_addr + cg * 32, rd);
+            tmem_wait_ld();
+            uint8_t* tile = sX + (it & 1) * TILE_BYTES;
+#pragma unroll
             for (int g = 0; g < 4; ++g) {
-                float pr[8], ds[8];
+                float* ds = reinterpret_cast<float*>(rd) + g * 8;
 #pragma unroll
                 for (int i = 0; i < 8; i += 4) {
-                    const float4 nl = st[(g * 8 + i) / 4], nd = st[(BWD_BQ + g * 8 + i) / 4];
-                    const float* s = reinterpret_cast<const float*>(rs + g * 8 + i);
-                    const float* d = reinterpret_cast<const float*>(rd + g * 8 + i);
-                    f2_unpack(f2_fma(f2_pack(s[0], s[1]), sc2, f2_pack(nl.x, nl.y)), pr[i], pr[i + 1]);
-                    f2_unpack(f2_fma(f2_pack(s[2], s[3]), sc2, f2_pack(nl.z, nl.w)), pr[i + 2], pr[i + 3]);
-                    f2_unpack(f2_add(f2_pack(d[0], d[1]), f2_pack(nd.x, nd.y)), ds[i], ds[i + 1]);
-                    f2_unpack(f2_add(f2_pack(d[2], d[3]), f2_pack(nd.z, nd.w)), ds[i + 2], ds[i + 3]);
+                    const float4 nd = st[(BWD_BQ + g * 8 + i) / 4];
+                    f2_unpack(f2_add(f2_pack(ds[i], ds[i + 1]), f2_pack(nd.x, nd.y)), ds[i], ds[i + 1]);
+                    f2_unpack(f2_add(f2_pack(ds[i + 2], ds[i + 3]), f2_pack(nd.z, nd.w)), ds[i + 2], ds[i + 3]);
                 }
 #pragma unroll
-                for (int i = 0; i < 8; ++i) pr[i] = ex2_approx(pr[i]);
-                if (need_mask) {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) pr[i] = g * 8 + i >= lo ? pr[i] : 0.f;
-                }
-#pragma unroll
-                for (int i = 0; i < 8; i += 2) f2_unpack(f2_mul(f2_pack(pr[i], pr[i + 1]), f2_pack(ds[i], ds[i + 1])), ds[i], ds[i + 1]);
+                for (int i = 0; i < 8; i += 2)
+                    f2_unpack(f2_mul(f2_pack(pr[g * 8 + i], pr[g * 8 + i + 1]), f2_pack(ds[i], ds[i + 1])), ds[i], ds[i + 1]);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {           // the packed pairs take the registers of the scores they came from
-                    rs[g * 4 + i] = f2_to_bf2(pr[2 * i], pr[2 * i + 1]);
+                    rs[g * 4 + i] = f2_to_bf2(pr[g * 8 + 2 * i], pr[g * 8 + 2 * i + 1]);
                     rd[g * 4 + i] = f2_to_bf2(ds[2 * i], ds[2 * i + 1]);
                 }
-                *reinterpret_cast<uint4*>(sdS + swz(row, cg * 4 + g)) =
+                *reinterpret_cast<uint4*>(tile + swz(row, cg * 4 + g)) =
                     make_uint4(rd[g * 4], rd[g * 4 + 1], rd[g * 4 + 2], rd[g * 4 + 3]);
             }
             tmem_st16(tS, rs);
             tmem_st16(tS + 16, rd);
-            if (fetch) stats[((it + 1) & 1) * BWD_STAT_FLOATS + threadIdx.x] = next;
+            if (fetch) stat_store(it + 1, next);
             tmem_wait_st();
             tc_fence_before();
             fence_proxy_async();                        // dS^T
@@ -861,16 +881,15 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             tmem_wait_ld();
             tc_fence_before();
             mbar_arrive(dq_free);
-            if (it > 0 && !mbar_wait(dqs_free, (it - 1) & 1, abort_flag)) { ok = false; break; }
-            if (lane < 16) {
-                uint8_t* atom = sdQ + cg * (TILE_BYTES / 2);
+            if (lane < 16) {                            // dS^T has been read by the product that made dQ
+                uint8_t* atom = tile + cg * (TILE_BYTES / 2);
 #pragma unroll
                 for (int g = 0; g < 8; ++g)
                     *reinterpret_cast<uint4*>(atom + swz(quarter * 16 + lane, g)) =
                         make_uint4(t[4 * g], t[4 * g + 1], t[4 * g + 2], t[4 * g + 3]);
             }
             fence_proxy_async();
-            mbar_arrive(dqs_full);
+            mbar_arrive(&dqs_full[it & 1]);
         }
         // dV, dK of this key block: this warp's 32 columns (64 bytes = two full sectors per row) straight from registers
         if (ok && mbar_wait(in_free, (n_it - 1) & 1, abort_flag)) {
@@ -898,7 +917,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tc_fence_before();
     __syncthreads();
     if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, CME_ERR_TIMEOUT);
-    if (warp == BWD_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, BWD_TMEM_COLS); }
+    if (warp == BWD_STORE_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, BWD_TMEM_COLS); }
 }
 
 // ------------------------------------------------------------------------------------------------------
@@ -1276,7 +1295,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         // between the arrival of S and the first exponential
         auto row_stats = [&](int it2, float& l2, float& d2) {
             const int qc2 = min(qblock(it2) * BQ + row, p.T - 1);
-            l2 = p.lse[(long long)bh * p.T + qc2] * LOG2E;
+            l2 = p.lse[(long long)bh * p.T + qc2];       // used untouched a block later, so that nothing waits for it here
             d2 = p.delta[(long long)bh * p.T + qc2];
         };
         float lse2_n = 0.f, dl_n = 0.f;
@@ -1284,7 +1303,7 @@ attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int it = 0; it < n_it && ok; ++it) {
             const int qi0 = qblock(it) * BQ;
             const int q = qi0 + row;
-            const float lse2 = lse2_n, dl = dl_n;
+            const float lse2 = lse2_n * LOG2E, dl = dl_n;
             if (it + 1 < n_it) row_stats(it + 1, lse2_n, dl_n);
             uint8_t* bufP = sP;
             uint8_t* bufS = sdS + (it & 1) * 2 * TILE_BYTES;
