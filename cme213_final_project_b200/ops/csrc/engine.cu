@@ -224,6 +224,18 @@ int gemm(const Engine& e, cudaStream_t st, int M, int N, int K, const void* A, l
     return cme_gemm(&g, e.d.gemm_backend, st);
 }
 
+// d ln1 of the models with separate Q, K and V: three products that accumulate into it, rounded after each.
+int gemm_sum3(const Engine& e, cudaStream_t st, int M, int N, int K, const void* A, long long sA, const void* B, long long sB, void* C) {
+    CmeGemm g{};
+    g.M = M; g.N = N; g.K = K; g.batch = 3;
+    g.A = A; g.lda = K; g.strideA = sA;
+    g.B = B; g.ldb = K; g.strideB = sB; g.b_trans = 1;
+    g.C = C; g.ldc = N; g.c_dtype = e.d.dtype; g.ab_dtype = e.d.dtype;
+    g.allow_tf32 = e.d.allow_tf32;
+    g.workspace = e.gemm_ws; g.workspace_bytes = e.gemm_ws_bytes;
+    return cme_gemm_sum3(&g, e.d.gemm_backend, st);
+}
+
 // A plain product of bf16 operands with an fp32 result (the reduced-precision feed-forward experiment).
 int gemm_lp(const Engine& e, cudaStream_t st, int M, int N, int K, const void* A, long long lda, int a_trans,
             const void* B, long long ldb, int b_trans, void* C, long long ldc, int accumulate = 0) {
@@ -715,9 +727,8 @@ CME_API int cme_engine_backward(void* h, const int* tokens, int accumulate, CmeB
             TRY(gemm(e, st, BT, D, 3 * D, e.dqkv, 3 * D, 0, e.P(s.Wqkv), 3 * D, 1, e.dln, D));
             TRY(gemm(e, ws, D, 3 * D, BT, a.ln1, D, 1, e.dqkv, 3 * D, 0, e.G(s.Wqkv), 3 * D, accumulate));
         } else {
-            const long long pl = (long long)BT * D * e.es, wm = (long long)D * D * e.es;
-            for (int i = 0; i < 3; ++i)
-                TRY(gemm(e, st, BT, D, D, e.dqkv + i * pl, D, 0, e.P(s.Wq) + i * wm, D, 1, e.dln, D, i > 0));
+            const long long pl = (long long)BT * D, wm = (long long)D * D;
+            TRY(gemm_sum3(e, st, BT, D, D, e.dqkv, pl, e.P(s.Wq), wm, e.dln));
             TRY(gemm(e, ws, D, D, BT, a.ln1, D, 1, e.dqkv, D, 0, e.G(s.Wq), D, accumulate, nullptr, 0, nullptr, 0,
                      nullptr, 0, nullptr, 0, 3, 0, (long long)BT * D, (long long)D * D));
         }

@@ -45,4 +45,6 @@ struct CmeGemm {
 
 int gemm_tcgen05_supported(const CmeGemm* g);
 int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream);
+extern "C" int cme_gemm(const CmeGemm* g, int backend, void* stream);
+extern "C" int cme_gemm_sum3(const CmeGemm* g, int backend, void* stream);     // see gemm_tcgen05.cu
 int gemm_simt_launch(const CmeGemm* g, cudaStream_t stream);

@@ -101,6 +101,10 @@ CME_GEMM_TC_EXTERN(192, false, true, SPEC_DMUL)
 CME_GEMM_TC_EXTERN(192, false, true, SPEC_DRELU)
 #endif
 
+#if CME_GEMM_TC_GROUP == -1 || CME_GEMM_TC_GROUP == 15     // three products, each rounded
+CME_GEMM_TC_EXTERN(64, false, false, SPEC_SUM3)
+#endif
+
 #ifdef CME_GEMM_TC_GROUP_DEFAULTED
 #undef CME_GEMM_TC_GROUP
 #undef CME_GEMM_TC_GROUP_DEFAULTED

@@ -38,6 +38,10 @@ constexpr int A_TILE_BYTES = BM * BK_BYTES;
 // Operand element type of a kernel variant: SPEC bit 14 set = fp32 storage multiplied as tf32 (kind::tf32), output
 // fp32.  The tile geometry is the same in bytes; only element counts and the instruction kind differ.
 constexpr bool spec_tf32(int spec) { return spec >= 0 && ((spec >> 14) & 1) != 0; }
+// SPEC bit 15 set = C is the sum of three products (the operands' batch entries), rounded to bf16 after each: what three products
+// that accumulate into C leave there, in one launch.
+constexpr bool spec_chain(int spec) { return spec >= 0 && ((spec >> 15) & 1) != 0; }
+constexpr int CHAIN = 3;
 constexpr int NUM_THREADS = 192;          // TMA warp + MMA warp + 4 epilogue warps
 constexpr int NUM_THREADS_WIDE = 320;     // ... + 8 epilogue warps (two per scheduler) for the arithmetic-heavy epilogues
 
@@ -72,7 +76,9 @@ template <int BN, bool PAIR, bool SIMPLE, int SPEC = -1> struct Cfg {
     static constexpr int B_TILE_BYTES = B_GROUPS * GW * BK_BYTES;
     static constexpr int load_bytes(bool b_mn) { return A_TILE_BYTES + (b_mn ? B_TILE_BYTES : BN_LOCAL * BK_BYTES); }
     static constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
-    static constexpr int TMEM_COLS = 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
+    static constexpr bool SUM3 = spec_chain(SPEC);
+    static constexpr int ACC_COLS = SUM3 ? CHAIN * BN : BN;   // accumulator columns of a tile
+    static constexpr int TMEM_COLS = 2 * ACC_COLS <= 128 ? 128 : 2 * ACC_COLS <= 256 ? 256 : 512;
     // Compile-time variants with a TMA-fed input or a second (pre-activation) output run eight epilogue warps, two
     // per warp scheduler, each set taking every other 64-column chunk: their dependent chains (TMEM load, shared
     // memory, MUFU) then overlap instead of leaving the scheduler idle.  Two buffers per warp there; three for the
@@ -94,6 +100,7 @@ template <int BN, bool PAIR, bool SIMPLE, int SPEC = -1> struct Cfg {
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + FIXED_BYTES;
     static_assert(STAGES >= 3, "too few main-loop stages");
     static_assert(SMEM_BYTES <= SMEM_LIMIT, "shared-memory carve-up exceeds what one CTA may have");
+    static_assert(2 * ACC_COLS <= 512 && (!SUM3 || (BN == 64 && !PAIR)), "three accumulators, twice, must fit TMEM");
     static_assert(TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "two accumulators must fit TMEM (power of two)");
     static_assert(STAGE_BYTES % 1024 == 0 && A_TILE_BYTES % 1024 == 0, "swizzled tiles need 1024-byte aligned bases");
     static_assert(BAR_BYTES >= (2 * 8 + 4 + EPI_WARPS * NB) * 8 + 8, "barrier block too small");
@@ -270,7 +277,8 @@ __device__ __forceinline__ void load8_guard(const __nv_bfloat16* rowp, int n, in
 //   bit 0 bias | bits 1-2 act | bits 3-4 dact | bit 5 residual | bit 6 accumulate | bit 7 aux_out |
 //   bits 8-9 in_kind | bit 10 aux_ring | bit 11 fp32 output (split-K partials; nothing else set) |
 //   bit 12 aux tensors hold the activation's derivative | bit 13 column sums of C |
-//   bit 14 fp32 operands multiplied as tf32 (with bit 11: fp32 output)
+//   bit 14 fp32 operands multiplied as tf32 (with bit 11: fp32 output) |
+//   bit 15 sum of three products, each rounded (nothing else set)
 constexpr int spec_pack(bool bias, int act, int dact, bool res, bool accum, bool aux, int in_kind, bool aux_ring,
                         bool aux_deriv = false, bool colsum = false) {
     return int(bias) | (act << 1) | (dact << 3) | (int(res) << 5) | (int(accum) << 6) | (int(aux) << 7) |
@@ -445,6 +453,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int tile0 = PAIR ? int(blockIdx.x >> 1) : int(blockIdx.x);
     const int tile_step = PAIR ? int(gridDim.x >> 1) : int(gridDim.x);
     constexpr int BMT = PAIR ? 2 * BM : BM;                  // rows of one scheduled tile
+    constexpr bool SUM3 = C::SUM3;
     // Programmatic dependent launch: everything above (barrier init, TMEM allocation, descriptor prefetch) may run
     // while the previous kernel of the stream is still finishing; its results are only touched after this point.
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -467,9 +476,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const int m0 = tm * BMT + int(cta_rank) * BM;
                 const int n0 = tn * BN + int(cta_rank) * C::BN_LOCAL;
                 const int kb0 = split * p.kb_per_split;
-                const int kb1 = min(kb0 + p.kb_per_split, p.num_kb);
-                const int za = p.a_batched ? bidx : 0, zb = p.b_batched ? bidx : 0;
-                for (int kb = kb0; kb < kb1; ++kb) {
+                const int kb1 = SUM3 ? CHAIN * p.num_kb : min(kb0 + p.kb_per_split, p.num_kb);
+                int za = p.a_batched ? bidx : 0, zb = p.b_batched ? bidx : 0;
+                for (int kk = kb0; kk < kb1; ++kk) {
+                    int kb = kk;
+                    if constexpr (SUM3) {                     // the k-blocks of the three products follow one another
+                        za = zb = kk >= 2 * p.num_kb ? 2 : kk >= p.num_kb ? 1 : 0;
+                        kb = kk - za * p.num_kb;
+                    }
                     if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
                     uint8_t* sA = smem + stage * C::STAGE_BYTES;
                     uint8_t* sB = sA + A_TILE_BYTES;
@@ -533,14 +547,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int tile = tile0; tile < total_tiles && ok; tile += tile_step, ++it) {
                 const int split = p.div_batch.div(p.div_mn.div(tile));
                 const int kb0 = split * p.kb_per_split;
-                const int kb1 = min(kb0 + p.kb_per_split, p.num_kb);
+                const int kb1 = SUM3 ? CHAIN * p.num_kb : min(kb0 + p.kb_per_split, p.num_kb);
                 const int buf = it & 1;
                 const uint32_t acc_phase = (it >> 1) & 1;
                 if (!mbar_wait(&tempty_bar[buf], acc_phase ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t tmem_d = tmem_base + buf * BN;
+                uint32_t tmem_d = tmem_base + buf * C::ACC_COLS;
                 uint32_t accf = 0;
                 for (int kb = kb0; kb < kb1; ++kb) {
+                    if constexpr (SUM3) {
+                        if (kb == p.num_kb || kb == 2 * p.num_kb) { tmem_d += BN; accf = 0; }
+                    }
                     if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t at = (uint32_t)(stage * C::STAGE_BYTES) >> 4;
@@ -680,7 +697,43 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const long long offc = zoff * p.strideC + (long long)row * p.ldc;
             const long long offr = (long long)bidx * p.strideC + (long long)row * p.ldres;
             const long long offa = (long long)bidx * p.strideC + (long long)row * p.ldaux;
-            const uint32_t tmem_row = tmem_base + (uint32_t(quarter * 32) << 16) + buf * BN;
+            const uint32_t tmem_row = tmem_base + (uint32_t(quarter * 32) << 16) + buf * C::ACC_COLS;
+            if constexpr (SUM3) {
+                uint8_t* sb = ring + (store_cnt & 1) * 4096;
+                if (lane == 0) tma_store_wait_read<1>();
+                __syncwarp();
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t r[CHAIN][32];
+#pragma unroll
+                    for (int c = 0; c < CHAIN; ++c) tmem_ld32(tmem_row + c * BN + h * 32, r[c]);
+                    tmem_wait_ld();
+                    if (h == 1) acc_release(buf);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int j = q * 8 + 2 * i;
+                            w[i] = f2_to_bf2(__uint_as_float(r[0][j]), __uint_as_float(r[0][j + 1]));
+#pragma unroll
+                            for (int c = 1; c < CHAIN; ++c) {
+                                const float2 o = bf2_to_f2(w[i]);
+                                w[i] = f2_to_bf2(__uint_as_float(r[c][j]) + o.x, __uint_as_float(r[c][j + 1]) + o.y);
+                            }
+                        }
+                        *reinterpret_cast<uint4*>(sb + lane * 128 + (((h * 4 + q) ^ (lane & 7)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_3d(&tmC, sb, n0, m0 + quarter * 32, 0);
+                    tma_store_commit();
+                }
+                ++store_cnt;
+                continue;
+            }
             if constexpr (SIMPLE) {
                 // Plain bf16 output (no fused arithmetic): the TMEM loads of chunk c+1 are in flight while chunk c is
                 // converted and staged, and the accumulator is handed back to the MMA warp as soon as the last load
@@ -966,6 +1019,7 @@ constexpr int SPEC_BIAS_GELU_AUXD = spec_pack(true, CME_ACT_GELU, 0, false, fals
 constexpr int SPEC_DMUL_COLSUM = spec_pack(false, 0, CME_ACT_GELU, false, false, false, 1, false, true, true);
 constexpr int SPEC_DMUL = spec_pack(false, 0, CME_ACT_GELU, false, false, false, 1, false, true, false);
 constexpr int SPEC_DRELU_COLSUM = spec_pack(false, 0, CME_ACT_RELU, false, false, false, 1, false, false, true);
+constexpr int SPEC_SUM3 = 1 << 15;
 constexpr int SPEC_ACC = spec_pack(false, 0, 0, false, true, false, 3, false);
 
 }  // namespace gemm_tc
