@@ -97,7 +97,20 @@ def lib() -> ctypes.CDLL:
     return l
 
 
-_wrappers_bound = None
+_wrappers_module = _wrappers_bound = None
+
+
+def _compiled():
+    """The module of compiled wrappers, for what calls no entry point of the library."""
+    global _wrappers_module
+    if _wrappers_module is None:
+        try:
+            from . import _wrappers
+        except ImportError as e:
+            raise NativeError(f"compiled wrappers not usable ({e}); run `python -m cme213_final_project_b200.ops.build`") from e
+        _wrappers.init(NativeError)
+        _wrappers_module = _wrappers
+    return _wrappers_module
 
 
 def _native():
@@ -105,10 +118,7 @@ def _native():
     global _wrappers_bound
     if _wrappers_bound is None:
         l = lib()
-        try:
-            from . import _wrappers
-        except ImportError as e:
-            raise NativeError(f"compiled wrappers not usable ({e}); run `python -m cme213_final_project_b200.ops.build`") from e
+        _wrappers = _compiled()
         _wrappers.bind(NativeError, {n: ctypes.cast(getattr(l, n), ctypes.c_void_p).value for n in _WRAPPED})
         _wrappers_bound = _wrappers
     return _wrappers_bound
@@ -208,40 +218,19 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bo
     take them all.
     """
     _cuda(a, b, out, bias, aux_out, aux_in, residual)
-    batch = 1
-    if a.dim() == 3:
-        batch = a.shape[0]
-    if b.dim() == 3:
-        batch = max(batch, b.shape[0])
-    a2, b2 = a.shape[-2:], b.shape[-2:]
-    M, K = (a2[1], a2[0]) if a_trans else (a2[0], a2[1])
-    Kb, N = (b2[1], b2[0]) if b_trans else (b2[0], b2[1])
-    if K != Kb:
-        raise NativeError(f"gemm: inner dimensions differ ({K} vs {Kb})")
-    odt = out_dtype or (out.dtype if out is not None else a.dtype)
-    if out is None:
-        shape = (batch, M, N) if (a.dim() == 3 or b.dim() == 3) else (M, N)
-        out = torch.empty(shape, dtype=odt, device=a.device)
-    ws = _scratch(a.device)
-    a3, b3 = a.dim() == 3, b.dim() == 3
-    slabs = part = None
-    if dbias is not None:
-        slabs = ctypes.c_int(0)
-        part = torch.empty((M + 31) // 32 * N, dtype=torch.float32, device=a.device)
-    g = CmeGemm(M, N, K, batch,
-                a.data_ptr(), a2[1], a2[0] * a2[1] if a3 else 0, int(a_trans),
-                b.data_ptr(), b2[1], b2[0] * b2[1] if b3 else 0, int(b_trans),
-                out.data_ptr(), N, M * N, _dt(out), _dt(a),
-                _a(bias), _a(residual), N, _a(aux_out), _a(aux_in), N,
-                ACT[act], ACT[dact], int(accumulate), _a(ws), 0 if ws is None else ws.numel() * 4, force_bn, force_splits,
-                int(aux_deriv), _a(part), None if slabs is None else ctypes.pointer(slabs), int(allow_tf32))
+    ws = _scratch(a.device)                           # goes back when the call has been issued
+    out, part, desc = _compiled().gemm_prepare(a, b, a_trans, b_trans, out, out_dtype, bias, ACT[act], aux_out, ACT[dact], aux_in,
+                                               residual, accumulate, force_bn, force_splits, aux_deriv, dbias is not None,
+                                               allow_tf32, ws)
+    g = CmeGemm.from_buffer(desc)
     _check(lib().cme_gemm(ctypes.byref(g), _GEMM_BACKENDS[backend], _st()))
     if dbias is not None:
-        gemm.last_colsum_slabs = slabs.value          # 0: the epilogue did not sum (tests look at this)
-        if slabs.value:
-            _check(lib().cme_colsum_slabs_finalize(_dt(dbias), _a(part), slabs.value, N, _a(dbias), 0, _st()))
+        slabs = ctypes.c_int.from_buffer(desc, ctypes.sizeof(CmeGemm)).value
+        gemm.last_colsum_slabs = slabs                # 0: the epilogue did not sum (tests look at this)
+        if slabs:
+            _check(lib().cme_colsum_slabs_finalize(_dt(dbias), _a(part), slabs, g.N, _a(dbias), 0, _st()))
         else:
-            dact_colsum(out.reshape(-1, N), want_g=False, dbias=dbias)
+            dact_colsum(out.reshape(-1, g.N), want_g=False, dbias=dbias)
     return out
 
 

@@ -53,7 +53,7 @@ def _build_wrappers(verbose: bool, force: bool) -> None:
     root = Path(torch.__file__).resolve().parent
     src, key = CSRC / "wrappers.cpp", BUILD / "wrappers.key"
     h = hashlib.sha256(f"{sys.version} {torch.__version__}".encode())
-    for p in (src, CSRC / "attention_desc.h"):
+    for p in (src, CSRC / "attention_desc.h", CSRC / "gemm_desc.h"):
         h.update(p.read_bytes())
     if not force and WRAPPERS.exists() and key.exists() and key.read_text() == h.hexdigest():
         return

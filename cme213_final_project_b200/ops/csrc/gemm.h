@@ -5,6 +5,7 @@
 // runs as separate kernels (bias+ReLU, bias+residual, ReLU-backward; activations.cu:84-199).
 #pragma once
 #include "common.h"
+#include "gemm_desc.h"
 
 enum CmeAct : int { CME_ACT_NONE = 0, CME_ACT_RELU = 1, CME_ACT_GELU = 2 };
 
@@ -22,26 +23,7 @@ enum CmeAct : int { CME_ACT_NONE = 0, CME_ACT_RELU = 1, CME_ACT_GELU = 2 };
 //   the kernel writes one fp32 row of partial sums per 32 rows of C, [ceil(M / 32)][N], and *colsum_slabs receives
 //   the number of such rows -- or 0 when the kernel that ran cannot produce them (the caller then sums C itself).
 //   cme_colsum_slabs_finalize adds the rows up in a fixed order.
-struct CmeGemm {
-    int M, N, K, batch;
-    const void* A; long long lda, strideA; int a_trans;
-    const void* B; long long ldb, strideB; int b_trans;
-    void* C; long long ldc, strideC; int c_dtype;        // CME_BF16 or CME_F32
-    int ab_dtype;                                         // CME_BF16, or CME_F32: exact on the SIMT kernel, tf32 tensor-core
-                                                          // math on the tcgen05 kernel when allow_tf32 is set
-    const void* bias;                                     // [N], same dtype as A/B, or null
-    const void* residual; long long ldres;                // [M, N] same dtype as C, or null (batch stride = strideC)
-    void* aux_out; const void* aux_in; long long ldaux;   // [M, N] same dtype as C
-    int act, dact, accumulate;
-    void* workspace; long long workspace_bytes;           // fp32 scratch for split-K partial sums (may be null)
-    int force_bn, force_splits;                           // 0 = choose automatically
-    int aux_deriv;                                        // aux tensors hold act'(pre-activation), see above
-    float* colsum; int* colsum_slabs;                     // optional column sums of C (device scratch, host count)
-    int allow_tf32;                                       // fp32 operands may be multiplied as tf32 (10-bit mantissa
-                                                          // inputs, fp32 accumulation), plain products with fp32 output:
-                                                          // 1: operands along K, or along M / N with K % 4 == 0 and within
-                                                          // half of the workspace; 2: all that the kernel reads; 0: none
-};
+// (struct CmeGemm: gemm_desc.h)
 
 int gemm_tcgen05_supported(const CmeGemm* g);
 int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream);

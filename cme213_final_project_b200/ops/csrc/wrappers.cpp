@@ -18,6 +18,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "attention_desc.h"
+#include "gemm_desc.h"
 
 #include <cmath>
 #include <cstring>
@@ -365,6 +366,92 @@ PyObject* embedding_bwd(PyObject*, PyObject* const* a, Py_ssize_t) {
     END_HANDLE_TH_ERRORS
 }
 
+// The steps of ops.gemm before its native call: shapes, the result, column sums and the descriptor, 5 of the 18 us that the call
+// took as Python statements.  Returns (out, column sums | None, descriptor in a bytearray, behind which lies the count that
+// colsum_slabs points to).
+// (a, b, a_trans, b_trans, out | None, out_dtype | None, bias | None, activation, aux_out | None, dact, aux_in | None, residual | None,
+//  accumulate, force_bn, force_splits, aux_deriv, column sums wanted, allow_tf32, scratch | None)
+PyObject* gemm_prepare(PyObject*, PyObject* const* o, Py_ssize_t) {
+    HANDLE_TH_ERRORS
+    auto any = [](PyObject* t) {
+        if (t == Py_None) return at::Tensor();
+        if (!THPVariable_Check(t)) fail(PyExc_TypeError, "native ops take tensors");
+        return THPVariable_Unpack(t);
+    };
+    auto number = [](PyObject* v) {                 // int(v)
+        PyObject* i = PyNumber_Long(v);
+        if (!i) throw python_error();
+        const long long n = PyLong_AsLongLong(i);
+        Py_DECREF(i);
+        if (n == -1 && PyErr_Occurred()) throw python_error();
+        return int32(n);
+    };
+    const at::Tensor a = any(o[0]), b = any(o[1]), bias = any(o[6]), aux_out = any(o[8]), aux_in = any(o[10]), res = any(o[11]),
+                     ws = any(o[18]);
+    if (!a.defined() || !b.defined()) fail(PyExc_TypeError, "native ops take tensors");
+    at::Tensor out = any(o[4]);
+    if (a.dim() < 2 || b.dim() < 2) fail(PyExc_IndexError, "gemm: operands have to be matrices");
+    const bool a3 = a.dim() == 3, b3 = b.dim() == 3;
+    long long batch = a3 ? a.size(0) : 1;
+    if (b3 && b.size(0) > batch) batch = b.size(0);
+    const long long a0 = a.size(-2), a1 = a.size(-1), b0 = b.size(-2), b1 = b.size(-1);
+    CmeGemm g;
+    std::memset(&g, 0, sizeof g);
+    g.a_trans = number(o[2]);
+    g.b_trans = number(o[3]);
+    const long long M = g.a_trans ? a1 : a0, K = g.a_trans ? a0 : a1, Kb = g.b_trans ? b1 : b0, N = g.b_trans ? b0 : b1;
+    if (K != Kb) fail(native_error, "gemm: inner dimensions differ (" + std::to_string(K) + " vs " + std::to_string(Kb) + ")");
+    if (!out.defined()) {
+        auto opt = a.options();
+        if (o[5] != Py_None) {
+            if (!THPDtype_Check(o[5])) fail(PyExc_TypeError, "gemm: out_dtype has to be a torch.dtype");
+            opt = opt.dtype(reinterpret_cast<THPDtype*>(o[5])->scalar_type);
+        }
+        out = a3 || b3 ? at::empty({batch, M, N}, opt) : at::empty({M, N}, opt);
+    }
+    g.ab_dtype = dtype(a);
+    g.c_dtype = dtype(out);
+    at::Tensor part;
+    if (truth(o[16])) part = at::empty({(M + 31) / 32 * N}, a.options().dtype(at::kFloat));
+    g.M = int32(M); g.N = int32(N); g.K = int32(K); g.batch = int32(batch);
+    g.A = ptr(a); g.lda = a1; g.strideA = a3 ? a0 * a1 : 0;
+    g.B = ptr(b); g.ldb = b1; g.strideB = b3 ? b0 * b1 : 0;
+    g.C = ptr(out); g.ldc = N; g.strideC = M * N;
+    g.bias = ptr(bias);
+    g.residual = ptr(res); g.ldres = N;
+    g.aux_out = ptr(aux_out); g.aux_in = ptr(aux_in); g.ldaux = N;
+    g.act = number(o[7]); g.dact = number(o[9]); g.accumulate = number(o[12]);
+    g.workspace = ptr(ws);
+    g.workspace_bytes = ws.defined() ? ws.numel() * 4 : 0;
+    g.force_bn = number(o[13]); g.force_splits = number(o[14]);
+    g.aux_deriv = number(o[15]);
+    g.allow_tf32 = number(o[17]);
+    PyObject* desc = PyByteArray_FromStringAndSize(nullptr, sizeof g + sizeof(int));
+    if (!desc) throw python_error();
+    char* at_desc = PyByteArray_AS_STRING(desc);
+    int* slabs = reinterpret_cast<int*>(at_desc + sizeof g);
+    *slabs = 0;
+    if (part.defined()) { g.colsum = (float*)ptr(part); g.colsum_slabs = slabs; }
+    std::memcpy(at_desc, &g, sizeof g);
+    PyObject* all = PyTuple_New(3);
+    if (!all) { Py_DECREF(desc); throw python_error(); }
+    PyTuple_SET_ITEM(all, 2, desc);
+    Py_ssize_t i = 0;
+    for (const at::Tensor* t : {static_cast<const at::Tensor*>(&out), static_cast<const at::Tensor*>(&part)}) {
+        PyObject* v = t->defined() ? THPVariable_Wrap(*t) : Py_NewRef(Py_None);
+        if (!v) { Py_DECREF(all); throw python_error(); }
+        PyTuple_SET_ITEM(all, i++, v);
+    }
+    return all;
+    END_HANDLE_TH_ERRORS
+}
+
+// (NativeError): for the functions that call no entry point
+PyObject* init(PyObject*, PyObject* const* a, Py_ssize_t) {
+    Py_XSETREF(native_error, Py_NewRef(a[0]));
+    Py_RETURN_NONE;
+}
+
 // (NativeError, {name: address}): what the functions above raise and call
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
@@ -394,7 +481,7 @@ PyObject* counted(PyObject* self, PyObject* const* a, Py_ssize_t n) {
     if (n != N) return PyErr_Format(PyExc_TypeError, "expected %d arguments, got %zd", N, n);
     return F(self, a, n);
 }
-PyMethodDef methods[] = {METHOD(bind, 2), METHOD(cross_entropy, 5), METHOD(attention_fwd, 9), METHOD(attention_bwd, 15),
+PyMethodDef methods[] = {METHOD(bind, 2), METHOD(init, 1), METHOD(gemm_prepare, 19), METHOD(cross_entropy, 5), METHOD(attention_fwd, 9), METHOD(attention_bwd, 15),
                          METHOD(layernorm_fwd, 6), METHOD(layernorm_bwd, 9), METHOD(bias_act_residual, 5), METHOD(dact_colsum, 6),
                          METHOD(embedding_fwd, 3), METHOD(embedding_bwd, 7), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_wrappers", nullptr, -1, methods};

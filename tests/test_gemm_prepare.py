@@ -1,0 +1,60 @@
+"""What ops.gemm hands to the native call for the operands that it accepts, and which it refuses."""
+import pytest
+import torch
+
+from cme213_final_project_b200 import ops
+
+
+@pytest.fixture
+def seen(monkeypatch):
+    calls = []
+
+    class Lib:
+        @staticmethod
+        def cme_gemm(desc, backend, stream):
+            calls.append(desc._obj)
+            return 0
+
+    monkeypatch.setattr(ops, "lib", lambda: Lib)
+    monkeypatch.setattr(ops, "_cuda", lambda *t: None)
+    monkeypatch.setattr(ops, "_st", lambda: 0)
+    return calls
+
+
+@pytest.mark.parametrize("sa,sb,at,bt,shape,strides", [
+    ((5, 7), (7, 3), 0, 0, (5, 3), (0, 0)), ((7, 5), (3, 7), 1, 1, (5, 3), (0, 0)), ((4, 5, 7), (7, 3), 0, 0, (4, 5, 3), (35, 0)),
+    ((5, 7), (4, 3, 7), 0, 1, (4, 5, 3), (0, 21)), ((4, 7, 5), (4, 7, 3), 1, 0, (4, 5, 3), (35, 21)), ((1, 5, 7), (2, 7, 3), 0, 0, (2, 5, 3), (35, 21))])
+def test_shapes_and_strides(seen, sa, sb, at, bt, shape, strides):
+    a, b = torch.zeros(sa), torch.zeros(sb, dtype=torch.float32)
+    out = ops.gemm(a, b, a_trans=at, b_trans=bt, out_dtype=torch.bfloat16)
+    g = seen[0]
+    assert tuple(out.shape) == shape and out.dtype == torch.bfloat16
+    assert (g.M, g.N, g.K, g.batch) == (5, 3, 7, shape[0] if len(shape) == 3 else 1)
+    assert (g.lda, g.ldb, g.ldc, g.strideA, g.strideB, g.strideC) == (sa[-1], sb[-1], 3, *strides, 15)
+    assert (g.A, g.B, g.C) == (a.data_ptr(), b.data_ptr(), out.data_ptr()) and (g.ab_dtype, g.c_dtype) == (ops.F32, ops.BF16)
+
+
+def test_optional_operands_and_choices(seen):
+    a, b, r, x = (torch.zeros(8, 8) for _ in range(4))
+    v, out = torch.zeros(8), torch.ones(8, 8)
+    assert ops.gemm(a, b, out=out, bias=v, act="gelu", aux_out=x, residual=r, accumulate=True, aux_deriv=True, backend="tcgen05",
+                    force_bn=128, force_splits=3, allow_tf32=2) is out
+    ops.gemm(a, b, dact="relu", aux_in=x, allow_tf32=False)
+    g, h = seen
+    assert (g.bias, g.residual, g.aux_out, g.aux_in, g.act, g.dact) == (v.data_ptr(), r.data_ptr(), x.data_ptr(), None, 2, 0)
+    assert (g.accumulate, g.aux_deriv, g.force_bn, g.force_splits, g.allow_tf32, g.ldres, g.ldaux) == (1, 1, 128, 3, 2, 8, 8)
+    assert (h.bias, h.residual, h.aux_out, h.aux_in, h.act, h.dact, h.accumulate, h.allow_tf32) == (None, None, None, x.data_ptr(), 0, 1, 0, 0)
+    assert g.workspace and g.workspace_bytes == 64 << 20 and not g.colsum and not g.colsum_slabs
+
+
+def test_refusals(seen):
+    a = torch.zeros(8, 8)
+    with pytest.raises(ops.NativeError, match=r"gemm: inner dimensions differ \(8 vs 4\)"):
+        ops.gemm(a, torch.zeros(4, 8))
+    with pytest.raises(IndexError):
+        ops.gemm(a, torch.zeros(8))
+    with pytest.raises(KeyError):
+        ops.gemm(a, a, act="?")
+    with pytest.raises(ops.NativeError, match="unsupported dtype torch.float16"):
+        ops.gemm(a.half(), a.half())
+    assert not seen
