@@ -347,15 +347,14 @@ struct AdamArgs {
 
 // The gradient's scale.  Partial sums of the squared norm are added by every block (1024 of them: a few loads from L2 and two
 // barriers, against a kernel of its own in front of this one).
-__device__ __forceinline__ float adam_grad_scale(const AdamArgs& a, float* scratch) {
+// `sq`: the first of them, or the squared norm itself.
+__device__ __forceinline__ float adam_grad_scale(const AdamArgs& a, float sq, float* scratch) {
     if (!a.normsq || a.clip_norm <= 0.f) return a.grad_scale;
-    float sq = 0.f;
     if (a.n_norm > 1) {
+        sq = 0.f;
         for (int i = threadIdx.x; i < a.n_norm; i += blockDim.x) sq += a.normsq[i];
         sq = block_sum(sq, scratch);
         if (a.norm_out && blockIdx.x == 0 && threadIdx.x == 0) *a.norm_out = sq;
-    } else {
-        sq = *a.normsq;
     }
     const float norm = sqrtf(sq) * a.grad_scale;
     return norm > a.clip_norm ? a.grad_scale * (a.clip_norm / norm) : a.grad_scale;
@@ -389,7 +388,7 @@ __global__ void __launch_bounds__(256) adam_kernel(const AdamArgs a) {
     const float lr = *a.lr;
     const float bc1 = 1.f - powf(a.beta1, (float)t), bc2 = 1.f - powf(a.beta2, (float)t);
     __shared__ float scratch[32];
-    const float gs = adam_grad_scale(a, scratch);
+    const float gs = adam_grad_scale(a, a.normsq ? *a.normsq : 0.f, scratch);
     const TG* grads = reinterpret_cast<const TG*>(a.grads);
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (long long)gridDim.x * blockDim.x) {
         const float g = to_f32<TG>(grads[i]) * gs;
@@ -408,39 +407,26 @@ __global__ void __launch_bounds__(256) adam_kernel(const AdamArgs a) {
 
 constexpr int ADAM_LIST = 512;             // ranges that a block keeps in shared memory (8 KB); longer lists are read in place
 
-// Four elements per thread-iteration (128-bit accesses on the fp32 state).  Requires 16-byte aligned arenas; the last n % 4
+// Four elements per thread and round (128-bit accesses on the fp32 state).  Requires 16-byte aligned arenas; the last n % 4
 // elements and groups in which a no-decay range begins or ends are decided element by element.  RANGES: there is weight
-// decay and a list of ranges.  124 M elements with bf16 gradients, 3.49 GB: 561 us without ranges, 556 us with 150, 0.96 of a
-// 6.54 TB/s copy (574 and 575 us with accesses marked as streaming, which pay at 10 M only, 46 for 49 us).
+// decay and a list of ranges.
+// Bound by memory: 124 M elements with bf16 gradients, 3.49 GB: 519 us (6.7 TB/s; 523 with 150 ranges), 535 with the norm's partial sums
+// to add up.  A block takes `rounds` x 256 consecutive groups, so that the blocks that run together, in their order, work on one window of
+// each array; as 2368 blocks that stride through all of it the same loop took 558 us.  Five blocks an SM: four 536 us, six 538 (spills
+// aside, more rows of DRAM open at once).
 template <typename TG, bool RANGES>
-__global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
+__global__ void __launch_bounds__(256, 5) adam_vec4_kernel(const AdamArgs a, const int rounds) {
     pdl_wait();
-    const int t = *a.step;
-    const float lr = *a.lr;
-    const float bc1 = 1.f - powf(a.beta1, (float)t), bc2 = 1.f - powf(a.beta2, (float)t);
-    const float ibc1 = 1.f / bc1, ibc2 = 1.f / bc2;
-    __shared__ float scratch[32];
-    const float gs = adam_grad_scale(a, scratch);
     const long long nv = a.n >> 2;
-    // The no-decay range at or after the element at hand stays in registers; where it is over, the next one is searched for
-    // in a copy of the list in shared memory.  From global memory that is a chain of dependent loads: all of the list where
-    // it was walked (150 ranges: 1 M elements 28 us, 16 M 113 us), seven loads a group where it was bisected (8.4 and 82 us).
-    __shared__ long long list[RANGES ? 2 * ADAM_LIST : 1];
-    const bool copied = a.n_nodecay <= ADAM_LIST;
-    if (RANGES && copied) {
-        for (int k = threadIdx.x; k < 2 * a.n_nodecay; k += blockDim.x) list[k] = a.nodecay[k];
-        __syncthreads();
-    }
-    const long long* ranges = copied ? list : a.nodecay;
-    const float keep = a.weight_decay > 0.f ? 1.f - lr * a.weight_decay : 1.f;
-    int seg = 0;
-    long long seg_start = 0, seg_end = 0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
+    const long long first = (long long)blockIdx.x * rounds * 256 + threadIdx.x;
+    const long long end = first + (long long)rounds * 256 < nv ? first + (long long)rounds * 256 : nv;
+    float4 m4, v4, p4;
+    float g[4];
+    auto load = [&](long long i) {
         const long long e = i << 2;
-        float g[4];
-        float4 m4 = *reinterpret_cast<const float4*>(a.m + e);
-        float4 v4 = *reinterpret_cast<const float4*>(a.v + e);
-        float4 p4 = *reinterpret_cast<const float4*>(a.master + e);
+        m4 = *reinterpret_cast<const float4*>(a.m + e);
+        v4 = *reinterpret_cast<const float4*>(a.v + e);
+        p4 = *reinterpret_cast<const float4*>(a.master + e);
         if constexpr (sizeof(TG) == 2) {
             const uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(a.grads) + e);
             float2 lo = bf2_to_f2(u.x), hi = bf2_to_f2(u.y);
@@ -449,6 +435,31 @@ __global__ void __launch_bounds__(256) adam_vec4_kernel(const AdamArgs a) {
             const float4 u = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.grads) + e);
             g[0] = u.x; g[1] = u.y; g[2] = u.z; g[3] = u.w;
         }
+    };
+    // every load of the set-up is in flight before the first result is used, and with them those of the first round
+    const int t = *a.step;
+    const float lr = *a.lr;
+    const float sq = a.normsq ? *a.normsq : 0.f;
+    if (first < end) load(first);
+    __shared__ float scratch[32], setup[2];
+    if (threadIdx.x < 2) setup[threadIdx.x] = 1.f / (1.f - powf(threadIdx.x ? a.beta2 : a.beta1, (float)t));
+    // The no-decay range at or after the element at hand stays in registers; where it is over, the next one is searched for
+    // in a copy of the list in shared memory.  From global memory that is a chain of dependent loads: all of the list where
+    // it was walked (150 ranges: 1 M elements 28 us, 16 M 113 us), seven loads a group where it was bisected (8.4 and 82 us).
+    __shared__ long long list[RANGES ? 2 * ADAM_LIST : 1];
+    const bool copied = a.n_nodecay <= ADAM_LIST;
+    if (RANGES && copied)
+        for (int k = threadIdx.x; k < 2 * a.n_nodecay; k += blockDim.x) list[k] = a.nodecay[k];
+    __syncthreads();
+    const float gs = adam_grad_scale(a, sq, scratch);
+    const long long* ranges = copied ? list : a.nodecay;
+    const float ibc1 = setup[0], ibc2 = setup[1];
+    const float keep = a.weight_decay > 0.f ? 1.f - lr * a.weight_decay : 1.f;
+    int seg = 0;
+    long long seg_start = 0, seg_end = 0;
+    for (long long i = first; i < end; i += 256) {
+        const long long e = i << 2;
+        if (i != first) load(i);
         float decay[4] = {keep, keep, keep, keep};
         if (RANGES) {
             auto advance = [&](long long to) {
@@ -619,13 +630,17 @@ CME_API int cme_adam_partials(int grad_dtype, float* master, void* compute_bf16,
     bool vec = n >= 4 && al(master, 16) && al(m, 16) && al(v, 16) && al(compute_bf16, 8) &&
                al(grads, grad_dtype == CME_BF16 ? 8 : 16);
     if (vec) {
-        blocks = (n / 4 + 255) / 256;
-        if (blocks > 148 * 16) blocks = 148 * 16;
+        // Rounds per block: its set-up (three scalars, two powers, the list of ranges) takes as long as a round, unless there are too few
+        // blocks to go round.  1 / 2 / 4 / 8 rounds: 124 M elements 580 / 521 / 519 / 523 us, 4 M 18.5 / 15.9 / 14.8 / 14.7, 1 M 6.8 / 5.9 /
+        // 7.0 / 9.3, 0.2 M 3.6 / 4.3 / 5.9 / 9.1.
+        const long long groups = (n / 4 + 255) / 256;
+        const int rounds = groups <= 148 * 3 ? 1 : groups <= 148 * 12 ? 2 : 4;
+        blocks = (groups + rounds - 1) / rounds;
         const bool ranges = weight_decay > 0.f && n_nodecay > 0;
         auto kernel = grad_dtype != CME_BF16 ? (ranges ? adam_vec4_kernel<float, true> : adam_vec4_kernel<float, false>)
                       : ranges               ? adam_vec4_kernel<__nv_bfloat16, true>
                                              : adam_vec4_kernel<__nv_bfloat16, false>;
-        CME_CUDA(cme_launch_dependent(kernel, dim3((int)blocks), dim3(256), 0, st, a));
+        CME_CUDA(cme_launch_dependent(kernel, dim3((int)blocks), dim3(256), 0, st, a, rounds));
     } else {
         CME_CUDA(cme_launch_dependent(grad_dtype == CME_BF16 ? adam_kernel<__nv_bfloat16> : adam_kernel<float>,
                                       dim3((int)blocks), dim3(256), 0, st, a));
