@@ -221,6 +221,7 @@ int gemm(const Engine& e, cudaStream_t st, int M, int N, int K, const void* A, l
     const bool on_side = e.side != nullptr && st == e.side, on_side2 = e.side2 != nullptr && st == e.side2;
     g.workspace = on_side ? e.gemm_ws_side : on_side2 ? e.gemm_ws_side2 : e.gemm_ws;
     g.workspace_bytes = on_side ? e.gemm_ws_side_bytes : on_side2 ? e.gemm_ws_side2_bytes : e.gemm_ws_bytes;
+    if (!e.d.fused_qkv) g.force_splits = gemm_kept_splits(&g);
     return cme_gemm(&g, e.d.gemm_backend, st);
 }
 
@@ -233,6 +234,9 @@ int gemm_sum3(const Engine& e, cudaStream_t st, int M, int N, int K, const void*
     g.C = C; g.ldc = N; g.c_dtype = e.d.dtype; g.ab_dtype = e.d.dtype;
     g.allow_tf32 = e.d.allow_tf32;
     g.workspace = e.gemm_ws; g.workspace_bytes = e.gemm_ws_bytes;
+    CmeGemm one = g;                  // each of the three has the splits that it has by itself; one launch makes them without
+    one.batch = 1;
+    g.force_splits = gemm_kept_splits(&one);
     return cme_gemm_sum3(&g, e.d.gemm_backend, st);
 }
 

@@ -27,6 +27,7 @@ enum CmeAct : int { CME_ACT_NONE = 0, CME_ACT_RELU = 1, CME_ACT_GELU = 2 };
 
 int gemm_tcgen05_supported(const CmeGemm* g);
 int gemm_tcgen05_launch(const CmeGemm* g, cudaStream_t stream);
+int gemm_kept_splits(const CmeGemm* g);
 extern "C" int cme_gemm(const CmeGemm* g, int backend, void* stream);
 extern "C" int cme_gemm_sum3(const CmeGemm* g, int backend, void* stream);     // see gemm_tcgen05.cu
 int gemm_simt_launch(const CmeGemm* g, cudaStream_t stream);

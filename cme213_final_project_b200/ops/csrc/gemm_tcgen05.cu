@@ -254,6 +254,55 @@ static void plan_tiles(int M, int N, int K, int batch, bool plain_epi, long long
     *bn_out = bn; *pair_out = pair; *splits_out = splits;
 }
 
+// K splits of a bf16 product whose sums keep their order from one version to the next.  The models with separate Q, K and V take
+// them: their gradients are clipped to norm 1 and Adam's first steps divide each by its own size, so one result that rounds the
+// other way can turn a step of a parameter round, and a run from the same seed ends 3 % elsewhere (width 512, 45 x 64 tokens, the
+// splits of plan_tiles).  So the number is that of the estimate these models have always had, with k-blocks at their former pace;
+// the tile's width, which changes no sum, comes from plan_tiles.  It is seldom the fastest: 512 x 512 x 2048 takes 8 splits where 4
+// are planned, and a step of width 512 over 45 x 64 tokens 212 us where the plan's splits take 201.
+static int kept_splits(int M, int N, int K, int batch, bool plain_epi, long long workspace_bytes, int num_sms, int max_pairs) {
+    const int num_kb = cme_cdiv(K, 64);
+    static const struct { int bn; bool pair; double per_step; } tiles[4] = {{256, true, 136.0}, {256, false, 168.0},
+                                                                            {128, false, 138.0}, {64, false, 140.0}};
+    double best = 1e30;
+    int best_s = 1;
+    for (const auto& t : tiles) {
+        if ((t.pair && (max_pairs <= 0 || M <= BM)) || (t.bn > 64 && N <= t.bn / 2)) continue;
+        const long long count = (long long)cme_cdiv(M, t.pair ? 2 * BM : BM) * cme_cdiv(N, t.bn) * batch;
+        const int slots = t.pair ? max_pairs : num_sms;
+        for (int s = 1; s <= 16; ++s) {
+            if (s > 1 && (!plain_epi || num_kb / s < 4 || (long long)s * batch * M * N * 4 > workspace_bytes)) break;
+            const double waves = (double)((count * s + slots - 1) / slots), kb = (double)cme_cdiv(num_kb, s);
+            double est = waves * ((kb + 2.0) * 4.0 * t.per_step + 6.0 * 4.0 * t.bn / 2.0) + (t.pair ? 2000.0 : 0.0);
+            if (s > 1) est += 6000.0 + (double)s * M * N * batch / num_sms / 16.0;
+            if (est < best) { best = est; best_s = s; }
+        }
+    }
+    return best_s;
+}
+
+static int pairs_of(CmeDeviceState* ds) {
+    if (ds->max_pairs < 0) {
+        const char* e = getenv("CME213_GEMM_PAIR");
+        ds->max_pairs = (e && e[0] == '0') ? 0 : query_max_pairs(ds->num_sms);
+    }
+    return ds->max_pairs;
+}
+
+// The same for a product's descriptor on the current device; 0: planned as any other.
+int gemm_kept_splits(const CmeGemm* g) {
+    CmeDeviceState* ds;
+    if (g->ab_dtype != CME_BF16 || cme_device_state(&ds)) return 0;
+    const bool plain_epi = !g->bias && !g->residual && !g->aux_out && !g->act && !g->dact;
+    return kept_splits(g->M, g->N, g->K, g->batch, plain_epi, g->workspace ? g->workspace_bytes : 0, ds->num_sms, pairs_of(ds));
+}
+
+// ... and without a device.
+CME_API int cme_gemm_kept_splits(int M, int N, int K, int batch, int plain_epilogue, long long workspace_bytes, int num_sms,
+                                 int max_pairs) {
+    return kept_splits(M, N, K, batch, plain_epilogue != 0, workspace_bytes, num_sms, max_pairs);
+}
+
 // The plan the launcher would choose for operands stored along K, without a device: `num_sms` SMs, `max_pairs` co-resident CTA
 // pairs (0 = no cluster launches).  out = {tile width, pair (0/1), splits}.
 CME_API int cme_gemm_plan(int M, int N, int K, int batch, int plain_epilogue, long long workspace_bytes, int num_sms,
@@ -317,7 +366,7 @@ int gemm_tcgen05_supported(const CmeGemm* g) {
 // three).
 CME_API int cme_gemm_sum3_planned(const CmeGemm* g) {
     if (g->batch != CHAIN || g->ab_dtype != CME_BF16 || g->c_dtype != CME_BF16 || !g->strideA || !g->strideB || g->bias || g->residual ||
-        g->aux_out || g->aux_in || g->act || g->dact || g->accumulate || g->force_bn || g->force_splits || g->ldc % 8 ||
+        g->aux_out || g->aux_in || g->act || g->dact || g->accumulate || g->force_bn || g->force_splits > 1 || g->ldc % 8 ||
         !gemm_tcgen05_supported(g))
         return 0;
     CmeDeviceState* ds;
@@ -326,7 +375,7 @@ CME_API int cme_gemm_sum3_planned(const CmeGemm* g) {
     bool pair = false;
     double one = 0.0, three = 0.0;
     const OperandLayout at = {g->a_trans != 0, g->b_trans == 0, g->lda * 2, g->ldb * 2};
-    plan_tiles(g->M, g->N, g->K, 1, false, 0, ds->num_sms, ds->max_pairs > 0 ? ds->max_pairs : 0, 0, 0, &bn, &pair, &splits, at, 64, &one);
+    plan_tiles(g->M, g->N, g->K, 1, false, 0, ds->num_sms, pairs_of(ds), 0, 0, &bn, &pair, &splits, at, 64, &one);
     bn = 64; splits = 0;
     plan_tiles(g->M, g->N, cme_cdiv(g->K, 64) * 64 * CHAIN, 1, false, 0, ds->num_sms, 0, 64, 0, &bn, &pair, &splits, at, 64, &three);
     return three < CHAIN * one;
@@ -342,11 +391,7 @@ static int gemm_tcgen05_run(const CmeGemm* g, cudaStream_t stream, bool sum3) {
         int rc0 = cme_device_state(&ds);
         if (rc0) return rc0;
     }
-    if (ds->max_pairs < 0) {
-        const char* e = getenv("CME213_GEMM_PAIR");
-        ds->max_pairs = (e && e[0] == '0') ? 0 : query_max_pairs(ds->num_sms);
-    }
-    const int g_num_sms = ds->num_sms, g_max_pairs = ds->max_pairs;
+    const int g_num_sms = ds->num_sms, g_max_pairs = pairs_of(ds);
     int* const g_status = ds->status + CME_STATUS_GEMM;
     const bool tf32 = g->ab_dtype == CME_F32;
     const int BK = tf32 ? 32 : 64;                            // K elements per 128-byte k-block
