@@ -18,9 +18,10 @@ namespace {
 // since a row's pitch is an odd number of 16-byte words.  Multiply-adds are packed pairs, fp32 tiles arrive by asynchronous
 // copies, all of a block's at once, the ones that the second product needs under the first.
 // The head size is padded with zeros to a multiple of 32 (template G = ceil(HD / 32)).
-// 32 x 4 heads x 64 tokens x head size 128, fp32, forward + backward: 13 + 27.6 us, 18 + 31 us with a warp for whole rows of the
-// forward, single multiply-adds and tiles loaded through registers one after the other (floor of both at the fp32 rate, 0.94 GFLOP
-// at 74 TFLOP/s: 13 us).  64 query rows a block instead of 32 in the forward: 12.8 us, no different.
+// 32 x 4 heads x 64 tokens x head size 128, fp32, forward + backward: 12.9 + 24.0 us; 18 + 31 with a warp for whole rows of the
+// forward, single multiply-adds and tiles loaded through registers one after the other, 12.9 + 27.8 with eight warps on each of the
+// backward's products (floor of both at the fp32 rate, 0.94 GFLOP at 74 TFLOP/s: 13 us).  64 query rows a block instead of 32 in the
+// forward: 12.8 us, no different.
 constexpr int CT = 64;               // rows streamed per step
 constexpr int WR = 16;               // rows a warp owns
 constexpr int LR = WR / 4;           // rows a lane has of them
@@ -58,7 +59,7 @@ __device__ __forceinline__ void load_rows(float* dst, const T* src, long long st
     static_assert(NR * 8 * G % NT == 0, "whole rounds");
 #pragma unroll 8
     for (int k = 0; k < NR * 8 * G / NT; ++k) {
-        const int i = threadIdx.x + k * NT, r = i / (8 * G), c = (i % (8 * G)) * 4;
+        const int i = threadIdx.x % NT + k * NT, r = i / (8 * G), c = (i % (8 * G)) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r0 + r < T_ && c < HD) {
             const T* p = src + (long long)(r0 + r) * st + c;
@@ -84,7 +85,7 @@ __device__ __forceinline__ void copy_rows(float* dst, const T* src, long long st
         const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
 #pragma unroll
         for (int k = 0; k < NR * 8 * G / NT; ++k) {
-            const int i = threadIdx.x + k * NT, r = i / (8 * G), c = (i % (8 * G)) * 4;
+            const int i = threadIdx.x % NT + k * NT, r = i / (8 * G), c = (i % (8 * G)) * 4;
             const bool in = r0 + r < T_ && c < HD;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + (uint32_t)(r * Pitch<G>::P + c) * 4u),
                          "l"(in ? src + (long long)(r0 + r) * st + c : src), "r"(in ? 16 : 0)
@@ -98,32 +99,32 @@ __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_
 // All but the last N committed groups of this thread have arrived.
 template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// s[i][j] = A[ty + 4 i] . B[tx + 8 j].  Packed pairs: the even and the odd elements are summed apart, two multiply-adds per
-// instruction, so that a scheduler with one or two warps has issue slots left for their loads.
-template <int G, int NJ>
-__device__ __forceinline__ void dot_rows(const float* A, const float* B, int ty, int tx, float (&s)[LR][NJ]) {
-    constexpr int P = Pitch<G>::P;
-    F32x2 t[LR][NJ];
+// s[i][j] = A[4 i] . B[8 j] over ND elements; A and B point at the lane's first rows.  Packed pairs: the even and the odd elements
+// are summed apart, two multiply-adds per instruction, so that a scheduler with one or two warps has issue slots left for their
+// loads.
+template <int P, int ND, int NJ, int NI>
+__device__ __forceinline__ void dot_tile(const float* A, const float* B, float (*s)[NJ]) {
+    F32x2 t[NI][NJ];
 #pragma unroll
-    for (int i = 0; i < LR; ++i)
+    for (int i = 0; i < NI; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) t[i][j] = f2_splat(0.f);
 #pragma unroll 2
-    for (int d = 0; d < 32 * G; d += 4) {
-        float4 a[LR];
+    for (int d = 0; d < ND; d += 4) {
+        float4 a[NI];
 #pragma unroll
-        for (int i = 0; i < LR; ++i) a[i] = *reinterpret_cast<const float4*>(A + (ty + 4 * i) * P + d);
+        for (int i = 0; i < NI; ++i) a[i] = *reinterpret_cast<const float4*>(A + 4 * i * P + d);
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-            const float4 b = *reinterpret_cast<const float4*>(B + (tx + 8 * j) * P + d);
+            const float4 b = *reinterpret_cast<const float4*>(B + 8 * j * P + d);
 #pragma unroll
-            for (int i = 0; i < LR; ++i)
+            for (int i = 0; i < NI; ++i)
                 t[i][j] = f2_fma(f2_pack(a[i].z, a[i].w), f2_pack(b.z, b.w),
                                  f2_fma(f2_pack(a[i].x, a[i].y), f2_pack(b.x, b.y), t[i][j]));
         }
     }
 #pragma unroll
-    for (int i = 0; i < LR; ++i) {
+    for (int i = 0; i < NI; ++i) {
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
             float even, odd;
@@ -144,16 +145,16 @@ template <> __device__ __forceinline__ void lds<2>(const float* p, float* f) {
     f[0] = v.x; f[1] = v.y;
 }
 
-// o[i][k] += w(i, j) * B[j][c0 + 8 VW k ...] over the CT streamed rows, c0 the lane's first column.  W: the weight tile, element
+// o[i][k] += w(i, j) * B[j][c0 + 8 VW k ...] over NJ streamed rows, c0 the lane's first column.  W: the weight tile, element
 // (row, j) at row * WROW + j * WCOL, its first row being the lane's.
-template <int G, int VW, int NK, int WROW, int WCOL>
-__device__ __forceinline__ void weighted_rows(const float* W, const float* B, float (&o)[LR][NK][VW]) {
+template <int G, int WROW, int WCOL, int NJ = CT, int NI, int NK, int VW>
+__device__ __forceinline__ void weighted_rows(const float* W, const float* B, float (&o)[NI][NK][VW]) {
     constexpr int P = Pitch<G>::P;
 #pragma unroll 2
-    for (int j = 0; j < CT; j += 4) {
-        float w[LR][4];
+    for (int j = 0; j < NJ; j += 4) {
+        float w[NI][4];
 #pragma unroll
-        for (int i = 0; i < LR; ++i) {
+        for (int i = 0; i < NI; ++i) {
             if (WCOL == 1) {
                 lds<4>(W + 4 * i * WROW + j, w[i]);
             } else {
@@ -168,7 +169,7 @@ __device__ __forceinline__ void weighted_rows(const float* W, const float* B, fl
                 float b[VW];
                 lds<VW>(B + (j + jj) * P + 8 * VW * k, b);
 #pragma unroll
-                for (int i = 0; i < LR; ++i)
+                for (int i = 0; i < NI; ++i)
 #pragma unroll
                     for (int c = 0; c < VW; c += 2)
                         f2_unpack(f2_fma(f2_splat(w[i][jj]), f2_pack(b[c], b[c + 1]), f2_pack(o[i][k][c], o[i][k][c + 1])),
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(NW * 64, fwd_blocks_per_sm<G, NW>()) attn_fwd_
         copies_wait<1>();
         __syncthreads();
         float s[LR][4];
-        dot_rows<G, 4>(sQ + w0 * P, sK + half * 32 * P, ty, tx, s);
+        dot_tile<P, 32 * G, 4, LR>(sQ + (w0 + ty) * P, sK + (half * 32 + tx) * P, s);
 #pragma unroll
         for (int i = 0; i < LR; ++i) {
             const int row = w0 + ty + 4 * i, q = q0 + row;
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(NW * 64, fwd_blocks_per_sm<G, NW>()) attn_fwd_
 #pragma unroll
                 for (int c = 0; c < VW; ++c) o[i][g][c] *= alpha[i];
         }
-        weighted_rows<G, VW, NK, SP, 1>(wP, sV + c0, o);
+        weighted_rows<G, SP, 1>(wP, sV + c0, o);
     }
 #pragma unroll
     for (int i = 0; i < LR; ++i) {
@@ -348,43 +349,51 @@ __global__ void __launch_bounds__(256) attn_delta_hd64_kernel(const CmeAttn a, f
     }
 }
 
-// delta[r] = sum_d dO[r][d] * O[r][d] for the rows whose dO tile has just been staged, one warp per row.  `sO`: the same rows of
-// O in shared memory, or null.
-template <typename T, int G>
-__device__ __forceinline__ void delta_rows(float* dst, const float* sdO, const float* sO, const T* o, long long ost, int r0, int T_,
-                                           int HD) {
-    constexpr int NW = BWD_THREADS / 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// delta[r] = sum_d dO[r][d] * O[r][d] for the CT rows whose tiles are staged, one warp per row, four warps.
+template <int G> __device__ __forceinline__ void delta_rows(float* dst, const float* sdO, const float* sO) {
+    constexpr int NW = BWD_THREADS / 64;
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % NW;
 #pragma unroll
     for (int k = 0; k < CT / NW; ++k) {
         const int r = warp + k * NW;
         float s = 0.f;
-        if (r0 + r < T_) {
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const int d = lane + 32 * g;
-                const int at = r * Pitch<G>::P + d;
-                if (d < HD) s = fmaf(sdO[at], sO ? sO[at] : to_f32<T>(o[(long long)(r0 + r) * ost + d]), s);
-            }
-        }
+        for (int g = 0; g < G; ++g) s = fmaf(sdO[r * Pitch<G>::P + lane + 32 * g], sO[r * Pitch<G>::P + lane + 32 * g], s);
         s = warp_sum(s);
         if (lane == 0) dst[r] = s;
     }
 }
 
 // blockIdx.z == 0: the block owns 64 keys and streams queries:    dV = sum_i P_ij dO_i,  dK = scale * sum_i dS_ij Q_i.
-//                  With one key block (T <= 64) it has all of dS as well and makes dQ too: five products instead of the
+//                  With one key block (T <= 64, ONE) it has all of dS as well and makes dQ too: five products instead of the
 //                  seven of the split form.
 // blockIdx.z == 1: the block owns 64 queries and streams keys:    dQ = scale * sum_j dS_ij K_j
 // Both kinds run in one launch, and delta = rowsum(dO * O) is made from the staged rows instead of by a kernel before.
-// Whether O is staged beside dO: fp32 heads wide enough for one block per SM anyway.
-template <typename T, int G> __host__ __device__ constexpr bool bwd_stages_o() { return sizeof(T) == 4 && G >= 3; }
-template <typename T, int G>
+//
+// The first four warps fetch Q and K, make P and then dV, the others fetch dO, V and O, make delta, dS and then dK: with four warps on
+// a 64 x 64 product a lane has 8 rows of it where eight warps leave 4, and so loads 12 words for 32 results a step instead of 8 for 16.
+// In dQ, a single product, they have half of the keys each.  A block that makes its scores once (ONE) and has the registers of a
+// whole SM goes to 8 x 8, the elements of the heads split between two warps.  Shared memory's share of five products of width 128
+// falls from 34800 clocks to 21200, next to 20500 of multiply-adds.  32 x 4 heads, fp32, us before and now: 64 tokens, head size 128
+// 27.8 and 24.0, 64 18.0 and 14.5, 32 13.5 and 10.8; 128 tokens 142 and 120, 69.3 and 67.7, 46.0 and 41.7.
+// O is staged as well, in the place of dS where its rows are no longer: loaded row by row into registers, under branches, it was a
+// chain of memory round trips (as were the log-sum-exps, read where a score was finished).
+template <int G> constexpr int bwd_tiles() { return 32 * G <= CT ? 4 : 5; }
+__device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory"); }
+template <typename T, int G, bool ONE>
 __global__ void __launch_bounds__(BWD_THREADS, G <= 2 ? 2 : 1) attn_bwd_kernel(const CmeAttn a, const bool vec) {
-    constexpr int P = Pitch<G>::P, NT = BWD_THREADS, RT = BWD_ROWS;
-    // a lane's columns: VW at half * 16 G + tx * VW, then every 8 VW
+    constexpr int P = Pitch<G>::P, NT = BWD_THREADS / 2, RT = BWD_ROWS, NI = 8;
+    constexpr int KS = ONE && G >= 3 ? 2 : 1;      // warps that share the elements of a score
+    constexpr int NP = ONE || G >= 3 ? NI : 4;     // rows of a score product at a time: two blocks per SM leave 128 registers
+    // delta after dP, whose product O's copies then run under; with one block per SM the other half would wait for it (24.9 us where
+    // 24.0 are below)
+    constexpr bool LATE = NP < NI;
+    // a lane's columns: VW at part * 16 G + tx * VW, then every 8 VW
     constexpr int VW = G % 2 == 0 ? 4 : 2, NK = 2 * G / VW;
-    static_assert(RT == CT && NT / 32 == 2 * RT / WR, "own and streamed tiles of one height, two warps per 16 rows");
+    static_assert(bwd_tiles<G>() == 5 || RT * P <= RT * SP, "O in the place of dS");
+    static_assert(RT == CT && NT / 32 * 32 * 32 == RT * CT, "own and streamed tiles of one height, four warps on 32 x 32 each");
+    static_assert(NT / 32 * 32 * NI * 4 <= RT * SP, "partial scores lie where the tile of P or dS will");
+    static_assert(BWD_THREADS * 4 * NK * VW <= CT * P, "half of dQ lies in the tile of the streamed rows");
     extern __shared__ __align__(16) float sm[];
     float* sA = sm;                    // own rows       K | Q
     float* sB = sA + RT * P;           //                V | dO
@@ -393,109 +402,154 @@ __global__ void __launch_bounds__(BWD_THREADS, G <= 2 ? 2 : 1) attn_bwd_kernel(c
     float* sP = sD + CT * P;           // [RT][SP] P (own row, streamed row)
     float* sS = sP + RT * SP;          // [RT][SP] dS
     float* sDl = sS + RT * SP;         // [CT] delta of the queries in shared memory
-    float* sO = bwd_stages_o<T, G>() ? sDl + CT : nullptr;        // O of the rows whose delta is made
+    float* sL = sDl + CT;              // [CT] log-sum-exp of the same queries
+    float* sO = bwd_tiles<G>() == 4 ? sS : sL + CT;        // O of the rows whose delta is made
     pdl_wait();
-    const bool kv = blockIdx.z == 0;
+    const bool kv = ONE || blockIdx.z == 0;
     const int bh = blockIdx.y, r0 = blockIdx.x * RT, HD = a.HD;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tx = lane & 7, ty = lane >> 3;
-    const int w0 = (warp & 3) * WR, half = warp >> 2, c0 = half * 16 * G + tx * VW;
+    const int half = warp >> 2, w0 = (warp & 1) * 32 + ty, part = (warp >> 1) & 1, c0 = part * 16 * G + tx * VW;
     const long long base = head_base(a, bh), obase = head_base_o(a, bh);
     const T* q = (const T*)a.q + base; const T* k = (const T*)a.k + base; const T* v = (const T*)a.v + base;
     const T* d_o = (const T*)a.d_o + obase; const T* o = (const T*)a.o + obase;
     const float* lse = a.lse + (long long)bh * a.T;
-    copy_rows<T, G, RT, NT>(sA, kv ? k : q, a.st, r0, a.T, HD, vec);
-    if (!kv) {
-        copy_rows<T, G, RT, NT>(sB, d_o, a.ost, r0, a.T, HD, vec);
-        if (sO) copy_rows<T, G, RT, NT>(sO, o, a.ost, r0, a.T, HD, vec);
-        copies_commit();
-    }
-    float acc1[LR][NK][VW], acc2[LR][NK][VW];
+    float acc[NI][NK][VW];
+    auto clear = [&] {
 #pragma unroll
-    for (int i = 0; i < LR; ++i)
+        for (int i = 0; i < NI; ++i)
 #pragma unroll
-        for (int g = 0; g < NK; ++g)
+            for (int g = 0; g < NK; ++g)
 #pragma unroll
-            for (int c = 0; c < VW; ++c) { acc1[i][g][c] = 0.f; acc2[i][g][c] = 0.f; }
-    if (!kv) {
-        copies_wait<0>();
-        __syncthreads();
-        delta_rows<T, G>(sDl, sB, sO, o, a.ost, r0, a.T, HD);
-    }
+                for (int c = 0; c < VW; ++c) acc[i][g][c] = 0.f;
+    };
+    if (!ONE) clear();
     // causal: queries see keys <= their index.  dQ blocks stop early; dK / dV blocks start late.
     const int s_begin = (kv && a.causal) ? r0 : 0;
     const int s_end = (!kv && a.causal) ? min(a.T, r0 + RT) : a.T;
     for (int s0 = s_begin; s0 < s_end; s0 += CT) {
-        __syncthreads();
-        copy_rows<T, G, CT, NT>(sC, kv ? q : k, a.st, s0, a.T, HD, vec);
-        copies_commit();
-        if (kv && s0 == s_begin) copy_rows<T, G, RT, NT>(sB, v, a.st, r0, a.T, HD, vec);
-        copy_rows<T, G, CT, NT>(sD, kv ? d_o : v, kv ? a.ost : a.st, s0, a.T, HD, vec);
-        if (kv && sO) copy_rows<T, G, CT, NT>(sO, o, a.ost, s0, a.T, HD, vec);
-        copies_commit();
-        copies_wait<1>();                          // the tiles of the first product; the others arrive meanwhile
-        __syncthreads();
-        float s[LR][4], dp[LR][4];
-        dot_rows<G, 4>(sA + w0 * P, sC + half * 32 * P, ty, tx, s);
-        copies_wait<0>();
-        __syncthreads();
-        if (kv) delta_rows<T, G>(sDl, sD, sO, o, a.ost, s0, a.T, HD);
-        dot_rows<G, 4>(sB + w0 * P, sD + half * 32 * P, ty, tx, dp);
-        if (kv) __syncthreads();                   // delta is written by all warps
-#pragma unroll
-        for (int i = 0; i < LR; ++i) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int own = w0 + ty + 4 * i, str = half * 32 + tx + 8 * j;
-                const int qi = kv ? s0 + str : r0 + own, ki = kv ? r0 + own : s0 + str;
-                const bool ok = qi < a.T && ki < a.T && (!a.causal || ki <= qi);
-                const float p = ok ? __expf(s[i][j] * a.scale - lse[qi]) : 0.f;
-                if (kv) sP[own * SP + str] = p;
-                sS[own * SP + str] = ok ? p * (dp[i][j] - sDl[kv ? str : own]) : 0.f;
-            }
-        }
-        __syncthreads();                           // the other half of these rows' scores is another warp's
-        const float* wP = sP + (w0 + ty) * SP;
-        const float* wS = sS + (w0 + ty) * SP;
-        if (kv) {
-            weighted_rows<G, VW, NK, SP, 1>(wP, sD + c0, acc1);        // dV += P^T dO
-            weighted_rows<G, VW, NK, SP, 1>(wS, sC + c0, acc2);        // dK += dS^T Q
+        const bool first = ONE || s0 == s_begin;
+        if (!first) __syncthreads();
+        if (half == 0) {
+            if (first) copy_rows<T, G, RT, NT>(sA, kv ? k : q, a.st, r0, a.T, HD, vec);
+            copy_rows<T, G, CT, NT>(sC, kv ? q : k, a.st, s0, a.T, HD, vec);
+            const int qi = (kv ? s0 : r0) + (int)threadIdx.x;
+            if ((kv || first) && threadIdx.x < CT) sL[threadIdx.x] = qi < a.T ? lse[qi] : 0.f;
         } else {
-            weighted_rows<G, VW, NK, SP, 1>(wS, sC + c0, acc1);        // dQ += dS K
+            if (first) copy_rows<T, G, RT, NT>(sB, kv ? v : d_o, kv ? a.st : a.ost, r0, a.T, HD, vec);
+            copy_rows<T, G, CT, NT>(sD, kv ? d_o : v, kv ? a.ost : a.st, s0, a.T, HD, vec);
+            if (LATE) copies_commit();
+            if (kv || first) copy_rows<T, G, CT, NT>(sO, o, a.ost, kv ? s0 : r0, a.T, HD, vec);
         }
-    }
+        copies_commit();
+        if (LATE && half) copies_wait<1>(); else copies_wait<0>();
+        half_sync(half);
+        if (!LATE && half && (kv || first)) delta_rows<G>(sDl, kv ? sD : sB, sO);
+        // S or dP: rows w0 + 4 i, columns part * 32 + tx + 8 j
+        const float* own = (half ? sB : sA) + w0 * P;
+        const float* str = (half ? sD : sC) + tx * P;
+        float s[NI][4];
+        if (KS == 1) {
 #pragma unroll
-    for (int i = 0; i < LR; ++i) {
-        const int r = r0 + w0 + ty + 4 * i;
-        if (r < a.T) {
-            const long long off = base + (long long)r * a.st;
+            for (int i = 0; i < NI; i += NP) dot_tile<P, 32 * G, 4, NP>(own + 4 * i * P, str + part * 32 * P, s + i);
+        } else {
+            float t[NI][8];                        // all 64 columns, half of the elements
+            dot_tile<P, 16 * G, 8, NI>(own + part * 16 * G, str + part * 16 * G, t);
+            float* mine = (half ? sS : sP) + (warp & 3) * (32 * NI * 4) + lane * 4;
+            const float* other = (half ? sS : sP) + ((warp & 3) ^ 2) * (32 * NI * 4) + lane * 4;
 #pragma unroll
-            for (int g = 0; g < NK; ++g) {
-                const int c = c0 + 8 * VW * g;
-                if (kv) {
-                    store_cols<T, VW>((T*)a.dv + off, c, HD, acc1[i][g], 1.f, vec);
-                    store_cols<T, VW>((T*)a.dk + off, c, HD, acc2[i][g], a.scale, vec);
-                } else {
-                    store_cols<T, VW>((T*)a.dq + off, c, HD, acc1[i][g], a.scale, vec);
-                }
+            for (int i = 0; i < NI; ++i)
+                *reinterpret_cast<float4*>(mine + i * 128) = part ? make_float4(t[i][0], t[i][1], t[i][2], t[i][3])
+                                                                  : make_float4(t[i][4], t[i][5], t[i][6], t[i][7]);
+            half_sync(half);
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                const float4 p = *reinterpret_cast<const float4*>(other + i * 128);
+                s[i][0] = (part ? t[i][4] : t[i][0]) + p.x;
+                s[i][1] = (part ? t[i][5] : t[i][1]) + p.y;
+                s[i][2] = (part ? t[i][6] : t[i][2]) + p.z;
+                s[i][3] = (part ? t[i][7] : t[i][3]) + p.w;
             }
+            half_sync(half);                       // they have been read: P and dS go to the same place
         }
+        if (LATE && half && (kv || first)) {
+            copies_wait<0>();
+            half_sync(half);
+            delta_rows<G>(sDl, kv ? sD : sB, sO);
+        }
+        auto seen = [&](int row, int col) {
+            const int qi = kv ? s0 + col : r0 + row, ki = kv ? r0 + row : s0 + col;
+            return qi < a.T && ki < a.T && (!a.causal || ki <= qi);
+        };
+        if (half == 0) {
+#pragma unroll
+            for (int i = 0; i < NI; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int row = w0 + 4 * i, col = part * 32 + tx + 8 * j;
+                    const float e = s[i][j] * a.scale - sL[kv ? col : row];
+                    sP[row * SP + col] = __expf(seen(row, col) ? e : -INFINITY);
+                }
+        }
+        __syncthreads();                           // P and, for dV, dO
+        if (half) {
+#pragma unroll
+            for (int i = 0; i < NI; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int row = w0 + 4 * i, col = part * 32 + tx + 8 * j;
+                    const float ds = sP[row * SP + col] * (s[i][j] - sDl[kv ? col : row]);
+                    sS[row * SP + col] = seen(row, col) ? ds : 0.f;
+                }
+        }
+        if (ONE) clear();
+        if (!kv) {
+            __syncthreads();
+            weighted_rows<G, SP, 1, CT / 2>(sS + w0 * SP + half * (CT / 2), sC + half * (CT / 2) * P + c0, acc);      // dQ += dS K
+        } else {
+            if (half) half_sync(half);
+            weighted_rows<G, SP, 1>((half ? sS : sP) + w0 * SP, (half ? sC : sD) + c0, acc);      // dV += P^T dO, dK += dS^T Q
+        }
+        if (ONE) break;
     }
-    if (gridDim.z == 1) {                          // T <= 64: dQ_i = scale * sum_j dS_ij K_j from the tile at hand
+    if (kv) {
 #pragma unroll
-        for (int i = 0; i < LR; ++i)
-#pragma unroll
-            for (int g = 0; g < NK; ++g)
-#pragma unroll
-                for (int c = 0; c < VW; ++c) acc1[i][g][c] = 0.f;
-        weighted_rows<G, VW, NK, 1, SP>(sS + w0 + ty, sA + c0, acc1);  // the tile read down its columns
-#pragma unroll
-        for (int i = 0; i < LR; ++i) {
-            const int r = w0 + ty + 4 * i;
+        for (int i = 0; i < NI; ++i) {
+            const int r = r0 + w0 + 4 * i;
             if (r < a.T)
 #pragma unroll
                 for (int g = 0; g < NK; ++g)
-                    store_cols<T, VW>((T*)a.dq + base + (long long)r * a.st, c0 + 8 * VW * g, HD, acc1[i][g], a.scale, vec);
+                    store_cols<T, VW>((T*)(half ? a.dk : a.dv) + base + (long long)r * a.st, c0 + 8 * VW * g, HD, acc[i][g],
+                                      half ? a.scale : 1.f, vec);
         }
+        if (!ONE) return;
+    }
+    __syncthreads();                               // dS is complete, the streamed rows have been read
+    if (ONE) {                                     // dQ_i = scale * sum_j dS_ij K_j: the tile read down its columns
+        clear();
+        weighted_rows<G, 1, SP, CT / 2>(sS + w0 + half * (CT / 2) * SP, sA + half * (CT / 2) * P + c0, acc);
+    }
+    // the halves' sums meet: each finishes four of a lane's rows
+    float* give = sC + threadIdx.x * VW;
+    const float* take = sC + (threadIdx.x ^ (BWD_THREADS / 2)) * VW;
+#pragma unroll
+    for (int i = 0; i < NI / 2; ++i)
+#pragma unroll
+        for (int g = 0; g < NK; ++g)
+#pragma unroll
+            for (int c = 0; c < VW; ++c) give[(i * NK + g) * BWD_THREADS * VW + c] = half ? acc[i][g][c] : acc[i + NI / 2][g][c];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NI / 2; ++i) {
+        const int r = r0 + w0 + 4 * (i + (half ? NI / 2 : 0));
+        if (r < a.T)
+#pragma unroll
+            for (int g = 0; g < NK; ++g) {
+                float sum[VW];
+#pragma unroll
+                for (int c = 0; c < VW; ++c)
+                    sum[c] = (half ? acc[i + NI / 2][g][c] : acc[i][g][c]) + take[(i * NK + g) * BWD_THREADS * VW + c];
+                store_cols<T, VW>((T*)a.dq + base + (long long)r * a.st, c0 + 8 * VW * g, HD, sum, a.scale, vec);
+            }
     }
 }
 
@@ -531,9 +585,9 @@ template <typename T, int G, int NW> int fwd_launch(const CmeAttn* a, cudaStream
 }
 template <typename T, int G> int bwd_launch(const CmeAttn* a, cudaStream_t st) {
     constexpr int P = Pitch<G>::P, RT = BWD_ROWS;
-    constexpr size_t smem = ((bwd_stages_o<T, G>() ? 5 : 4) * RT * P + 2 * RT * SP + CT) * sizeof(float);
+    constexpr size_t smem = (bwd_tiles<G>() * RT * P + 2 * RT * SP + 2 * CT) * sizeof(float);
     static_assert(smem <= 227 * 1024, "one block's shared memory");
-    auto k = attn_bwd_kernel<T, G>;
+    auto k = a->T <= RT ? attn_bwd_kernel<T, G, true> : attn_bwd_kernel<T, G, false>;
     int rc = allow_smem(k, smem);
     if (rc) return rc;
     CME_CUDA(cme_launch_dependent(k, dim3(cme_cdiv(a->T, RT), a->nb * a->nh, a->T <= RT ? 1 : 2), dim3(BWD_THREADS), smem,
