@@ -107,13 +107,14 @@ cross_entropy_bf16_vec_kernel(const __nv_bfloat16* __restrict__ logits, const in
     }
 }
 
-// Same contract, for rows of at most CEV_THREADS * CER_MAXV 16-byte vectors (53248 bf16: GPT-2's padded vocabulary
-// fits): the row lives in registers from its single read to its single write.  Pass 1 finds the maximum, pass 2
-// evaluates exp(x - max) once per element and keeps it as fp16 in the registers that held the logits (values in
-// (0, 1], 11 significant bits -- finer than the bf16 the gradient is stored in), pass 3 only scales.  One
+// Same contract, for rows of at most THREADS * NV 16-byte vectors: the row lives in registers from its single read to its single
+// write.  Pass 1 finds the maximum, pass 2 evaluates exp(x - max) once per element and keeps it as fp16 in the registers that held
+// the logits (values in (0, 1], 11 significant bits -- finer than the bf16 the gradient is stored in), pass 3 only scales.  One
 // exponential per element instead of two: the kernel is otherwise bound by the special-function unit as much as by
 // memory (100 K exponentials per row).
-constexpr int CER_MAXV = 13;
+// A block's time is a chain of load, maximum, exponentials, sum and store with a barrier between each, so what counts is that all of
+// its loads are on their way at once and that enough rows share an SM.  The loads are asm in a loop of their own: left to the
+// compiler they alternate with the maxima (8192 x 50304: 311 us, 265 so, 6.2 TB/s).  NV is what the row needs: see ce_rows.
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
@@ -121,32 +122,49 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
 __device__ __forceinline__ float2 unpack_h2(uint32_t w) {
     return __half22float2(*reinterpret_cast<const __half2*>(&w));
 }
-__global__ void __launch_bounds__(CEV_THREADS)
+template <int THREADS, int NV, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS)
 cross_entropy_bf16_reg_kernel(const __nv_bfloat16* __restrict__ logits, const int* __restrict__ targets,
                               __nv_bfloat16* dlogits, float* __restrict__ losses, int V, long long ld,
                               float grad_scale, float prob_eps) {
     __shared__ float scratch[32];
+    __shared__ int target;
+    constexpr bool ONE = NV > 10;    // the target is in one thread's register only: with it in all, 64 don't hold a longer row
+    pdl_wait();                      // (8192 x 50304: 280 us, 265 so; with shorter rows the other way round, 59 for 55 at 20000)
+    int tgt = 0;
+    if (!ONE || threadIdx.x == 0) tgt = targets[blockIdx.x];
     const long long off = (long long)blockIdx.x * ld;
     const uint4* row = reinterpret_cast<const uint4*>(logits + off);
     const int nv = V / 8;
-    uint4 r[CER_MAXV];
+    uint4 r[NV];
     float m = -INFINITY;
 #pragma unroll
-    for (int k = 0; k < CER_MAXV; ++k) {
-        const int i = threadIdx.x + k * CEV_THREADS;
-        if (i < nv) {
-            r[k] = row[i];
+    for (int k = 0; k < NV; ++k) {
+        const int i = threadIdx.x + k * THREADS;
+        if (i < nv)
+            asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r[k].x), "=r"(r[k].y), "=r"(r[k].z), "=r"(r[k].w)
+                         : "l"(row + i));
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        if (threadIdx.x + k * THREADS < nv) {
             float x[8];
             unpack8(r[k], x);
 #pragma unroll
             for (int j = 0; j < 8; ++j) m = fmaxf(m, x[j]);
         }
     }
+    __shared__ float xt;
+    tgt = tgt < 0 ? 0 : (tgt >= V ? V - 1 : tgt);
+    if (threadIdx.x == 0) {          // read before the barriers: after them the row is overwritten in place
+        xt = __bfloat162float(logits[off + tgt]);
+        target = tgt;
+    }
     const float row_max = block_max(m, scratch);
     float s = 0.f;
 #pragma unroll
-    for (int k = 0; k < CER_MAXV; ++k) {
-        if (threadIdx.x + k * CEV_THREADS < nv) {
+    for (int k = 0; k < NV; ++k) {
+        if (threadIdx.x + k * THREADS < nv) {
             float x[8];
             unpack8(r[k], x);
 #pragma unroll
@@ -156,24 +174,20 @@ cross_entropy_bf16_reg_kernel(const __nv_bfloat16* __restrict__ logits, const in
     }
     const float denom = block_sum(s, scratch);
     const float inv = 1.f / (denom + prob_eps);
-    int tgt = targets[blockIdx.x];
-    tgt = tgt < 0 ? 0 : (tgt >= V ? V - 1 : tgt);
     if (threadIdx.x == 0) {
-        const float xt = __bfloat162float(logits[off + tgt]);
         const float p = __expf(xt - row_max) * inv;
         losses[blockIdx.x] = prob_eps > 0.f ? -logf(p + prob_eps) : -(xt - row_max - logf(denom));
     }
-    __syncthreads();                 // the target's logit has been read before the row is overwritten in place
     if (dlogits) {
         uint4* g = reinterpret_cast<uint4*>(dlogits + off);
         const float sc = inv * grad_scale;
 #pragma unroll
-        for (int k = 0; k < CER_MAXV; ++k) {
-            const int i = threadIdx.x + k * CEV_THREADS;
+        for (int k = 0; k < NV; ++k) {
+            const int i = threadIdx.x + k * THREADS;
             if (i < nv) {
                 const float2 a = unpack_h2(r[k].x), b = unpack_h2(r[k].y), c = unpack_h2(r[k].z), d = unpack_h2(r[k].w);
                 float x[8] = {a.x * sc, a.y * sc, b.x * sc, b.y * sc, c.x * sc, c.y * sc, d.x * sc, d.y * sc};
-                const int t = tgt - i * 8;
+                const int t = (ONE ? target : tgt) - i * 8;
                 if (t >= 0 && t < 8) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
@@ -185,6 +199,33 @@ cross_entropy_bf16_reg_kernel(const __nv_bfloat16* __restrict__ logits, const in
     }
 }
 
+template <int THREADS, int NV, int BLOCKS>
+cudaError_t ce_rows_launch(const __nv_bfloat16* logits, const int* targets, __nv_bfloat16* dlogits, float* losses, int rows, int V,
+                           long long ld, float grad_scale, float prob_eps, cudaStream_t st) {
+    return cme_launch_dependent(cross_entropy_bf16_reg_kernel<THREADS, NV, BLOCKS>, dim3(rows), dim3(THREADS), 0, st, logits, targets,
+                                dlogits, losses, V, ld, grad_scale, prob_eps);
+}
+// By the length of the row: registers for it with the fewest idle threads, of the widths that a sweep of 28 forms left (rows x V, us
+// with one form for all before, and now): 8192 x 2048 100 -> 14.5, 8192 x 4096 113 -> 25, 8192 x 8192 130 -> 43, 4096 x 12288
+// 74 -> 35, 4096 x 20480 91 -> 56, 4096 x 28672 109 -> 83, 600 x 8192 13 -> 6.0.  Copy bandwidth would take 10, 20, 40, 30, 50, 71, 3.
+constexpr int CER_MAX_V = 512 * 13 * 8;
+cudaError_t ce_rows(const __nv_bfloat16* logits, const int* targets, __nv_bfloat16* dlogits, float* losses, int rows, int V,
+                    long long ld, float grad_scale, float prob_eps, cudaStream_t st) {
+#define CME_CER(T, NV, B) if (V <= T * NV * 8) return ce_rows_launch<T, NV, B>(logits, targets, dlogits, losses, rows, V, ld, grad_scale, prob_eps, st)
+    CME_CER(64, 4, 16);
+    CME_CER(128, 4, 12);
+    CME_CER(128, 6, 10);
+    CME_CER(128, 8, 10);
+    CME_CER(256, 6, 5);
+    CME_CER(256, 8, 5);
+    CME_CER(256, 10, 4);
+    CME_CER(256, 13, 4);
+    CME_CER(512, 8, 2);
+    CME_CER(512, 10, 2);
+    CME_CER(512, 13, 2);
+#undef CME_CER
+    return cudaErrorInvalidValue;
+}
 // Rows of at most WARPS * 32 * NV elements of any length, alignment and type, held in registers from their one read to
 // their one write: WARPS == 1 gives every warp a row (8 rows per block), else a block of WARPS warps shares one.
 // Character vocabularies are a few elements per lane: what bounds them is the latency of one row's chain of load,
@@ -525,10 +566,8 @@ CME_API int cme_cross_entropy(int dtype, const void* logits, const int* targets,
     const bool vec = dtype == CME_BF16 && V % 8 == 0 && ld % 8 == 0 && V >= 2048 &&
                      (reinterpret_cast<uintptr_t>(logits) & 15) == 0 &&
                      (!dlogits || (reinterpret_cast<uintptr_t>(dlogits) & 15) == 0);
-    if (vec && V / 8 <= CEV_THREADS * CER_MAXV) {
-        cross_entropy_bf16_reg_kernel<<<rows, CEV_THREADS, 0, st>>>((const __nv_bfloat16*)logits, targets,
-                                                                   (__nv_bfloat16*)dlogits, losses, V, ld, grad_scale,
-                                                                   prob_eps);
+    if (vec && V <= CER_MAX_V) {
+        CME_CUDA(ce_rows((const __nv_bfloat16*)logits, targets, (__nv_bfloat16*)dlogits, losses, rows, V, ld, grad_scale, prob_eps, st));
     } else if (vec) {
         const size_t row_bytes = (size_t)V * 2;
         const int cache = row_bytes <= 110 * 1024;          // two blocks per SM still fit
