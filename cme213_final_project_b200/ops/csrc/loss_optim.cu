@@ -234,7 +234,7 @@ cudaError_t ce_rows(const __nv_bfloat16* logits, const int* targets, __nv_bfloat
 // 16384 rows of 65 bf16 logits: 5.3 us, 27.8 us with a block per row.
 // One exponential per element (the general kernel evaluates it once for the sum and again for the gradient).
 template <typename T, int NV, int WARPS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(WARPS == 1 ? 256 : WARPS * 32)
 cross_entropy_short_kernel(const T* __restrict__ logits, const int* __restrict__ targets, T* dlogits,
                            float* __restrict__ losses, int rows, int V, long long ld, float grad_scale, float prob_eps) {
     __shared__ float scratch[32];
@@ -277,10 +277,14 @@ cross_entropy_short_kernel(const T* __restrict__ logits, const int* __restrict__
 template <typename T, int NV, int WARPS>
 cudaError_t ce_short_launch(const void* logits, const int* targets, void* dlogits, float* losses, int rows, int V,
                             long long ld, float grad_scale, float prob_eps, cudaStream_t st) {
-    return cme_launch_dependent(cross_entropy_short_kernel<T, NV, WARPS>, dim3(WARPS == 1 ? cme_cdiv(rows, 8) : rows), dim3(256), 0,
+    return cme_launch_dependent(cross_entropy_short_kernel<T, NV, WARPS>, dim3(WARPS == 1 ? cme_cdiv(rows, 8) : rows),
+                                dim3(WARPS == 1 ? 256 : WARPS * 32), 0,
                                 st, (const T*)logits, targets, (T*)dlogits, losses, rows, V, ld, grad_scale, prob_eps);
 }
-// One warp per row up to 1024 elements (32 registers a lane), one block per row up to 4096 (16 registers a thread).
+// One to four warps per row, the fewest whose lanes hold it in 32 registers, and of these as few as it fills: a second half of empty
+// registers costs as much as a full one, and eight warps wait for one another longer than four (bf16, us with 32 registers up to 1024,
+// then 8 warps of 8 or 16, and now: 16384 x 620 22.9 and 14.6, x 1001 25.8 and 23.0, x 1250 51.8 and 26.8, x 2001 54.6 and 38.5,
+// x 2500 85.3 and 50.3, 8192 x 4001 47.8 and 39.0, 1000 x 1501 5.2 and 4.1; fp32 alike).
 constexpr int CES_MAX_V = 4096;
 template <typename T>
 cudaError_t ce_short(const void* logits, const int* targets, void* dlogits, float* losses, int rows, int V, long long ld,
@@ -290,9 +294,15 @@ cudaError_t ce_short(const void* logits, const int* targets, void* dlogits, floa
     if (V <= 128) return CME_CES(4, 1);
     if (V <= 256) return CME_CES(8, 1);
     if (V <= 512) return CME_CES(16, 1);
-    if (V <= 1024) return CME_CES(32, 1);
-    if (V <= 2048) return CME_CES(8, 8);
-    return CME_CES(16, 8);
+    if (V <= 640) return CME_CES(20, 1);
+    if (V <= 768) return CME_CES(12, 2);
+    if (V <= 1024) return CME_CES(16, 2);
+    if (V <= 1280) return CME_CES(20, 2);
+    if (V <= 1536) return CME_CES(24, 2);
+    if (V <= 2048) return CME_CES(32, 2);
+    if (V <= 2560) return CME_CES(20, 4);
+    if (V <= 3072) return CME_CES(24, 4);
+    return CME_CES(32, 4);
 #undef CME_CES
 }
 

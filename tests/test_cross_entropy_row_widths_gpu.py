@@ -1,4 +1,4 @@
-"""Cross-entropy of bf16 rows held in registers, at both edges of each width's range, against float64 PyTorch."""
+"""Cross-entropy of rows held in registers, at both edges of each width's range, against float64 PyTorch."""
 import pytest
 import torch
 
@@ -33,3 +33,23 @@ def test_row_widths(V, inplace):
     bound = want.abs() * (2.0 ** -8 + 2.0 ** -11 + 2.0 ** -16) + 2.0 ** -24
     bound[pick, targets.long()] += 2.0 ** -11
     assert (err <= bound).all()
+
+
+@pytest.mark.parametrize("V", [512, 513, 640, 641, 768, 769, 1023, 1025, 1280, 1281, 1536, 1537, 2047, 2049, 2559, 2561, 3071, 3073, 4095])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_short_row_widths(V, dtype):
+    from cme213_final_project_b200 import ops
+    rows = 11
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = (torch.randn(rows, V, generator=g, device="cuda") * 3).to(dtype)
+    targets = torch.randint(0, V, (rows,), generator=g, device="cuda", dtype=torch.int32)
+    targets[0], targets[1] = 0, V - 1
+    ref, pick = x.double(), torch.arange(rows, device="cuda")
+    want = torch.softmax(ref, 1)
+    want[pick, targets.long()] -= 1
+    _, grad, losses = ops.cross_entropy(x.clone(), targets, inplace=True)
+    assert (losses.double() - (torch.logsumexp(ref, 1) - ref[pick, targets.long()])).abs().max().item() < 20 * 2.0 ** -19
+    # exponential, sum and products to 2^-16; a bf16 result rounded once; the target's element is p - 1 with the error of p <= 1
+    bound = want.abs() * (2.0 ** -16 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0))
+    bound[pick, targets.long()] += 2.0 ** -16
+    assert ((grad.double() * rows - want).abs() <= bound).all()
