@@ -40,6 +40,10 @@ template <> __device__ __forceinline__ void unpack_raw<float>(const uint4& r, fl
 }
 template <> __device__ __forceinline__ void unpack_raw<__nv_bfloat16>(const uint4& r, float* f) { unpack8(r, f); }
 
+__device__ __forceinline__ void load_raw(uint4& r, const void* p) {
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+}
+
 // Rows travel through a ring of shared-memory stages: all of its stages but one are ahead of the row a warp works on (three
 // stages; two in the backward of four vectors per lane).  A lane copies exactly the 16-byte words it will read itself, so
 // waiting for its own copies is all the synchronisation there is.  Registers alone keep one row in flight per warp, and the
@@ -82,9 +86,8 @@ __device__ __forceinline__ void row_scale(float (&o)[W], const float (&x)[W], co
         f2_unpack(f2_fma(f2_mul(f2_add(f2_pack(x[j], x[j + 1]), nmean), rstd), f2_pack(g[j], g[j + 1]), f2_pack(bt[j], bt[j + 1])),
                   o[j], o[j + 1]);
 }
-// y = LN(a [+ b]) * gamma + beta; optionally writes r = a + b, mean and rstd.  Rows of at most 32 * NV 16-byte vectors, one
-// warp per row, the grid what is resident at once.  Bound by memory: 16384 x 768 bf16 from memory with the residual add and
-// its sum stored (101 MB) 19.1 us; with one row per warp and four vectors per lane whatever the row's length, 22.0 us.
+// y = LN(a [+ b]) * gamma + beta; optionally writes r = a + b, mean and rstd.  fp32 rows of at most 32 * NV 16-byte vectors, one
+// warp per row, the grid what is resident at once.
 template <typename T, int NV>
 __global__ void __launch_bounds__(LN_WARPS * 32, NV <= 3 ? 3 : 2)
 ln_fwd_vec_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ r_out, const T* __restrict__ gamma,
@@ -161,9 +164,12 @@ ln_fwd_vec_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restric
     }
 }
 
-// Same bits with one row per warp, from global memory to registers.
+// Same bits with one row per warp, from global memory to registers.  Bound by memory: bf16 16384 x 768 with the residual add and its
+// sum stored (101 MB) 15.9 us, what a copy takes.  The loads of a bf16 row are asm ahead of all else: left to the compiler, which puts
+// each under its sum and store, it took 17.6, and with the rows in a ring of asynchronous copies, as fp32 ones are, 18.7.  Four blocks
+// an SM: with five or six forced the longest rows spill (16384 x 1024 22.3, 24.5 and 31.3).
 template <typename T, int NV>
-__global__ void __launch_bounds__(LN_WARPS * 32)
+__global__ void __launch_bounds__(LN_WARPS * 32, sizeof(T) == 2 ? 4 : 0)      // 0: left to the compiler
 ln_fwd_row_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ r_out, const T* __restrict__ gamma,
                   const T* __restrict__ beta, T* __restrict__ y, float* __restrict__ mean_out,
                   float* __restrict__ rstd_out, int rows, int D, float eps) {
@@ -173,16 +179,26 @@ ln_fwd_row_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restric
     const int row = blockIdx.x * LN_WARPS + (threadIdx.x >> 5);
     if (row >= rows) return;
     const long long off = (long long)row * D;
+    constexpr bool FIRST = sizeof(T) == 2;
+    uint4 ra[NV], rb[NV];
+    if (FIRST) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+            if (lane + 32 * i < nvec) {
+                load_raw(ra[i], a + off + (lane + 32 * i) * W);
+                if (b) load_raw(rb[i], b + off + (lane + 32 * i) * W);
+            }
+    }
     float x[NV][W];
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const int v = lane + 32 * i;
         if (v < nvec) {
-            load_vec<T>(a + off + v * W, x[i]);
+            if (FIRST) unpack_raw<T>(ra[i], x[i]); else load_vec<T>(a + off + v * W, x[i]);
             if (b) {
                 float t[W];
-                load_vec<T>(b + off + v * W, t);
+                if (FIRST) unpack_raw<T>(rb[i], t); else load_vec<T>(b + off + v * W, t);
                 row_add(x[i], t);
                 if (r_out) store_vec<T>(r_out + off + v * W, x[i]);
             }
@@ -521,32 +537,35 @@ inline int even_grid(int rows, int resident) {
 template <typename T, int NV>
 int ln_fwd_vec_launch(const T* a, const T* b, T* r, const T* g, const T* be, T* y, float* mean, float* rstd, int rows, int D,
                       float eps, cudaStream_t st) {
-    // The ring pays while the grid is a round or two (bf16, residual, us row by row / ring: 2048 x 768 4.2 / 4.0, 2048 x 1024
-    // 7.0 / 4.6) and where the rows come from memory and not from L2 (65536 x 768 43 / 41, 65536 x 1024 64 / 56).  Between the
-    // two more warps are worth more: 8192 x 768 from L2 5.8 / 6.5, 16384 x 512 6.7 / 8.3, 16384 x 1024 12.1 / 14.6, 8192 x 384
-    // fp32 4.0 / 5.2.  fp32 rows beyond L2 are faster row by row as well (65536 x 384, residual, 64 / 73).
+    // bf16 row by row whatever the size (with residual, us ring / row by row, from memory: 2048 x 768 3.7 / 3.5, 4096 x 768 6.6 / 5.8,
+    // 8192 x 384 6.7 / 6.1, 16384 x 1024 25.0 / 22.3; from L2: 8192 x 1024 10.8 / 8.2, 65536 x 1024 98 / 82).  fp32 rows are twice as
+    // many words a lane, and there the ring pays while the grid is a round or two (2048 x 512, residual, row by row / ring 4.5 / 4.4),
+    // and from memory up to 90 MB.  Between the two more warps are worth more (8192 x 384 from L2 4.0 / 5.2), and beyond L2 as well
+    // (65536 x 384, residual, 64 / 73).
     const double in_bytes = (double)rows * D * sizeof(T) * (b ? 2 : 1);
-    if (rows >= 8192 && (in_bytes <= 36e6 || (sizeof(T) == 4 && in_bytes >= 90e6))) {
+    if (sizeof(T) == 2 || (rows >= 8192 && (in_bytes <= 36e6 || in_bytes >= 90e6))) {
         CME_CUDA(cme_launch_dependent(ln_fwd_row_kernel<T, NV>, dim3(cme_cdiv(rows, LN_WARPS)), dim3(LN_WARPS * 32), 0, st, a, b,
                                       r, g, be, y, mean, rstd, rows, D, eps));
         CME_LAUNCH_CHECK();
         return CME_OK;
     }
-    const size_t smem = (size_t)LN_WARPS * LN_STAGES * (b ? 2 : 1) * NV * 512;
-    auto k = ln_fwd_vec_kernel<T, NV>;
-    static int resident[2][CME_MAX_DEVICES];       // [residual][device]
-    int dev = 0;
-    CME_CUDA(cudaGetDevice(&dev));
-    int& res = resident[b != nullptr][dev % CME_MAX_DEVICES];
-    if (!res) {
-        int n = 0;
-        const int rc = resident_blocks(k, smem, &n);
-        if (rc) return rc;
-        res = n;
+    if constexpr (sizeof(T) == 4) {
+        const size_t smem = (size_t)LN_WARPS * LN_STAGES * (b ? 2 : 1) * NV * 512;
+        auto k = ln_fwd_vec_kernel<T, NV>;
+        static int resident[2][CME_MAX_DEVICES];       // [residual][device]
+        int dev = 0;
+        CME_CUDA(cudaGetDevice(&dev));
+        int& res = resident[b != nullptr][dev % CME_MAX_DEVICES];
+        if (!res) {
+            int n = 0;
+            const int rc = resident_blocks(k, smem, &n);
+            if (rc) return rc;
+            res = n;
+        }
+        CME_CUDA(cme_launch_dependent(k, dim3(even_grid(rows, res)), dim3(LN_WARPS * 32), smem, st, a, b, r, g, be, y, mean, rstd,
+                                      rows, D, eps));
+        CME_LAUNCH_CHECK();
     }
-    CME_CUDA(cme_launch_dependent(k, dim3(even_grid(rows, res)), dim3(LN_WARPS * 32), smem, st, a, b, r, g, be, y, mean, rstd,
-                                  rows, D, eps));
-    CME_LAUNCH_CHECK();
     return CME_OK;
 }
 
