@@ -23,8 +23,8 @@
 //     highest key block stores its part, each lower one adds its own when the tile's counter says it is its turn,
 //     and key block 0, whose turn is last, adds the sum to its part in registers, scales, casts and writes dQ --
 //     bit-reproducible, no clearing or conversion pass, but the chain of turns makes CTAs wait for one another.  Whole backward in
-//     modes 0 / 1 / 2: 16 x 12 heads x 1024 tokens 183 / 283 / 279 us causal, 290 / 500 / 389 all keys; 64 x 6 x 256 causal
-//     58 / 78 / 107.
+//     modes 0 / 1 / 2: 16 x 12 heads x 1024 tokens 146 / 259 / 276 us causal, 227 / 473 / 369 all keys; 64 x 6 x 256 causal
+//     48 / 69 / 98.
 // Grids that fill the GPU take small CTAs, several to an SM; others, and the backward's modes 1 and 2, 128 x 128 blocks.
 // Every mbarrier wait is bounded; on expiry the CTA flags the status word, frees TMEM and returns.
 #include "attention.h"
@@ -336,7 +336,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // Forward of grids that leave the small CTAs above without neighbours (fwd_wide)
 // ------------------------------------------------------------------------------------------------------
 // 128 keys per step in a CTA of which two fit an SM: S_j is copied to registers, the tensor core makes S_{j+1} while softmax_j runs, and P
-// has columns of its own.  Alone on its SM, a CTA gets through its keys in 0.6 of the time that the small one takes.
+// has columns of its own.  Alone on its SM, a CTA gets through its keys in 0.7 of the time that the small one takes.
 // shared: Q 16K | K[3] 48K | V[3] 48K | barriers      (P never passes through shared memory)
 constexpr int FWD_WIDE_STAGES = 3;           // a K / V tile is requested two blocks ahead of its use: its ~1200-clock
                                            // latency no longer delays the next S product
@@ -1470,12 +1470,14 @@ int attention_tc_supported(const CmeAttn* a) {
 // Which kernel a call takes, by how it fills the SMs.  ctas: 128-row tiles of all heads; the small CTAs share an SM by four (forward)
 // or two (backward), the wide ones by two or one.  Times in us, wide / small, heads x tokens.
 //
-// Forward.  Up to two tiles per SM the small CTAs run without enough neighbours: 16 x 1024 14.1 / 26.1 causal, 24 x 582 11.1 / 18.0,
-// 128 x 256 8.8 / 9.7, 192 x 128 6.5 / 7.3 (with 129 to 192 tokens up to one: 64 x 192 7.4 / 7.9, 96 x 192 8.8 / 7.9).  Beyond, causal
-// calls take the small ones (192 x 256 14.0 / 11.0, 96 x 1024 40 / 32.6) but for long sequences just beyond (48 x 1024 23.5 / 27.4;
-// 64 x 1024 30.1 / 28.6).  With all keys both do a full GPU's work at one rate, and what counts is the last wave: to six tiles per SM
-// the wide ones (64 x 1024 33.8 / 37.2, 96 x 1024 49.8 / 57.7, 128 x 582 33.7 / 37.5; 192 x 582 49 / 43), then where that of the small
-// ones would be a quarter full (160 x 1024 81 / 86).
+// Forward.  Up to two tiles per SM the small CTAs run without enough neighbours: 16 x 1024 13.1 / 19.2 causal, 24 x 582 9.9 / 13.3,
+// 192 x 128 6.3 / 6.8, 128 x 256 8.2 / 8.2 (with 129 to 192 tokens up to one: 64 x 192 6.9 / 6.7, 96 x 192 7.9 / 7.0).  Beyond, causal
+// calls take the small ones (192 x 256 12.1 / 9.8, 96 x 1024 36.3 / 29.2) but for long sequences just beyond.  With all keys both do a
+// full GPU's work at one rate, and the last wave decides: to six tiles per SM the wide ones (64 x 1024 32.5 / 33.6, 80 x 1024 41.3 / 43.7;
+// 192 x 582 42.7 / 38.0), then where that of the small ones would be a quarter full.
+// The lines were drawn before the small CTAs issued their products faster; near them the small ones are ahead by now (causal 48 x 1024
+// 22.6 / 20.8, 64 x 1024 27.6 / 22.7; all keys 96 x 1024 48.1 / 47.5, 160 x 1024 71.9 / 68.9).  They stay, because which kernel
+// runs shows in the last bits of the results.
 bool fwd_wide(long long ctas, int T, bool causal, int sms) {
     if (T > 128 && T <= 192) return ctas <= sms;
     if (ctas <= 2ll * sms) return true;
@@ -1483,12 +1485,12 @@ bool fwd_wide(long long ctas, int T, bool causal, int sms) {
     const long long last = ctas % (4ll * sms);
     return (T > 512 && ctas <= 6ll * sms) || (T > 768 && ctas > 8ll * sms && last > 0 && last <= sms);
 }
-// Backward.  One tile per SM: 16 x 1024 24.1 / 38.9, 24 x 582 17.0 / 25.9, 64 x 256 10.2 / 13.1, 128 x 128 8.5 / 9.0.  Two per SM: the
-// small ones win (96 x 256 17.1 / 15.2, all keys 24 x 1024 47.6 / 46.2), causal not beyond 448 tokens (24 and 32 x 1024 35.0 / 41.3 and
-// 41.7 / 42.7, 48 x 582 28.3 / 28.7), since the wide CTAs of light tiles make room for others.  With all keys and an odd number, the small
-// ones' last wave is half empty: three 48 x 1024 71 / 86, 64 x 582 48 / 55, 192 x 256 28.8 / 30.2, but 192 x 192 26.8 / 22.4; five 80 x 1024
-// 121 / 126, 128 x 582 82 / 83.  Else the small ones (causal 48 x 1024 53 / 48, 96 x 1024 93 / 80.5; all keys 96 x 1024 148 / 132,
-// 128 x 1024 178 / 173).
+// Backward.  One tile per SM: 16 x 1024 20.9 / 28.4, 24 x 582 15.2 / 19.4, 64 x 256 10.1 / 10.7, 128 x 128 8.2 / 7.9.  Two per SM: the
+// small ones (96 x 256 16.9 / 12.6, all keys 24 x 1024 40.9 / 36.6), causal not beyond 448 tokens.  With all keys and an odd number the
+// small ones' last wave is half empty (48 x 1024 61.8 / 63.0, 64 x 582 42.7 / 42.2; 192 x 192 26.0 / 19.0).  Else the small ones (causal
+// 48 x 1024 47.6 / 38.8, 96 x 1024 83.5 / 65.5; all keys 96 x 1024 125 / 106, 128 x 1024 149 / 138).  These lines, too, are older than
+// the faster small CTAs (causal 32 x 1024 36.5 / 31.9, 48 x 582 25.8 / 21.6; all keys 192 x 256 28.3 / 22.8, 80 x 1024 103 / 97, 128 x 582
+// 72.5 / 65.2) and stay.
 bool bwd_wide(long long ctas, int T, bool causal, int sms) {
     const long long waves = (ctas + sms - 1) / sms;
     if (causal) return waves <= 1 || (waves == 2 && T > 448);
