@@ -12,18 +12,18 @@ namespace {
 
 // What bounds these kernels is the fp32 multiply-add rate and, next to it, shared-memory reads: a 16-byte load per lane
 // takes the SM's shared memory four clocks, in which its schedulers issue sixteen multiply-adds.  So every product is
-// register-tiled.  The warps form groups of 16 rows x 2 halves -- of the streamed rows in the score products, of the head's
-// columns in the others; a lane has 4 of the rows (ty + 4 i) and every eighth streamed row of its half (tx + 8 j), or VW
-// consecutive columns in 8 VW, so that a lane's 4-row tiles of two outputs fit its registers.  No load has a bank conflict,
-// since a row's pitch is an odd number of 16-byte words.  Multiply-adds are packed pairs, fp32 tiles arrive by asynchronous
-// copies, all of a block's at once, the ones that the second product needs under the first.
+// register-tiled.  In the forward the warps form groups of 16 rows x 2 halves -- of the streamed rows in the score products, of the
+// head's columns in the others; a lane has 4 of the rows (ty + 4 i) and every eighth streamed row of its half (tx + 8 j), or VW
+// consecutive columns in 8 VW.  In the backward four warps have a product (attn_bwd_kernel) and a lane 8 rows.  No load has a bank
+// conflict, since a row's pitch is an odd number of 16-byte words.  Multiply-adds are packed pairs, fp32 tiles arrive by asynchronous
+// copies, all that a group of warps needs at once; in the forward V's under the first product.
 // The head size is padded with zeros to a multiple of 32 (template G = ceil(HD / 32)).
 // 32 x 4 heads x 64 tokens x head size 128, fp32, forward + backward: 12.9 + 24.0 us; 18 + 31 with a warp for whole rows of the
 // forward, single multiply-adds and tiles loaded through registers one after the other, 12.9 + 27.8 with eight warps on each of the
 // backward's products (floor of both at the fp32 rate, 0.94 GFLOP at 74 TFLOP/s: 13 us).  64 query rows a block instead of 32 in the
 // forward: 12.8 us, no different.
 constexpr int CT = 64;               // rows streamed per step
-constexpr int WR = 16;               // rows a warp owns
+constexpr int WR = 16;               // rows a warp of the forward owns
 constexpr int LR = WR / 4;           // rows a lane has of them
 constexpr int SP = CT + 4;           // pitch of the probability tiles
 constexpr int MAX_HD = 128;
