@@ -584,11 +584,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     if constexpr (PAIR) mma_commit_pair(&tfull_bar[buf], 3); else mma_commit(&tfull_bar[buf]);
                 }
             }
-            if (!PAIR && ok) {                          // the accumulators of the last two tiles have been read
-                tmem_free = true;
-                for (int i = it > 1 ? it - 2 : 0; i < it; ++i)
-                    tmem_free = tmem_free && mbar_wait(&tempty_bar[i & 1], (i >> 1) & 1, abort_flag);
-            }
+            // The accumulators of the last two tiles have been read.  A pair's leader waits as well: the peer's arrivals on these
+            // barriers are stores to this CTA's shared memory, which has to exist until they are there.
+            for (int i = it > 1 ? it - 2 : 0; i < it && ok; ++i) ok = mbar_wait(&tempty_bar[i & 1], (i >> 1) & 1, abort_flag);
+            tmem_free = !PAIR && ok;
         }
         // freed under the last tile's stores, not after them (256 clocks); a pair's CTAs free theirs together
         if constexpr (!PAIR) {
@@ -952,7 +951,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     __syncwarp();
     tc_fence_before();
-    // A pair leaves together: neither CTA may exit while the other can still signal its barriers or read its tiles.
+    // A pair leaves together: neither CTA may exit while the other's products still read its tiles or signal its barriers.  Those are
+    // over when both have seen their last accumulator complete, and the peer's arrivals at the leader when its MMA thread has seen them
+    // (above), so this meeting has no memory to order: each CTA comes to it after its own waits.
     __syncthreads();
     if constexpr (PAIR) cluster_sync_relaxed();
     if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, CME_ERR_TIMEOUT);

@@ -202,12 +202,14 @@ __device__ __forceinline__ uint32_t mapa_u32(const void* p, uint32_t rank) {
     return out;
 }
 // Meeting points of the cluster's threads that order no memory.  What must be seen across is ordered by its own means (barrier
-// words by fence_barrier_init, tensor memory by the tcgen05 fences); a release at cluster scope waits for all of the thread's earlier
-// stores, 1000-2000 clocks.
+// words by fence_barrier_init, tensor memory by the tcgen05 fences, arrivals by waits for them); a release at cluster scope waits for all
+// of the thread's earlier stores, 1000-2000 clocks.
 __device__ __forceinline__ void cluster_sync_relaxed() {
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
-// An arrival on another CTA's barrier, with the default release at CTA scope, for the same reason.
+// An arrival on another CTA's barrier, with the default release at CTA scope: it hands over tensor memory, whose loads tcgen05.wait::ld
+// has completed before, and no word of memory that the other CTA reads.  It is a store to that CTA, which has to wait for it on the
+// barrier itself before it may exit: cluster_sync_relaxed does not order it.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
