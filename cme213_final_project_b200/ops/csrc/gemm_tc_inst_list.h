@@ -91,6 +91,7 @@ CME_GEMM_TC_EXTERN(192, false, true, SPEC_BIAS)
 #if CME_GEMM_TC_GROUP == -1 || CME_GEMM_TC_GROUP == 13     // CTA pair, 192 columns: compile-time epilogues
 CME_GEMM_TC_EXTERN(192, false, true, SPEC_RES)
 CME_GEMM_TC_EXTERN(192, false, true, SPEC_BIAS_RES)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_BIAS_GELU_AUX)
 CME_GEMM_TC_EXTERN(192, false, true, SPEC_BIAS_RELU)
 CME_GEMM_TC_EXTERN(192, false, true, SPEC_DRELU_COLSUM)
 #endif
@@ -99,6 +100,7 @@ CME_GEMM_TC_EXTERN(192, false, true, SPEC_BIAS_GELU_AUXD)
 CME_GEMM_TC_EXTERN(192, false, true, SPEC_DMUL_COLSUM)
 CME_GEMM_TC_EXTERN(192, false, true, SPEC_DMUL)
 CME_GEMM_TC_EXTERN(192, false, true, SPEC_DRELU)
+CME_GEMM_TC_EXTERN(192, false, true, SPEC_DGELU)
 #endif
 
 #if CME_GEMM_TC_GROUP == -1 || CME_GEMM_TC_GROUP == 15     // three products, each rounded
