@@ -281,14 +281,16 @@ cudaError_t ce_short_launch(const void* logits, const int* targets, void* dlogit
                                 dim3(WARPS == 1 ? 256 : WARPS * 32), 0,
                                 st, (const T*)logits, targets, (T*)dlogits, losses, rows, V, ld, grad_scale, prob_eps);
 }
-// One to four warps per row, the fewest whose lanes hold it in 32 registers, and of these as few as it fills: a second half of empty
-// registers costs as much as a full one, and eight warps wait for one another longer than four (bf16, us with 32 registers up to 1024,
-// then 8 warps of 8 or 16, and now: 16384 x 620 22.9 and 14.6, x 1001 25.8 and 23.0, x 1250 51.8 and 26.8, x 2001 54.6 and 38.5,
-// x 2500 85.3 and 50.3, 8192 x 4001 47.8 and 39.0, 1000 x 1501 5.2 and 4.1; fp32 alike).
+// One to four warps per row, so that a lane has at most 32 registers of it, and of these as few as the row fills: a second half of
+// empty registers costs as much as a full one, eight warps wait for one another longer than four, and two of 12 or 16 registers are
+// faster than one of 24 or 32 (bf16, us with 32 registers up to 1024, then 8 warps of 8 or 16, and so: 16384 x 620 22.9 and 14.6,
+// x 1001 25.8 and 23.0, x 1250 51.8 and 26.8, x 2001 54.6 and 38.5, x 2500 85.3 and 50.3, 8192 x 4001 47.8 and 39.0; fp32 alike).
+// Up to two rows per SM nothing overlaps a row's chain, and eight warps have the shorter one (128 x 2001 3.44 us, 4.02 with two
+// warps; 296 x 4001 4.43 and 4.77; 400 x 1501 4.1 and 4.3, x 2500 4.7 and 4.1, 600 x 3001 6.3 and 5.3).
 constexpr int CES_MAX_V = 4096;
 template <typename T>
 cudaError_t ce_short(const void* logits, const int* targets, void* dlogits, float* losses, int rows, int V, long long ld,
-                     float grad_scale, float prob_eps, cudaStream_t st) {
+                     float grad_scale, float prob_eps, int sms, cudaStream_t st) {
 #define CME_CES(NV, WARPS) ce_short_launch<T, NV, WARPS>(logits, targets, dlogits, losses, rows, V, ld, grad_scale, prob_eps, st)
     if (V <= 64) return CME_CES(2, 1);
     if (V <= 128) return CME_CES(4, 1);
@@ -297,6 +299,7 @@ cudaError_t ce_short(const void* logits, const int* targets, void* dlogits, floa
     if (V <= 640) return CME_CES(20, 1);
     if (V <= 768) return CME_CES(12, 2);
     if (V <= 1024) return CME_CES(16, 2);
+    if (rows <= 2 * sms) return V <= 2048 ? CME_CES(8, 8) : CME_CES(16, 8);
     if (V <= 1280) return CME_CES(20, 2);
     if (V <= 1536) return CME_CES(24, 2);
     if (V <= 2048) return CME_CES(32, 2);
@@ -590,8 +593,13 @@ CME_API int cme_cross_entropy(int dtype, const void* logits, const int* targets,
         cross_entropy_bf16_vec_kernel<<<rows, CEV_THREADS, cache ? row_bytes : 0, st>>>(
             (const __nv_bfloat16*)logits, targets, (__nv_bfloat16*)dlogits, losses, V, ld, grad_scale, prob_eps, cache);
     } else if (V <= CES_MAX_V) {
-        CME_CUDA(dtype == CME_BF16 ? ce_short<__nv_bfloat16>(logits, targets, dlogits, losses, rows, V, ld, grad_scale, prob_eps, st)
-                                   : ce_short<float>(logits, targets, dlogits, losses, rows, V, ld, grad_scale, prob_eps, st));
+        int sms = 0;
+        if (V > 1024) {
+            const int rc = cme_num_sms(&sms);
+            if (rc) return rc;
+        }
+        CME_CUDA(dtype == CME_BF16 ? ce_short<__nv_bfloat16>(logits, targets, dlogits, losses, rows, V, ld, grad_scale, prob_eps, sms, st)
+                                   : ce_short<float>(logits, targets, dlogits, losses, rows, V, ld, grad_scale, prob_eps, sms, st));
     } else if (dtype == CME_BF16)
         cross_entropy_kernel<__nv_bfloat16><<<rows, CE_THREADS, 0, st>>>((const __nv_bfloat16*)logits, targets,
                                                                          (__nv_bfloat16*)dlogits, losses, V, ld,

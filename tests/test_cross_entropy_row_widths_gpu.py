@@ -37,9 +37,9 @@ def test_row_widths(V, inplace):
 
 @pytest.mark.parametrize("V", [512, 513, 640, 641, 768, 769, 1023, 1025, 1280, 1281, 1536, 1537, 2047, 2049, 2559, 2561, 3071, 3073, 4095])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-def test_short_row_widths(V, dtype):
+@pytest.mark.parametrize("rows", [11, 297])        # eight warps share a row of more than 1024 up to two rows per SM, fewer beyond
+def test_short_row_widths(V, dtype, rows):
     from cme213_final_project_b200 import ops
-    rows = 11
     g = torch.Generator(device="cuda").manual_seed(V)
     x = (torch.randn(rows, V, generator=g, device="cuda") * 3).to(dtype)
     targets = torch.randint(0, V, (rows,), generator=g, device="cuda", dtype=torch.int32)
