@@ -459,6 +459,7 @@ __global__ void __launch_bounds__(256) adam_kernel(const AdamArgs a) {
 }
 
 
+constexpr int ADAM_BLOCKS_PER_SM = 5;
 constexpr int ADAM_LIST = 512;             // ranges that a block keeps in shared memory (8 KB); longer lists are read in place
 
 // Four elements per thread and round (128-bit accesses on the fp32 state).  Requires 16-byte aligned arenas; the last n % 4
@@ -469,7 +470,7 @@ constexpr int ADAM_LIST = 512;             // ranges that a block keeps in share
 // each array; as 2368 blocks that stride through all of it the same loop took 558 us.  Five blocks an SM: four 536 us, six 538 (spills
 // aside, more rows of DRAM open at once).
 template <typename TG, bool RANGES>
-__global__ void __launch_bounds__(256, 5) adam_vec4_kernel(const AdamArgs a, const int rounds) {
+__global__ void __launch_bounds__(256, ADAM_BLOCKS_PER_SM) adam_vec4_kernel(const AdamArgs a, const int rounds) {
     pdl_wait();
     const long long nv = a.n >> 2;
     const long long first = (long long)blockIdx.x * rounds * 256 + threadIdx.x;
@@ -687,11 +688,18 @@ CME_API int cme_adam_partials(int grad_dtype, float* master, void* compute_bf16,
     bool vec = n >= 4 && al(master, 16) && al(m, 16) && al(v, 16) && al(compute_bf16, 8) &&
                al(grads, grad_dtype == CME_BF16 ? 8 : 16);
     if (vec) {
-        // Rounds per block: its set-up (three scalars, two powers, the list of ranges) takes as long as a round, unless there are too few
-        // blocks to go round.  1 / 2 / 4 / 8 rounds: 124 M elements 580 / 521 / 519 / 523 us, 4 M 18.5 / 15.9 / 14.8 / 14.7, 1 M 6.8 / 5.9 /
-        // 7.0 / 9.3, 0.2 M 3.6 / 4.3 / 5.9 / 9.1.
+        // Rounds per block: its set-up (three scalars, two powers, the list of ranges, the norm's partial sums) takes as long as a round,
+        // so the fewest that let all blocks run at once, five per SM, up to four; beyond that a second wave costs as much as it is full,
+        // and three rounds are within 3 % of the best everywhere.  us with 1 / 2 / 3 / 4 / 8 rounds, bf16 gradients, no ranges or clipping:
+        // 0.46 M elements 2.9 / 3.4 / 4.0 / 4.4 / 6.9, 1 M 4.8 / 4.6 / 5.0 / 5.3 / 7.1, 1.8 M 7.0 / 7.0 / 6.4 / 6.6 / 8.4, 2.5 M from memory
+        // 10.3 / 9.6 / 10.3 / 9.4 / 11.8, 4 M 18.9 / 19.0 / 19.5 / 21.0 / 20.4, with ranges and the norm's partial sums 26.5 / 24.2 / 23.6 /
+        // 25.6 / 23.3; 40 M with both 223 / 188 / 179 / 178 / 179.
         const long long groups = (n / 4 + 255) / 256;
-        const int rounds = groups <= 148 * 3 ? 1 : groups <= 148 * 12 ? 2 : 4;
+        int sms = 0;
+        const int rc = cme_num_sms(&sms);
+        if (rc) return rc;
+        const long long fit = (groups + ADAM_BLOCKS_PER_SM * sms - 1) / (ADAM_BLOCKS_PER_SM * sms);
+        const int rounds = fit <= 4 ? (int)fit : 3;
         blocks = (groups + rounds - 1) / rounds;
         const bool ranges = weight_decay > 0.f && n_nodecay > 0;
         auto kernel = grad_dtype != CME_BF16 ? (ranges ? adam_vec4_kernel<float, true> : adam_vec4_kernel<float, false>)

@@ -1,4 +1,5 @@
-"""The optimizer where the rounds per block change (454 656 and 1 818 624 elements), and where the last block and round are not full."""
+"""The optimizer where the rounds per block change (multiples of 757 760 elements up to four), and where the last block and round are
+not full."""
 import pytest
 import torch
 
@@ -7,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("clip,ranges", [(0.0, False), (0.01, True)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("n", [4, 1023, 1024, 1029, 454_655, 454_656, 454_661, 1_818_624, 1_818_629, 1_820_676, 4_000_003])
+@pytest.mark.parametrize("n", [4, 1023, 1024, 1029, 454_655, 454_656, 454_661, 757_760, 757_761, 1_515_520, 1_515_525, 1_818_624,
+                               1_818_629, 1_820_676, 2_273_284, 3_031_040, 3_031_041, 4_000_003])
 def test_every_element_is_updated_once(n, dtype, clip, ranges):
     from cme213_final_project_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(1)
