@@ -391,9 +391,11 @@ PyObject* gemm_prepare(PyObject*, PyObject* const* o, Py_ssize_t) {
     if (!a.defined() || !b.defined()) fail(PyExc_TypeError, "native ops take tensors");
     at::Tensor out = any(o[4]);
     if (a.dim() < 2 || b.dim() < 2) fail(PyExc_IndexError, "gemm: operands have to be matrices");
+    // a leading size of 1 is shared by the entries of the other operand, as a matrix is
     const bool a3 = a.dim() == 3, b3 = b.dim() == 3;
-    long long batch = a3 ? a.size(0) : 1;
-    if (b3 && b.size(0) > batch) batch = b.size(0);
+    const long long na = a3 ? a.size(0) : 1, nb = b3 ? b.size(0) : 1, batch = na == 1 ? nb : na;
+    if (nb != 1 && nb != batch)
+        fail(native_error, "gemm: operands of " + std::to_string(na) + " and " + std::to_string(nb) + " matrices");
     const long long a0 = a.size(-2), a1 = a.size(-1), b0 = b.size(-2), b1 = b.size(-1);
     CmeGemm g;
     std::memset(&g, 0, sizeof g);
@@ -414,8 +416,8 @@ PyObject* gemm_prepare(PyObject*, PyObject* const* o, Py_ssize_t) {
     at::Tensor part;
     if (truth(o[16])) part = at::empty({(M + 31) / 32 * N}, a.options().dtype(at::kFloat));
     g.M = int32(M); g.N = int32(N); g.K = int32(K); g.batch = int32(batch);
-    g.A = ptr(a); g.lda = a1; g.strideA = a3 ? a0 * a1 : 0;
-    g.B = ptr(b); g.ldb = b1; g.strideB = b3 ? b0 * b1 : 0;
+    g.A = ptr(a); g.lda = a1; g.strideA = na == batch && a3 ? a0 * a1 : 0;
+    g.B = ptr(b); g.ldb = b1; g.strideB = nb == batch && b3 ? b0 * b1 : 0;
     g.C = ptr(out); g.ldc = N; g.strideC = M * N;
     g.bias = ptr(bias);
     g.residual = ptr(res); g.ldres = N;

@@ -23,7 +23,8 @@ def seen(monkeypatch):
 
 @pytest.mark.parametrize("sa,sb,at,bt,shape,strides", [
     ((5, 7), (7, 3), 0, 0, (5, 3), (0, 0)), ((7, 5), (3, 7), 1, 1, (5, 3), (0, 0)), ((4, 5, 7), (7, 3), 0, 0, (4, 5, 3), (35, 0)),
-    ((5, 7), (4, 3, 7), 0, 1, (4, 5, 3), (0, 21)), ((4, 7, 5), (4, 7, 3), 1, 0, (4, 5, 3), (35, 21)), ((1, 5, 7), (2, 7, 3), 0, 0, (2, 5, 3), (35, 21))])
+    ((5, 7), (4, 3, 7), 0, 1, (4, 5, 3), (0, 21)), ((4, 7, 5), (4, 7, 3), 1, 0, (4, 5, 3), (35, 21)), ((1, 5, 7), (2, 7, 3), 0, 0, (2, 5, 3), (0, 21)),
+    ((3, 7, 5), (1, 3, 7), 1, 1, (3, 5, 3), (35, 0)), ((1, 5, 7), (1, 7, 3), 0, 0, (1, 5, 3), (35, 21))])
 def test_shapes_and_strides(seen, sa, sb, at, bt, shape, strides):
     a, b = torch.zeros(sa), torch.zeros(sb, dtype=torch.float32)
     out = ops.gemm(a, b, a_trans=at, b_trans=bt, out_dtype=torch.bfloat16)
@@ -58,3 +59,22 @@ def test_refusals(seen):
     with pytest.raises(ops.NativeError, match="unsupported dtype torch.float16"):
         ops.gemm(a.half(), a.half())
     assert not seen
+
+
+@pytest.mark.parametrize("sa,sb", [((2, 5, 7), (3, 7, 3)), ((3, 5, 7), (2, 7, 3)), ((0, 5, 7), (2, 7, 3)), ((2, 5, 7), (0, 7, 3))])
+def test_batches_that_do_not_match(seen, sa, sb):
+    """A descriptor has one number of matrices: entries beyond an operand's own lie outside its memory."""
+    with pytest.raises(ops.NativeError, match=f"operands of {sa[0]} and {sb[0]} matrices"):
+        ops.gemm(torch.zeros(sa), torch.zeros(sb))
+    assert not seen
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("backend", ["tcgen05", "simt"])
+@pytest.mark.parametrize("na,nb", [(1, 3), (3, 1), (3, 3)])
+def test_one_matrix_is_shared(na, nb, backend):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a, b = (torch.randn(s, generator=g, device="cuda").to(torch.bfloat16) for s in ((na, 72, 64), (nb, 64, 40)))
+    got = ops.gemm(a, b, backend=backend)
+    want = torch.stack([ops.gemm(a[i % na].contiguous(), b[i % nb].contiguous(), backend=backend) for i in range(3)])
+    assert torch.equal(got, want)
