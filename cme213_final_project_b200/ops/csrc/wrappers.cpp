@@ -413,6 +413,23 @@ PyObject* gemm_prepare(PyObject*, PyObject* const* o, Py_ssize_t) {
     }
     g.ab_dtype = dtype(a);
     g.c_dtype = dtype(out);
+    g.act = number(o[7]); g.dact = number(o[9]);
+    // the kernels take as many elements of these types as the descriptor says, whatever the tensors hold
+    auto holds = [](const char* name, const at::Tensor& t, const at::Tensor& typed, const char* whose, long long count) {
+        if (!t.defined()) return;
+        if (t.scalar_type() != typed.scalar_type()) fail(native_error, std::string("gemm: ") + name + " has to have the type of " + whose);
+        if (t.numel() < count)
+            fail(native_error, std::string("gemm: ") + name + " has " + std::to_string(t.numel()) + " of " + std::to_string(count) +
+                                   " elements");
+    };
+    const long long elements = batch * M * N;
+    holds("b", b, a, "a", 0);
+    holds("out", out, out, "out", elements);
+    holds("bias", bias, a, "a", N);
+    holds("residual", res, out, "out", elements);
+    holds("aux_out", aux_out, out, "out", elements);
+    if (g.dact && !aux_in.defined()) fail(native_error, "gemm: dact needs aux_in");
+    if (g.dact) holds("aux_in", aux_in, out, "out", elements);
     at::Tensor part;
     if (truth(o[16])) part = at::empty({(M + 31) / 32 * N}, a.options().dtype(at::kFloat));
     g.M = int32(M); g.N = int32(N); g.K = int32(K); g.batch = int32(batch);
@@ -422,7 +439,7 @@ PyObject* gemm_prepare(PyObject*, PyObject* const* o, Py_ssize_t) {
     g.bias = ptr(bias);
     g.residual = ptr(res); g.ldres = N;
     g.aux_out = ptr(aux_out); g.aux_in = ptr(aux_in); g.ldaux = N;
-    g.act = number(o[7]); g.dact = number(o[9]); g.accumulate = number(o[12]);
+    g.accumulate = number(o[12]);
     g.workspace = ptr(ws);
     g.workspace_bytes = ws.defined() ? ws.numel() * 4 : 0;
     g.force_bn = number(o[13]); g.force_splits = number(o[14]);

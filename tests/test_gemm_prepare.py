@@ -69,6 +69,30 @@ def test_batches_that_do_not_match(seen, sa, sb):
     assert not seen
 
 
+@pytest.mark.parametrize("kw,what", [
+    ({"out": torch.zeros(7, 8)}, "out has 56 of 64"), ({"bias": torch.zeros(7)}, "bias has 7 of 8"),
+    ({"residual": torch.zeros(8, 7)}, "residual has 56 of 64"), ({"aux_out": torch.zeros(8)}, "aux_out has 8 of 64"),
+    ({"dact": "relu", "aux_in": torch.zeros(8)}, "aux_in has 8 of 64"), ({"dact": "relu"}, "dact needs aux_in"),
+    ({"bias": torch.zeros(8).bfloat16()}, "bias has to have the type of a"),
+    ({"residual": torch.zeros(8, 8).bfloat16()}, "residual has to have the type of out"),
+    ({"out_dtype": torch.bfloat16, "aux_out": torch.zeros(8, 8)}, "aux_out has to have the type of out"),
+    ({"out": torch.zeros(8, 8).bfloat16(), "dact": "relu", "aux_in": torch.zeros(8, 8)}, "aux_in has to have the type of out"),
+    ({"b": torch.zeros(8, 8).bfloat16()}, "b has to have the type of a")])
+def test_operands_that_the_kernels_would_leave(seen, kw, what):
+    with pytest.raises(ops.NativeError, match=what):
+        ops.gemm(torch.zeros(8, 8), **{"b": torch.zeros(8, 8), **kw})
+    assert not seen
+
+
+def test_operands_of_other_shapes(seen):
+    """What holds enough elements is taken as before, whatever its shape; an auxiliary input without use is not looked at."""
+    a, b = torch.zeros(2, 4, 8), torch.zeros(8, 8)
+    out = torch.zeros(100)
+    assert ops.gemm(a, b, out=out, bias=torch.zeros(1, 9), residual=torch.zeros(64), aux_in=torch.zeros(1)) is out
+    assert ops.gemm(b, b.clone(), out_dtype=torch.bfloat16, bias=torch.zeros(8), residual=torch.zeros(8, 8).bfloat16()).shape == (8, 8)
+    assert len(seen) == 2
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("backend", ["tcgen05", "simt"])
 @pytest.mark.parametrize("na,nb", [(1, 3), (3, 1), (3, 3)])
