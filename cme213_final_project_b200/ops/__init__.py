@@ -217,10 +217,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bo
     of four and such operands of at most 32 MB together, and ``auto`` multiplies the others exactly; ``allow_tf32=2`` lets it
     take them all.
     """
-    _cuda(a, b, out, bias, aux_out, aux_in, residual)
+    _cuda(a, b, out, bias, aux_out, aux_in, residual, dbias)
     ws = _scratch(a.device)                           # goes back when the call has been issued
     out, part, desc = _compiled().gemm_prepare(a, b, a_trans, b_trans, out, out_dtype, bias, ACT[act], aux_out, ACT[dact], aux_in,
-                                               residual, accumulate, force_bn, force_splits, aux_deriv, dbias is not None,
+                                               residual, accumulate, force_bn, force_splits, aux_deriv, dbias,
                                                allow_tf32, ws)
     g = CmeGemm.from_buffer(desc)
     _check(lib().cme_gemm(ctypes.byref(g), _GEMM_BACKENDS[backend], _st()))
@@ -230,7 +230,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_trans: bool = False, b_trans: bo
         if slabs:
             _check(lib().cme_colsum_slabs_finalize(_dt(dbias), _a(part), slabs, g.N, _a(dbias), 0, _st()))
         else:
-            dact_colsum(out.reshape(-1, g.N), want_g=False, dbias=dbias)
+            rows = out.view(-1)[:g.batch * g.M * g.N].view(-1, g.N)
+            if dbias.dtype == out.dtype:
+                dact_colsum(rows, want_g=False, dbias=dbias)
+            else:                                     # that pass writes the type that it reads: in fp32, then cast
+                sums = dact_colsum(rows if rows.dtype == torch.float32 else cast(rows, torch.float32), want_g=False)[1]
+                dbias.view(-1)[:g.N].copy_(sums)
     return out
 
 

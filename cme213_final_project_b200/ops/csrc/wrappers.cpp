@@ -370,7 +370,7 @@ PyObject* embedding_bwd(PyObject*, PyObject* const* a, Py_ssize_t) {
 // took as Python statements.  Returns (out, column sums | None, descriptor in a bytearray, behind which lies the count that
 // colsum_slabs points to).
 // (a, b, a_trans, b_trans, out | None, out_dtype | None, bias | None, activation, aux_out | None, dact, aux_in | None, residual | None,
-//  accumulate, force_bn, force_splits, aux_deriv, column sums wanted, allow_tf32, scratch | None)
+//  accumulate, force_bn, force_splits, aux_deriv, dbias | None, allow_tf32, scratch | None)
 PyObject* gemm_prepare(PyObject*, PyObject* const* o, Py_ssize_t) {
     HANDLE_TH_ERRORS
     auto any = [](PyObject* t) {
@@ -431,7 +431,11 @@ PyObject* gemm_prepare(PyObject*, PyObject* const* o, Py_ssize_t) {
     if (g.dact && !aux_in.defined()) fail(native_error, "gemm: dact needs aux_in");
     if (g.dact) holds("aux_in", aux_in, out, "out", elements);
     at::Tensor part;
-    if (truth(o[16])) part = at::empty({(M + 31) / 32 * N}, a.options().dtype(at::kFloat));
+    if (const at::Tensor sums = any(o[16]); sums.defined()) {
+        dtype(sums);                                // one of the two types
+        holds("dbias", sums, sums, "dbias", N);
+        part = at::empty({(M + 31) / 32 * N}, a.options().dtype(at::kFloat));
+    }
     g.M = int32(M); g.N = int32(N); g.K = int32(K); g.batch = int32(batch);
     g.A = ptr(a); g.lda = a1; g.strideA = na == batch && a3 ? a0 * a1 : 0;
     g.B = ptr(b); g.ldb = b1; g.strideB = nb == batch && b3 ? b0 * b1 : 0;

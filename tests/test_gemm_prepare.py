@@ -77,7 +77,8 @@ def test_batches_that_do_not_match(seen, sa, sb):
     ({"residual": torch.zeros(8, 8).bfloat16()}, "residual has to have the type of out"),
     ({"out_dtype": torch.bfloat16, "aux_out": torch.zeros(8, 8)}, "aux_out has to have the type of out"),
     ({"out": torch.zeros(8, 8).bfloat16(), "dact": "relu", "aux_in": torch.zeros(8, 8)}, "aux_in has to have the type of out"),
-    ({"b": torch.zeros(8, 8).bfloat16()}, "b has to have the type of a")])
+    ({"b": torch.zeros(8, 8).bfloat16()}, "b has to have the type of a"), ({"dbias": torch.zeros(7)}, "dbias has 7 of 8"),
+    ({"dbias": torch.zeros(8).half()}, "unsupported dtype")])
 def test_operands_that_the_kernels_would_leave(seen, kw, what):
     with pytest.raises(ops.NativeError, match=what):
         ops.gemm(torch.zeros(8, 8), **{"b": torch.zeros(8, 8), **kw})
@@ -102,3 +103,22 @@ def test_one_matrix_is_shared(na, nb, backend):
     got = ops.gemm(a, b, backend=backend)
     want = torch.stack([ops.gemm(a[i % na].contiguous(), b[i % nb].contiguous(), backend=backend) for i in range(3)])
     assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("backend", ["auto", "simt"])              # with column sums from the epilogue, and from a pass of their own
+@pytest.mark.parametrize("out_dtype,sum_dtype", [(torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
+def test_column_sums_of_another_type(out_dtype, sum_dtype, backend):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a, b, x = (torch.randn(s, generator=g, device="cuda") for s in ((96, 64), (64, 40), (96, 40)))
+    around = torch.full((3 * 40,), 7.0, dtype=sum_dtype, device="cuda")
+    kw = {"dact": "relu", "aux_in": x.to(out_dtype)} if out_dtype == torch.bfloat16 else {}
+    room = torch.full((100, 40), 9.0, dtype=out_dtype, device="cuda")           # more than the product fills
+    ops.gemm(a.bfloat16(), b.bfloat16(), out=room, dbias=around[40:80], backend=backend, **kw)
+    assert (room[96:] == 9).all()
+    out = room[:96]
+    want, size = out.double().sum(0), out.double().abs().sum(0)
+    # sums of 96 in fp32 (of the epilogue's unrounded values, a bf16 result's are 2^-8 off each), rounded once
+    bound = size * (96 * 2.0 ** -24 + (2.0 ** -8 if out_dtype == torch.bfloat16 else 0)) + want.abs() * (2.0 ** -8 if sum_dtype == torch.bfloat16 else 0)
+    assert ((around[40:80].double() - want).abs() <= bound).all()
+    assert (around[:40] == 7).all() and (around[80:] == 7).all()
