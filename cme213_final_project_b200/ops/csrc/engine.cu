@@ -221,7 +221,7 @@ int gemm(const Engine& e, cudaStream_t st, int M, int N, int K, const void* A, l
     const bool on_side = e.side != nullptr && st == e.side, on_side2 = e.side2 != nullptr && st == e.side2;
     g.workspace = on_side ? e.gemm_ws_side : on_side2 ? e.gemm_ws_side2 : e.gemm_ws;
     g.workspace_bytes = on_side ? e.gemm_ws_side_bytes : on_side2 ? e.gemm_ws_side2_bytes : e.gemm_ws_bytes;
-    if (!e.d.fused_qkv) g.force_splits = gemm_kept_splits(&g);
+    g.force_splits = gemm_kept_splits(&g);
     return cme_gemm(&g, e.d.gemm_backend, st);
 }
 

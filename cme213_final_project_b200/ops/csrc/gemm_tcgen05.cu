@@ -254,12 +254,12 @@ static void plan_tiles(int M, int N, int K, int batch, bool plain_epi, long long
     *bn_out = bn; *pair_out = pair; *splits_out = splits;
 }
 
-// K splits of a bf16 product whose sums keep their order from one version to the next.  The models with separate Q, K and V take
-// them: their gradients are clipped to norm 1 and Adam's first steps divide each by its own size, so one result that rounds the
-// other way can turn a step of a parameter round, and a run from the same seed ends 3 % elsewhere (width 512, 45 x 64 tokens, the
-// splits of plan_tiles).  So the number is that of the estimate these models have always had, with k-blocks at their former pace;
-// the tile's width, which changes no sum, comes from plan_tiles.  It is seldom the fastest: 512 x 512 x 2048 takes 8 splits where 4
-// are planned, and a step of width 512 over 45 x 64 tokens 212 us where the plan's splits take 201.
+// K splits of the engine's bf16 products.  A training step keeps the order of its sums from one version to the next: Adam's first steps
+// divide each gradient by its own size, so one result that rounds the other way can turn a step of a parameter round, and a run from
+// the same seed ends 3 % elsewhere (parity model of width 512, 45 x 64 tokens, the splits of plan_tiles).  So the number is that of the
+// estimate that the engine has always had, with k-blocks at their former pace; the tile's width, which changes no sum, comes from
+// plan_tiles.  us a step with these splits / with the plan's: char-gpt 2114 / 2115, GPT-2 small 15240 / 15180, width 512 over 45 x 64
+// tokens 212 / 201 (512 x 512 x 2048 takes 8 splits where 4 are planned).
 static int kept_splits(int M, int N, int K, int batch, bool plain_epi, long long workspace_bytes, int num_sms, int max_pairs) {
     const int num_kb = cme_cdiv(K, 64);
     static const struct { int bn; bool pair; double per_step; } tiles[4] = {{256, true, 136.0}, {256, false, 168.0},

@@ -1,4 +1,4 @@
-"""K splits of the models with separate Q, K and V: the order of their sums stays as it was, whatever the planner learns."""
+"""K splits of the engine's bf16 products: the order of a training step's sums stays as it was, whatever the planner learns."""
 import ctypes
 
 import pytest
@@ -10,7 +10,7 @@ from cme213_final_project_b200 import ops
     (128, 512, 1024, 1, 1, 64 << 20, 4), (256, 256, 2560, 3, 1, 64 << 20, 10), (512, 512, 2048, 1, 1, 64 << 20, 8),
     (1600, 512, 2048, 1, 1, 64 << 20, 5), (512, 512, 3840, 3, 1, 64 << 20, 6), (2048, 512, 3584, 1, 1, 64 << 20, 4),
     (512, 512, 2048, 1, 0, 64 << 20, 1), (512, 512, 2048, 1, 1, 3 << 20, 3), (512, 128, 192, 1, 1, 64 << 20, 1),
-    (2048, 128, 128, 1, 1, 64 << 20, 1)])
+    (2048, 128, 128, 1, 1, 64 << 20, 1), (384, 1152, 16384, 1, 1, 64 << 20, 9), (768, 2304, 16384, 1, 1, 64 << 20, 5)])
 def test_splits_stay(M, N, K, batch, plain, ws, splits):
     lib = ops.host_lib()
     if lib is None:
