@@ -52,3 +52,17 @@ def test_splits(splits):
     a, b = _mk((2048, 512), 7), _mk((2048, 400), 8)
     (got, want), _ = _both(a, b, a_trans=True, force_splits=splits)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("sa,sb", [((3, 520, 72), (3, 72, 200)), ((3, 520, 72), (72, 200)), ((520, 72), (3, 72, 200))])
+def test_batches(sa, sb):
+    """Several matrices, and one operand for all of them; plain, and with epilogue operands that arrive by TMA."""
+    a, b, x = _mk(sa, 9), _mk(sb, 10), _mk((3, 520, 200), 11)
+    for kw in ({}, {"residual": x}, {"dact": "gelu", "aux_in": x}, {"dact": "relu", "aux_in": x}, {"out": x.clone, "accumulate": True},
+               {"act": "gelu", "aux_out": lambda: torch.empty_like(x)}, {"out_dtype": torch.float32}):
+        (got, want), (u, v) = _both(a, b, **kw)
+        assert torch.equal(got, want), kw.keys()
+        assert "aux_out" not in u or torch.equal(u["aux_out"], v["aux_out"])
+        if not kw:
+            ref = a.float() @ b.float()
+            assert (got.float() - ref).abs().max().item() <= 2 ** -8 * ref.abs().max().item()

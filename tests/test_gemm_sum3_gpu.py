@@ -30,3 +30,26 @@ def test_same_bits_as_three_products(M, N, K, one_launch, a_trans, b_trans):
     torch.cuda.synchronize()
     assert ops.gemm_check_status() == 0
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 192, 512), (200, 72, 1032)])
+@pytest.mark.parametrize("kind,splits,allow_tf32", [("bf16", 4, 0), ("bf16", 1, 0), ("fp32", 0, 0), ("fp32", 0, 2), ("fp32", 3, 2)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_products_that_go_one_by_one(M, N, K, kind, splits, allow_tf32, accumulate):
+    """What one launch does not make -- split reductions, fp32 storage exact and as tf32, a sum on top of C -- is made by three."""
+    from cme213_final_project_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(2)
+    dt = torch.bfloat16 if kind == "bf16" else torch.float32
+    a, b, c = (torch.randn(s, generator=g, device="cuda").to(dt) for s in ((3, M, K), (3, N, K), (M, N)))
+    kw = {"b_trans": True, "force_splits": splits, "allow_tf32": allow_tf32}
+    want, out = c.clone(), c.clone()
+    for i in range(3):
+        ops.gemm(a[i], b[i], out=want, accumulate=accumulate or i > 0, **kw)
+    ws = torch.empty(16 << 20, device="cuda")
+    d = ops.CmeGemm(M, N, K, 3, a.data_ptr(), K, M * K, 0, b.data_ptr(), K, N * K, 1, out.data_ptr(), N, 0, ops._dt(out), ops._dt(a))
+    d.accumulate, d.force_splits, d.allow_tf32, d.workspace, d.workspace_bytes = int(accumulate), splits, allow_tf32, ws.data_ptr(), 64 << 20
+    assert not ops.lib().cme_gemm_sum3_planned(ctypes.byref(d)) or (kind, splits, accumulate) == ("bf16", 1, False)
+    assert ops.lib().cme_gemm_sum3(ctypes.byref(d), 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    assert ops.gemm_check_status() == 0
+    assert torch.equal(out, want)
