@@ -1475,9 +1475,9 @@ int attention_tc_supported(const CmeAttn* a) {
 // calls take the small ones (192 x 256 12.1 / 9.8, 96 x 1024 36.3 / 29.2) but for long sequences just beyond.  With all keys both do a
 // full GPU's work at one rate, and the last wave decides: to six tiles per SM the wide ones (64 x 1024 32.5 / 33.6, 80 x 1024 41.3 / 43.7;
 // 192 x 582 42.7 / 38.0), then where that of the small ones would be a quarter full.
-// The lines were drawn before the small CTAs issued their products faster; near them the small ones are ahead by now (causal 48 x 1024
-// 22.6 / 20.8, 64 x 1024 27.6 / 22.7; all keys 96 x 1024 48.1 / 47.5, 160 x 1024 71.9 / 68.9).  They stay, because which kernel
-// runs shows in the last bits of the results.
+// The lines were drawn before the small CTAs issued their products faster; near them the small ones are ahead by now (where the
+// wide ones run: causal 48 x 1024 22.6 / 20.8; all keys 96 x 1024 48.1 / 47.5, 160 x 1024 71.9 / 68.9).  They have not been drawn anew:
+// which kernel runs shows in the last bits of the results.
 bool fwd_wide(long long ctas, int T, bool causal, int sms) {
     if (T > 128 && T <= 192) return ctas <= sms;
     if (ctas <= 2ll * sms) return true;
